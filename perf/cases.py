@@ -209,3 +209,40 @@ def run(state):
     if not s["backward"]:
         return o
     return (o.detach(), *torch.autograd.grad(o, (s["q"], s["k"], s["v"]), s["do"]))
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, in 64 bits: whole rows of the score matrix, as many at a time as fit in 1 GB."""
+    c, s = case, prepare(case, seed)
+    B, H, M, N, D = c["B"], c["H"], c["M"], c["N"], c["D"]
+    group, gap, scale = H // c["Hk"], max(0, N - M), 1.0 / D ** 0.5
+    new = {"device": "cuda", "dtype": torch.float64}
+    o = torch.zeros(B, H, M, D, **new)
+    dq, dk, dv = (torch.zeros(B, h, n, D, **new) if c["backward"] else None for h, n in ((H, M), (c["Hk"], N), (c["Hk"], N)))
+    keys = torch.arange(N, device="cuda")
+    step = max(1, min(M, (1 << 27) // N))
+    with torch.no_grad():
+        for b in range(B):
+            for h in range(H):
+                hk = h // group
+                k, v = s["k"][b, hk].double(), s["v"][b, hk].double()
+                for i in range(0, M, step):
+                    rows = slice(i, min(i + step, M))
+                    last = min(N, rows.stop + gap) if c["causal"] else N  # no row of these sees a later key
+                    q = s["q"][b, h, rows].double()
+                    p = (q @ k[:last].T).mul_(scale)
+                    if c["causal"]:
+                        p.masked_fill_(keys[None, :last] > torch.arange(rows.start, rows.stop, device="cuda")[:, None] + gap, -torch.inf)
+                    if s["eq"] is not None:
+                        eq, ek = s["eq"][b, h, rows, None], s["ek"][b, h, None, :last]
+                        p.masked_fill_((eq < 0) & (eq != ek), -torch.inf)
+                    p.sub_(p.amax(1, keepdim=True).clamp_(min=-1e300)).exp_()
+                    p.div_(p.sum(1, keepdim=True).clamp_(min=1e-300))  # a row without keys gives zeros
+                    o[b, h, rows] = p @ v[:last]
+                    if c["backward"]:
+                        do = s["do"][b, h, rows].double()
+                        dv[b, hk, :last] += p.T @ do
+                        ds = (do @ v[:last].T).sub_((do * o[b, h, rows]).sum(1, keepdim=True)).mul_(p)
+                        dq[b, h, rows] = (ds @ k[:last]).mul_(scale)
+                        dk[b, hk, :last] += (ds.T @ q).mul_(scale)
+    return (o, dq, dk, dv) if c["backward"] else o
