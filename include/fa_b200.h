@@ -109,6 +109,18 @@ int fa_plan_build(const fa_problem* p, const fa_ids* eq, const fa_ids* ek, void*
 int fa_fwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v,
            const fa_tensor* o, float* lse, const void* plan, int32_t* status, void* stream);
 
+/* The same forward for calls without ids (mode 0, 16-bit types) that are too few to fill the GPU, a decoded token or
+ * a short block of queries against long keys: the keys of each query block are cut into `splits` runs that
+ * different SMs work on, their fp32 results go to `workspace` (16-byte aligned, at least fa_fwd_workspace_bytes)
+ * and a second kernel merges them. fa_fwd_splits returns the number that pays on the current device (1: call
+ * fa_fwd, or pass splits = 1 and no workspace); more than one per 128 keys is refused, as is any splitting of other
+ * calls (FA_ERR_UNSUPPORTED). The workspace is free again when the launches are done. */
+int fa_fwd_splits(const fa_problem* p);
+int fa_fwd_workspace_bytes(const fa_problem* p, int32_t splits, size_t* bytes);
+int fa_fwd_split(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
+                 float* lse, const void* plan, int32_t splits, void* workspace, size_t workspace_bytes, int32_t* status,
+                 void* stream);
+
 /* delta[b,h,i] = sum_d o*do in fp32 (replaces flash_triton.py:585); delta is
  * [B, H, fa_padded_rows(M)], padding rows are written as 0. */
 int fa_bwd_delta(const fa_problem* p, const fa_tensor* o, const fa_tensor* d_o, float* delta, void* stream);

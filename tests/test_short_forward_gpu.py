@@ -1,0 +1,91 @@
+"""Forward calls without ids that are short of work: query heads of a group packed into one tile, keys cut into
+runs that are merged afterwards. Against plain attention in 64 bits; the bound is the parity tests' rule for 16-bit
+results (2e-2, or one rounding step of the result where that is larger)."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # B, H, Hk, M, N, D, causal
+    (1, 8, 2, 1, 128, 64, True),      # one token, one tile of keys
+    (2, 8, 1, 1, 4500, 128, True),    # a group of 8, ragged keys, split
+    (1, 64, 8, 1, 700, 32, False),
+    (16, 32, 8, 1, 1000, 128, True),  # packed, not split
+    (1, 6, 2, 50, 3000, 64, True),    # a group of 3 in tiles of 2 heads: the second tile is half empty
+    (1, 16, 4, 32, 9000, 128, True),  # a full tile of packed rows
+    (1, 12, 4, 64, 64, 128, True),    # two heads a tile, diagonal inside it
+    (1, 8, 8, 65, 5000, 64, True),    # no packing, split
+    (1, 4, 4, 300, 7777, 128, True),  # three query blocks a head, split
+    (1, 4, 4, 1000, 4096, 16, False),
+    (1, 2, 1, 3, 40000, 128, True),
+]
+
+
+@pytest.fixture(scope="module")
+def fb():
+    import flash_b200
+    return flash_b200
+
+
+def _exact(q, k, v, causal):
+    G, M, N = q.shape[1] // k.shape[1], q.shape[2], k.shape[2]
+    q, k, v = q.double(), k.double().repeat_interleave(G, 1), v.double().repeat_interleave(G, 1)
+    s = q @ k.transpose(2, 3) / q.shape[3] ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(M, N, dtype=torch.bool, device=q.device).triu(N - M + 1), -torch.inf)
+    return torch.softmax(s, 3) @ v, torch.logsumexp(s, 3) / torch.log(torch.tensor(2.0, device=q.device, dtype=torch.float64))
+
+
+def _close(got, want, what):
+    err, want = (got.double() - want).abs(), want.abs()
+    bound = torch.where(want < 2.56, torch.full_like(want, 2e-2), want * 2.0 ** -7)
+    assert bool((err <= bound).all()), (what, err.max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(str(int(x)) for x in c))
+def test_short_forward(fb, case, dtype):
+    B, H, Hk, M, N, D, causal = case
+    g = torch.Generator(device="cuda").manual_seed(M * N)
+    # q as a projection leaves it ([B, M, H, D] transposed), k and v contiguous
+    q = torch.randn(B, M, H, D, generator=g, device="cuda").to(dtype).transpose(1, 2).requires_grad_()
+    k, v = [torch.randn(B, Hk, N, D, generator=g, device="cuda").to(dtype).requires_grad_() for _ in range(2)]
+    do = torch.randn(B, H, M, D, generator=g, device="cuda").to(dtype)
+    o = fb.attention(q, k, v, causal)
+    o.backward(do)
+    fb.check_status()
+    qe, ke, ve = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    oe, _ = _exact(qe, ke, ve, causal)
+    oe.backward(do.double())
+    for what, got, want in (("o", o, oe), ("dq", q.grad, qe.grad), ("dk", k.grad, ke.grad), ("dv", v.grad, ve.grad)):
+        _close(got.detach(), want.detach(), what)
+
+
+@pytest.mark.parametrize("splits", [1, 2, 5, 16])
+def test_any_number_of_runs(fb, splits):
+    """Also numbers the rule would not take, among them runs that the causal bound leaves without keys; lse too."""
+    from flash_b200 import _lib, ops
+    B, H, Hk, M, N, D = 2, 4, 2, 300, 2048, 64
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, o = torch.randn(B, H, M, D, generator=g, device="cuda").bfloat16(), torch.empty(B, H, M, D, device="cuda", dtype=torch.bfloat16)
+    k, v = [torch.randn(B, Hk, N, D, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    prob = ops._problem(B, H, Hk, M, N, D, q.dtype, True, 0, 1, D ** -0.5)
+    lse = torch.full((B, H, 384), float("nan"), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n = ctypes.c_size_t(0)
+    assert lib.fa_fwd_workspace_bytes(ctypes.byref(prob), splits, ctypes.byref(n)) == 0
+    assert (n.value == 0) == (splits == 1)
+    work = torch.full((max(4, n.value // 4),), float("nan"), device="cuda")
+    tq, tk, tv, to = [ops._tensor(t) for t in (q, k, v, o)]
+    args = [ctypes.byref(x) for x in (prob, tq, tk, tv, to)]
+    if splits > 1:
+        assert lib.fa_fwd_split(*args, lse.data_ptr(), None, splits, work.data_ptr(), n.value - 4, status.data_ptr(), ops._stream()) == 6
+    assert lib.fa_fwd_split(*args, lse.data_ptr(), None, 17, work.data_ptr(), 1 << 40, status.data_ptr(), ops._stream()) == 2
+    assert lib.fa_fwd_split(*args, lse.data_ptr(), None, splits, work.data_ptr(), n.value, status.data_ptr(), ops._stream()) == 0
+    oe, le = _exact(q, k, v, True)
+    _close(o, oe, "o")
+    assert (lse[..., :M].double() - le).abs().max().item() < 1e-4 and bool(torch.isfinite(lse).all())
+    assert int(status.item()) == 0

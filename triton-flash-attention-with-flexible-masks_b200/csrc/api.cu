@@ -12,6 +12,7 @@ cudaError_t launch_plan_build(const void*, const int64_t*, int, const void*, con
 cudaError_t launch_debug_mask(const MaskArgs&, uint8_t*, uint8_t*, cudaStream_t);
 cudaError_t launch_fwd(int, bool, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&,
                        const FwdParams&, int, cudaStream_t);
+cudaError_t launch_fwd_combine(bool, const CombineParams&, cudaStream_t);
 cudaError_t launch_bwd_delta(const DeltaParams&, cudaStream_t);
 cudaError_t launch_bwd_dkdv(int, bool, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&,
                             const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const DkdvParams&, int,
@@ -114,6 +115,34 @@ int make_map(CUtensorMap* out, const fa_tensor* t, int dtype, int B, int H, int 
     return r == CUDA_SUCCESS ? FA_OK : FA_ERR_TENSORMAP;
 }
 
+// 5-D map over the q / o of a packed or split forward: [B, Hk, G, M, D] with G = H / Hk, box = 64 elements of D x
+// `rows` queries x `pack` heads of a group; otherwise as make_map.
+int make_map_grouped(CUtensorMap* out, const fa_tensor* t, const fa_problem* p, int rows, int pack) {
+    EncodeFn fn = encode_fn();
+    if (!fn) return FA_ERR_NO_DRIVER;
+    const int G = p->H / p->Hk;
+    const cuuint64_t dims[5] = {cuuint64_t(p->D), cuuint64_t(p->M), cuuint64_t(G), cuuint64_t(p->Hk), cuuint64_t(p->B)};
+    const int64_t sl = (p->M > 1) ? t->stride[2] : p->D;
+    const int64_t sh = (p->H > 1) ? t->stride[1] : sl * p->M;
+    const int64_t sb = (p->B > 1) ? t->stride[0] : sh * p->H;
+    const cuuint64_t strides[4] = {cuuint64_t(sl) * 2, cuuint64_t(sh) * 2, cuuint64_t(sh) * G * 2, cuuint64_t(sb) * 2};
+    const cuuint32_t box[5] = {64, cuuint32_t(rows), cuuint32_t(pack), 1, 1};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r =
+        fn(out, p->dtype == FA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, t->ptr,
+           dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? FA_OK : FA_ERR_TENSORMAP;
+}
+
+// Query heads of a group that share one 128-row tile in the forward: as many as fit, for calls without ids whose
+// queries fill at most half a tile.
+int fwd_pack(const fa_problem* p) {
+    const int G = p->H / p->Hk;
+    if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32 || p->M > fa::kBlk / 2) return 1;
+    return G < fa::kBlk / p->M ? G : fa::kBlk / p->M;
+}
+
 constexpr size_t kCtrWords = 128;  // size of the plan's counter section (PlanLayout::off_ctr)
 
 // Debug switches, read from the environment at every call so that a test can flip them:
@@ -196,6 +225,31 @@ int sm_count() {
         cached[dev] = n;
     }
     return cached[dev];
+}
+
+// Runs into which the forward cuts each item's key tiles, for calls without ids that have fewer items than the GPU
+// has SMs. A round of items costs its tiles plus about 4 tile times of fill, drain and epilogue; the second
+// kernel and the fp32 rows cost about 6 more. At most two items per SM, which bounds the workspace at 20 MB.
+int fwd_splits(const fa_problem* p, int sms) {
+    if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32) return 1;
+    const int pack = fwd_pack(p);
+    const int64_t items = int64_t(fa::cdiv(p->M, fa::kBlk)) * p->Hk * fa::cdiv(p->H / p->Hk, pack) * p->B;
+    if (items >= sms) return 1;
+    const int T = fa::cdiv(p->N, fa::kBlk);
+    int best = 1, best_cost = T + 4;
+    for (int ns = 2; ns <= T / 2 && items * ns <= 2 * sms; ++ns) {
+        const int rounds = int((items * ns + sms - 1) / sms);
+        const int cost = rounds * (fa::cdiv(T, ns) + 4) + 6;
+        if (cost < best_cost) best = ns, best_cost = cost;
+    }
+    return best;
+}
+
+// fp32 rows and log-sum-exps of all runs
+size_t fwd_workspace_bytes(const fa_problem* p, int ns) {
+    if (ns <= 1) return 0;
+    const size_t rows = size_t(p->B) * p->H * p->M;
+    return (rows * ns * (p->D > 64 ? 128 : 64) + rows * ns) * sizeof(float);
 }
 
 // fp32 inputs: which = 0 forward, 1 delta, 2 dK / dV, 3 dQ; absent tensors are null
@@ -286,12 +340,37 @@ int fa_plan_build(const fa_problem* p, const fa_ids* eq, const fa_ids* ek, void*
     return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 
+int fa_fwd_splits(const fa_problem* p) {
+    if (check_problem(p)) return 1;
+    const int sms = sm_count();
+    return sms > 0 ? fwd_splits(p, sms) : 1;
+}
+
+int fa_fwd_workspace_bytes(const fa_problem* p, int32_t splits, size_t* bytes) {
+    if (!bytes || splits < 1) return FA_ERR_BAD_ARG;
+    const int rc = check_problem(p);
+    if (rc) return rc;
+    *bytes = fwd_workspace_bytes(p, splits);
+    return FA_OK;
+}
+
 int fa_fwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
            float* lse, const void* plan, int32_t* status, void* stream) {
+    return fa_fwd_split(p, q, k, v, o, lse, plan, 1, nullptr, 0, status, stream);
+}
+
+int fa_fwd_split(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
+                 float* lse, const void* plan, int32_t splits, void* workspace, size_t workspace_bytes, int32_t* status,
+                 void* stream) {
     int rc = check_problem(p);
     if (rc) return rc;
-    if (!lse || !status) return FA_ERR_BAD_ARG;
+    if (!lse || !status || splits < 1) return FA_ERR_BAD_ARG;
     if (!aligned16(lse)) return FA_ERR_ALIGNMENT;
+    if (splits > 1) {
+        if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32 || splits > fa::cdiv(p->N, fa::kBlk)) return FA_ERR_UNSUPPORTED;
+        if (!workspace || workspace_bytes < fwd_workspace_bytes(p, splits)) return FA_ERR_PLAN_SIZE;
+        if (!aligned16(workspace)) return FA_ERR_ALIGNMENT;
+    }
     if (p->dtype == FA_FP32) return run_f32(0, p, q, k, v, o, nullptr, nullptr, nullptr, nullptr, lse, nullptr, plan, stream);
     if ((rc = check_tensor(q, p->B, p->H, p->M))) return rc;
     if ((rc = check_tensor(k, p->B, p->Hk, p->N))) return rc;
@@ -299,24 +378,36 @@ int fa_fwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa
     if ((rc = check_tensor(o, p->B, p->H, p->M))) return rc;
     fa::FwdParams fp;
     if ((rc = make_mask(&fp.mask, p, plan))) return rc;
+    fp.G = p->H / p->Hk;
+    fp.pack = fwd_pack(p);
+    fp.ns = splits;
+    const int box_rows = fp.pack > 1 ? p->M : fa::kBlk;
+    fp.rows = box_rows * fp.pack;
+    const bool grouped = fp.pack > 1 || fp.ns > 1;
     CUtensorMap tq, tk, tv, to;
-    if ((rc = make_map(&tq, q, p->dtype, p->B, p->H, p->M, p->D))) return rc;
+    if ((rc = grouped ? make_map_grouped(&tq, q, p, box_rows, fp.pack) : make_map(&tq, q, p->dtype, p->B, p->H, p->M, p->D))) return rc;
     if ((rc = make_map(&tk, k, p->dtype, p->B, p->Hk, p->N, p->D))) return rc;
     if ((rc = make_map(&tv, v, p->dtype, p->B, p->Hk, p->N, p->D))) return rc;
-    if ((rc = make_map(&to, o, p->dtype, p->B, p->H, p->M, p->D))) return rc;
+    if ((rc = grouped ? make_map_grouped(&to, o, p, box_rows, fp.pack) : make_map(&to, o, p->dtype, p->B, p->H, p->M, p->D))) return rc;
     const int sms = sm_count();
     if (sms <= 0) return FA_ERR_LAUNCH;
     fp.lse = lse;
     fp.H = p->H;
     fp.B = p->B;
-    fp.G = p->H / p->Hk;
-    fp.gh = head_group(p, p->H * p->B);
+    fp.gh = head_group(p, p->Hk * fa::cdiv(fp.G, fp.pack) * p->B);
     fp.by_length = (p->mode == FA_MODE1_DOC && int64_t(fa::cdiv(p->M, fa::kBlk) * p->H * p->B) < 32 * int64_t(sms)) ? 1 : 0;
     fp.scale_log2 = p->sm_scale * kLog2e;
     fp.status = status;
     fp.wait_limit = wait_limit_clocks();
-    const cudaError_t e =
-        fa::launch_fwd(p->D, p->dtype == FA_BF16, tq, tk, tv, to, fp, sms, static_cast<cudaStream_t>(stream));
+    const int64_t rows = int64_t(p->B) * p->H * p->M;
+    const int dk = p->D > 64 ? 128 : 64;
+    fp.part_o = static_cast<float*>(workspace);
+    fp.part_lse = splits > 1 ? fp.part_o + rows * splits * dk : nullptr;
+    cudaError_t e = fa::launch_fwd(p->D, p->dtype == FA_BF16, tq, tk, tv, to, fp, sms, static_cast<cudaStream_t>(stream));
+    if (e == cudaSuccess && splits > 1) {
+        fa::CombineParams cp{fp.part_o, fp.part_lse, out_view(o), lse, p->B, p->H, p->M, p->D, dk, splits, fa::pad128(p->M), status};
+        e = fa::launch_fwd_combine(p->dtype == FA_BF16, cp, static_cast<cudaStream_t>(stream));
+    }
     return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 

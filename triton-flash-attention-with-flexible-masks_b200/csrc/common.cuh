@@ -210,6 +210,25 @@ __device__ __forceinline__ void nan_fill_outputs(uint8_t* tile, int nbox, const 
     }
 }
 
+// The same for the 5-D output map (D, M, G, Hk, B) of the forward's packed calls.
+__device__ __forceinline__ void nan_fill_short(uint8_t* tile, int nbox, const CUtensorMap* m, int n_blk, int n_g, int pack,
+                                               int n_hk, int n_b) {
+    constexpr int kBox = kBlk * 64 * 2;
+    for (int i = threadIdx.x; i < nbox * kBox / 16; i += blockDim.x)
+        reinterpret_cast<uint4*>(tile)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    fence_proxy_async();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int n = n_blk * n_g * n_hk * n_b;
+        for (int j = blockIdx.x; j < n; j += gridDim.x) {
+            const int blk = j % n_blk, g = (j / n_blk) % n_g, hk = (j / (n_blk * n_g)) % n_hk, b = j / (n_blk * n_g * n_hk);
+            for (int x = 0; x < nbox; ++x) tma_store_5d(m, smem_u32(tile) + x * kBox, x * 64, blk * kBlk, g * pack, hk, b);
+            tma_store_commit();
+        }
+        tma_store_wait_all();
+    }
+}
+
 // Device-side view of a [B, H, L, D] tensor for plain (non-TMA) stores.
 struct OutTensor {
     void* ptr;

@@ -27,6 +27,7 @@
 #include <type_traits>
 #include "common.cuh"
 #include "params.cuh"
+#include <type_traits>
 
 namespace fa {
 
@@ -55,7 +56,17 @@ struct FwdSmem {
     static constexpr int total = off_misc + 16;
 };
 
-template <int D, bool BF16>
+// SHORT: calls without ids whose items are too few or too empty for one item per (query block, head, batch).
+// Two things are added (fwd_short_pack and fwd_splits in api.cu say when):
+//  - p.pack query heads of one kv head share a tile, row g * M + i = query i of the g-th of them (at most 128
+//    rows: one decoded token of 4 heads reads the keys and values once instead of four times). The Q and O maps
+//    are 5-D, (D, M, G, Hk, B), and a box holds p.rows rows; tile rows past them are never loaded, hold whatever
+//    was there and only ever reach results that are not stored. Warps without a valid row skip the softmax.
+//  - an item's tiles are cut into p.ns runs that are items of their own. With ns > 1 the normalised fp32 rows
+//    and their log-sum-exp go to the workspace, and fwd_combine_kernel merges them.
+// Such calls are bound by reading K and V (16 tokens of 32 / 8 heads of 128 against 4500 keys: 295 MB, 45 us at the
+// copy rate; 171 us with a tile per head, 63 us packed) or, with few heads, by the longest item's chain of tiles.
+template <int D, bool BF16, bool SHORT>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdParams p) {
@@ -67,8 +78,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 
     const MaskArgs& mk = p.mask;
     const int nQ = mk.L.nQ;
-    const int HB = p.H * p.B;
-    const int n_items = nQ * HB;
+    const int nG = SHORT ? cdiv(p.G, p.pack) : 1;  // tiles' worth of query heads per kv head
+    const int HP = SHORT ? p.H / p.G * nG : p.H;   // heads, or packs of heads, per batch
+    const int HB = HP * p.B;
+    const int ns = SHORT ? p.ns : 1;
+    const int n_items = nQ * HB * ns;
     unsigned int* ctr = mk.ctr ? mk.ctr + CTR_FWD : nullptr;
 
     volatile int* misc = reinterpret_cast<volatile int*>(smem + S::off_misc);  // [0] tmem, [1] abort
@@ -113,7 +127,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
     // an earlier launch on this device ran into a time-out that the host has not yet cleared
-    if (aborted && (sbase & 1023u) == 0) nan_fill_outputs(smem + S::off_q, S::NBOX, &tmO, nullptr, nQ, p.H, p.B);
+    if (aborted && (sbase & 1023u) == 0) {
+        if constexpr (!SHORT) nan_fill_outputs(smem + S::off_q, S::NBOX, &tmO, nullptr, nQ, p.H, p.B);
+        else if (ns == 1) nan_fill_short(smem + S::off_q, S::NBOX, &tmO, nQ, nG, p.pack, p.H / p.G, p.B);
+        // (with ns > 1 the combine kernel fills the output)
+    }
 
     auto sQ = [&](int s) { return sbase + S::off_q + uint32_t(s) * S::TILE; };
     auto sK = [&](int s) { return sbase + S::off_k + uint32_t(s) * S::TILE; };
@@ -128,8 +146,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         const int grp = j / per, rem = j - grp * per;
         const int gsz = min(p.gh, HB - grp * p.gh);  // heads in this group (the last one may be smaller)
         const int pos = rem / gsz, bh = grp * p.gh + (rem - pos * gsz);
-        b = bh / p.H;
-        h = bh - b * p.H;
+        b = bh / HP;
+        h = bh - b * HP;
         // few items per CTA: longest first (sorted in the plan), so that no long item is left for the end
         qb = p.by_length ? mk.plan[mk.L.off_ordq + (int64_t(b) * mk.He + (mk.He == 1 ? 0 : h)) * nQ + pos] : nQ - 1 - pos;
     };
@@ -163,11 +181,17 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     break;
                 }
                 int qb, h, b;
-                decode(j, qb, h, b);
+                const int sp = SHORT ? j % ns : 0;  // which run of the item's tiles
+                decode(SHORT ? j / ns : j, qb, h, b);
                 const int he = (mk.He == 1) ? 0 : h;
                 int lo, hi;
                 kv_range(mk, b, he, qb, lo, hi);
                 int n = hi - lo;
+                if constexpr (SHORT) {  // no ids: every tile of the range is visited
+                    const int first = int(int64_t(n) * sp / ns);
+                    n = int(int64_t(n) * (sp + 1) / ns) - first;
+                    lo += first;
+                }
                 if (n > kListCap) n = kListCap;  // the host refuses problems that could exceed the cap
                 uint16_t* list = reinterpret_cast<uint16_t*>(smem + S::off_list) + s * kListCap;
                 int T = 0;
@@ -208,7 +232,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     const int s = kk & 1;
                     if (!mbar_wait(BAR(B_OSTAGED + s), (kk >> 1) & 1, ab, ST_WAIT_TIMEOUT + 13)) return false;
                     const int qb = item_qb[s], h = item_h[s], b = item_b[s];
-                    for (int x = 0; x < S::NBOX; ++x) tma_store_4d(&tmO, sQ(s) + x * S::BOX, x * 64, qb * kBlk, h, b);
+                    if constexpr (SHORT) {
+                        if (ns > 1) return true;  // the rows went to the workspace
+                        for (int x = 0; x < S::NBOX; ++x)
+                            tma_store_5d(&tmO, sQ(s) + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
+                    } else {
+                        for (int x = 0; x < S::NBOX; ++x) tma_store_4d(&tmO, sQ(s) + x * S::BOX, x * 64, qb * kBlk, h, b);
+                    }
                     tma_store_commit();
                     tma_store_wait_read();
                     return true;
@@ -221,15 +251,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     if (j < 0) break;
                     const uint16_t* list = list_of(s);
                     const int qb = info[s * 8 + 4], h = info[s * 8 + 5], b = info[s * 8 + 6];
-                    const int hk = h / p.G;
+                    const int hk = SHORT ? h / nG : h / p.G;
                     const int he = (mk.He == 1) ? 0 : h;
                     // the slot still holds the staged O tile of item k-2: send it off first
                     if (use > 0) ok = store_o(k - 2);
                     if (!ok) break;
                     item_qb[s] = qb; item_h[s] = h; item_b[s] = b;
-                    mbar_expect_tx(BAR(B_QFULL + s), S::TILE);
-                    for (int x = 0; x < S::NBOX; ++x)
-                        tma_load_4d(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, h, b);
+                    if constexpr (SHORT) {
+                        mbar_expect_tx(BAR(B_QFULL + s), uint32_t(p.rows) * 128u * S::NBOX);
+                        for (int x = 0; x < S::NBOX; ++x)
+                            tma_load_5d(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, (h % nG) * p.pack, hk, b);
+                    } else {
+                        mbar_expect_tx(BAR(B_QFULL + s), S::TILE);
+                        for (int x = 0; x < S::NBOX; ++x)
+                            tma_load_4d(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, h, b);
+                    }
                     for (int t = 0; t <= T && ok; ++t) {  // K runs one tile ahead of V
                         if (t < T) {
                             const int kb = lo + (list[t] & 1023);
@@ -375,7 +411,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             if (j < 0) break;
             const uint16_t* list = list_of(s);
             const int qb = info[s * 8 + 4], h = info[s * 8 + 5], b = info[s * 8 + 6];
-            const int row = qb * kBlk + r;
+            // this thread's query: row of the head, and (SHORT) which head of the group
+            const int g_row = SHORT && p.pack > 1 ? r / mk.M : 0;
+            const int row = qb * kBlk + r - g_row * mk.M;
+            const int g_own = SHORT ? (h % nG) * p.pack + g_row : 0;
+            const bool valid = !SHORT || (row < mk.M && g_row < p.pack && g_own < p.G);
+            const bool active = !SHORT || __any_sync(0xffffffffu, valid);  // does this warp hold a query at all?
             const int qc = reinterpret_cast<const int*>(smem + S::off_qc)[s * kBlk + r];
             float m_run = -INFINITY, l_run = 0.f;
             int n_my = 0;
@@ -394,6 +435,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 alive = __all_sync(0xffffffffu, alive);
                 if (!alive) break;
                 tc_fence_after();
+                if (SHORT && !active) {  // no row of this warp is a query: its lanes of P and O are never stored
+                    if (turns) {
+                        alive = mbar_wait(BAR(B_TURN + w), nturn & 1, ab, ST_WAIT_TIMEOUT + 10);
+                        alive = __all_sync(0xffffffffu, alive);
+                        if (!alive) break;
+                        ++nturn;
+                    }
+                    mbar_arrive(BAR(B_PHALF0 + w));
+                    mbar_arrive(BAR(B_PHALF1 + w));
+                    if (turns && (t0 == 0 ? (n_my < n_other) : (n_my + 1 < n_other))) mbar_arrive(BAR(B_TURN + (w ^ 1)));
+                    continue;
+                }
                 uint32_t sr[128];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) tmem_ld32(tS + uint32_t(q) * 32u, sr + q * 32);
@@ -569,12 +622,29 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             const bool healthy = alive && (misc[1] == 0);
             if (w == 0 && healthy) {
                 const float lse = (lt > 0.f) ? fmaf(mt, c, log2f(lt)) : -INFINITY;
-                p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + row] = lse;
+                if constexpr (SHORT) {
+                    const int64_t bh0 = int64_t(b) * p.H + int64_t(h / nG) * p.G;
+                    if (ns > 1) {
+                        if (valid) p.part_lse[((bh0 + g_own) * mk.M + row) * ns + j % ns] = lse;
+                    } else {
+                        if (valid) p.lse[(bh0 + g_own) * mk.L.Mpad + row] = lse;
+                        // the rows past M that pad the buffer
+                        for (int g = (h % nG) * p.pack; g < min(p.G, (h % nG + 1) * p.pack); ++g)
+                            if (qb * kBlk + r >= mk.M) p.lse[(bh0 + g) * mk.L.Mpad + qb * kBlk + r] = 0.f;
+                    }
+                } else {
+                    p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + row] = lse;
+                }
             }
             // this thread's half row: columns [w*D/2, (w+1)*D/2) of both accumulators
             constexpr int HALF = D / 2;
             const uint32_t c0 = uint32_t(w) * HALF;
             uint32_t outw[HALF / 2];
+            float* part = nullptr;  // this thread's half row in the workspace (SHORT, ns > 1)
+            if constexpr (SHORT) {
+                if (ns > 1 && valid && healthy)
+                    part = p.part_o + ((int64_t(j % ns) * p.B * p.H + int64_t(b) * p.H + int64_t(h / nG) * p.G + g_own) * mk.M + row) * D + c0;
+            }
 #pragma unroll
             for (int q = 0; q < HALF / 32; ++q) {
                 uint32_t x0[32], x1[32];
@@ -594,6 +664,17 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         v1 = fmaf(__uint_as_float(x1[2 * x + 1]), f1, v1);
                     }
                     outw[16 * q + x] = pack2<BF16>(v0, v1);
+                    if constexpr (SHORT) {
+                        x0[2 * x] = __float_as_uint(v0);
+                        x0[2 * x + 1] = __float_as_uint(v1);
+                    }
+                }
+                if constexpr (SHORT) {
+                    if (part) {
+#pragma unroll
+                        for (int x = 0; x < 8; ++x)
+                            *reinterpret_cast<uint4*>(part + 32 * q + 4 * x) = make_uint4(x0[4 * x], x0[4 * x + 1], x0[4 * x + 2], x0[4 * x + 3]);
+                    }
                 }
             }
             // both accumulators have been read: the MMA issuers may start the next item's P*V
@@ -637,15 +718,63 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     }
 }
 
+// Merges the ns partial results of a split forward: O = sum_s w_s O_s with w_s = 2^(lse_s - lse), lse the log2-sum
+// over the parts. One warp per row; lane l owns columns l, l + 32, ... (D <= 128), all sums
+// in fp32 in the order of the parts. Bound by latency: at most a few MB are read, all of them from L2.
+template <bool BF16>
+__global__ void __launch_bounds__(256) fwd_combine_kernel(const CombineParams p) {
+    const int64_t row = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);  // of the [B, H, M] rows
+    const int lane = threadIdx.x & 31;
+    const int64_t rows = int64_t(p.B) * p.H * p.M;
+    if (row >= rows) return;
+    const int64_t bh = row / p.M;
+    const int i = int(row - bh * p.M);
+    float* lse = p.lse + bh * p.Mpad;
+    if (i == p.M - 1)  // the rows past M that pad the buffer
+        for (int64_t x = p.M + lane; x < p.Mpad; x += 32) lse[x] = 0.f;
+    const bool failed = status_is_fatal(*p.status);  // the forward left no parts: NaN, as the other kernels do
+    float mx = -INFINITY;
+    for (int s = lane; s < p.ns; s += 32) mx = fmaxf(mx, p.part_lse[row * p.ns + s]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float acc[4] = {0.f, 0.f, 0.f, 0.f}, total = 0.f;
+    if (mx != -INFINITY) {
+#pragma unroll 4
+        for (int s = 0; s < p.ns; ++s) {
+            const float wgt = fast_exp2(p.part_lse[row * p.ns + s] - mx);  // an empty part: 2^-inf = 0
+            const float* po = p.part_o + (int64_t(s) * rows + row) * p.Dk;
+            total += wgt;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (lane + 32 * k < p.D) acc[k] = fmaf(wgt, po[lane + 32 * k], acc[k]);
+        }
+    }
+    const float inv = total > 0.f ? 1.f / total : 0.f;
+    const int b = int(bh / p.H), h = int(bh - int64_t(b) * p.H);
+    uint16_t* out = static_cast<uint16_t*>(p.o.ptr) + int64_t(b) * p.o.sb + int64_t(h) * p.o.sh + int64_t(i) * p.o.sl;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (lane + 32 * k < p.D) out[lane + 32 * k] = failed ? uint16_t(0xffff) : uint16_t(pack2<BF16>(acc[k] * inv, 0.f));
+    if (lane == 0) lse[i] = total > 0.f ? mx + log2f(total) : -INFINITY;
+}
+
+cudaError_t launch_fwd_combine(bool bf16, const CombineParams& p, cudaStream_t stream) {
+    const unsigned grid = unsigned((int64_t(p.B) * p.H * p.M + 7) / 8);
+    if (bf16) fwd_combine_kernel<true><<<grid, 256, 0, stream>>>(p);
+    else fwd_combine_kernel<false><<<grid, 256, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
 // ---- host launcher (called from api.cu) -------------------------------------------------
-template <int D, bool BF16>
+template <int D, bool BF16, bool SHORT>
 static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                                 const CUtensorMap& to, const FwdParams& p, int num_sms, cudaStream_t stream) {
-    auto kern = fwd_kernel<D, BF16>;
+    auto kern = fwd_kernel<D, BF16, SHORT>;
     constexpr int smem = FwdSmem<D>::total;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const int n_items = p.mask.L.nQ * p.H * p.B;
+    const int heads = SHORT ? p.H / p.G * cdiv(p.G, p.pack) : p.H;
+    const int n_items = p.mask.L.nQ * heads * p.B * (SHORT ? p.ns : 1);
     dim3 grid(n_items < num_sms ? n_items : num_sms);
     kern<<<grid, kAttnThreads, smem, stream>>>(tq, tk, tv, to, p);
     return cudaGetLastError();
@@ -654,10 +783,16 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
 
 cudaError_t launch_fwd(int D, bool bf16, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                        const CUtensorMap& to, const FwdParams& p, int num_sms, cudaStream_t stream) {
-    if (D == 128) return bf16 ? launch_fwd_t<128, true>(tq, tk, tv, to, p, num_sms, stream)
-                              : launch_fwd_t<128, false>(tq, tk, tv, to, p, num_sms, stream);
-    return bf16 ? launch_fwd_t<64, true>(tq, tk, tv, to, p, num_sms, stream)
-                : launch_fwd_t<64, false>(tq, tk, tv, to, p, num_sms, stream);
+    auto pick = [&](auto d, auto shrt) {
+        constexpr int kD = decltype(d)::value;
+        constexpr bool kShort = decltype(shrt)::value;
+        return bf16 ? launch_fwd_t<kD, true, kShort>(tq, tk, tv, to, p, num_sms, stream)
+                    : launch_fwd_t<kD, false, kShort>(tq, tk, tv, to, p, num_sms, stream);
+    };
+    using std::integral_constant;
+    const bool shrt = p.pack > 1 || p.ns > 1;
+    if (D == 128) return shrt ? pick(integral_constant<int, 128>{}, std::true_type{}) : pick(integral_constant<int, 128>{}, std::false_type{});
+    return shrt ? pick(integral_constant<int, 64>{}, std::true_type{}) : pick(integral_constant<int, 64>{}, std::false_type{});
 }
 
 }  // namespace fa

@@ -16,6 +16,22 @@ struct FwdParams {
     float scale_log2;  // sm_scale * log2(e)
     int* status;
     long long wait_limit;  // SM clocks a bounded wait may last
+    // calls without ids that are short of items (fwd_kernel, SHORT)
+    int pack;         // query heads of a group that share a tile; 1: none
+    int rows;         // rows of a Q / O box
+    int ns;           // runs an item's tiles are cut into; 1: none
+    float* part_o;    // [ns, B, H, M, 64 or 128] normalised rows of each run (ns > 1)
+    float* part_lse;  // [B, H, M, ns]
+};
+
+struct CombineParams {
+    const float* part_o;
+    const float* part_lse;
+    OutTensor o;
+    float* lse;  // [B, H, Mpad]
+    int B, H, M, D, Dk, ns;  // Dk: columns of a row of part_o
+    int64_t Mpad;
+    const int* status;
 };
 
 struct DeltaParams {

@@ -124,6 +124,8 @@ def attention_host(q, k, v, do=None, causal=False, sm_scale=None, eq=None, ek=No
         def cut(t, lo, hi):
             return t[lo:hi] if dim == 0 else t[:, lo:hi]
 
+        # the slices cut their keys as the whole call would: the same bits, whatever the number of slices
+        splits = ops.forward_splits(B, H, Hk, M, k.shape[2], D, q.dtype, causal, score_func_mode) if direct else 1
         finished = []  # per slice: the event after its kernels
         for (qa, qb, ka, kb) in slices:
             if 0 < _HOST_AHEAD <= len(finished):
@@ -153,6 +155,7 @@ def attention_host(q, k, v, do=None, causal=False, sm_scale=None, eq=None, ek=No
                     k_ = k_.expand(dq_.shape[0], dq_.shape[1], k.shape[2]) if k_.shape[1] == 1 else k_
                 if direct:
                     ctx = _Ctx()
+                    ctx.fwd_splits = splits
                     o = ops.FlashAttention.forward(ctx, dq_, dk_, dv_, causal, sm_scale, e, k_, score_func_mode)
                     results = [("o", o, qa, qb)]
                     if backward:

@@ -153,6 +153,11 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+def forward_splits(B, H, Hk, M, N, D, dtype, causal, mode):
+    """Into how many runs the forward of this call cuts the keys of a query block (fa_fwd_splits)."""
+    return _lib.load().fa_fwd_splits(ctypes.byref(_problem(B, H, Hk, M, N, D, dtype, causal, mode, 1, 1.0)))
+
+
 def build_plan(prob, eq, ek, status):
     """Mask plan: int32 device buffer consumed by the forward and backward kernels. With ids it
     holds their codes and block statistics; without (eq is None) only the kernels' work counters."""
@@ -221,10 +226,19 @@ class FlashAttention(torch.autograd.Function):
             Mpad = lib.fa_padded_rows(M)
             L = torch.empty((B, H, Mpad), device=q.device, dtype=torch.float32)
             tq, tk, tv, to = _tensor(q), _tensor(k), _tensor(v), _tensor(Out)
-            with _Timed("fwd"):
-                _lib.check(lib.fa_fwd(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
-                                      ctypes.byref(to), L.data_ptr(), plan.data_ptr() if plan is not None else None,
-                                      status.data_ptr(), _stream()), "fa_fwd")
+            # calls that cannot fill the GPU cut their keys into runs (attention_host sets the number of the
+            # whole call, so that a slice computes the same bits)
+            splits = getattr(ctx, "fwd_splits", 0) or lib.fa_fwd_splits(ctypes.byref(prob))
+            work, work_ptr, work_bytes = None, None, 0
+            if splits > 1:
+                nbytes = ctypes.c_size_t(0)
+                _lib.check(lib.fa_fwd_workspace_bytes(ctypes.byref(prob), splits, ctypes.byref(nbytes)), "fa_fwd_workspace_bytes")
+                work = torch.empty(nbytes.value // 4, dtype=torch.float32, device=q.device)
+                work_ptr, work_bytes = work.data_ptr(), nbytes.value
+            with _Timed("fwd", 2 if splits > 1 else 1):
+                _lib.check(lib.fa_fwd_split(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
+                                            ctypes.byref(to), L.data_ptr(), plan.data_ptr() if plan is not None else None,
+                                            splits, work_ptr, work_bytes, status.data_ptr(), _stream()), "fa_fwd_split")
             if _SYNC_STATUS:
                 check_status(q.device)
         # autograd context (flash_triton.py:558-562); eq/ek are kept for the saved-tensor contract,
