@@ -1,0 +1,45 @@
+"""fp32 kernels at the edges of their 32-row CTAs and 64-column tiles, every head dim, with ids that leave whole tiles
+unvisited, against plain attention in 64 bits (1e-4, the fp32 tests' bound)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("offset", [0, 1], ids=["aligned", "odd base"])
+@pytest.mark.parametrize("D", [16, 32, 64, 128])
+@pytest.mark.parametrize("M,N,causal,mode,per_head", [
+    (1, 63, True, 0, False), (31, 64, True, 0, False), (33, 65, True, 1, False), (64, 64, False, 1, True),
+    (127, 129, True, 1, True), (130, 700, True, 1, False), (513, 513, True, 1, True), (200, 77, False, 0, False)])
+def test_tile_edges(M, N, causal, mode, per_head, D, offset):
+    import flash_b200 as fb
+    B, H, Hk = 2, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(M + N + D)
+
+    def rows(h, n):  # with an odd base the rows are only 4-byte aligned
+        x = torch.randn(B * h * n * D + offset, generator=g, device="cuda")[offset:].view(B, h, n, D)
+        return x.detach().requires_grad_()
+
+    q, k, v, do = rows(H, M), rows(Hk, N), rows(Hk, N), rows(H, M).detach()
+    eq = ek = None
+    keep = torch.ones(B, H, M, N, dtype=torch.bool, device="cuda")
+    if mode == 1:
+        heads = H if per_head else 1
+        # documents of 50 to 180 tokens, so that tiles of 64 between them are skipped, and a few ids that see everything
+        ends = torch.cumsum(torch.randint(50, 180, (B, heads, 20), generator=g, device="cuda"), 2)
+        ek = -1 - (torch.arange(N, device="cuda")[:, None] >= ends[:, :, None, :]).sum(3)
+        ek[torch.rand(ek.shape, generator=g, device="cuda") < 0.02] = 3
+        eq = ek[..., torch.arange(M, device="cuda") + N - M] if N >= M else ek[..., torch.randint(0, N, (M,), generator=g, device="cuda")]
+        eq, ek = eq.expand(B, H, M), ek.expand(B, H, N)
+        keep &= (eq[..., None] >= 0) | (eq[..., None] == ek[..., None, :])
+    if causal:
+        keep &= torch.ones(M, N, dtype=torch.bool, device="cuda").tril(N - M)
+    o = fb.attention(q, k, v, causal, None, eq, ek, mode)
+    o.backward(do)
+    fb.check_status()
+    qe, ke, ve = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    s = (qe @ ke.repeat_interleave(2, 1).transpose(2, 3) / D ** 0.5).masked_fill(~keep, -torch.inf)
+    oe = torch.softmax(s, 3) @ ve.repeat_interleave(2, 1)
+    oe.backward(do.double())
+    for what, got, want in (("o", o, oe), ("dq", q.grad, qe.grad), ("dk", k.grad, ke.grad), ("dv", v.grad, ve.grad)):
+        assert (got.double() - want).abs().max().item() < 1e-4, what

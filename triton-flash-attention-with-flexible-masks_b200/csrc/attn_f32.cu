@@ -3,84 +3,163 @@
 // asked of fp32 results, so fp32 tensors take the kernels below: the same flash-attention recurrence
 // (flash_triton.py:94-133 forward, :250-311 dK/dV, :387-423 dQ), the same mask plan, tile
 // classification and per-entry predicate as the 16-bit kernels, but all arithmetic in fp32 FMAs.
-// They cover every head dim the reference accepts (16, 32, 64, 128) and are meant for checks and
-// small problems, not for speed.
+// They cover every head dim the reference accepts (16, 32, 64, 128).
 //
-// One CTA = 128 threads = 4 warps works on 32 "rows" (queries in the forward and dQ kernels, keys
-// in the dK/dV kernel) against tiles of 32 "columns"; warp w owns rows 8w..8w+7, lane = column.
-// Two building blocks on shared-memory tiles with rows padded to D + 4 floats:
-//   rows_dot_cols: s[r] = sum_d A[row r][d] * B[col lane][d]   (A broadcast, B one row per lane)
-//   rows_acc:      acc[r][k] += sum_c P[row r][c] * V[c][lane + 32 k]
+// One CTA = 8 warps works on 32 "rows" (queries in the forward and dQ kernels, keys in the dK/dV kernel) against
+// tiles of 64 "columns", which cp.async brings into the other of two shared-memory stages while a tile is worked
+// on. Warp w owns rows 4w..4w+3 from the scores to the result: half a warp has two rows, lane x of the half has
+// columns x, x + 16, x + 32, x + 48 of the scores (2 x 4 products in registers) and D / 16 columns of the result,
+// so the softmax needs shuffles over 16 lanes and no barrier, and P passes through the warp's own shared rows.
+// These calls are a few hundred rows of a few heads: what bounds them is the chain of tiles of the longest CTA,
+// in it the shared-memory reads (10 wavefronts per 32 FMAs of a warp). 32 rows rather than 64 keep 8 heads of 512 at
+// 128 CTAs.
 #include "../../include/fa_b200.h"
 #include "common.cuh"
 #include "params.cuh"
 
 namespace fa {
 
-constexpr int kT = 32;  // rows per CTA and columns per tile
+constexpr int kR = 32;          // rows per CTA
+constexpr int kC = 64;          // columns per tile
+constexpr int kF32Threads = 256;
+constexpr int kLdP = kC + 4;    // pitch of the P tile
 
 template <int D>
 struct F32Smem {
-    static constexpr int LD = D + 4;
-    static constexpr int tile = kT * LD;  // floats
+    static constexpr int LD = D + 4;  // pitch: 8 lanes that read 16 bytes each of neighbouring rows hit all 32 banks
+    static constexpr int rows = kR * LD, cols = kC * LD, p = kR * kLdP;  // floats
+    static constexpr int vec = 3 * kC;                                   // per column: id code, lse, delta
 };
 
-// loads rows [r0, r0 + 32) of a [L, D] slice into a padded tile; rows >= L are zero
-template <int D>
-__device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t sl, int r0, int L) {
-    constexpr int LD = F32Smem<D>::LD;
-    for (int i = threadIdx.x; i < kT * (D / 4); i += blockDim.x) {
-        const int r = i / (D / 4), c4 = i % (D / 4);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r0 + r < L) {
-            const float* p = src + int64_t(r0 + r) * sl + 4 * c4;
-            if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) v = *reinterpret_cast<const float4*>(p);
-            else v = make_float4(p[0], p[1], p[2], p[3]);
-        }
-        *reinterpret_cast<float4*>(dst + r * LD + 4 * c4) = v;
-    }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool real) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(real ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ bool rows_aligned(const float* base, int64_t sl) {
+    return (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (sl & 3) == 0;
 }
 
-template <int D>
-__device__ __forceinline__ void rows_dot_cols(const float* A, const float* Bt, int warp, int lane, float (&s)[8]) {
+// starts the copy of rows [r0, r0 + NR) of a [L, D] slice into a padded tile; rows >= L become zero. Tensors are only
+// promised to be 4-byte aligned: `vec` says that every row of this one starts on 16 bytes.
+template <int D, int NR>
+__device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t sl, bool vec, int r0, int L) {
     constexpr int LD = F32Smem<D>::LD;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) s[r] = 0.f;
+    if (vec) {
 #pragma unroll 4
-    for (int d4 = 0; d4 < D / 4; ++d4) {
-        const float4 b = *reinterpret_cast<const float4*>(Bt + lane * LD + 4 * d4);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float4 a = *reinterpret_cast<const float4*>(A + (8 * warp + r) * LD + 4 * d4);
-            s[r] = fmaf(a.x, b.x, s[r]);
-            s[r] = fmaf(a.y, b.y, s[r]);
-            s[r] = fmaf(a.z, b.z, s[r]);
-            s[r] = fmaf(a.w, b.w, s[r]);
+        for (int i = threadIdx.x; i < NR * (D / 4); i += kF32Threads) {
+            const int r = i / (D / 4), c = i % (D / 4) * 4;
+            const bool real = r0 + r < L;
+            cp_async16(smem_u32(dst + r * LD + c), real ? src + int64_t(r0 + r) * sl + c : src, real);
         }
-    }
-}
-
-template <int D>
-__device__ __forceinline__ void rows_acc(const float* P, const float* V, int warp, int lane, float (&acc)[8][(D + 31) / 32]) {
-    constexpr int LD = F32Smem<D>::LD;
-    constexpr int NK = (D + 31) / 32;
+    } else {
 #pragma unroll 4
-    for (int c = 0; c < kT; ++c) {
-        float v[NK];
-#pragma unroll
-        for (int k = 0; k < NK; ++k) v[k] = (lane + 32 * k < D) ? V[c * LD + lane + 32 * k] : 0.f;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float p = P[(8 * warp + r) * kT + c];
-#pragma unroll
-            for (int k = 0; k < NK; ++k) acc[r][k] = fmaf(p, v[k], acc[r][k]);
+        for (int i = threadIdx.x; i < NR * D; i += kF32Threads) {
+            const int r = i / D, c = i % D;
+            const bool real = r0 + r < L;
+            cp_async4(smem_u32(dst + r * LD + c), real ? src + int64_t(r0 + r) * sl + c : src, real);
         }
     }
 }
 
-__device__ __forceinline__ float warp_max(float x) {
+// s[r][c] = row (r0 + r) of A . row (x + 16 c) of B; even and odd elements are summed apart (packed FMAs)
+template <int D>
+__device__ __forceinline__ void rows_dot_cols(const float* A, const float* Bt, int r0, int x, float (&s)[2][4]) {
+    constexpr int LD = F32Smem<D>::LD;
+    uint64_t t[2][4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) t[r][c] = 0;
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+        ulonglong2 a[2], b[4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) a[r] = *reinterpret_cast<const ulonglong2*>(A + (r0 + r) * LD + d);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const ulonglong2*>(Bt + (x + 16 * c) * LD + d);
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) t[r][c] = fma_f2(a[r].y, b[c].y, fma_f2(a[r].x, b[c].x, t[r][c]));
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            float lo, hi;
+            unpack_f2(t[r][c], lo, hi);
+            s[r][c] = lo + hi;
+        }
+}
+
+// result columns of lane x: D = 128: 4x..4x+3 and 64 + 4x..; 64: 4x..4x+3; 32: 2x, 2x+1; 16: x
+template <int D>
+struct Own {
+    static constexpr int N = D / 16, W = N < 4 ? N : 4;  // columns per lane, consecutive ones
+    static __device__ __forceinline__ int col(int x, int k) { return k / W * 64 + x * W + k % W; }
+    static __device__ __forceinline__ void load(const float* row, int x, float (&v)[N]) {
+        if constexpr (W == 4) {
+#pragma unroll
+            for (int k = 0; k < N; k += 4) {
+                const float4 t = *reinterpret_cast<const float4*>(row + col(x, k));
+                v[k] = t.x; v[k + 1] = t.y; v[k + 2] = t.z; v[k + 3] = t.w;
+            }
+        } else if constexpr (W == 2) {
+            const float2 t = *reinterpret_cast<const float2*>(row + 2 * x);
+            v[0] = t.x; v[1] = t.y;
+        } else {
+            v[0] = row[x];
+        }
+    }
+    static __device__ __forceinline__ void store(float* row, int x, bool vec, const float (&v)[N], float f) {
+        if (W == 4 && vec) {
+#pragma unroll
+            for (int k = 0; k < N; k += 4)
+                *reinterpret_cast<float4*>(row + col(x, k)) = make_float4(v[k] * f, v[(k + 1) % N] * f, v[(k + 2) % N] * f, v[(k + 3) % N] * f);
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k) row[col(x, k)] = v[k] * f;
+        }
+    }
+};
+
+// acc[r][k] += sum_c P[r0 + r][c] * V[c][own column k]
+template <int D>
+__device__ __forceinline__ void rows_acc(const float* P, const float* V, int r0, int x, float (&acc)[2][D / 16]) {
+    constexpr int LD = F32Smem<D>::LD;
+#pragma unroll 2
+    for (int c = 0; c < kC; c += 4) {
+        const float4 p0 = *reinterpret_cast<const float4*>(P + r0 * kLdP + c);
+        const float4 p1 = *reinterpret_cast<const float4*>(P + (r0 + 1) * kLdP + c);
+        const float w0[4] = {p0.x, p0.y, p0.z, p0.w}, w1[4] = {p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+            float v[D / 16];
+            Own<D>::load(V + (c + cc) * LD, x, v);
+#pragma unroll
+            for (int k = 0; k < D / 16; ++k) {
+                acc[0][k] = fmaf(w0[cc], v[k], acc[0][k]);
+                acc[1][k] = fmaf(w1[cc], v[k], acc[1][k]);
+            }
+        }
+    }
+}
+
+// over the 16 lanes that share a row
+__device__ __forceinline__ float half_max(float x) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    return x;
+}
+__device__ __forceinline__ float half_sum(float x) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     return x;
 }
 __device__ __forceinline__ float warp_sum(float x) {
@@ -89,9 +168,16 @@ __device__ __forceinline__ float warp_sum(float x) {
     return x;
 }
 
-// does the 128 x 128 block that holds rows i0.. and columns j0.. contain an unmasked entry at all?
-__device__ __forceinline__ bool block_visited(const MaskArgs& mk, int b, int he, int i0, int j0) {
-    return (classify_from_plan(mk, b, he, i0 / kBlk, j0 / kBlk) & TILE_VISIT) != 0;
+// visited[o] for every 128-block o of the other side; the caller synchronises
+__device__ __forceinline__ void find_visited(uint8_t* visited, const MaskArgs& mk, int b, int he, bool rows_are_queries, int own) {
+    const int n = rows_are_queries ? mk.L.nK : mk.L.nQ;
+    for (int o = threadIdx.x; o < n; o += kF32Threads)
+        visited[o] = (classify_from_plan(mk, b, he, rows_are_queries ? own : o, rows_are_queries ? o : own) & TILE_VISIT) != 0;
+}
+// first column >= c (a multiple of kC) of a visited block, or end
+__device__ __forceinline__ int next_tile(const uint8_t* visited, int c, int end) {
+    while (c < end && !visited[c / kBlk]) c = c / kBlk * kBlk + kBlk;
+    return c;
 }
 
 __device__ __forceinline__ int code_q(const MaskArgs& mk, int b, int he, int i) {
@@ -105,69 +191,90 @@ __device__ __forceinline__ int code_k(const MaskArgs& mk, int b, int he, int j) 
 // forward: grid (ceil(M / 32), H, B)
 // ---------------------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(128) f32_fwd_kernel(const F32Params p) {
+__global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p) {
+    using S = F32Smem<D>;
     extern __shared__ __align__(16) float sm[];
     float* Qs = sm;
-    float* Ks = Qs + F32Smem<D>::tile;
-    float* Vs = Ks + F32Smem<D>::tile;
-    float* Ps = Vs + F32Smem<D>::tile;  // [32][32]
-    constexpr int NK = (D + 31) / 32;
+    float* KVs = Qs + S::rows;            // two stages of K, V
+    float* Ps = KVs + 4 * S::cols;
+    int* codes = reinterpret_cast<int*>(Ps + S::p);  // two stages
+    __shared__ uint8_t visited[kListCap];
     const MaskArgs& mk = p.mask;
-    const int i0 = blockIdx.x * kT, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;
+    const int i0 = int(gridDim.x - 1 - blockIdx.x) * kR, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;  // long rows first
     const int he = (mk.He == 1) ? 0 : h;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    load_tile<D>(Qs, p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh, p.q.sl, i0, mk.M);
-    float m[8], l[8], acc[8][NK];
-    int qc[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        m[r] = -INFINITY;
-        l[r] = 0.f;
-        qc[r] = code_q(mk, b, he, i0 + 8 * warp + r);
-#pragma unroll
-        for (int k = 0; k < NK; ++k) acc[r][k] = 0.f;
-    }
-    const int hi = mk.causal ? min(mk.N, i0 + kT + mk.gap) : mk.N;  // keys beyond the last row's causal bound
+    const int lane = threadIdx.x & 31, x = lane & 15, r0 = (threadIdx.x >> 5) * 4 + (lane >> 4) * 2;
+    const float* qbase = p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh;
     const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
     const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
-    for (int j0 = 0; j0 < hi; j0 += kT) {
-        if (!block_visited(mk, b, he, i0, j0)) continue;  // uniform for the CTA
-        __syncthreads();
-        load_tile<D>(Ks, kbase, p.k.sl, j0, mk.N);
-        load_tile<D>(Vs, vbase, p.v.sl, j0, mk.N);
-        __syncthreads();
-        const int j = j0 + lane;
-        const int kc = code_k(mk, b, he, j);
-        float s[8];
-        rows_dot_cols<D>(Qs, Ks, warp, lane, s);
+    const bool kvec = rows_aligned(kbase, p.k.sl), vvec = rows_aligned(vbase, p.v.sl);
+    const int32_t* kcodes = mk.mode == 1 ? mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad : nullptr;
+    auto fetch = [&](int j0, int st) {
+        load_tile<D, kC>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, mk.N);
+        load_tile<D, kC>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, mk.N);
+        if (kcodes && threadIdx.x < kC) cp_async4(smem_u32(codes + st * kC + threadIdx.x), kcodes + j0 + threadIdx.x, true);
+    };
+    load_tile<D, kR>(Qs, qbase, p.q.sl, rows_aligned(qbase, p.q.sl), i0, mk.M);
+    find_visited(visited, mk, b, he, true, i0 / kBlk);
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[2][D / 16];
+    int qc[2];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int i = i0 + 8 * warp + r;
-            const bool keep = keep_entry(i, j, qc[r], kc, mk.N, mk.gap, mk.causal, mk.mode);
-            const float sv = keep ? s[r] * p.scale : -INFINITY;
-            const float mn = fmaxf(m[r], warp_max(sv));
+    for (int r = 0; r < 2; ++r) {
+        qc[r] = code_q(mk, b, he, i0 + r0 + r);
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) acc[r][k] = 0.f;
+    }
+    const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;  // keys beyond the last row's causal bound
+    __syncthreads();
+    int j0 = next_tile(visited, 0, end);
+    if (j0 < end) fetch(j0, 0);
+    cp_async_commit();
+    for (int st = 0; j0 < end; st ^= 1) {
+        const int jn = next_tile(visited, j0 + kC, end);
+        if (jn < end) fetch(jn, st ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* Ks = KVs + st * 2 * S::cols;
+        float s[2][4];
+        rows_dot_cols<D>(Qs, Ks, r0, x, s);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int i = i0 + r0 + r;
+            float mx = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int j = j0 + x + 16 * c;
+                const bool keep = keep_entry(i, j, qc[r], kcodes ? codes[st * kC + x + 16 * c] : 0, mk.N, mk.gap, mk.causal, mk.mode);
+                s[r][c] = keep ? s[r][c] * p.scale : -INFINITY;
+                mx = fmaxf(mx, s[r][c]);
+            }
+            const float mn = fmaxf(m[r], half_max(mx));
             const float alpha = (m[r] == -INFINITY) ? 0.f : expf(m[r] - mn);
-            const float pe = (sv == -INFINITY) ? 0.f : expf(sv - mn);
-            l[r] = l[r] * alpha + warp_sum(pe);
             m[r] = mn;
+            l[r] *= alpha;
 #pragma unroll
-            for (int k = 0; k < NK; ++k) acc[r][k] *= alpha;
-            Ps[(8 * warp + r) * kT + lane] = pe;
+            for (int k = 0; k < D / 16; ++k) acc[r][k] *= alpha;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float pe = (s[r][c] == -INFINITY) ? 0.f : expf(s[r][c] - mn);
+                l[r] += pe;
+                Ps[(r0 + r) * kLdP + x + 16 * c] = pe;
+            }
         }
         __syncwarp();
-        rows_acc<D>(Ps, Vs, warp, lane, acc);
-        __syncwarp();
+        rows_acc<D>(Ps, Ks + S::cols, r0, x, acc);
+        __syncthreads();  // the stage may be refilled
+        j0 = jn;
     }
+    float* obase = p.o.ptr + int64_t(b) * p.o.sb + int64_t(h) * p.o.sh;
+    const bool ovec = rows_aligned(obase, p.o.sl);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int i = i0 + 8 * warp + r;
+    for (int r = 0; r < 2; ++r) {
+        const int i = i0 + r0 + r;
+        const float lt = half_sum(l[r]);
         if (i >= mk.M) continue;
-        const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
-        float* po = p.o.ptr + int64_t(b) * p.o.sb + int64_t(h) * p.o.sh + int64_t(i) * p.o.sl;
-#pragma unroll
-        for (int k = 0; k < NK; ++k)
-            if (lane + 32 * k < D) po[lane + 32 * k] = acc[r][k] * inv;
-        if (lane == 0) p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + i] = l[r] > 0.f ? m[r] + logf(l[r]) : -INFINITY;
+        Own<D>::store(obase + int64_t(i) * p.o.sl, x, ovec, acc[r], lt > 0.f ? 1.f / lt : 0.f);
+        if (x == 0) p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + i] = lt > 0.f ? m[r] + logf(lt) : -INFINITY;
     }
 }
 
@@ -191,66 +298,81 @@ __global__ void __launch_bounds__(128) f32_delta_kernel(const F32Params p) {
 // dQ: grid (ceil(M / 32), H, B). rows = queries, columns = keys
 // ---------------------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(128) f32_bwd_dq_kernel(const F32Params p) {
+__global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params p) {
+    using S = F32Smem<D>;
     extern __shared__ __align__(16) float sm[];
     float* Qs = sm;
-    float* dOs = Qs + F32Smem<D>::tile;
-    float* Ks = dOs + F32Smem<D>::tile;
-    float* Vs = Ks + F32Smem<D>::tile;
-    float* Ps = Vs + F32Smem<D>::tile;
-    constexpr int NK = (D + 31) / 32;
+    float* dOs = Qs + S::rows;
+    float* KVs = dOs + S::rows;           // two stages of K, V
+    float* Ps = KVs + 4 * S::cols;
+    int* codes = reinterpret_cast<int*>(Ps + S::p);
+    __shared__ uint8_t visited[kListCap];
     const MaskArgs& mk = p.mask;
-    const int i0 = blockIdx.x * kT, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;
+    const int i0 = int(gridDim.x - 1 - blockIdx.x) * kR, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;
     const int he = (mk.He == 1) ? 0 : h;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    load_tile<D>(Qs, p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh, p.q.sl, i0, mk.M);
-    load_tile<D>(dOs, p.d_o.ptr + int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh, p.d_o.sl, i0, mk.M);
-    float acc[8][NK], lse[8], dl[8];
-    int qc[8];
+    const int lane = threadIdx.x & 31, x = lane & 15, r0 = (threadIdx.x >> 5) * 4 + (lane >> 4) * 2;
+    const float* qbase = p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh;
+    const float* dobase = p.d_o.ptr + int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh;
+    const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
+    const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
+    const bool kvec = rows_aligned(kbase, p.k.sl), vvec = rows_aligned(vbase, p.v.sl);
+    const int32_t* kcodes = mk.mode == 1 ? mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad : nullptr;
+    auto fetch = [&](int j0, int st) {
+        load_tile<D, kC>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, mk.N);
+        load_tile<D, kC>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, mk.N);
+        if (kcodes && threadIdx.x < kC) cp_async4(smem_u32(codes + st * kC + threadIdx.x), kcodes + j0 + threadIdx.x, true);
+    };
+    load_tile<D, kR>(Qs, qbase, p.q.sl, rows_aligned(qbase, p.q.sl), i0, mk.M);
+    load_tile<D, kR>(dOs, dobase, p.d_o.sl, rows_aligned(dobase, p.d_o.sl), i0, mk.M);
+    find_visited(visited, mk, b, he, true, i0 / kBlk);
+    float acc[2][D / 16], lse[2], dl[2];
+    int qc[2];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int i = i0 + 8 * warp + r;
+    for (int r = 0; r < 2; ++r) {
+        const int i = i0 + r0 + r;
         const int64_t ro = (int64_t(b) * p.H + h) * mk.L.Mpad + i;
         lse[r] = (i < mk.M) ? p.lse[ro] : -INFINITY;
         dl[r] = (i < mk.M) ? p.delta[ro] : 0.f;
         qc[r] = code_q(mk, b, he, i);
 #pragma unroll
-        for (int k = 0; k < NK; ++k) acc[r][k] = 0.f;
+        for (int k = 0; k < D / 16; ++k) acc[r][k] = 0.f;
     }
-    const int hi = mk.causal ? min(mk.N, i0 + kT + mk.gap) : mk.N;
-    const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
-    const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
-    for (int j0 = 0; j0 < hi; j0 += kT) {
-        if (!block_visited(mk, b, he, i0, j0)) continue;
+    const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;
+    __syncthreads();
+    int j0 = next_tile(visited, 0, end);
+    if (j0 < end) fetch(j0, 0);
+    cp_async_commit();
+    for (int st = 0; j0 < end; st ^= 1) {
+        const int jn = next_tile(visited, j0 + kC, end);
+        if (jn < end) fetch(jn, st ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
         __syncthreads();
-        load_tile<D>(Ks, kbase, p.k.sl, j0, mk.N);
-        load_tile<D>(Vs, vbase, p.v.sl, j0, mk.N);
-        __syncthreads();
-        const int j = j0 + lane;
-        const int kc = code_k(mk, b, he, j);
-        float s[8], dp[8];
-        rows_dot_cols<D>(Qs, Ks, warp, lane, s);
-        rows_dot_cols<D>(dOs, Vs, warp, lane, dp);
+        const float* Ks = KVs + st * 2 * S::cols;
+        float s[2][4], dp[2][4];
+        rows_dot_cols<D>(Qs, Ks, r0, x, s);
+        rows_dot_cols<D>(dOs, Ks + S::cols, r0, x, dp);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int i = i0 + 8 * warp + r;
-            const bool keep = (i < mk.M) && keep_entry(i, j, qc[r], kc, mk.N, mk.gap, mk.causal, mk.mode);
-            const float pe = keep ? expf(s[r] * p.scale - lse[r]) : 0.f;  // a kept entry has a finite lse
-            Ps[(8 * warp + r) * kT + lane] = pe * (dp[r] - dl[r]);       // dS (flash_triton.py:301)
+        for (int r = 0; r < 2; ++r) {
+            const int i = i0 + r0 + r;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int j = j0 + x + 16 * c;
+                const bool keep = (i < mk.M) && keep_entry(i, j, qc[r], kcodes ? codes[st * kC + x + 16 * c] : 0, mk.N, mk.gap, mk.causal, mk.mode);
+                const float pe = keep ? expf(s[r][c] * p.scale - lse[r]) : 0.f;  // a kept entry has a finite lse
+                Ps[(r0 + r) * kLdP + x + 16 * c] = keep ? pe * (dp[r][c] - dl[r]) : 0.f;  // dS (flash_triton.py:301)
+            }
         }
         __syncwarp();
-        rows_acc<D>(Ps, Ks, warp, lane, acc);  // dQ += dS K (flash_triton.py:420)
-        __syncwarp();
+        rows_acc<D>(Ps, Ks, r0, x, acc);  // dQ += dS K (flash_triton.py:420)
+        __syncthreads();
+        j0 = jn;
     }
+    float* dqbase = p.dq.ptr + int64_t(b) * p.dq.sb + int64_t(h) * p.dq.sh;
+    const bool dqvec = rows_aligned(dqbase, p.dq.sl);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int i = i0 + 8 * warp + r;
-        if (i >= mk.M) continue;
-        float* pq = p.dq.ptr + int64_t(b) * p.dq.sb + int64_t(h) * p.dq.sh + int64_t(i) * p.dq.sl;
-#pragma unroll
-        for (int k = 0; k < NK; ++k)
-            if (lane + 32 * k < D) pq[lane + 32 * k] = acc[r][k] * p.scale;  // flash_triton.py:425
-    }
+    for (int r = 0; r < 2; ++r)
+        if (i0 + r0 + r < mk.M) Own<D>::store(dqbase + int64_t(i0 + r0 + r) * p.dq.sl, x, dqvec, acc[r], p.scale);  // flash_triton.py:425
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -258,105 +380,123 @@ __global__ void __launch_bounds__(128) f32_bwd_dq_kernel(const F32Params p) {
 // are walked one after the other, so the group sum (flash_triton.py:635-637) needs no second pass
 // ---------------------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(128) f32_bwd_dkdv_kernel(const F32Params p) {
+__global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Params p) {
+    using S = F32Smem<D>;
     extern __shared__ __align__(16) float sm[];
     float* Ks = sm;
-    float* Vs = Ks + F32Smem<D>::tile;
-    float* Qs = Vs + F32Smem<D>::tile;
-    float* dOs = Qs + F32Smem<D>::tile;
-    float* Ps = dOs + F32Smem<D>::tile;
-    constexpr int NK = (D + 31) / 32;
+    float* Vs = Ks + S::rows;
+    float* QDs = Vs + S::rows;            // two stages of Q, dO
+    float* Ps = QDs + 4 * S::cols;
+    float* vecs = Ps + S::p;              // two stages of id code, lse, delta per query
+    __shared__ uint8_t visited[kListCap];
     const MaskArgs& mk = p.mask;
-    const int j0 = blockIdx.x * kT, hk = blockIdx.y, b = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    load_tile<D>(Ks, p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh, p.k.sl, j0, mk.N);
-    load_tile<D>(Vs, p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh, p.v.sl, j0, mk.N);
-    float dk[8][NK], dv[8][NK];
+    const int j0 = blockIdx.x * kR, hk = blockIdx.y, b = blockIdx.z;
+    const int lane = threadIdx.x & 31, x = lane & 15, r0 = (threadIdx.x >> 5) * 4 + (lane >> 4) * 2;
+    const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
+    const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
+    load_tile<D, kR>(Ks, kbase, p.k.sl, rows_aligned(kbase, p.k.sl), j0, mk.N);
+    load_tile<D, kR>(Vs, vbase, p.v.sl, rows_aligned(vbase, p.v.sl), j0, mk.N);
+    float dk[2][D / 16], dv[2][D / 16];
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int k = 0; k < NK; ++k) dk[r][k] = dv[r][k] = 0.f;
+        for (int k = 0; k < D / 16; ++k) dk[r][k] = dv[r][k] = 0.f;
     // first query row that can see key j0 under the causal mask (flash_triton.py:214-218)
-    const int lo = mk.causal ? max(0, j0 - mk.gap) / kT * kT : 0;
+    const int first = mk.causal ? max(0, j0 - mk.gap) / kC * kC : 0;
     for (int g = 0; g < p.G; ++g) {
         const int h = hk * p.G + g;
         const int he = (mk.He == 1) ? 0 : h;
-        int kc[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) kc[r] = code_k(mk, b, he, j0 + 8 * warp + r);
         const float* qbase = p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh;
         const float* dobase = p.d_o.ptr + int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh;
-        for (int i0 = lo; i0 < mk.M; i0 += kT) {
-            if (!block_visited(mk, b, he, i0, j0)) continue;
-            __syncthreads();
-            load_tile<D>(Qs, qbase, p.q.sl, i0, mk.M);
-            load_tile<D>(dOs, dobase, p.d_o.sl, i0, mk.M);
-            __syncthreads();
-            const int i = i0 + lane;
-            const int64_t ro = (int64_t(b) * p.H + h) * mk.L.Mpad + i;
-            const float lse = (i < mk.M) ? p.lse[ro] : -INFINITY;
-            const float dl = (i < mk.M) ? p.delta[ro] : 0.f;
-            const int qc = code_q(mk, b, he, i);
-            float s[8], dp[8];
-            rows_dot_cols<D>(Ks, Qs, warp, lane, s);    // S^T
-            rows_dot_cols<D>(Vs, dOs, warp, lane, dp);  // dP^T
-            float pe[8];
+        const bool qvec = rows_aligned(qbase, p.q.sl), dovec = rows_aligned(dobase, p.d_o.sl);
+        const int64_t ro = (int64_t(b) * p.H + h) * mk.L.Mpad;
+        const int32_t* qcodes = mk.mode == 1 ? mk.plan + mk.L.off_qc + (int64_t(b) * mk.He + he) * mk.L.Mpad : nullptr;
+        auto fetch = [&](int i0, int st) {
+            load_tile<D, kC>(QDs + st * 2 * S::cols, qbase, p.q.sl, qvec, i0, mk.M);
+            load_tile<D, kC>(QDs + (st * 2 + 1) * S::cols, dobase, p.d_o.sl, dovec, i0, mk.M);
+            if (threadIdx.x < S::vec) {  // the per-row buffers are padded to 128 rows; what pads them is not used
+                const int t = threadIdx.x % kC, what = threadIdx.x / kC;
+                const void* src = what == 0 ? static_cast<const void*>(qcodes) : what == 1 ? p.lse + ro : p.delta + ro;
+                if (src) cp_async4(smem_u32(vecs + st * S::vec + threadIdx.x), static_cast<const float*>(src) + i0 + t, true);
+            }
+        };
+        if (g == 0 || mk.He != 1) find_visited(visited, mk, b, he, false, j0 / kBlk);
+        int kc[2];
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int j = j0 + 8 * warp + r;
-                const bool keep = (i < mk.M) && keep_entry(i, j, qc, kc[r], mk.N, mk.gap, mk.causal, mk.mode);
-                pe[r] = keep ? expf(s[r] * p.scale - lse) : 0.f;
-                Ps[(8 * warp + r) * kT + lane] = pe[r];
+        for (int r = 0; r < 2; ++r) kc[r] = code_k(mk, b, he, j0 + r0 + r);
+        __syncthreads();
+        int i0 = next_tile(visited, first, mk.M);
+        if (i0 < mk.M) fetch(i0, 0);
+        cp_async_commit();
+        for (int st = 0; i0 < mk.M; st ^= 1) {
+            const int in = next_tile(visited, i0 + kC, mk.M);
+            if (in < mk.M) fetch(in, st ^ 1);
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+            const float* Qs = QDs + st * 2 * S::cols;
+            const float* dOs = Qs + S::cols;
+            const float* vec = vecs + st * S::vec;
+            float s[2][4], dp[2][4];
+            rows_dot_cols<D>(Ks, Qs, r0, x, s);    // S^T
+            rows_dot_cols<D>(Vs, dOs, r0, x, dp);  // dP^T
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int i = i0 + x + 16 * c;
+                const int qc = qcodes ? __float_as_int(vec[x + 16 * c]) : 0;
+                const float lse = vec[kC + x + 16 * c], dl = vec[2 * kC + x + 16 * c];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const bool keep = (i < mk.M) && keep_entry(i, j0 + r0 + r, qc, kc[r], mk.N, mk.gap, mk.causal, mk.mode);
+                    const float pe = keep ? expf(s[r][c] * p.scale - lse) : 0.f;
+                    Ps[(r0 + r) * kLdP + x + 16 * c] = pe;
+                    dp[r][c] = keep ? pe * (dp[r][c] - dl) : 0.f;
+                }
             }
             __syncwarp();
-            rows_acc<D>(Ps, dOs, warp, lane, dv);  // dV += P^T dO (flash_triton.py:291)
+            rows_acc<D>(Ps, dOs, r0, x, dv);  // dV += P^T dO (flash_triton.py:291)
             __syncwarp();
 #pragma unroll
-            for (int r = 0; r < 8; ++r) Ps[(8 * warp + r) * kT + lane] = pe[r] * (dp[r] - dl);
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) Ps[(r0 + r) * kLdP + x + 16 * c] = dp[r][c];
             __syncwarp();
-            rows_acc<D>(Ps, Qs, warp, lane, dk);   // dK += dS^T Q (flash_triton.py:308)
-            __syncwarp();
+            rows_acc<D>(Ps, Qs, r0, x, dk);   // dK += dS^T Q (flash_triton.py:308)
+            __syncthreads();
+            i0 = in;
         }
     }
+    cp_async_wait<0>();
+    float* dkbase = p.dk.ptr + int64_t(b) * p.dk.sb + int64_t(hk) * p.dk.sh;
+    float* dvbase = p.dv.ptr + int64_t(b) * p.dv.sb + int64_t(hk) * p.dv.sh;
+    const bool dkvec = rows_aligned(dkbase, p.dk.sl), dvvec = rows_aligned(dvbase, p.dv.sl);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int j = j0 + 8 * warp + r;
+    for (int r = 0; r < 2; ++r) {
+        const int j = j0 + r0 + r;
         if (j >= mk.N) continue;
-        float* pk = p.dk.ptr + int64_t(b) * p.dk.sb + int64_t(hk) * p.dk.sh + int64_t(j) * p.dk.sl;
-        float* pv = p.dv.ptr + int64_t(b) * p.dv.sb + int64_t(hk) * p.dv.sh + int64_t(j) * p.dv.sl;
-#pragma unroll
-        for (int k = 0; k < NK; ++k)
-            if (lane + 32 * k < D) {
-                pk[lane + 32 * k] = dk[r][k] * p.scale;  // flash_triton.py:313
-                pv[lane + 32 * k] = dv[r][k];
-            }
+        Own<D>::store(dkbase + int64_t(j) * p.dk.sl, x, dkvec, dk[r], p.scale);  // flash_triton.py:313
+        Own<D>::store(dvbase + int64_t(j) * p.dv.sl, x, dvvec, dv[r], 1.f);
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 template <int D>
 static cudaError_t launch_f32_t(int which, const F32Params& p, cudaStream_t stream) {
+    using S = F32Smem<D>;
     const MaskArgs& mk = p.mask;
-    constexpr int tile = F32Smem<D>::tile;
-    cudaError_t e = cudaSuccess;
-    if (which == 0) {
-        const int smem = (3 * tile + kT * kT) * 4;
-        e = cudaFuncSetAttribute(f32_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int fwd_smem = (S::rows + 4 * S::cols + S::p + 2 * kC) * 4;
+    constexpr int bwd_smem = (2 * S::rows + 4 * S::cols + S::p + 2 * S::vec) * 4;
+    static_assert(bwd_smem + kListCap <= 232448, "shared memory budget");
+    auto run = [&](auto kern, int smem, int rows, int heads) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
-        f32_fwd_kernel<D><<<dim3(cdiv(mk.M, kT), p.H, p.B), 128, smem, stream>>>(p);
-    } else if (which == 1) {
-        f32_delta_kernel<D><<<dim3(unsigned(mk.L.Mpad / 4), p.H, p.B), 128, 0, stream>>>(p);
-    } else if (which == 2) {
-        const int smem = (4 * tile + kT * kT) * 4;
-        e = cudaFuncSetAttribute(f32_bwd_dkdv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        f32_bwd_dkdv_kernel<D><<<dim3(cdiv(mk.N, kT), p.Hk, p.B), 128, smem, stream>>>(p);
-    } else {
-        const int smem = (4 * tile + kT * kT) * 4;
-        e = cudaFuncSetAttribute(f32_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        f32_bwd_dq_kernel<D><<<dim3(cdiv(mk.M, kT), p.H, p.B), 128, smem, stream>>>(p);
-    }
+        kern<<<dim3(cdiv(rows, kR), heads, p.B), kF32Threads, smem, stream>>>(p);
+        return cudaGetLastError();
+    };
+    if (which == 0) return run(f32_fwd_kernel<D>, fwd_smem, mk.M, p.H);
+    if (which == 2) return run(f32_bwd_dkdv_kernel<D>, bwd_smem, mk.N, p.Hk);
+    if (which == 3) return run(f32_bwd_dq_kernel<D>, bwd_smem, mk.M, p.H);
+    f32_delta_kernel<D><<<dim3(unsigned(mk.L.Mpad / 4), p.H, p.B), 128, 0, stream>>>(p);
     return cudaGetLastError();
 }
 
