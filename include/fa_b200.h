@@ -91,6 +91,10 @@ int64_t fa_padded_rows(int32_t M);
  * counters of the attention kernels only; such a plan is optional). */
 int fa_plan_bytes(const fa_problem* p, size_t* bytes);
 
+/* 1 if a plan would not change how the launches for this problem share out their work: no ids, and no launch
+ * (with `backward` != 0, of the backward too) has more items than the current device has SMs. */
+int fa_plan_optional(const fa_problem* p, int32_t backward);
+
 /* Builds the mask plan from eq [B,H,M] / ek [B,H,N]: 32-bit id codes, per-128-block id
  * min/max, per-block ranges of blocks that hold at least one unmasked entry, and a few work
  * counters through which the CTAs of fa_fwd / fa_bwd_dkdv / fa_bwd_dq share out their work.
@@ -135,6 +139,11 @@ int fa_bwd_dkdv(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, con
 int fa_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v,
               const fa_tensor* d_o, const float* lse, const float* delta, const fa_tensor* dq,
               const void* plan, int32_t* status, void* stream);
+
+/* fa_bwd_delta, fa_bwd_dkdv and fa_bwd_dq in this order; stops at the first that fails. */
+int fa_bwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
+           const fa_tensor* d_o, const float* lse, float* delta, const fa_tensor* dq, const fa_tensor* dk,
+           const fa_tensor* dv, const void* plan, int32_t* status, void* stream);
 
 /* Debug: materialise the kernels' decisions. keep is [B, id_heads, M, N] bytes (1 = unmasked),
  * produced by the same device predicate the attention kernels use; tile_class is

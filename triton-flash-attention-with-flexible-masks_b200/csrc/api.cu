@@ -316,6 +316,15 @@ int fa_plan_bytes(const fa_problem* p, size_t* bytes) {
     return FA_OK;
 }
 
+int fa_plan_optional(const fa_problem* p, int32_t backward) {
+    if (check_problem(p) || p->mode != FA_MODE0_NOPE) return 0;
+    if (p->dtype == FA_FP32) return 1;
+    const int sms = sm_count();
+    const int64_t nq = int64_t(fa::cdiv(p->M, fa::kBlk)) * p->B, nk = int64_t(fa::cdiv(p->N, fa::kBlk)) * p->B;
+    const bool fwd = nq * p->Hk * fa::cdiv(p->H / p->Hk, fwd_pack(p)) <= sms;
+    return fwd && (!backward || (nq * p->H <= sms && nk * p->Hk <= sms));
+}
+
 int fa_plan_build(const fa_problem* p, const fa_ids* eq, const fa_ids* ek, void* plan, size_t plan_bytes,
                   int32_t* status, void* stream) {
     const int rc = check_problem(p);
@@ -515,6 +524,15 @@ int fa_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const
     const cudaError_t e =
         fa::launch_bwd_dq(p->D, p->dtype == FA_BF16, tq, tk, tv, tdo, tdq, qp, sms, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+}
+
+int fa_bwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
+           const fa_tensor* d_o, const float* lse, float* delta, const fa_tensor* dq, const fa_tensor* dk, const fa_tensor* dv,
+           const void* plan, int32_t* status, void* stream) {
+    int rc = fa_bwd_delta(p, o, d_o, delta, stream);
+    if (!rc) rc = fa_bwd_dkdv(p, q, k, v, d_o, lse, delta, dk, dv, plan, status, stream);
+    if (!rc) rc = fa_bwd_dq(p, q, k, v, d_o, lse, delta, dq, plan, status, stream);
+    return rc;
 }
 
 uint32_t fa_classify_tile(int32_t M, int32_t N, int32_t causal, int32_t mode, int32_t qb, int32_t kb, int32_t qmin,

@@ -678,7 +678,8 @@ static cudaError_t launch_dkdv_t(const CUtensorMap& tq, const CUtensorMap& tk, c
                                  const DkdvParams& p, int num_sms, cudaStream_t stream) {
     auto kern = bwd_dkdv_kernel<D, BF16>;
     constexpr int smem = DkdvSmem<D>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<uint64_t> allowed{0};
+    cudaError_t e = allow_smem(kern, smem, allowed);
     if (e != cudaSuccess) return e;
     const int n_items = p.mask.L.nK * p.Hk * p.B;
     const int grid = n_items < num_sms ? n_items : num_sms;

@@ -554,7 +554,8 @@ static cudaError_t launch_dq_t(const CUtensorMap& tq, const CUtensorMap& tk, con
                                cudaStream_t stream) {
     auto kern = bwd_dq_kernel<D, BF16>;
     constexpr int smem = DqSmem<D>::total;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<uint64_t> allowed{0};
+    cudaError_t e = allow_smem(kern, smem, allowed);
     if (e != cudaSuccess) return e;
     const int n_items = p.mask.L.nQ * p.H * p.B;
     const int grid = n_items < num_sms ? n_items : num_sms;

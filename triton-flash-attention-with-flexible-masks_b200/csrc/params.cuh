@@ -1,5 +1,6 @@
 // Kernel parameter blocks, filled by api.cu.
 #pragma once
+#include <atomic>
 #include "common.cuh"
 
 namespace fa {
@@ -80,6 +81,20 @@ struct F32Params {
     int B, H, Hk, G;
     float scale;
 };
+
+// Lets kernels of this launch site use `bytes` of dynamic shared memory. The attribute belongs to the device: it is set
+// once per device (always to the same value, so a race between two first calls is harmless). One `done` per kernel.
+template <class Kernel>
+inline cudaError_t allow_smem(Kernel kern, int bytes, std::atomic<uint64_t>& done) {
+    int dev = -1;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = (dev >= 0 && dev < 64) ? uint64_t(1) << dev : 0;
+    if (bit && (done.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
+    const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (r == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return r;
+}
 
 // Ordered compaction of per-tile flags (list[i] = flags of tile lo+i) into the visited list:
 // entry = (i) | flags << 10. One warp; returns the number of visited tiles.

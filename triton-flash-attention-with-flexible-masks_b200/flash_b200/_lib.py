@@ -16,6 +16,7 @@ EXPORTS = (
     "fa_version", "fa_error_string", "fa_padded_rows", "fa_plan_bytes", "fa_plan_build", "fa_fwd",
     "fa_bwd_delta", "fa_bwd_dkdv", "fa_bwd_dq", "fa_debug_mask", "fa_classify_tile", "fa_fwd_static_plan",
     "fa_debug_wait_timeout", "fa_group_rows", "fa_permute_rows", "fa_fwd_splits", "fa_fwd_workspace_bytes", "fa_fwd_split",
+    "fa_plan_optional", "fa_bwd",
 )
 
 
@@ -68,6 +69,10 @@ def load():
     lib.fa_fwd_workspace_bytes.argtypes = [P, ctypes.c_int32, ctypes.POINTER(ctypes.c_size_t)]
     lib.fa_fwd_split.restype = i32
     lib.fa_fwd_split.argtypes = [P, T, T, T, T, vp, vp, ctypes.c_int32, vp, ctypes.c_size_t, vp, vp]
+    lib.fa_plan_optional.restype = i32
+    lib.fa_plan_optional.argtypes = [P, ctypes.c_int32]
+    lib.fa_bwd.restype = i32
+    lib.fa_bwd.argtypes = [P, T, T, T, T, T, vp, vp, T, T, T, vp, vp, vp]
     lib.fa_bwd_delta.restype = i32
     lib.fa_bwd_delta.argtypes = [P, T, T, vp, vp]
     lib.fa_bwd_dkdv.restype = i32

@@ -73,6 +73,8 @@ class _Ctx:
     directly, which saves the autograd bookkeeping and the hop to the engine's thread per slice (the
     host's time per slice decides how fine the slices can be)."""
 
+    needs_input_grad = (True, True, True)
+
     def save_for_backward(self, *tensors):
         self.saved_tensors = tensors
 

@@ -5,6 +5,7 @@ signature, defaults, assertions, saved-tensor contract and return convention; th
 launches are replaced by calls into libfa_b200.so (hand-written sm_100a kernels). There is no
 Triton, no dispatch over back-ends and no CPU path: CPU tensors raise.
 """
+import contextlib
 import ctypes
 import math
 import os
@@ -29,28 +30,39 @@ LAUNCHES = 0
 
 
 class _Timed:
-    """Brackets one C-ABI call with CUDA events on the current stream when PROFILE is a list."""
+    """Brackets one C-ABI call with CUDA events on the current stream when PROFILE is a list (`_timed`)."""
 
-    def __init__(self, name, kernels=1):
-        self.name, self.kernels = name, kernels
+    def __init__(self, name):
+        self.name = name
 
     def __enter__(self):
-        global LAUNCHES
-        LAUNCHES += self.kernels
-        if PROFILE is not None:
-            # inside a CUDA graph capture the events become record nodes of the graph, re-recorded by
-            # every replay and readable after it
-            ext = torch.cuda.is_current_stream_capturing()
-            self.e0 = torch.cuda.Event(enable_timing=True, external=ext)
-            self.e1 = torch.cuda.Event(enable_timing=True, external=ext)
-            self.e0.record()
+        # inside a CUDA graph capture the events become record nodes of the graph, re-recorded by
+        # every replay and readable after it
+        ext = torch.cuda.is_current_stream_capturing()
+        self.e0 = torch.cuda.Event(enable_timing=True, external=ext)
+        self.e1 = torch.cuda.Event(enable_timing=True, external=ext)
+        self.e0.record()
         return self
 
     def __exit__(self, *exc):
+        self.e1.record()
         if PROFILE is not None:
-            self.e1.record()
             PROFILE.append((self.name, self.e0, self.e1))
         return False
+
+
+_UNTIMED = contextlib.nullcontext()
+
+
+def _timed(name, kernels=1):
+    global LAUNCHES
+    LAUNCHES += kernels
+    return _UNTIMED if PROFILE is None else _Timed(name)
+
+
+def _current(device):
+    """A context in which `device` is the current one; nothing to do, and nothing paid, if it is already."""
+    return _UNTIMED if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _status_word(device):
@@ -93,7 +105,10 @@ def check_status(device=None):
 def maybe_contiguous(x):
     """flash_triton.py:435-437, extended by the TMA rules: last stride 1, 16-byte aligned base,
     other strides positive multiples of 8 elements."""
-    ok = x.stride(-1) == 1 and x.data_ptr() % 16 == 0
+    ok = x.data_ptr() % 16 == 0
+    if ok and x.is_contiguous() and x.shape[-1] % 8 == 0:
+        return x
+    ok = ok and x.stride(-1) == 1
     if ok:
         for size, stride in zip(x.shape[:-1], x.stride()[:-1]):
             if size > 1 and (stride <= 0 or stride % 8 != 0):
@@ -111,20 +126,11 @@ def _same_device(ref, **tensors):
 
 
 def _tensor(x):
-    t = _lib.Tensor()
-    t.ptr = x.data_ptr()
-    for i in range(4):
-        t.stride[i] = x.stride(i)
-    return t
+    return _lib.Tensor(x.data_ptr(), x.stride())
 
 
 def _ids(x):
-    i = _lib.Ids()
-    i.ptr = x.data_ptr()
-    for d in range(3):
-        i.stride[d] = x.stride(d)
-    i.dtype = _lib.FA_ID_INT32 if x.dtype == torch.int32 else _lib.FA_ID_INT64
-    return i
+    return _lib.Ids(x.data_ptr(), x.stride(), _lib.FA_ID_INT32 if x.dtype == torch.int32 else _lib.FA_ID_INT64)
 
 
 def _id_tensor(e, B, H, L, name):
@@ -137,20 +143,14 @@ def _id_tensor(e, B, H, L, name):
 
 
 def _problem(B, H, Hk, M, N, D, dtype, causal, mode, id_heads, sm_scale):
-    p = _lib.Problem()
-    p.B, p.H, p.Hk, p.M, p.N, p.D = B, H, Hk, M, N, D
     if dtype not in _DTYPES:
         raise NotImplementedError(f"flash_b200 supports bf16, fp16 and fp32 inputs, got {dtype}")
-    p.dtype = _DTYPES[dtype]
-    p.causal = 1 if causal else 0
-    p.mode = int(mode)
-    p.id_heads = id_heads
-    p.sm_scale = float(sm_scale)
-    return p
+    return _lib.Problem(B, H, Hk, M, N, D, _DTYPES[dtype], 1 if causal else 0, int(mode), id_heads, float(sm_scale))
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device, as the library takes it."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def forward_splits(B, H, Hk, M, N, D, dtype, causal, mode):
@@ -163,15 +163,15 @@ def build_plan(prob, eq, ek, status):
     holds their codes and block statistics; without (eq is None) only the kernels' work counters."""
     lib = _lib.load()
     nbytes = ctypes.c_size_t(0)
-    _lib.check(lib.fa_plan_bytes(ctypes.byref(prob), ctypes.byref(nbytes)), "fa_plan_bytes")
+    _lib.check(lib.fa_plan_bytes(prob, ctypes.byref(nbytes)), "fa_plan_bytes")
     plan = torch.empty(max(nbytes.value // 4, 1), dtype=torch.int32, device=status.device)
     if eq is None:
-        _lib.check(lib.fa_plan_build(ctypes.byref(prob), None, None, plan.data_ptr(), nbytes.value,
+        _lib.check(lib.fa_plan_build(prob, None, None, plan.data_ptr(), nbytes.value,
                                      status.data_ptr(), _stream()), "fa_plan_build")
         return plan
     ieq, iek = _ids(eq), _ids(ek)
-    with _Timed("plan", 3):
-        _lib.check(lib.fa_plan_build(ctypes.byref(prob), ctypes.byref(ieq), ctypes.byref(iek), plan.data_ptr(),
+    with _timed("plan", 3):
+        _lib.check(lib.fa_plan_build(prob, ieq, iek, plan.data_ptr(),
                                      nbytes.value, status.data_ptr(), _stream()), "fa_plan_build")
     return plan
 
@@ -199,7 +199,9 @@ class FlashAttention(torch.autograd.Function):
         assert score_func_mode in (SCORE_FUNC_MODE0_NOPE, SCORE_FUNC_MODE1_DOC)
         if not q.is_cuda:
             raise RuntimeError("flash_b200 runs on CUDA tensors only (there is no CPU implementation)")
-        _same_device(q, k=k, v=v, eq=eq, ek=ek)
+        device = q.device
+        if k.device != device or v.device != device or (eq is not None and (eq.device != device or ek.device != device)):
+            _same_device(q, k=k, v=v, eq=eq, ek=ek)
         if k.dtype != q.dtype or v.dtype != q.dtype:
             raise ValueError(f"flash_b200: q, k, v must share one dtype, got {q.dtype}, {k.dtype}, {v.dtype}")
         if sm_scale is None:
@@ -213,32 +215,32 @@ class FlashAttention(torch.autograd.Function):
             ek = _id_tensor(ek, B, H, N, "ek")
             broadcast = (H == 1) or (eq.stride(1) == 0 and ek.stride(1) == 0)
             id_heads = 1 if broadcast else H
-        with torch.cuda.device(q.device):
+        with _current(device):
             prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, id_heads, sm_scale)
-            status = _status_word(q.device)
+            status = _status_word(device)
             if score_func_mode == SCORE_FUNC_MODE1_DOC:
                 plan = build_plan(prob, eq, ek, status)
+            elif lib.fa_plan_optional(prob, any(ctx.needs_input_grad[:3])):
+                plan = None  # no more items than SMs: nothing to count
             else:
                 plan = build_plan(prob, None, None, status)
             Out = torch.empty_like(q)
             if maybe_contiguous(Out) is not Out:
-                Out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-            Mpad = lib.fa_padded_rows(M)
-            L = torch.empty((B, H, Mpad), device=q.device, dtype=torch.float32)
-            tq, tk, tv, to = _tensor(q), _tensor(k), _tensor(v), _tensor(Out)
+                Out = torch.empty(q.shape, dtype=q.dtype, device=device)
+            L = torch.empty((B, H, (M + 127) // 128 * 128), device=device, dtype=torch.float32)
             # calls that cannot fill the GPU cut their keys into runs (attention_host sets the number of the
             # whole call, so that a slice computes the same bits)
-            splits = getattr(ctx, "fwd_splits", 0) or lib.fa_fwd_splits(ctypes.byref(prob))
+            splits = getattr(ctx, "fwd_splits", 0) or lib.fa_fwd_splits(prob)
             work, work_ptr, work_bytes = None, None, 0
             if splits > 1:
                 nbytes = ctypes.c_size_t(0)
-                _lib.check(lib.fa_fwd_workspace_bytes(ctypes.byref(prob), splits, ctypes.byref(nbytes)), "fa_fwd_workspace_bytes")
-                work = torch.empty(nbytes.value // 4, dtype=torch.float32, device=q.device)
+                _lib.check(lib.fa_fwd_workspace_bytes(prob, splits, ctypes.byref(nbytes)), "fa_fwd_workspace_bytes")
+                work = torch.empty(nbytes.value // 4, dtype=torch.float32, device=device)
                 work_ptr, work_bytes = work.data_ptr(), nbytes.value
-            with _Timed("fwd", 2 if splits > 1 else 1):
-                _lib.check(lib.fa_fwd_split(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
-                                            ctypes.byref(to), L.data_ptr(), plan.data_ptr() if plan is not None else None,
-                                            splits, work_ptr, work_bytes, status.data_ptr(), _stream()), "fa_fwd_split")
+            with _timed("fwd", 2 if splits > 1 else 1):
+                _lib.check(lib.fa_fwd_split(prob, _tensor(q), _tensor(k), _tensor(v), _tensor(Out), L.data_ptr(),
+                                            plan.data_ptr() if plan is not None else None, splits, work_ptr, work_bytes,
+                                            status.data_ptr(), _stream()), "fa_fwd_split")
             if _SYNC_STATUS:
                 check_status(q.device)
         # autograd context (flash_triton.py:558-562); eq/ek are kept for the saved-tensor contract,
@@ -264,36 +266,37 @@ class FlashAttention(torch.autograd.Function):
         B, H, M, D, N, Hk, num_groups, MN_GAP = ctx.shapes
         score_func_mode, = ctx.score_func_info
         plan = ctx.plan
-        _same_device(q, do=do)
+        device = q.device
+        if do.device != device:
+            _same_device(q, do=do)
         if do.dtype != q.dtype:
             do = do.to(q.dtype)
         do = maybe_contiguous(do)
-        with torch.cuda.device(q.device):
+        with _current(device):
             prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, ctx.id_heads, sm_scale)
-            status = _status_word(q.device)
+            status = _status_word(device)
             stream = _stream()
             plan_ptr = plan.data_ptr() if plan is not None else None
-            tq, tk, tv, to, tdo = _tensor(q), _tensor(k), _tensor(v), _tensor(o), _tensor(do)
-            # delta = rowsum(o * do) (flash_triton.py:584-592)
             delta = torch.empty_like(L)
-            with _Timed("delta"):
-                _lib.check(lib.fa_bwd_delta(ctypes.byref(prob), ctypes.byref(to), ctypes.byref(tdo), delta.data_ptr(),
-                                            stream), "fa_bwd_delta")
-            # dk, dv (flash_triton.py:594-614, group sum of :635-637 done inside the kernel)
-            dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=q.device)
-            dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=q.device)
-            tdk, tdv = _tensor(dk), _tensor(dv)
-            with _Timed("dkdv"):
-                _lib.check(lib.fa_bwd_dkdv(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
-                                           ctypes.byref(tdo), L.data_ptr(), delta.data_ptr(), ctypes.byref(tdk),
-                                           ctypes.byref(tdv), plan_ptr, status.data_ptr(), stream), "fa_bwd_dkdv")
-            # dq (flash_triton.py:616-634); every row is written by the kernel
-            dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-            tdq = _tensor(dq)
-            with _Timed("dq"):
-                _lib.check(lib.fa_bwd_dq(ctypes.byref(prob), ctypes.byref(tq), ctypes.byref(tk), ctypes.byref(tv),
-                                         ctypes.byref(tdo), L.data_ptr(), delta.data_ptr(), ctypes.byref(tdq), plan_ptr,
-                                         status.data_ptr(), stream), "fa_bwd_dq")
+            dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=device)
+            dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=device)
+            dq = torch.empty(q.shape, dtype=q.dtype, device=device)
+            tq, tk, tv, to, tdo = _tensor(q), _tensor(k), _tensor(v), _tensor(o), _tensor(do)
+            tdq, tdk, tdv = _tensor(dq), _tensor(dk), _tensor(dv)
+            lp, dp, sp = L.data_ptr(), delta.data_ptr(), status.data_ptr()
+            if PROFILE is None:  # the three kernels in one call
+                with _timed("bwd", 3):
+                    _lib.check(lib.fa_bwd(prob, tq, tk, tv, to, tdo, lp, dp, tdq, tdk, tdv, plan_ptr, sp, stream), "fa_bwd")
+            else:
+                # delta = rowsum(o * do) (flash_triton.py:584-592)
+                with _timed("delta"):
+                    _lib.check(lib.fa_bwd_delta(prob, to, tdo, dp, stream), "fa_bwd_delta")
+                # dk, dv (flash_triton.py:594-614, group sum of :635-637 done inside the kernel)
+                with _timed("dkdv"):
+                    _lib.check(lib.fa_bwd_dkdv(prob, tq, tk, tv, tdo, lp, dp, tdk, tdv, plan_ptr, sp, stream), "fa_bwd_dkdv")
+                # dq (flash_triton.py:616-634); every row is written by the kernel
+                with _timed("dq"):
+                    _lib.check(lib.fa_bwd_dq(prob, tq, tk, tv, tdo, lp, dp, tdq, plan_ptr, sp, stream), "fa_bwd_dq")
             if _SYNC_STATUS:
                 check_status(q.device)
         return dq, dk, dv, None, None, None, None, None
@@ -316,11 +319,11 @@ def _permute_rows(x, index, id_heads):
     x = maybe_contiguous(x)
     B, H, M, D = x.shape
     out = torch.empty((B, H, M, D), dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
+    with _current(x.device):
         prob = _problem(B, H, H, M, M, D, x.dtype, False, SCORE_FUNC_MODE1_DOC, id_heads, 1.0)
         tx, to = _tensor(x), _tensor(out)
-        with _Timed("permute"):
-            _lib.check(lib.fa_permute_rows(ctypes.byref(prob), ctypes.byref(tx), ctypes.byref(to), index.data_ptr(),
+        with _timed("permute"):
+            _lib.check(lib.fa_permute_rows(prob, tx, to, index.data_ptr(),
                                            _stream()), "fa_permute_rows")
     return out
 
@@ -346,13 +349,13 @@ def group_rows(eq, B, H, M):
     lib = _lib.load()
     eq = _id_tensor(eq, B, H, M, "eq")
     id_heads = 1 if (H == 1 or eq.stride(1) == 0) else H
-    with torch.cuda.device(eq.device):
+    with _current(eq.device):
         out = torch.empty((3, B, id_heads, M), dtype=torch.int32, device=eq.device)
         prob = _problem(B, H, H, M, M, 64, torch.bfloat16, False, SCORE_FUNC_MODE1_DOC, id_heads, 1.0)
         ieq = _ids(eq)
         status = _status_word(eq.device)
-        with _Timed("group"):
-            _lib.check(lib.fa_group_rows(ctypes.byref(prob), ctypes.byref(ieq), out[0].data_ptr(), out[1].data_ptr(),
+        with _timed("group"):
+            _lib.check(lib.fa_group_rows(prob, ieq, out[0].data_ptr(), out[1].data_ptr(),
                                          out[2].data_ptr(), status.data_ptr(), _stream()), "fa_group_rows")
     return out[0], out[1], out[2], id_heads
 
@@ -405,6 +408,6 @@ def debug_mask(B, H, M, N, causal, eq=None, ek=None, score_func_mode=SCORE_FUNC_
         nQ, nK = (M + 127) // 128, (N + 127) // 128
         keep = torch.zeros((B, He, M, N), dtype=torch.uint8, device=device)
         cls = torch.zeros((B, He, nQ, nK), dtype=torch.uint8, device=device)
-        _lib.check(lib.fa_debug_mask(ctypes.byref(prob), plan.data_ptr() if plan is not None else None,
+        _lib.check(lib.fa_debug_mask(prob, plan.data_ptr() if plan is not None else None,
                                      keep.data_ptr(), cls.data_ptr(), _stream()), "fa_debug_mask")
     return keep.bool(), cls
