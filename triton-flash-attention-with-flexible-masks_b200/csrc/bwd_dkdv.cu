@@ -55,25 +55,21 @@ struct DkdvSmem {
 static_assert(DkdvSmem<128>::total <= 232448 && DkdvSmem<64>::total <= 232448, "shared memory budget");
 
 // Per-candidate code kept in shared memory (2 bits): 0 not visited, 1 visited without id check,
-// 2 id check, 3 id check and the query codes of the block are monotone. Whether a tile needs the
-// range check (causal bound and / or query tail) follows from its coordinates alone.
-enum : uint32_t { KC_SKIP = 0u, KC_PLAIN = 1u, KC_DOC = 2u, KC_DOCMONO = 3u };
+// 2 id check. Whether a tile needs the range check (causal bound and / or query tail) follows from its
+// coordinates alone.
+enum : uint32_t { KC_SKIP = 0u, KC_PLAIN = 1u, KC_DOC = 2u };
 
 // Flags of tile (qb, kb) for all query heads of one kv head at once. When the heads disagree
 // (ids given per head) the id check is forced, entry by entry, which is always exact.
 __device__ __forceinline__ uint32_t classify_group(const MaskArgs& mk, int b, int hk, int G, int qb, int kb) {
     if (mk.He == 1 || G == 1) return classify_from_plan(mk, b, mk.He == 1 ? 0 : hk * G, qb, kb);
-    uint32_t f = 0, mono = TILE_KMONO | TILE_QMONO;
+    uint32_t f = 0;
     bool all = true;
     for (int g = 0; g < G; ++g) {
         const uint32_t fg = classify_from_plan(mk, b, hk * G + g, qb, kb);
-        if (fg & TILE_VISIT) { f |= fg; mono &= fg; } else all = false;
+        if (fg & TILE_VISIT) f |= fg; else all = false;
     }
-    // the chunk shortcuts of the id check may only be taken if the codes are monotone for every head
-    // that the check is applied to (a head that reports no id check does not report its monotony)
-    f &= ~(TILE_KMONO | TILE_QMONO);
     if (f && !all) f |= TILE_DOC;
-    else f |= mono;
     return f;
 }
 
@@ -232,7 +228,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         if (c >= n) break;
                         const uint32_t f = classify_group(mk, b, hk, G, lo + c, kb);
                         uint32_t code = KC_SKIP;
-                        if (f & TILE_VISIT) code = !(f & TILE_DOC) ? KC_PLAIN : (f & TILE_QMONO) ? KC_DOCMONO : KC_DOC;
+                        if (f & TILE_VISIT) code = (f & TILE_DOC) ? KC_DOC : KC_PLAIN;
                         cnt += (code != KC_SKIP);
                         byte |= code << (2 * e);
                     }
@@ -454,14 +450,33 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             int kc = 0, kc_g = -1;  // this key's code for the current query head
             for (int it = 0; it < NIT && ok; ++it, wk.advance(cg, cc)) {
                 const int he = (mk.He == 1) ? 0 : hk * G + cg;
-                const uint32_t code = wk.code(cc);
-                const bool fl_doc = code >= KC_DOC;
+                const bool fl_doc = wk.code(cc) == KC_DOC;
                 const int qb0 = (lo + cc) * kBlk;
                 const bool fl_range = (mk.causal && (k0 + kBlk > mk.N || k1 - 1 > qb0 + mk.gap)) || (qb0 + kBlk > mk.M);
                 const int q0 = qb0 + cbase;  // first query row of this thread's columns
                 const int gi = gt + it, st = gi % NST;
                 const float* vlse = reinterpret_cast<const float*>(smem + S::off_vec + st * S::VEC) + cbase;
                 const float* vdelta = vlse + kBlk;
+
+                // keep(x) = (cmin <= x < cmax) & (qc[x] >= 0 | qc[x] == kc) as 32-bit masks, worked out before the
+                // scores are there
+                const bool flagged = fl_range || fl_doc;
+                uint32_t keep[2] = {~0u, ~0u};
+                if (flagged) {
+                    if (fl_doc) {
+                        const int64_t bh_ids = int64_t(b) * mk.He + he;
+                        if (kc_g != cg) { kc = __ldg(mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + j); kc_g = cg; }
+                        const int* qcs = mk.plan + mk.L.off_qc + bh_ids * mk.L.Mpad + q0;
+                        const int qc0 = __ldg(qcs + lane), qc1 = __ldg(qcs + 32 + lane);
+                        keep[0] = lanes_equal(qc0, kc) | __ballot_sync(0xffffffffu, qc0 >= 0);
+                        keep[1] = lanes_equal(qc1, kc) | __ballot_sync(0xffffffffu, qc1 >= 0);
+                    }
+                    if (fl_range) {
+                        const int cmin = mk.causal ? (j - mk.gap) - q0 : 0, cmax = mk.M - q0;
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) keep[q] &= first_bits(cmax - 32 * q) & ~first_bits(cmin - 32 * q);
+                    }
+                }
 
                 ok = mbar_wait(BAR(B_QFULL + st), (gi / NST) & 1, ab, ST_WAIT_TIMEOUT + 49);
                 if (ok) ok = mbar_wait(BAR(B_SFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 50);
@@ -475,12 +490,18 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 tc_fence_before();
                 mbar_arrive(BAR(B_SFREE));  // the next S^T may now overwrite the columns
                 float* pr = reinterpret_cast<float*>(sr);
-                {
-                    // P^T = exp2(S^T*c - LSE) on packed pairs. A fully masked row has LSE = -inf and only
-                    // occurs in flagged tiles.
-                    const uint64_t c2 = pack_f2(c, c);
+                // P^T = exp2(S^T*c - LSE) on packed pairs, 0 where masked. A fully masked row has LSE = -inf and only
+                // occurs in flagged tiles.
+                const uint64_t c2 = pack_f2(c, c);
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) {
+                for (int h2 = 0; h2 < 2; ++h2) {
+                    if (flagged && !__any_sync(0xffffffffu, keep[h2] != 0u)) {
+#pragma unroll
+                        for (int x = 0; x < 32; ++x) pr[32 * h2 + x] = 0.f;
+                        continue;
+                    }
+#pragma unroll
+                    for (int q = 8 * h2; q < 8 * h2 + 8; ++q) {
                         const float4 l4 = *reinterpret_cast<const float4*>(vlse + 4 * q);
                         float x0, x1, x2, x3;
                         unpack_f2(fma_f2(pack_f2(pr[4 * q + 0], pr[4 * q + 1]), c2, pack_f2(-l4.x, -l4.y)), x0, x1);
@@ -490,55 +511,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         pr[4 * q + 2] = fast_exp2(x2);
                         pr[4 * q + 3] = fast_exp2(x3);
                     }
-                }
-                if (fl_range || fl_doc) {
-                    // keep(x) = (cmin <= x < cmax) & (qc[x] >= 0 | qc[x] == kc), per 32-query chunk where
-                    // the chunk lies on one side of the range and (monotone query codes) is one document
-                    int cmin = -0x40000000, cmax = 64;
-                    if (fl_range) {
-                        if (mk.causal) cmin = (j - mk.gap) - q0;
-                        cmax = min(64, mk.M - q0);
-                    }
-                    const int* qcs = nullptr;
-                    if (fl_doc) {
-                        const int64_t bh_ids = int64_t(b) * mk.He + he;
-                        if (kc_g != cg) { kc = mk.plan[mk.L.off_kc + bh_ids * mk.L.Npad + j]; kc_g = cg; }
-                        qcs = mk.plan + mk.L.off_qc + bh_ids * mk.L.Mpad + q0;
-                    }
+                    if (flagged && __any_sync(0xffffffffu, keep[h2] != ~0u)) {
 #pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        int state = 0;  // this key in chunk q: 0 keep all, 1 mask all, 2 entry by entry
-                        if (32 * q >= cmax || 32 * q + 31 < cmin) state = 1;
-                        else if (32 * q < cmin || 32 * q + 31 >= cmax) state = 2;
-                        if (fl_doc && state != 1) {
-                            if (code == KC_DOCMONO) {
-                                const int qf = __ldg(qcs + 32 * q), ql = __ldg(qcs + 32 * q + 31);
-                                if (qf != ql) state = 2;
-                                else if (!(qf >= 0 || qf == kc)) state = 1;
-                            } else {
-                                state = 2;
-                            }
-                        }
-                        if (!__any_sync(0xffffffffu, state == 2)) {
-                            if (state == 1) {
-#pragma unroll
-                                for (int x = 0; x < 32; ++x) pr[32 * q + x] = 0.f;
-                            }
-                        } else if (fl_doc) {
-                            const int4* qc4 = reinterpret_cast<const int4*>(qcs + 32 * q);
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) {
-                                const int4 qc = __ldg(qc4 + u);
-                                const int x = 32 * q + 4 * u;
-                                pr[x + 0] = ((qc.x >= 0 || qc.x == kc) && x + 0 >= cmin && x + 0 < cmax) ? pr[x + 0] : 0.f;
-                                pr[x + 1] = ((qc.y >= 0 || qc.y == kc) && x + 1 >= cmin && x + 1 < cmax) ? pr[x + 1] : 0.f;
-                                pr[x + 2] = ((qc.z >= 0 || qc.z == kc) && x + 2 >= cmin && x + 2 < cmax) ? pr[x + 2] : 0.f;
-                                pr[x + 3] = ((qc.w >= 0 || qc.w == kc) && x + 3 >= cmin && x + 3 < cmax) ? pr[x + 3] : 0.f;
-                            }
-                        } else {
-#pragma unroll
-                            for (int x = 0; x < 32; ++x) pr[32 * q + x] = (32 * q + x >= cmin && 32 * q + x < cmax) ? pr[32 * q + x] : 0.f;
-                        }
+                        for (int x = 0; x < 32; ++x) pr[32 * h2 + x] = (keep[h2] & (1u << x)) ? pr[32 * h2 + x] : 0.f;
                     }
                 }
                 // P^T (input dtype) -> shared memory, K-major 128-byte-swizzled rows: this thread's 64

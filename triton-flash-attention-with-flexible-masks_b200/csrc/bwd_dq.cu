@@ -410,6 +410,26 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 const bool fl_bound = (kb0 + kBlk > mk.N) || (mk.causal && kb1 - 1 > q0 + mk.gap);
                 const int k0 = kb0 + cbase;  // first key column of this thread
                 const uint32_t tS = tmem + lane_base + uint32_t(gi & 1) * 128u + uint32_t(cbase);
+                // keep(x) = (x <= lim) & (qc >= 0 | kc[x] == qc) as 32-bit masks, worked out before the scores are there
+                const bool flagged = fl_bound || fl_doc;
+                uint32_t keep[2] = {~0u, ~0u};
+                if (flagged) {
+                    if (fl_doc) {
+                        const int* kcs = mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + k0;
+                        const int kc0 = __ldg(kcs + lane), kc1 = __ldg(kcs + 32 + lane);
+                        const uint32_t same0 = lanes_equal(kc0, qc), same1 = lanes_equal(kc1, qc);
+                        if (qc < 0) {  // a row with qc >= 0 passes the id check everywhere
+                            keep[0] = same0;
+                            keep[1] = same1;
+                        }
+                    }
+                    if (fl_bound) {
+                        int jmax = mk.N - 1;
+                        if (mk.causal) jmax = min(jmax, row + mk.gap);
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) keep[q] &= first_bits(jmax + 1 - k0 - 32 * q);
+                    }
+                }
                 ok = mbar_wait(BAR(B_SFULL + (gi & 1)), (gi >> 1) & 1, ab, ST_WAIT_TIMEOUT + 27);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
@@ -419,37 +439,25 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 tmem_ld32(tS + 32u, sr + 32);
                 tc_wait_ld();
                 float* pr = reinterpret_cast<float*>(sr);
-                {
-                    // P = exp2(S*c - LSE) on packed pairs
-                    const uint64_t c2 = pack_f2(c, c), nl2 = pack_f2(-lse, -lse);
+                // P = exp2(S*c - LSE) on packed pairs, 0 where masked
+                const uint64_t c2 = pack_f2(c, c), nl2 = pack_f2(-lse, -lse);
 #pragma unroll
-                    for (int x = 0; x < 32; ++x) {
+                for (int q = 0; q < 2; ++q) {
+                    if (flagged && !__any_sync(0xffffffffu, keep[q] != 0u)) {
+#pragma unroll
+                        for (int x = 0; x < 32; ++x) pr[32 * q + x] = 0.f;
+                        continue;
+                    }
+#pragma unroll
+                    for (int x = 16 * q; x < 16 * q + 16; ++x) {
                         float x0, x1;
                         unpack_f2(fma_f2(pack_f2(pr[2 * x], pr[2 * x + 1]), c2, nl2), x0, x1);
                         pr[2 * x] = fast_exp2(x0);
                         pr[2 * x + 1] = fast_exp2(x1);
                     }
-                }
-                if (fl_bound || fl_doc) {
-                    int lim = 63;
-                    if (fl_bound) {
-                        int jmax = mk.N - 1;
-                        if (mk.causal) jmax = min(jmax, row + mk.gap);
-                        lim = jmax - k0;
-                    }
-                    if (fl_doc && qc < 0) {
-                        const int4* kc4 = reinterpret_cast<const int4*>(mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + k0);
+                    if (flagged && __any_sync(0xffffffffu, keep[q] != ~0u)) {
 #pragma unroll
-                        for (int q = 0; q < 16; ++q) {
-                            const int4 kc = __ldg(kc4 + q);
-                            pr[4 * q + 0] = (kc.x == qc && 4 * q + 0 <= lim) ? pr[4 * q + 0] : 0.f;
-                            pr[4 * q + 1] = (kc.y == qc && 4 * q + 1 <= lim) ? pr[4 * q + 1] : 0.f;
-                            pr[4 * q + 2] = (kc.z == qc && 4 * q + 2 <= lim) ? pr[4 * q + 2] : 0.f;
-                            pr[4 * q + 3] = (kc.w == qc && 4 * q + 3 <= lim) ? pr[4 * q + 3] : 0.f;
-                        }
-                    } else {
-#pragma unroll
-                        for (int x = 0; x < 64; ++x) pr[x] = (x <= lim) ? pr[x] : 0.f;
+                        for (int x = 0; x < 32; ++x) pr[32 * q + x] = (keep[q] & (1u << x)) ? pr[32 * q + x] : 0.f;
                     }
                 }
                 ok = mbar_wait(BAR(B_DPFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 28);
