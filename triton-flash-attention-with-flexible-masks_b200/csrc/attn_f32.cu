@@ -7,12 +7,12 @@
 //
 // One CTA = 8 warps works on 32 "rows" (queries in the forward and dQ kernels, keys in the dK/dV kernel) against
 // tiles of 64 "columns", which cp.async brings into the other of two shared-memory stages while a tile is worked
-// on. Warp w owns rows 4w..4w+3 from the scores to the result: half a warp has two rows, lane x of the half has
-// columns x, x + 16, x + 32, x + 48 of the scores (2 x 4 products in registers) and D / 16 columns of the result,
-// so the softmax needs shuffles over 16 lanes and no barrier, and P passes through the warp's own shared rows.
-// These calls are a few hundred rows of a few heads: what bounds them is the chain of tiles of the longest CTA,
-// in it the shared-memory reads (10 wavefronts per 32 FMAs of a warp). 32 rows rather than 64 keep 8 heads of 512 at
-// 128 CTAs.
+// on. Warp w owns rows 4w..4w+3 from the scores to the result: lane x has columns x and x + 32 of the scores (4 x 2
+// products in registers) and D / 32 columns of the result, so the softmax needs no barrier and P passes through the
+// warp's own shared rows. These calls are a few hundred rows of a few heads: what bounds them is the chain of tiles
+// of the longest CTA, in it the shared-memory reads. A 16-byte read takes one pass per 8 lanes even where lanes repeat
+// an address, so all lanes of a warp share the rows (one pass) and none shares a column: 12 passes per 32 FMAs of a
+// warp, about half of what half-warps with two rows each took. 32 rows rather than 64 keep 8 heads of 512 at 128 CTAs.
 #include "../../include/fa_b200.h"
 #include "common.cuh"
 #include "params.cuh"
@@ -67,99 +67,99 @@ __device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t 
     }
 }
 
-// s[r][c] = row (r0 + r) of A . row (x + 16 c) of B; even and odd elements are summed apart (packed FMAs)
+// s[r][c] = row (r0 + r) of A . row (x + 32 c) of B; even and odd elements are summed apart (packed FMAs)
 template <int D>
-__device__ __forceinline__ void rows_dot_cols(const float* A, const float* Bt, int r0, int x, float (&s)[2][4]) {
+__device__ __forceinline__ void rows_dot_cols(const float* A, const float* Bt, int r0, int x, float (&s)[4][2]) {
     constexpr int LD = F32Smem<D>::LD;
-    uint64_t t[2][4];
+    uint64_t t[4][2];
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) t[r][c] = 0;
+        for (int c = 0; c < 2; ++c) t[r][c] = 0;
 #pragma unroll 4
     for (int d = 0; d < D; d += 4) {
-        ulonglong2 a[2], b[4];
+        ulonglong2 a[4], b[2];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) a[r] = *reinterpret_cast<const ulonglong2*>(A + (r0 + r) * LD + d);
+        for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const ulonglong2*>(A + (r0 + r) * LD + d);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const ulonglong2*>(Bt + (x + 16 * c) * LD + d);
+        for (int c = 0; c < 2; ++c) b[c] = *reinterpret_cast<const ulonglong2*>(Bt + (x + 32 * c) * LD + d);
 #pragma unroll
-        for (int r = 0; r < 2; ++r)
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) t[r][c] = fma_f2(a[r].y, b[c].y, fma_f2(a[r].x, b[c].x, t[r][c]));
+            for (int c = 0; c < 2; ++c) t[r][c] = fma_f2(a[r].y, b[c].y, fma_f2(a[r].x, b[c].x, t[r][c]));
     }
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2; ++c) {
             float lo, hi;
             unpack_f2(t[r][c], lo, hi);
             s[r][c] = lo + hi;
         }
 }
 
-// result columns of lane x: D = 128: 4x..4x+3 and 64 + 4x..; 64: 4x..4x+3; 32: 2x, 2x+1; 16: x
+// result columns of lane x, consecutive: 4x.. (D = 128), 2x.. (64), x (32), x of the lanes below 16 (16)
 template <int D>
 struct Own {
-    static constexpr int N = D / 16, W = N < 4 ? N : 4;  // columns per lane, consecutive ones
-    static __device__ __forceinline__ int col(int x, int k) { return k / W * 64 + x * W + k % W; }
+    static constexpr int N = D < 32 ? 1 : D / 32;
+    static __device__ __forceinline__ bool has(int x) { return D >= 32 || x < D; }
     static __device__ __forceinline__ void load(const float* row, int x, float (&v)[N]) {
-        if constexpr (W == 4) {
-#pragma unroll
-            for (int k = 0; k < N; k += 4) {
-                const float4 t = *reinterpret_cast<const float4*>(row + col(x, k));
-                v[k] = t.x; v[k + 1] = t.y; v[k + 2] = t.z; v[k + 3] = t.w;
-            }
-        } else if constexpr (W == 2) {
+        if constexpr (N == 4) {
+            const float4 t = *reinterpret_cast<const float4*>(row + 4 * x);
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else if constexpr (N == 2) {
             const float2 t = *reinterpret_cast<const float2*>(row + 2 * x);
             v[0] = t.x; v[1] = t.y;
         } else {
-            v[0] = row[x];
+            v[0] = row[D >= 32 ? x : x % D];
         }
     }
     static __device__ __forceinline__ void store(float* row, int x, bool vec, const float (&v)[N], float f) {
-        if (W == 4 && vec) {
+        if constexpr (N == 4) {
+            if (vec) {
+                *reinterpret_cast<float4*>(row + 4 * x) = make_float4(v[0] * f, v[1] * f, v[2] * f, v[3] * f);
+                return;
+            }
+        } else if constexpr (N == 2) {
+            if (vec) {
+                *reinterpret_cast<float2*>(row + 2 * x) = make_float2(v[0] * f, v[1] * f);
+                return;
+            }
+        }
+        if (has(x)) {
 #pragma unroll
-            for (int k = 0; k < N; k += 4)
-                *reinterpret_cast<float4*>(row + col(x, k)) = make_float4(v[k] * f, v[(k + 1) % N] * f, v[(k + 2) % N] * f, v[(k + 3) % N] * f);
-        } else {
-#pragma unroll
-            for (int k = 0; k < N; ++k) row[col(x, k)] = v[k] * f;
+            for (int k = 0; k < N; ++k) row[N * x + k] = v[k] * f;
         }
     }
 };
 
 // acc[r][k] += sum_c P[r0 + r][c] * V[c][own column k]
 template <int D>
-__device__ __forceinline__ void rows_acc(const float* P, const float* V, int r0, int x, float (&acc)[2][D / 16]) {
+__device__ __forceinline__ void rows_acc(const float* P, const float* V, int r0, int x, float (&acc)[4][Own<D>::N]) {
     constexpr int LD = F32Smem<D>::LD;
-#pragma unroll 2
+#pragma unroll 4
     for (int c = 0; c < kC; c += 4) {
-        const float4 p0 = *reinterpret_cast<const float4*>(P + r0 * kLdP + c);
-        const float4 p1 = *reinterpret_cast<const float4*>(P + (r0 + 1) * kLdP + c);
-        const float w0[4] = {p0.x, p0.y, p0.z, p0.w}, w1[4] = {p1.x, p1.y, p1.z, p1.w};
+        float w[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float4 p = *reinterpret_cast<const float4*>(P + (r0 + r) * kLdP + c);
+            w[r][0] = p.x; w[r][1] = p.y; w[r][2] = p.z; w[r][3] = p.w;
+        }
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
-            float v[D / 16];
+            float v[Own<D>::N];
             Own<D>::load(V + (c + cc) * LD, x, v);
 #pragma unroll
-            for (int k = 0; k < D / 16; ++k) {
-                acc[0][k] = fmaf(w0[cc], v[k], acc[0][k]);
-                acc[1][k] = fmaf(w1[cc], v[k], acc[1][k]);
-            }
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int k = 0; k < Own<D>::N; ++k) acc[r][k] = fmaf(w[r][cc], v[k], acc[r][k]);
         }
     }
 }
 
-// over the 16 lanes that share a row
-__device__ __forceinline__ float half_max(float x) {
+__device__ __forceinline__ float warp_max(float x) {
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
-__device__ __forceinline__ float half_sum(float x) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
     return x;
 }
 __device__ __forceinline__ float warp_sum(float x) {
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
     const MaskArgs& mk = p.mask;
     const int i0 = int(gridDim.x - 1 - blockIdx.x) * kR, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;  // long rows first
     const int he = (mk.He == 1) ? 0 : h;
-    const int lane = threadIdx.x & 31, x = lane & 15, r0 = (threadIdx.x >> 5) * 4 + (lane >> 4) * 2;
+    const int x = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * 4;
     const float* qbase = p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh;
     const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
     const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
@@ -215,13 +215,15 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
     };
     load_tile<D, kR>(Qs, qbase, p.q.sl, rows_aligned(qbase, p.q.sl), i0, mk.M);
     find_visited(visited, mk, b, he, true, i0 / kBlk);
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[2][D / 16];
-    int qc[2];
+    float m[4], l[4], acc[4][Own<D>::N];
+    int qc[4];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < 4; ++r) {
+        m[r] = -INFINITY;
+        l[r] = 0.f;
         qc[r] = code_q(mk, b, he, i0 + r0 + r);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) acc[r][k] = 0.f;
+        for (int k = 0; k < Own<D>::N; ++k) acc[r][k] = 0.f;
     }
     const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;  // keys beyond the last row's causal bound
     __syncthreads();
@@ -235,30 +237,30 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
         cp_async_wait<1>();
         __syncthreads();
         const float* Ks = KVs + st * 2 * S::cols;
-        float s[2][4];
+        float s[4][2];
         rows_dot_cols<D>(Qs, Ks, r0, x, s);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
+        for (int r = 0; r < 4; ++r) {
             const int i = i0 + r0 + r;
             float mx = -INFINITY;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = j0 + x + 16 * c;
-                const bool keep = keep_entry(i, j, qc[r], kcodes ? codes[st * kC + x + 16 * c] : 0, mk.N, mk.gap, mk.causal, mk.mode);
+            for (int c = 0; c < 2; ++c) {
+                const int j = j0 + x + 32 * c;
+                const bool keep = keep_entry(i, j, qc[r], kcodes ? codes[st * kC + x + 32 * c] : 0, mk.N, mk.gap, mk.causal, mk.mode);
                 s[r][c] = keep ? s[r][c] * p.scale : -INFINITY;
                 mx = fmaxf(mx, s[r][c]);
             }
-            const float mn = fmaxf(m[r], half_max(mx));
+            const float mn = fmaxf(m[r], warp_max(mx));
             const float alpha = (m[r] == -INFINITY) ? 0.f : expf(m[r] - mn);
             m[r] = mn;
             l[r] *= alpha;
 #pragma unroll
-            for (int k = 0; k < D / 16; ++k) acc[r][k] *= alpha;
+            for (int k = 0; k < Own<D>::N; ++k) acc[r][k] *= alpha;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 2; ++c) {
                 const float pe = (s[r][c] == -INFINITY) ? 0.f : expf(s[r][c] - mn);
                 l[r] += pe;
-                Ps[(r0 + r) * kLdP + x + 16 * c] = pe;
+                Ps[(r0 + r) * kLdP + x + 32 * c] = pe;
             }
         }
         __syncwarp();
@@ -269,9 +271,9 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
     float* obase = p.o.ptr + int64_t(b) * p.o.sb + int64_t(h) * p.o.sh;
     const bool ovec = rows_aligned(obase, p.o.sl);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < 4; ++r) {
         const int i = i0 + r0 + r;
-        const float lt = half_sum(l[r]);
+        const float lt = warp_sum(l[r]);
         if (i >= mk.M) continue;
         Own<D>::store(obase + int64_t(i) * p.o.sl, x, ovec, acc[r], lt > 0.f ? 1.f / lt : 0.f);
         if (x == 0) p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + i] = lt > 0.f ? m[r] + logf(lt) : -INFINITY;
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
     const MaskArgs& mk = p.mask;
     const int i0 = int(gridDim.x - 1 - blockIdx.x) * kR, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;
     const int he = (mk.He == 1) ? 0 : h;
-    const int lane = threadIdx.x & 31, x = lane & 15, r0 = (threadIdx.x >> 5) * 4 + (lane >> 4) * 2;
+    const int x = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * 4;
     const float* qbase = p.q.ptr + int64_t(b) * p.q.sb + int64_t(h) * p.q.sh;
     const float* dobase = p.d_o.ptr + int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh;
     const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
@@ -325,17 +327,17 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
     load_tile<D, kR>(Qs, qbase, p.q.sl, rows_aligned(qbase, p.q.sl), i0, mk.M);
     load_tile<D, kR>(dOs, dobase, p.d_o.sl, rows_aligned(dobase, p.d_o.sl), i0, mk.M);
     find_visited(visited, mk, b, he, true, i0 / kBlk);
-    float acc[2][D / 16], lse[2], dl[2];
-    int qc[2];
+    float acc[4][Own<D>::N], lse[4], dl[4];
+    int qc[4];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < 4; ++r) {
         const int i = i0 + r0 + r;
         const int64_t ro = (int64_t(b) * p.H + h) * mk.L.Mpad + i;
         lse[r] = (i < mk.M) ? p.lse[ro] : -INFINITY;
         dl[r] = (i < mk.M) ? p.delta[ro] : 0.f;
         qc[r] = code_q(mk, b, he, i);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) acc[r][k] = 0.f;
+        for (int k = 0; k < Own<D>::N; ++k) acc[r][k] = 0.f;
     }
     const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;
     __syncthreads();
@@ -349,18 +351,18 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
         cp_async_wait<1>();
         __syncthreads();
         const float* Ks = KVs + st * 2 * S::cols;
-        float s[2][4], dp[2][4];
+        float s[4][2], dp[4][2];
         rows_dot_cols<D>(Qs, Ks, r0, x, s);
         rows_dot_cols<D>(dOs, Ks + S::cols, r0, x, dp);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
+        for (int r = 0; r < 4; ++r) {
             const int i = i0 + r0 + r;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = j0 + x + 16 * c;
-                const bool keep = (i < mk.M) && keep_entry(i, j, qc[r], kcodes ? codes[st * kC + x + 16 * c] : 0, mk.N, mk.gap, mk.causal, mk.mode);
+            for (int c = 0; c < 2; ++c) {
+                const int j = j0 + x + 32 * c;
+                const bool keep = (i < mk.M) && keep_entry(i, j, qc[r], kcodes ? codes[st * kC + x + 32 * c] : 0, mk.N, mk.gap, mk.causal, mk.mode);
                 const float pe = keep ? expf(s[r][c] * p.scale - lse[r]) : 0.f;  // a kept entry has a finite lse
-                Ps[(r0 + r) * kLdP + x + 16 * c] = keep ? pe * (dp[r][c] - dl[r]) : 0.f;  // dS (flash_triton.py:301)
+                Ps[(r0 + r) * kLdP + x + 32 * c] = keep ? pe * (dp[r][c] - dl[r]) : 0.f;  // dS (flash_triton.py:301)
             }
         }
         __syncwarp();
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
     float* dqbase = p.dq.ptr + int64_t(b) * p.dq.sb + int64_t(h) * p.dq.sh;
     const bool dqvec = rows_aligned(dqbase, p.dq.sl);
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 4; ++r)
         if (i0 + r0 + r < mk.M) Own<D>::store(dqbase + int64_t(i0 + r0 + r) * p.dq.sl, x, dqvec, acc[r], p.scale);  // flash_triton.py:425
 }
 
@@ -391,16 +393,16 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
     __shared__ uint8_t visited[kListCap];
     const MaskArgs& mk = p.mask;
     const int j0 = blockIdx.x * kR, hk = blockIdx.y, b = blockIdx.z;
-    const int lane = threadIdx.x & 31, x = lane & 15, r0 = (threadIdx.x >> 5) * 4 + (lane >> 4) * 2;
+    const int x = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * 4;
     const float* kbase = p.k.ptr + int64_t(b) * p.k.sb + int64_t(hk) * p.k.sh;
     const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
     load_tile<D, kR>(Ks, kbase, p.k.sl, rows_aligned(kbase, p.k.sl), j0, mk.N);
     load_tile<D, kR>(Vs, vbase, p.v.sl, rows_aligned(vbase, p.v.sl), j0, mk.N);
-    float dk[2][D / 16], dv[2][D / 16];
+    float dk[4][Own<D>::N], dv[4][Own<D>::N];
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) dk[r][k] = dv[r][k] = 0.f;
+        for (int k = 0; k < Own<D>::N; ++k) dk[r][k] = dv[r][k] = 0.f;
     // first query row that can see key j0 under the causal mask (flash_triton.py:214-218)
     const int first = mk.causal ? max(0, j0 - mk.gap) / kC * kC : 0;
     for (int g = 0; g < p.G; ++g) {
@@ -421,9 +423,9 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
             }
         };
         if (g == 0 || mk.He != 1) find_visited(visited, mk, b, he, false, j0 / kBlk);
-        int kc[2];
+        int kc[4];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) kc[r] = code_k(mk, b, he, j0 + r0 + r);
+        for (int r = 0; r < 4; ++r) kc[r] = code_k(mk, b, he, j0 + r0 + r);
         __syncthreads();
         int i0 = next_tile(visited, first, mk.M);
         if (i0 < mk.M) fetch(i0, 0);
@@ -437,19 +439,19 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
             const float* Qs = QDs + st * 2 * S::cols;
             const float* dOs = Qs + S::cols;
             const float* vec = vecs + st * S::vec;
-            float s[2][4], dp[2][4];
+            float s[4][2], dp[4][2];
             rows_dot_cols<D>(Ks, Qs, r0, x, s);    // S^T
             rows_dot_cols<D>(Vs, dOs, r0, x, dp);  // dP^T
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int i = i0 + x + 16 * c;
-                const int qc = qcodes ? __float_as_int(vec[x + 16 * c]) : 0;
-                const float lse = vec[kC + x + 16 * c], dl = vec[2 * kC + x + 16 * c];
+            for (int c = 0; c < 2; ++c) {
+                const int i = i0 + x + 32 * c;
+                const int qc = qcodes ? __float_as_int(vec[x + 32 * c]) : 0;
+                const float lse = vec[kC + x + 32 * c], dl = vec[2 * kC + x + 32 * c];
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
+                for (int r = 0; r < 4; ++r) {
                     const bool keep = (i < mk.M) && keep_entry(i, j0 + r0 + r, qc, kc[r], mk.N, mk.gap, mk.causal, mk.mode);
                     const float pe = keep ? expf(s[r][c] * p.scale - lse) : 0.f;
-                    Ps[(r0 + r) * kLdP + x + 16 * c] = pe;
+                    Ps[(r0 + r) * kLdP + x + 32 * c] = pe;
                     dp[r][c] = keep ? pe * (dp[r][c] - dl) : 0.f;
                 }
             }
@@ -457,9 +459,9 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
             rows_acc<D>(Ps, dOs, r0, x, dv);  // dV += P^T dO (flash_triton.py:291)
             __syncwarp();
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int r = 0; r < 2; ++r) Ps[(r0 + r) * kLdP + x + 16 * c] = dp[r][c];
+                for (int r = 0; r < 4; ++r) Ps[(r0 + r) * kLdP + x + 32 * c] = dp[r][c];
             __syncwarp();
             rows_acc<D>(Ps, Qs, r0, x, dk);   // dK += dS^T Q (flash_triton.py:308)
             __syncthreads();
@@ -471,7 +473,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
     float* dvbase = p.dv.ptr + int64_t(b) * p.dv.sb + int64_t(hk) * p.dv.sh;
     const bool dkvec = rows_aligned(dkbase, p.dk.sl), dvvec = rows_aligned(dvbase, p.dv.sl);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
+    for (int r = 0; r < 4; ++r) {
         const int j = j0 + r0 + r;
         if (j >= mk.N) continue;
         Own<D>::store(dkbase + int64_t(j) * p.dk.sl, x, dkvec, dk[r], p.scale);  // flash_triton.py:313
