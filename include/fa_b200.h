@@ -140,7 +140,8 @@ int fa_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const
               const fa_tensor* d_o, const float* lse, const float* delta, const fa_tensor* dq,
               const void* plan, int32_t* status, void* stream);
 
-/* fa_bwd_delta, fa_bwd_dkdv and fa_bwd_dq in this order; stops at the first that fails. */
+/* fa_bwd_delta, fa_bwd_dkdv and fa_bwd_dq in this order; stops at the first that fails. The dQ kernel (16-bit types)
+ * is launched so that it may start on SMs that the dK/dV kernel has left; it ends after it. */
 int fa_bwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
            const fa_tensor* d_o, const float* lse, float* delta, const fa_tensor* dq, const fa_tensor* dk,
            const fa_tensor* dv, const void* plan, int32_t* status, void* stream);

@@ -18,7 +18,7 @@ cudaError_t launch_bwd_dkdv(int, bool, const CUtensorMap&, const CUtensorMap&, c
                             const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const DkdvParams&, int,
                             cudaStream_t);
 cudaError_t launch_bwd_dq(int, bool, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&,
-                          const CUtensorMap&, const CUtensorMap&, const DqParams&, int, cudaStream_t);
+                          const CUtensorMap&, const CUtensorMap&, const DqParams&, int, bool, cudaStream_t);
 
 // fp32 path (attn_f32.cu)
 cudaError_t launch_f32(int which, int D, const F32Params& p, cudaStream_t stream);
@@ -276,6 +276,47 @@ int run_f32(int which, const fa_problem* p, const fa_tensor* q, const fa_tensor*
     return fa::launch_f32(which, p->D, fp, static_cast<cudaStream_t>(stream)) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 
+int run_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* d_o,
+              const float* lse, const float* delta, const fa_tensor* dq, const void* plan, int32_t* status,
+               bool overlap, void* stream) {
+    int rc = check_problem(p);
+    if (rc) return rc;
+    if (!lse || !delta || !status) return FA_ERR_BAD_ARG;
+    if (!aligned16(lse) || !aligned16(delta)) return FA_ERR_ALIGNMENT;  // read with bulk copies
+    if (p->dtype == FA_FP32)
+        return run_f32(3, p, q, k, v, nullptr, d_o, dq, nullptr, nullptr, const_cast<float*>(lse), const_cast<float*>(delta), plan, stream);
+    if ((rc = check_tensor(q, p->B, p->H, p->M))) return rc;
+    if ((rc = check_tensor(d_o, p->B, p->H, p->M))) return rc;
+    if ((rc = check_tensor(dq, p->B, p->H, p->M))) return rc;
+    if ((rc = check_tensor(k, p->B, p->Hk, p->N))) return rc;
+    if ((rc = check_tensor(v, p->B, p->Hk, p->N))) return rc;
+    fa::DqParams qp;
+    if ((rc = make_mask(&qp.mask, p, plan))) return rc;
+    CUtensorMap tq, tk, tv, tdo;
+    if ((rc = make_map(&tq, q, p->dtype, p->B, p->H, p->M, p->D))) return rc;
+    if ((rc = make_map(&tdo, d_o, p->dtype, p->B, p->H, p->M, p->D))) return rc;
+    if ((rc = make_map(&tk, k, p->dtype, p->B, p->Hk, p->N, p->D))) return rc;
+    if ((rc = make_map(&tv, v, p->dtype, p->B, p->Hk, p->N, p->D))) return rc;
+    CUtensorMap tdq;
+    if ((rc = make_map(&tdq, dq, p->dtype, p->B, p->H, p->M, p->D))) return rc;
+    const int sms = sm_count();
+    if (sms <= 0) return FA_ERR_LAUNCH;
+    qp.lse = lse;
+    qp.delta = delta;
+    qp.B = p->B;
+    qp.H = p->H;
+    qp.G = p->H / p->Hk;
+    qp.gh = head_group(p, p->H * p->B);
+    qp.by_length = (p->mode == FA_MODE1_DOC && int64_t(fa::cdiv(p->M, fa::kBlk) * p->H * p->B) < 32 * int64_t(sms)) ? 1 : 0;
+    qp.scale_log2 = p->sm_scale * kLog2e;
+    qp.sm_scale = p->sm_scale;
+    qp.status = status;
+    qp.wait_limit = wait_limit_clocks();
+    const cudaError_t e =
+        fa::launch_bwd_dq(p->D, p->dtype == FA_BF16, tq, tk, tv, tdo, tdq, qp, sms, overlap, static_cast<cudaStream_t>(stream));
+    return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+}
+
 }  // namespace
 
 extern "C" {
@@ -488,42 +529,7 @@ int fa_bwd_dkdv(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, con
 int fa_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* d_o,
               const float* lse, const float* delta, const fa_tensor* dq, const void* plan, int32_t* status,
               void* stream) {
-    int rc = check_problem(p);
-    if (rc) return rc;
-    if (!lse || !delta || !status) return FA_ERR_BAD_ARG;
-    if (!aligned16(lse) || !aligned16(delta)) return FA_ERR_ALIGNMENT;  // read with bulk copies
-    if (p->dtype == FA_FP32)
-        return run_f32(3, p, q, k, v, nullptr, d_o, dq, nullptr, nullptr, const_cast<float*>(lse), const_cast<float*>(delta), plan, stream);
-    if ((rc = check_tensor(q, p->B, p->H, p->M))) return rc;
-    if ((rc = check_tensor(d_o, p->B, p->H, p->M))) return rc;
-    if ((rc = check_tensor(dq, p->B, p->H, p->M))) return rc;
-    if ((rc = check_tensor(k, p->B, p->Hk, p->N))) return rc;
-    if ((rc = check_tensor(v, p->B, p->Hk, p->N))) return rc;
-    fa::DqParams qp;
-    if ((rc = make_mask(&qp.mask, p, plan))) return rc;
-    CUtensorMap tq, tk, tv, tdo;
-    if ((rc = make_map(&tq, q, p->dtype, p->B, p->H, p->M, p->D))) return rc;
-    if ((rc = make_map(&tdo, d_o, p->dtype, p->B, p->H, p->M, p->D))) return rc;
-    if ((rc = make_map(&tk, k, p->dtype, p->B, p->Hk, p->N, p->D))) return rc;
-    if ((rc = make_map(&tv, v, p->dtype, p->B, p->Hk, p->N, p->D))) return rc;
-    CUtensorMap tdq;
-    if ((rc = make_map(&tdq, dq, p->dtype, p->B, p->H, p->M, p->D))) return rc;
-    const int sms = sm_count();
-    if (sms <= 0) return FA_ERR_LAUNCH;
-    qp.lse = lse;
-    qp.delta = delta;
-    qp.B = p->B;
-    qp.H = p->H;
-    qp.G = p->H / p->Hk;
-    qp.gh = head_group(p, p->H * p->B);
-    qp.by_length = (p->mode == FA_MODE1_DOC && int64_t(fa::cdiv(p->M, fa::kBlk) * p->H * p->B) < 32 * int64_t(sms)) ? 1 : 0;
-    qp.scale_log2 = p->sm_scale * kLog2e;
-    qp.sm_scale = p->sm_scale;
-    qp.status = status;
-    qp.wait_limit = wait_limit_clocks();
-    const cudaError_t e =
-        fa::launch_bwd_dq(p->D, p->dtype == FA_BF16, tq, tk, tv, tdo, tdq, qp, sms, static_cast<cudaStream_t>(stream));
-    return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+    return run_bwd_dq(p, q, k, v, d_o, lse, delta, dq, plan, status, false, stream);
 }
 
 int fa_bwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
@@ -531,7 +537,7 @@ int fa_bwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa
            const void* plan, int32_t* status, void* stream) {
     int rc = fa_bwd_delta(p, o, d_o, delta, stream);
     if (!rc) rc = fa_bwd_dkdv(p, q, k, v, d_o, lse, delta, dk, dv, plan, status, stream);
-    if (!rc) rc = fa_bwd_dq(p, q, k, v, d_o, lse, delta, dq, plan, status, stream);
+    if (!rc) rc = run_bwd_dq(p, q, k, v, d_o, lse, delta, dq, plan, status, true, stream);
     return rc;
 }
 

@@ -163,6 +163,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
         fence_mbar_init();
+        launch_dependents();  // fa_bwd's dQ kernel reads nothing that this one writes
     }
     if (warp == 9) {
         tmem_alloc(sbase + S::off_misc, 512);

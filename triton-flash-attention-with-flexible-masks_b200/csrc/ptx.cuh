@@ -257,6 +257,11 @@ __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// Programmatic launch: the next kernel of the stream, if it was launched that way, may start once every block of this
+// grid has said so (or left); and the wait, in that kernel, for the kernel before it to be complete. No-ops otherwise.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------------------
 // descriptors
 // ----------------------------------------------------------------------------------------
