@@ -230,6 +230,11 @@ int sm_count() {
 // Runs into which the forward cuts each item's key tiles, for calls without ids that have fewer items than the GPU
 // has SMs. A round of items costs its tiles plus about 4 tile times of fill, drain and epilogue; the second
 // kernel and the fp32 rows cost about 6 more. At most two items per SM, which bounds the workspace at 20 MB.
+// One token, 32 / 8 heads of 128, us with 1 run and with the number taken here: 32768 keys 240, 37.7 (18 runs; best of
+// 1, 2, 4, 8, 16: 37.0 with 16); 4096 keys 36.5, 16.7 (16; best); 1024 keys 14.9 (1; best 12.6 with 4); 4 sequences
+// of 8192 keys 67.5, 34.1 (4; best); 8 of them 71.2, 52.0 (2; best). 300 queries against 9000 keys: 16 / 4 heads 77.4, 39.9
+// (3; 2 runs 49.2, 4 runs 56.9), 32 / 8 heads 78.0, 71.8 (3; 2 runs 94.1, 4 runs 82.0). 1000 x 1000 of 8 heads of 64: 14.6
+// (1; 2 runs 18.1).
 int fwd_splits(const fa_problem* p, int sms) {
     if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32) return 1;
     const int pack = fwd_pack(p);
