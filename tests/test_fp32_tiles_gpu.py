@@ -43,3 +43,33 @@ def test_tile_edges(M, N, causal, mode, per_head, D, offset):
     oe.backward(do.double())
     for what, got, want in (("o", o, oe), ("dq", q.grad, qe.grad), ("dk", k.grad, ke.grad), ("dv", v.grad, ve.grad)):
         assert (got.double() - want).abs().max().item() < 1e-4, what
+
+
+@pytest.mark.parametrize("D", [16, 64, 128])
+@pytest.mark.parametrize("G,sees", [(2, (0, 1)), (2, (1, 0)), (4, (0, 1, 1, 1)), (4, (1, 0, 0, 1)), (4, (1, 1, 1, 0)), (4, (0, 0, 0, 0))])
+def test_heads_of_a_group_that_see_nothing_of_a_key_block(G, sees, D, monkeypatch):
+    """Ids per head: some heads of a group have no query in the document that fills the first and the third block of
+    keys, so dK / dV finds no tile for them there and goes straight on to the next head."""
+    import flash_b200 as fb
+    monkeypatch.setattr(fb.ops, "GROUP_QUERIES", False)  # the caller's order of queries, so that every block is mixed
+    B, Hk, M, N = 2, 3, 1500, 500
+    H = G * Hk
+    g = torch.Generator(device="cuda").manual_seed(G + D)
+    q, k, v, do = [torch.randn(B, h, n, D, generator=g, device="cuda") for h, n in ((H, M), (Hk, N), (Hk, N), (H, M))]
+    ek = (-1 - torch.arange(N, device="cuda") // 128 % 2).expand(B, H, N)
+    eq = -2 + torch.randint(0, 2, (B, H, M), generator=g, device="cuda")
+    for h in range(H):
+        if not sees[h % G]:
+            eq[:, h] = -2
+    keep = eq[..., None] == ek[..., None, :]
+    for t in (q, k, v):
+        t.requires_grad_()
+    o = fb.attention(q, k, v, False, None, eq, ek, 1)
+    o.backward(do)
+    fb.check_status()
+    qe, ke, ve = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    s = (qe @ ke.repeat_interleave(G, 1).transpose(2, 3) / D ** 0.5).masked_fill(~keep, -torch.inf)
+    oe = torch.softmax(s, 3) @ ve.repeat_interleave(G, 1)
+    oe.backward(do.double())
+    for what, got, want in (("o", o, oe), ("dq", q.grad, qe.grad), ("dk", k.grad, ke.grad), ("dv", v.grad, ve.grad)):
+        assert (got.double() - want).abs().max().item() < 1e-4, what

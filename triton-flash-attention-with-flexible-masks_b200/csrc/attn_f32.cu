@@ -422,7 +422,12 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
                 if (src) cp_async4(smem_u32(vecs + st * S::vec + threadIdx.x), static_cast<const float*>(src) + i0 + t, true);
             }
         };
-        if (g == 0 || mk.He != 1) find_visited(visited, mk, b, he, false, j0 / kBlk);
+        if (g == 0 || mk.He != 1) {
+            // A head without a visible tile has passed no barrier since its next_tile: without this one a fast warp
+            // would rewrite the table while a slow one reads it, and the two would take different numbers of tiles.
+            if (g > 0) __syncthreads();
+            find_visited(visited, mk, b, he, false, j0 / kBlk);
+        }
         int kc[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) kc[r] = code_k(mk, b, he, j0 + r0 + r);
