@@ -89,3 +89,53 @@ def test_any_number_of_runs(fb, splits):
     _close(o, oe, "o")
     assert (lse[..., :M].double() - le).abs().max().item() < 1e-4 and bool(torch.isfinite(lse).all())
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("what", ["nan in k", "overflowing score", "all of a run is nan", "nan in v", "inf in v", "-inf scores"])
+@pytest.mark.parametrize("M,G", [(1, 4), (40, 2), (200, 1)])
+def test_values_that_are_not_finite_do_not_get_lost_in_a_run(fb, M, G, what):
+    """A call cut into runs gives such rows as the call of one run does: zeros with an lse of -inf where a score is NaN,
+    NaN with an lse of -inf where one is +inf, NaN or an infinity where only a value is."""
+    from flash_b200 import _lib, ops
+    B, Hk, N, D, splits = 2, 2, 1500, 64, 4
+    H = G * Hk
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    q = torch.randn(B, H, M, D, generator=g, device="cuda").bfloat16()
+    k, v = [torch.randn(B, Hk, N, D, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    if what == "nan in k":
+        k[1, 0, 700, 3] = float("nan")
+    elif what == "overflowing score":  # +inf for one half of the rows, -inf for the other
+        k[1, 0, 700] = 0
+        k[1, 0, 700, 0] = 3e38
+        odd = (torch.arange(G, device="cuda")[:, None] + torch.arange(M, device="cuda")) % 2
+        q[1, :G, :, 0] = (4 - 8 * odd).bfloat16()
+    elif what == "all of a run is nan":
+        k[1, 0, 256:768] = float("nan")
+    elif what == "-inf scores":
+        q[1, :G, :, 0] = 1
+        k[1, 0, 512:900, 0] = -float("inf")
+    else:
+        v[1, 0, 700, 3] = float(what.split()[0])
+    prob = ops._problem(B, H, Hk, M, N, D, q.dtype, True, 0, 1, D ** -0.5)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n = ctypes.c_size_t(0)
+    assert lib.fa_fwd_workspace_bytes(ctypes.byref(prob), splits, ctypes.byref(n)) == 0
+    work = torch.empty(n.value // 4, device="cuda")
+    results = []
+    for ns in (1, splits):
+        o, lse = torch.empty_like(q), torch.empty(B, H, -(-M // 128) * 128, device="cuda")
+        assert lib.fa_fwd_split(prob, ops._tensor(q), ops._tensor(k), ops._tensor(v), ops._tensor(o), lse.data_ptr(), None, ns,
+                                work.data_ptr(), n.value, status.data_ptr(), ops._stream()) == 0
+        results.append((o.double(), lse[..., :M].double()))
+    assert int(status.item()) == 0
+    (o1, l1), (o2, l2) = results
+    dead = l1 == -torch.inf
+    if "v" not in what.split()[-1:] and what != "-inf scores":  # the case does what it says: rows of the group are lost
+        assert bool(dead[1, :G].any()) and bool(((o1[dead] == 0) | torch.isnan(o1[dead])).all())
+    assert torch.equal(dead, l2 == -torch.inf)
+    assert bool(((l1 - l2).abs() < 1e-4 + 1e-6 * l1.abs())[~dead].all())
+    assert torch.equal(torch.isnan(o1), torch.isnan(o2))
+    assert torch.equal(o1.nan_to_num(0, 0, 0).ne(0).any(3), o2.nan_to_num(0, 0, 0).ne(0).any(3))
+    fine = torch.isfinite(o1) & torch.isfinite(o2)
+    _close(o2[fine], o1[fine], "o")

@@ -625,7 +625,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 if constexpr (SHORT) {
                     const int64_t bh0 = int64_t(b) * p.H + int64_t(h / nG) * p.G;
                     if (ns > 1) {
-                        if (valid) p.part_lse[((bh0 + g_own) * mk.M + row) * ns + j % ns] = lse;
+                        // a run that went NaN says so: -inf would pass for a run without keys
+                        if (valid) p.part_lse[((bh0 + g_own) * mk.M + row) * ns + j % ns] = (lt == lt) ? lse : lt;
                     } else {
                         if (valid) p.lse[(bh0 + g_own) * mk.L.Mpad + row] = lse;
                         // the rows past M that pad the buffer
@@ -719,8 +720,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 }
 
 // Merges the ns partial results of a split forward: O = sum_s w_s O_s with w_s = 2^(lse_s - lse), lse the log2-sum
-// over the parts. One warp per row; lane l owns columns l, l + 32, ... (D <= 128), all sums
-// in fp32 in the order of the parts. Bound by latency: at most a few MB are read, all of them from L2.
+// over the parts. A part whose lse is NaN or +inf (a NaN or an infinity among its scores) makes the row its own, as in a
+// call of one run: zeros or NaN, with an lse of -inf. One warp per row; lane l owns columns l, l + 32, ... (D <= 128), all sums
+// in fp32 in the order of the parts. Bound by latency: at most 20 MB are read (fwd_splits in api.cu), mostly from L2.
 template <bool BF16>
 __global__ void __launch_bounds__(256) fwd_combine_kernel(const CombineParams p) {
     const int64_t row = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);  // of the [B, H, M] rows
@@ -734,14 +736,22 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const CombineParams p)
         for (int64_t x = p.M + lane; x < p.Mpad; x += 32) lse[x] = 0.f;
     const bool failed = status_is_fatal(*p.status);  // the forward left no parts: NaN, as the other kernels do
     float mx = -INFINITY;
-    for (int s = lane; s < p.ns; s += 32) mx = fmaxf(mx, p.part_lse[row * p.ns + s]);
+    bool spoilt = false;
+    for (int s = lane; s < p.ns; s += 32) {
+        const float x = p.part_lse[row * p.ns + s];
+        spoilt |= !(x < INFINITY);
+        mx = fmaxf(mx, x);
+    }
+    spoilt = __any_sync(0xffffffffu, spoilt);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float acc[4] = {0.f, 0.f, 0.f, 0.f}, total = 0.f;
-    if (mx != -INFINITY) {
+    if (mx != -INFINITY || spoilt) {
 #pragma unroll 4
         for (int s = 0; s < p.ns; ++s) {
-            const float wgt = fast_exp2(p.part_lse[row * p.ns + s] - mx);  // an empty part: 2^-inf = 0
+            const float x = p.part_lse[row * p.ns + s];
+            const float wgt = !spoilt ? fast_exp2(x - mx) : x < INFINITY ? 0.f : 1.f;  // an empty part: 2^-inf = 0
+            if (spoilt && wgt == 0.f) continue;
             const float* po = p.part_o + (int64_t(s) * rows + row) * p.Dk;
             total += wgt;
 #pragma unroll
@@ -755,7 +765,7 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const CombineParams p)
 #pragma unroll
     for (int k = 0; k < 4; ++k)
         if (lane + 32 * k < p.D) out[lane + 32 * k] = failed ? uint16_t(0xffff) : uint16_t(pack2<BF16>(acc[k] * inv, 0.f));
-    if (lane == 0) lse[i] = total > 0.f ? mx + log2f(total) : -INFINITY;
+    if (lane == 0) lse[i] = (total > 0.f && !spoilt) ? mx + log2f(total) : -INFINITY;
 }
 
 cudaError_t launch_fwd_combine(bool bf16, const CombineParams& p, cudaStream_t stream) {
