@@ -73,3 +73,35 @@ def test_heads_of_a_group_that_see_nothing_of_a_key_block(G, sees, D, monkeypatc
     oe.backward(do.double())
     for what, got, want in (("o", o, oe), ("dq", q.grad, qe.grad), ("dk", k.grad, ke.grad), ("dv", v.grad, ve.grad)):
         assert (got.double() - want).abs().max().item() < 1e-4, what
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["k", "v", "q", "do"])
+@pytest.mark.parametrize("gap", [0, 64])
+def test_values_that_the_causal_mask_hides_from_a_whole_block_of_rows(gap, where, value):
+    """A NaN or an infinity in a key that no query of a block of 32 may see (or in a query that sees no key of a block)
+    leaves that block's results alone, although a tile of 64 columns holds it."""
+    import flash_b200 as fb
+    B, H, M, D = 1, 2, 192, 64
+    N = M + gap
+    g = torch.Generator(device="cuda").manual_seed(gap)
+    t = {n: torch.randn(B, H, l, D, generator=g, device="cuda") for n, l in (("q", M), ("k", N), ("v", N), ("do", M))}
+    for n in ("q", "k", "v"):
+        t[n].requires_grad_()
+
+    def step():
+        o = fb.attention(t["q"], t["k"], t["v"], True)
+        return (o.detach(), *torch.autograd.grad(o, (t["q"], t["k"], t["v"]), t["do"]))
+
+    clean = step()
+    with torch.no_grad():
+        # key 100 + gap is in the second half of a tile that queries 64..95 work on, query 70 in the first half of one
+        # that keys 96 + gap.. work on
+        t[where][0, 1, 100 + gap if where in "kv" else 70] = value
+    o, dq, dk, dv = step()
+    fb.check_status()
+    if where in "kv":
+        assert torch.equal(o[:, :, :96], clean[0][:, :, :96]) and torch.equal(dq[:, :, :96], clean[1][:, :, :96])
+    else:
+        rows = slice(96 + gap, None)
+        assert torch.equal(dk[:, :, rows], clean[2][:, :, rows]) and torch.equal(dv[:, :, rows], clean[3][:, :, rows])

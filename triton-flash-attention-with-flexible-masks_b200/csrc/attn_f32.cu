@@ -45,23 +45,25 @@ __device__ __forceinline__ bool rows_aligned(const float* base, int64_t sl) {
     return (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (sl & 3) == 0;
 }
 
-// starts the copy of rows [r0, r0 + NR) of a [L, D] slice into a padded tile; rows >= L become zero. Tensors are only
-// promised to be 4-byte aligned: `vec` says that every row of this one starts on 16 bytes.
+// starts the copy of rows [r0, r0 + NR) of a slice into a padded tile; rows outside [lo, hi) become zero: those outside
+// the tensor, and those that the causal mask hides from the whole CTA, for their products with a P of 0 would be NaN
+// where they hold a NaN or an infinity. Tensors are only promised to be 4-byte aligned: `vec` says that every row of
+// this one starts on 16 bytes.
 template <int D, int NR>
-__device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t sl, bool vec, int r0, int L) {
+__device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t sl, bool vec, int r0, int hi, int lo = 0) {
     constexpr int LD = F32Smem<D>::LD;
     if (vec) {
 #pragma unroll 4
         for (int i = threadIdx.x; i < NR * (D / 4); i += kF32Threads) {
             const int r = i / (D / 4), c = i % (D / 4) * 4;
-            const bool real = r0 + r < L;
+            const bool real = r0 + r >= lo && r0 + r < hi;
             cp_async16(smem_u32(dst + r * LD + c), real ? src + int64_t(r0 + r) * sl + c : src, real);
         }
     } else {
 #pragma unroll 4
         for (int i = threadIdx.x; i < NR * D; i += kF32Threads) {
             const int r = i / D, c = i % D;
-            const bool real = r0 + r < L;
+            const bool real = r0 + r >= lo && r0 + r < hi;
             cp_async4(smem_u32(dst + r * LD + c), real ? src + int64_t(r0 + r) * sl + c : src, real);
         }
     }
@@ -208,9 +210,10 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
     const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
     const bool kvec = rows_aligned(kbase, p.k.sl), vvec = rows_aligned(vbase, p.v.sl);
     const int32_t* kcodes = mk.mode == 1 ? mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad : nullptr;
+    const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;  // keys beyond the last row's causal bound
     auto fetch = [&](int j0, int st) {
-        load_tile<D, kC>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, mk.N);
-        load_tile<D, kC>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, mk.N);
+        load_tile<D, kC>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, end);
+        load_tile<D, kC>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, end);
         if (kcodes && threadIdx.x < kC) cp_async4(smem_u32(codes + st * kC + threadIdx.x), kcodes + j0 + threadIdx.x, true);
     };
     load_tile<D, kR>(Qs, qbase, p.q.sl, rows_aligned(qbase, p.q.sl), i0, mk.M);
@@ -225,7 +228,6 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
 #pragma unroll
         for (int k = 0; k < Own<D>::N; ++k) acc[r][k] = 0.f;
     }
-    const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;  // keys beyond the last row's causal bound
     __syncthreads();
     int j0 = next_tile(visited, 0, end);
     if (j0 < end) fetch(j0, 0);
@@ -319,9 +321,10 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
     const float* vbase = p.v.ptr + int64_t(b) * p.v.sb + int64_t(hk) * p.v.sh;
     const bool kvec = rows_aligned(kbase, p.k.sl), vvec = rows_aligned(vbase, p.v.sl);
     const int32_t* kcodes = mk.mode == 1 ? mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad : nullptr;
+    const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;  // keys beyond the last row's causal bound
     auto fetch = [&](int j0, int st) {
-        load_tile<D, kC>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, mk.N);
-        load_tile<D, kC>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, mk.N);
+        load_tile<D, kC>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, end);
+        load_tile<D, kC>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, end);
         if (kcodes && threadIdx.x < kC) cp_async4(smem_u32(codes + st * kC + threadIdx.x), kcodes + j0 + threadIdx.x, true);
     };
     load_tile<D, kR>(Qs, qbase, p.q.sl, rows_aligned(qbase, p.q.sl), i0, mk.M);
@@ -339,7 +342,6 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
 #pragma unroll
         for (int k = 0; k < Own<D>::N; ++k) acc[r][k] = 0.f;
     }
-    const int end = mk.causal ? min(mk.N, i0 + kR + mk.gap) : mk.N;
     __syncthreads();
     int j0 = next_tile(visited, 0, end);
     if (j0 < end) fetch(j0, 0);
@@ -404,7 +406,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
 #pragma unroll
         for (int k = 0; k < Own<D>::N; ++k) dk[r][k] = dv[r][k] = 0.f;
     // first query row that can see key j0 under the causal mask (flash_triton.py:214-218)
-    const int first = mk.causal ? max(0, j0 - mk.gap) / kC * kC : 0;
+    const int first = mk.causal ? max(0, j0 - mk.gap) : 0;
     for (int g = 0; g < p.G; ++g) {
         const int h = hk * p.G + g;
         const int he = (mk.He == 1) ? 0 : h;
@@ -414,8 +416,8 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
         const int64_t ro = (int64_t(b) * p.H + h) * mk.L.Mpad;
         const int32_t* qcodes = mk.mode == 1 ? mk.plan + mk.L.off_qc + (int64_t(b) * mk.He + he) * mk.L.Mpad : nullptr;
         auto fetch = [&](int i0, int st) {
-            load_tile<D, kC>(QDs + st * 2 * S::cols, qbase, p.q.sl, qvec, i0, mk.M);
-            load_tile<D, kC>(QDs + (st * 2 + 1) * S::cols, dobase, p.d_o.sl, dovec, i0, mk.M);
+            load_tile<D, kC>(QDs + st * 2 * S::cols, qbase, p.q.sl, qvec, i0, mk.M, first);
+            load_tile<D, kC>(QDs + (st * 2 + 1) * S::cols, dobase, p.d_o.sl, dovec, i0, mk.M, first);
             if (threadIdx.x < S::vec) {  // the per-row buffers are padded to 128 rows; what pads them is not used
                 const int t = threadIdx.x % kC, what = threadIdx.x / kC;
                 const void* src = what == 0 ? static_cast<const void*>(qcodes) : what == 1 ? p.lse + ro : p.delta + ro;
@@ -432,7 +434,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
 #pragma unroll
         for (int r = 0; r < 4; ++r) kc[r] = code_k(mk, b, he, j0 + r0 + r);
         __syncthreads();
-        int i0 = next_tile(visited, first, mk.M);
+        int i0 = next_tile(visited, first / kC * kC, mk.M);
         if (i0 < mk.M) fetch(i0, 0);
         cp_async_commit();
         for (int st = 0; i0 < mk.M; st ^= 1) {
