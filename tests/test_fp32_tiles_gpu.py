@@ -105,3 +105,32 @@ def test_values_that_the_causal_mask_hides_from_a_whole_block_of_rows(gap, where
     else:
         rows = slice(96 + gap, None)
         assert torch.equal(dk[:, :, rows], clean[2][:, :, rows]) and torch.equal(dv[:, :, rows], clean[3][:, :, rows])
+
+
+@pytest.mark.parametrize("D", [16, 128])
+def test_blocks_without_a_visible_tile(D):
+    """Many CTAs that load their rows and find nothing to do, between others that do: zeros, and the others undisturbed."""
+    import flash_b200 as fb
+    B, H, L = 8, 8, 1024
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v, do = [torch.randn(B, H, L, D, generator=g, device="cuda").requires_grad_() for _ in range(4)]
+    ek = (-1 - torch.arange(L, device="cuda") // 256).expand(B, H, L)
+    blind = torch.arange(L, device="cuda") // 128 % 2 == 1  # every other block of queries is in no document
+    eq = torch.where(blind, torch.full_like(ek, -9), ek)
+
+    def step():
+        o = fb.attention(q, k, v, True, None, eq, ek, 1)
+        return (o, *torch.autograd.grad(o, (q, k, v), do))
+
+    o, dq, dk, dv = step()
+    fb.check_status()
+    assert bool((o[:, :, blind] == 0).all()) and bool((dq[:, :, blind] == 0).all())
+    qe, ke, ve = [t[:2].detach().double().requires_grad_() for t in (q, k, v)]
+    keep = ((eq[:2, :, :, None] == ek[:2, :, None]) & torch.ones(L, L, dtype=torch.bool, device="cuda").tril())[:, :, ~blind]
+    s = (qe[:, :, ~blind] @ ke.transpose(2, 3) / D ** 0.5).masked_fill(~keep, -torch.inf)
+    oe = torch.softmax(s, 3) @ ve
+    want = torch.autograd.grad(oe, (qe, ke, ve), do[:2, :, ~blind].double())
+    for got, x in ((o[:2, :, ~blind], oe), (dq[:2], want[0]), (dk[:2], want[1]), (dv[:2], want[2])):
+        assert (got.double() - x).abs().max().item() < 1e-4
+    for a, b in zip((o, dq, dk, dv), step()):
+        assert torch.equal(a, b)

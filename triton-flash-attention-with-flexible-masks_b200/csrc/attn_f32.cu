@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
         __syncthreads();  // the stage may be refilled
         j0 = jn;
     }
+    cp_async_wait<0>();  // a block without a visible tile has not waited for its Q
     float* obase = p.o.ptr + int64_t(b) * p.o.sb + int64_t(h) * p.o.sh;
     const bool ovec = rows_aligned(obase, p.o.sl);
 #pragma unroll
@@ -372,6 +373,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
         __syncthreads();
         j0 = jn;
     }
+    cp_async_wait<0>();
     float* dqbase = p.dq.ptr + int64_t(b) * p.dq.sb + int64_t(h) * p.dq.sh;
     const bool dqvec = rows_aligned(dqbase, p.dq.sl);
 #pragma unroll
