@@ -53,6 +53,7 @@ struct DkdvSmem {
     static constexpr int total = off_misc + 16;
 };
 static_assert(DkdvSmem<128>::total <= 232448 && DkdvSmem<64>::total <= 232448, "shared memory budget");
+static_assert(DkdvSmem<128>::total > 116736 && DkdvSmem<64>::total > 116736, "shares an SM with a dQ CTA");
 
 // Per-candidate code kept in shared memory (2 bits): 0 not visited, 1 visited without id check,
 // 2 id check. Whether a tile needs the range check (causal bound and / or query tail) follows from its

@@ -43,6 +43,9 @@ struct DqSmem {
     static constexpr int total = off_misc + 16;
 };
 static_assert(DqSmem<128>::total <= 232448 && DqSmem<64>::total <= 232448, "shared memory budget");
+// With the dK/dV kernel's CTAs (more than half of it as well) none of these fits on one SM: an overlapping launch never
+// takes tensor memory that a dK/dV CTA still has to allocate.
+static_assert(DqSmem<128>::total > 116736 && DqSmem<64>::total > 116736, "shares an SM");
 
 // Per-candidate code kept in shared memory (2 bits): 0 not visited, 1 visited without id check,
 // 2 id check. Whether a tile needs the bound check (key tail, causal diagonal) follows from its
@@ -132,8 +135,22 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     tc_fence_after();
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
-    // an earlier launch on this device ran into a time-out that the host has not yet cleared
-    if (aborted && (sbase & 1023u) == 0) nan_fill_outputs(smem + S::off_q, S::NBOX, &tmdQ, nullptr, nQ, p.H, p.B);
+    // Item k of this CTA. Items are handed out in order from a counter in the plan (any CTA takes the next one: the work
+    // per item varies with the mask); without counters (no plan given) they are dealt out round robin in alternating
+    // direction, which evens out their sorted lengths.
+    auto take = [&](int k) {
+        if (ctr) return int(atomicAdd(ctr, 1u));
+        return k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
+    };
+    // An earlier launch on this device ran into a time-out that the host has not yet cleared. A launch that overlaps the
+    // dK/dV kernel may have CTAs that started before that kernel's time-out and CTAs that started after it, so those
+    // that see it fill the items that they would have computed, and only those.
+    if (aborted && (sbase & 1023u) == 0)
+        nan_fill_items(smem + S::off_q, S::NBOX, &tmdQ, [&](int k, int& qb, int& h, int& b) {
+            const int j = take(k);
+            if (j < n_items) decode(j, qb, h, b);
+            return j < n_items;
+        });
 
     if (warp >= 8) {
         setmaxnreg_dec<56>();
@@ -141,10 +158,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         } else if (warp == 11) {
             // ------------------------------ scheduler ------------------------------
             // Item k goes to slot k & 1: range [lo, lo + n) of candidate key blocks, a 2-bit code per
-            // candidate, the number of visited tiles, the item index (-1: no more items). Items are
-            // handed out in order from a counter in the plan (any CTA takes the next one: the work
-            // per item varies with the mask); without counters (no plan given) they are dealt out
-            // round robin in alternating direction, which evens out their sorted lengths.
+            // candidate, the number of visited tiles, the item index (-1: no more items).
             bool ok = true;
             for (int k = 0;; ++k) {
                 const int s = k & 1, use = k >> 1;
@@ -152,10 +166,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 int j = 0;
-                if (lane == 0) {
-                    if (ctr) j = int(atomicAdd(ctr, 1u));
-                    else j = k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
-                }
+                if (lane == 0) j = take(k);
                 j = __shfl_sync(0xffffffffu, j, 0);
                 if (j >= n_items) {
                     if (lane == 0) {

@@ -237,6 +237,25 @@ __device__ __forceinline__ void nan_fill_outputs(uint8_t* tile, int nbox, const 
     }
 }
 
+// The same, item by item: next(k, blk, h, b) gives the k-th tile to fill, or false behind the last one. For a launch whose
+// CTAs may disagree about the status word: a CTA that has seen it fills what it would have computed.
+template <class Next>
+__device__ __forceinline__ void nan_fill_items(uint8_t* tile, int nbox, const CUtensorMap* m, Next next) {
+    constexpr int kBox = kBlk * 64 * 2;
+    for (int i = threadIdx.x; i < nbox * kBox / 16; i += blockDim.x)
+        reinterpret_cast<uint4*>(tile)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    fence_proxy_async();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int blk, h, b;
+        for (int k = 0; next(k, blk, h, b); ++k) {
+            for (int x = 0; x < nbox; ++x) tma_store_4d(m, smem_u32(tile) + x * kBox, x * 64, blk * kBlk, h, b);
+            tma_store_commit();
+        }
+        tma_store_wait_all();
+    }
+}
+
 // The same for the 5-D output map (D, M, G, Hk, B) of the forward's packed calls.
 __device__ __forceinline__ void nan_fill_short(uint8_t* tile, int nbox, const CUtensorMap* m, int n_blk, int n_g, int pack,
                                                int n_hk, int n_b) {
