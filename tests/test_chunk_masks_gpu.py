@@ -42,3 +42,50 @@ def test_backward_chunk_masks(M, N, causal, ndoc, run, per_head, D):
         bound = 6 * 2.0 ** -9 * (norm + norm.square().mean().sqrt())
         err = (got.detach().double() - want).norm(dim=3)
         assert bool((err <= bound).all()), (what, (err / bound).max().item())
+
+
+@pytest.mark.parametrize("M,N,causal,ndoc,run,per_head,D", [
+    (300, 300, True, 5, 1, False, 64),     # five codes a chunk, six with an id that attends everywhere: some blocks either way
+    (300, 300, True, 40, 1, True, 128),    # up to 32 codes
+    (1000, 1300, True, 30, 10, False, 64),
+    (120, 500, False, 6, 1, True, 128)])
+def test_walk_and_compare_give_the_same_bits(M, N, causal, ndoc, run, per_head, D, monkeypatch):
+    """The plan's flag of a block with many distinct codes decides how the backward compares its codes, and nothing else."""
+    import flash_b200 as fb
+    from flash_b200 import ops
+    B, H, Hk = 2, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(N + ndoc)
+    q, k, v, do = [torch.randn(B, h, n, D, generator=g, device="cuda").bfloat16() for h, n in ((H, M), (Hk, N), (Hk, N), (H, M))]
+    ek = -1 - torch.randint(0, ndoc, (B, H if per_head else 1, N // run + 1), generator=g, device="cuda").repeat_interleave(run, 2)[..., :N]
+    ek[torch.rand(ek.shape, generator=g, device="cuda") < 0.03] = 5
+    eq, ek = ek[..., N - M:].expand(B, H, M), ek.expand(B, H, N)
+    for t in (q, k, v):
+        t.requires_grad_()
+    build, flags = ops.build_plan, []
+
+    def build_with(many):
+        def made(*args):
+            plan = build(*args)
+            rows, nq, nk = B * (H if per_head else 1), -(-M // 128), -(-N // 128)
+            up = lambda n: -(-n // 128) * 128
+            at = rows * 128 * (nq + nk) + 4 * up(rows * nq) + 4 * up(rows * nk)  # codes, min / max, ranges
+            qf, kf = plan[at:at + rows * nq], plan[at + up(rows * nq):at + up(rows * nq) + rows * nk]
+            flags.extend((qf.clone(), kf.clone()))
+            for f in (qf, kf):
+                if many is not None:
+                    f.copy_(f & 1 | (2 if many else 0))
+            return plan
+        return made
+
+    results = []
+    for many in (None, False, True):
+        monkeypatch.setattr(ops, "build_plan", build_with(many))
+        results.append(torch.autograd.grad(fb.attention(q, k, v, causal, None, eq, ek, 1), (q, k, v), do))
+    fb.check_status()
+    # the flags are the rule's: more than five distinct codes in 32 rows (padding of the last block included)
+    codes = torch.nn.functional.pad(torch.where(eq >= 0, torch.full_like(eq, 1 << 40), eq)[:, :H if per_head else 1], (0, -M % 128), value=1 << 40)
+    chunks = codes.reshape(-1, 32).sort(1).values
+    want = ((chunks.diff(dim=1) != 0).sum(1) + 1 > 5).view(-1, 4).any(1)
+    assert torch.equal((flags[0] & 2) != 0, want.view(-1))
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))

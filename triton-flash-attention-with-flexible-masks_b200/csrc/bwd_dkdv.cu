@@ -56,9 +56,9 @@ static_assert(DkdvSmem<128>::total <= 232448 && DkdvSmem<64>::total <= 232448, "
 static_assert(DkdvSmem<128>::total > 116736 && DkdvSmem<64>::total > 116736, "shares an SM with a dQ CTA");
 
 // Per-candidate code kept in shared memory (2 bits): 0 not visited, 1 visited without id check,
-// 2 id check. Whether a tile needs the range check (causal bound and / or query tail) follows from its
-// coordinates alone.
-enum : uint32_t { KC_SKIP = 0u, KC_PLAIN = 1u, KC_DOC = 2u };
+// 2 id check, 3 id check with many codes in the query block. Whether a tile needs the range check (causal bound
+// and / or query tail) follows from its coordinates alone.
+enum : uint32_t { KC_SKIP = 0u, KC_PLAIN = 1u, KC_DOC = 2u, KC_DOCMANY = 3u };
 
 // Flags of tile (qb, kb) for all query heads of one kv head at once. When the heads disagree
 // (ids given per head) the id check is forced, entry by entry, which is always exact.
@@ -230,7 +230,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         if (c >= n) break;
                         const uint32_t f = classify_group(mk, b, hk, G, lo + c, kb);
                         uint32_t code = KC_SKIP;
-                        if (f & TILE_VISIT) code = (f & TILE_DOC) ? KC_DOC : KC_PLAIN;
+                        if (f & TILE_VISIT) code = !(f & TILE_DOC) ? KC_PLAIN : (f & TILE_QMANY) ? KC_DOCMANY : KC_DOC;
                         cnt += (code != KC_SKIP);
                         byte |= code << (2 * e);
                     }
@@ -452,7 +452,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             int kc = 0, kc_g = -1;  // this key's code for the current query head
             for (int it = 0; it < NIT && ok; ++it, wk.advance(cg, cc)) {
                 const int he = (mk.He == 1) ? 0 : hk * G + cg;
-                const bool fl_doc = wk.code(cc) == KC_DOC;
+                const uint32_t code = wk.code(cc);
+                const bool fl_doc = code >= KC_DOC, many = code == KC_DOCMANY;
                 const int qb0 = (lo + cc) * kBlk;
                 const bool fl_range = (mk.causal && (k0 + kBlk > mk.N || k1 - 1 > qb0 + mk.gap)) || (qb0 + kBlk > mk.M);
                 const int q0 = qb0 + cbase;  // first query row of this thread's columns
@@ -470,8 +471,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         if (kc_g != cg) { kc = __ldg(mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + j); kc_g = cg; }
                         const int* qcs = mk.plan + mk.L.off_qc + bh_ids * mk.L.Mpad + q0;
                         const int qc0 = __ldg(qcs + lane), qc1 = __ldg(qcs + 32 + lane);
-                        keep[0] = lanes_equal(qc0, kc) | __ballot_sync(0xffffffffu, qc0 >= 0);
-                        keep[1] = lanes_equal(qc1, kc) | __ballot_sync(0xffffffffu, qc1 >= 0);
+                        keep[0] = codes_equal(qcs, qc0, kc, many) | __ballot_sync(0xffffffffu, qc0 >= 0);
+                        keep[1] = codes_equal(qcs + 32, qc1, kc, many) | __ballot_sync(0xffffffffu, qc1 >= 0);
                     }
                     if (fl_range) {
                         const int cmin = mk.causal ? (j - mk.gap) - q0 : 0, cmax = mk.M - q0;

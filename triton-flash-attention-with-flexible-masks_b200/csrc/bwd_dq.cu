@@ -48,9 +48,9 @@ static_assert(DqSmem<128>::total <= 232448 && DqSmem<64>::total <= 232448, "shar
 static_assert(DqSmem<128>::total > 116736 && DqSmem<64>::total > 116736, "shares an SM");
 
 // Per-candidate code kept in shared memory (2 bits): 0 not visited, 1 visited without id check,
-// 2 id check. Whether a tile needs the bound check (key tail, causal diagonal) follows from its
-// coordinates alone.
-enum : uint32_t { QC_SKIP = 0u, QC_PLAIN = 1u, QC_DOC = 2u };
+// 2 id check, 3 id check with many codes in the key block. Whether a tile needs the bound check (key tail,
+// causal diagonal) follows from its coordinates alone.
+enum : uint32_t { QC_SKIP = 0u, QC_PLAIN = 1u, QC_DOC = 2u, QC_DOCMANY = 3u };
 
 struct DqWalk {
     const uint8_t* fl;
@@ -190,7 +190,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                         const int c = 4 * i + e;
                         if (c >= n) break;
                         const uint32_t f = classify_from_plan(mk, b, he, qb, lo + c);
-                        const uint32_t code = !(f & TILE_VISIT) ? QC_SKIP : (f & TILE_DOC) ? QC_DOC : QC_PLAIN;
+                        uint32_t code = QC_SKIP;
+                        if (f & TILE_VISIT) code = !(f & TILE_DOC) ? QC_PLAIN : (f & TILE_KMANY) ? QC_DOCMANY : QC_DOC;
                         cnt += (code != QC_SKIP);
                         byte |= code << (2 * e);
                     }
@@ -415,7 +416,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             int cc = wk.first_from(0);
             for (int t = 0; t < T && ok; ++t, cc = wk.first_from(cc + 1)) {
                 const int gi = gt + t;
-                const bool fl_doc = wk.code(cc) == QC_DOC;
+                const uint32_t code = wk.code(cc);
+                const bool fl_doc = code >= QC_DOC, many = code == QC_DOCMANY;
                 const int kb0 = (lo + cc) * kBlk;
                 const int kb1 = min(kb0 + kBlk, mk.N);
                 const bool fl_bound = (kb0 + kBlk > mk.N) || (mk.causal && kb1 - 1 > q0 + mk.gap);
@@ -428,7 +430,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     if (fl_doc) {
                         const int* kcs = mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + k0;
                         const int kc0 = __ldg(kcs + lane), kc1 = __ldg(kcs + 32 + lane);
-                        const uint32_t same0 = lanes_equal(kc0, qc), same1 = lanes_equal(kc1, qc);
+                        const uint32_t same0 = codes_equal(kcs, kc0, qc, many), same1 = codes_equal(kcs + 32, kc1, qc, many);
                         if (qc < 0) {  // a row with qc >= 0 passes the id check everywhere
                             keep[0] = same0;
                             keep[1] = same1;

@@ -26,9 +26,10 @@ __host__ __device__ inline int64_t pad128(int64_t x) { return (x + 127) / 128 * 
 //   kmin, kmax [B, He, nK]   min / max key code per block of 128 keys
 //   kv_lo, kv_hi [B, He, nQ] range of key blocks with an unmasked entry, per query block
 //   q_lo, q_hi   [B, He, nK] range of query blocks with an unmasked entry, per key block
-//   qmono [B, He, nQ], kmono [B, He, nK]  1 if the codes of the block (all 128 stored codes, padding of a
-//                ragged last block included) are monotone (non-decreasing or non-increasing), i.e. equal
-//                codes are adjacent: the usual packed-documents layout
+//   qflags [B, He, nQ], kflags [B, He, nK]  of the 128 stored codes of a block, padding of a ragged last block
+//                included: BF_MONO if they are monotone (non-decreasing or non-increasing), i.e. equal codes are
+//                adjacent, the usual packed-documents layout; BF_MANY if some 32 of them (aligned) hold more than
+//                kWalkCodes distinct codes
 //   ord_q [B, He, nQ], ord_k [B, He, nK]  the blocks of a head sorted by the length of their visit range,
 //                longest first (ties: from the long end of a causal head)
 //   ctr [128]    work counters of the persistent kernels (item counter, finished-CTA counter per kernel);
@@ -37,7 +38,7 @@ __host__ __device__ inline int64_t pad128(int64_t x) { return (x + 127) / 128 * 
 struct PlanLayout {
     int B, He, M, N, nQ, nK;
     int64_t Mpad, Npad;
-    int64_t off_qc, off_kc, off_qmin, off_qmax, off_kmin, off_kmax, off_kvlo, off_kvhi, off_qlo, off_qhi, off_qmono, off_kmono, off_ordq, off_ordk, off_ctr;
+    int64_t off_qc, off_kc, off_qmin, off_qmax, off_kmin, off_kmax, off_kvlo, off_kvhi, off_qlo, off_qhi, off_qflags, off_kflags, off_ordq, off_ordk, off_ctr;
     int64_t total;  // int32 elements
 
     __host__ __device__ PlanLayout() {}
@@ -57,8 +58,8 @@ struct PlanLayout {
         off_kvhi = o; o += pad128(bh * nQ);
         off_qlo = o;  o += pad128(bh * nK);
         off_qhi = o;  o += pad128(bh * nK);
-        off_qmono = o; o += pad128(bh * nQ);
-        off_kmono = o; o += pad128(bh * nK);
+        off_qflags = o; o += pad128(bh * nQ);
+        off_kflags = o; o += pad128(bh * nK);
         off_ordq = o;  o += pad128(bh * nQ);
         off_ordk = o;  o += pad128(bh * nK);
         off_ctr = o;   o += 128;
@@ -83,6 +84,9 @@ enum : int {
     DBG_ALL_PARTIAL = 2,  // evaluate the bound and the id rule entry by entry on every visited tile
 };
 
+enum : int { BF_MONO = 1, BF_MANY = 2 };  // flags of a block's codes
+constexpr int kWalkCodes = 5;
+
 enum { CTR_FWD = 0, CTR_DKDV = 2, CTR_DQ = 4 };  // pairs {next item, CTAs finished} inside the plan's ctr section
 
 enum : uint32_t {
@@ -91,7 +95,9 @@ enum : uint32_t {
     TILE_DOC = 4u,     // needs the per-entry id check
     TILE_QTAIL = 8u,   // holds rows >= M (matters to the backward kernels only)
     TILE_KMONO = 16u,  // key codes of the block are monotone: a 32-key chunk is uniform iff its ends are equal
-    TILE_QMONO = 32u,  // same for the query codes of the block
+    TILE_QMONO = 32u,  // same for the query codes of the block (reported by fa_debug_mask only)
+    TILE_KMANY = 64u,  // 32 keys of the block hold many distinct codes (BF_MANY)
+    TILE_QMANY = 128u, // same for the query codes of the block
 };
 
 // Classification of tile (qb, kb) from the block statistics. Conservative: a tile is skipped
@@ -117,14 +123,17 @@ __host__ __device__ inline uint32_t classify_tile(int qb, int kb, int M, int N, 
     return f;
 }
 
+// All loads are issued together: they are on the way of a kernel's first tile. Bits that a caller does not look at cost none.
 __device__ __forceinline__ uint32_t classify_from_plan(const MaskArgs& a, int b, int he, int qb, int kb) {
-    int qmin = 0, qmax = 0, kmin = 0, kmax = 0;
+    int qmin = 0, qmax = 0, kmin = 0, kmax = 0, qf = 0, kf = 0;
     if (a.mode == 1) {
         const int64_t bh = int64_t(b) * a.He + he;
         qmin = a.plan[a.L.off_qmin + bh * a.L.nQ + qb];
         qmax = a.plan[a.L.off_qmax + bh * a.L.nQ + qb];
         kmin = a.plan[a.L.off_kmin + bh * a.L.nK + kb];
         kmax = a.plan[a.L.off_kmax + bh * a.L.nK + kb];
+        qf = a.plan[a.L.off_qflags + bh * a.L.nQ + qb];
+        kf = a.plan[a.L.off_kflags + bh * a.L.nK + kb];
     }
     uint32_t f = classify_tile(qb, kb, a.M, a.N, a.gap, a.causal, a.mode, qmin, qmax, kmin, kmax);
     if (a.debug) {
@@ -134,10 +143,9 @@ __device__ __forceinline__ uint32_t classify_from_plan(const MaskArgs& a, int b,
         }
         if ((a.debug & DBG_ALL_PARTIAL) && f) return f | TILE_BOUND | (a.mode == 1 ? TILE_DOC : 0u);
     }
-    if (a.mode == 1 && (f & TILE_DOC)) {
-        const int64_t bh = int64_t(b) * a.He + he;
-        if (a.plan[a.L.off_kmono + bh * a.L.nK + kb]) f |= TILE_KMONO;
-        if (a.plan[a.L.off_qmono + bh * a.L.nQ + qb]) f |= TILE_QMONO;
+    if (f & TILE_DOC) {
+        f |= ((kf & BF_MONO) ? TILE_KMONO : 0u) | ((kf & BF_MANY) ? TILE_KMANY : 0u);
+        f |= ((qf & BF_MONO) ? TILE_QMONO : 0u) | ((qf & BF_MANY) ? TILE_QMANY : 0u);
     }
     return f;
 }
@@ -192,21 +200,31 @@ __device__ __forceinline__ bool keep_entry(int i, int j, int qc, int kc, int N, 
 // The forward keeps its compares: the same masks there cost dense tiles 2 % (registers) for 2 % on packed ones.
 __device__ __forceinline__ uint32_t first_bits(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1u; }
 
-// Bit x of the result: lane x's `code` equals this thread's `own`. Walks the distinct codes of the chunk (one to three
-// with packed documents); a chunk with more than six is compared lane by lane. All lanes of the warp take part.
-__device__ __forceinline__ uint32_t lanes_equal(int code, int own) {
-    uint32_t todo = ~0u, mine = 0u;
+// Bit x of the result: codes[x] (32 of them, 16-byte aligned; `code` is the lane's own) equals this thread's `own`. All
+// lanes of the warp take part. A walk over the distinct codes of the chunk costs a shuffle and a vote for each (one to
+// three with packed documents); reading and comparing all 32 costs the same whatever they are. `many`, from the plan's
+// BF_MANY, says which: backward of 4 x 16 heads x 4096 x 128 with ids drawn at random from 4 (walk) 1095 us, from 6, 8
+// or 40 (compare) 1077 us, and 1182, 1504 and 1504 us with a walk of at most six codes and shuffles beyond; random
+// runs of 10 (four or five codes, walk) 961 us, 1007 us with a compare; compares after the scores: 1163 us for all.
+__device__ __forceinline__ uint32_t codes_equal(const int32_t* codes, int code, int own, bool many) {
+    uint32_t mine = 0u;
+    if (many) {
+        const int4* c4 = reinterpret_cast<const int4*>(codes);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int4 c = __ldg(c4 + u);
+            mine |= (c.x == own ? 1u << (4 * u) : 0u) | (c.y == own ? 2u << (4 * u) : 0u) |
+                    (c.z == own ? 4u << (4 * u) : 0u) | (c.w == own ? 8u << (4 * u) : 0u);
+        }
+        return mine;
+    }
+    uint32_t todo = ~0u;
 #pragma unroll 1
-    for (int k = 0; k < 6 && todo; ++k) {
+    while (todo) {
         const int c = __shfl_sync(~0u, code, __ffs(todo) - 1);
         const uint32_t m = __ballot_sync(~0u, code == c);
         if (own == c) mine = m;
         todo &= ~m;
-    }
-    if (todo) {
-        mine = 0u;
-#pragma unroll 4
-        for (int x = 0; x < 32; ++x) mine |= uint32_t(__shfl_sync(~0u, code, x) == own) << x;
     }
     return mine;
 }

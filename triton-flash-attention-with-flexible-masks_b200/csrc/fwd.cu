@@ -197,7 +197,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 int T = 0;
                 for (int base = 0; base < n; base += 32) {
                     const int i = base + lane;
-                    const uint32_t f = (i < n) ? classify_from_plan(mk, b, he, qb, lo + i) : 0u;
+                    const uint32_t f = (i < n) ? classify_from_plan(mk, b, he, qb, lo + i) & (TILE_VISIT | TILE_BOUND | TILE_DOC | TILE_KMONO) : 0u;
                     const uint32_t m = __ballot_sync(0xffffffffu, (f & TILE_VISIT) != 0);
                     if (f & TILE_VISIT) list[T + __popc(m & ((1u << lane) - 1u))] = uint16_t(uint32_t(i) | (f << 10));
                     T += __popc(m);

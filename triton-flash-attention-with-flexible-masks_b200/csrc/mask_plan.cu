@@ -84,15 +84,17 @@ __global__ void __launch_bounds__(128) plan_codes_kernel(IdsView eq, IdsView ek,
         rise = code > codes[threadIdx.x - 1];
         fall = code < codes[threadIdx.x - 1];
     }
-    const int any_rise = block_reduce_max(rise, scratch);
-    const int any_fall = block_reduce_max(fall, scratch);
-    const int mono = !(any_rise && any_fall);
+    const bool leads = __ffs(__match_any_sync(0xffffffffu, code)) - 1 == int(threadIdx.x & 31);  // first of its code in the warp
+    const bool many = __popc(__ballot_sync(0xffffffffu, leads)) > kWalkCodes;
+    const int any_rise = __syncthreads_or(rise), any_fall = __syncthreads_or(fall);
+    const int flags = ((any_rise && any_fall) ? 0 : BF_MONO) | (__syncthreads_or(many) ? BF_MANY : 0);
     if (threadIdx.x == 0) {
-        plan[(is_q ? L.off_qmono + bh * L.nQ : L.off_kmono + bh * L.nK) + blk] = mono;
         if (is_q) {
+            plan[L.off_qflags + bh * L.nQ + blk] = flags;
             plan[L.off_qmin + bh * L.nQ + blk] = mn;
             plan[L.off_qmax + bh * L.nQ + blk] = mx;
         } else {
+            plan[L.off_kflags + bh * L.nK + blk] = flags;
             plan[L.off_kmin + bh * L.nK + blk] = mn;
             plan[L.off_kmax + bh * L.nK + blk] = mx;
         }
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(128) debug_mask_kernel(MaskArgs a, uint8_t* ke
     uint32_t f = classify_from_plan(a, b, he, qb, kb);
     const bool in_range = (kb >= lo && kb < hi) && (qb >= qlo && qb < qhi);
     if (!in_range) f = 0;
-    if (tile_class && threadIdx.x == 0) tile_class[(bh * a.L.nQ + qb) * a.L.nK + kb] = uint8_t(f);
+    if (tile_class && threadIdx.x == 0) tile_class[(bh * a.L.nQ + qb) * a.L.nK + kb] = uint8_t(f & 63u);  // the bits above are a matter of speed
     if (!keep) return;
     const int i = qb * kBlk + threadIdx.x;
     if (i >= a.M) return;
