@@ -91,8 +91,10 @@ int64_t fa_padded_rows(int32_t M);
  * counters of the attention kernels only; such a plan is optional). */
 int fa_plan_bytes(const fa_problem* p, size_t* bytes);
 
-/* 1 if a plan would not change how the launches for this problem share out their work: no ids, and no launch
- * (with `backward` != 0, of the backward too) has more items than the current device has SMs. */
+/* 1 if a plan would gain the launches for this problem nothing: no ids, and no launch (with `backward` != 0, of the
+ * backward too) has more items than the current device has SMs. The runs of a split forward are not counted: there are
+ * at most two per SM if fa_fwd_splits set their number, all nearly as long, and dealing them out in a fixed order takes
+ * no longer than through a plan's counters. Results are the same bits with and without a plan. */
 int fa_plan_optional(const fa_problem* p, int32_t backward);
 
 /* Builds the mask plan from eq [B,H,M] / ek [B,H,N]: 32-bit id codes, per-128-block id

@@ -139,3 +139,30 @@ def test_values_that_are_not_finite_do_not_get_lost_in_a_run(fb, M, G, what):
     assert torch.equal(o1.nan_to_num(0, 0, 0).ne(0).any(3), o2.nan_to_num(0, 0, 0).ne(0).any(3))
     fine = torch.isfinite(o1) & torch.isfinite(o2)
     _close(o2[fine], o1[fine], "o")
+
+
+@pytest.mark.parametrize("M,N,splits", [(300, 9000, 3), (1, 4000, 11)])
+def test_runs_are_dealt_out_alike_with_and_without_a_plan(fb, M, N, splits):
+    """A split call for which a plan is optional, with more runs than SMs: the same bits either way, twice with one plan."""
+    from flash_b200 import _lib, ops
+    B, H, Hk, D = 4, 32, 8, 64
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q = torch.randn(B if M == 1 else 1, H, M, D, generator=g, device="cuda").bfloat16()
+    B = q.shape[0]
+    k, v = [torch.randn(B, Hk, N, D, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    prob = ops._problem(B, H, Hk, M, N, D, q.dtype, True, 0, 1, D ** -0.5)
+    assert lib.fa_plan_optional(prob, 0) == 1
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n = ctypes.c_size_t(0)
+    assert lib.fa_fwd_workspace_bytes(prob, splits, ctypes.byref(n)) == 0
+    work = torch.empty(n.value // 4, device="cuda")
+    plan = ops.build_plan(prob, None, None, status)
+    results = []
+    for p in (None, plan.data_ptr(), plan.data_ptr()):
+        o, lse = torch.empty_like(q), torch.empty(B, H, -(-M // 128) * 128, device="cuda")
+        assert lib.fa_fwd_split(prob, ops._tensor(q), ops._tensor(k), ops._tensor(v), ops._tensor(o), lse.data_ptr(), p, splits,
+                                work.data_ptr(), n.value, status.data_ptr(), ops._stream()) == 0
+        results.append((o, lse))
+    assert int(status.item()) == 0
+    assert all(torch.equal(o, results[0][0]) and torch.equal(lse, results[0][1]) for o, lse in results[1:])

@@ -221,7 +221,7 @@ class FlashAttention(torch.autograd.Function):
             if score_func_mode == SCORE_FUNC_MODE1_DOC:
                 plan = build_plan(prob, eq, ek, status)
             elif lib.fa_plan_optional(prob, any(ctx.needs_input_grad[:3])):
-                plan = None  # no more items than SMs: nothing to count
+                plan = None  # so few items that counters would not pay
             else:
                 plan = build_plan(prob, None, None, status)
             Out = torch.empty_like(q)
