@@ -328,11 +328,11 @@ def run_ours(args):
 
         # The timed step is one CUDA graph of the step's calls (plan, forward, backward): a rank's share of
         # the step is short (0.5 ms at 8 GPUs) and Python enqueues it more slowly than the GPU runs it when
-        # the host is busy, which a graph replay does not depend on. With one rank the per-kernel events
-        # are captured into the timed graph as event-record nodes and read after every timed replay.
-        # They cost about 4 us each, too much for the short steps of several ranks: there the timed graph
-        # has none and the per-kernel times come from one replay of a second graph (with the events) right
-        # after the timed region. --no-graph times plain eager calls (every step carries its own events).
+        # the host is busy, which a graph replay does not depend on. It is captured without per-kernel events:
+        # they cost about 4 us each, and with them the backward's kernels are launched one by one (dQ does not
+        # start beside dK / dV), which is not what a user's step does. The per-kernel times come from a
+        # second graph, which has the events, replayed after the timed region. --no-graph times plain eager
+        # calls, and the per-kernel times come from further eager steps.
         for _ in range(warmup):
             flush.zero_()
             step()
@@ -346,18 +346,16 @@ def run_ours(args):
                 with torch.cuda.stream(side):
                     step()
                 torch.cuda.current_stream().wait_stream(side)
-                graph_prof = torch.cuda.CUDAGraph()
-                ops.PROFILE = []
+                graph = torch.cuda.CUDAGraph()
                 l0 = ops.LAUNCHES
-                with torch.cuda.graph(graph_prof):
+                with torch.cuda.graph(graph):
                     step()
                 launches_per_step = ops.LAUNCHES - l0
+                graph_prof = torch.cuda.CUDAGraph()
+                ops.PROFILE = []
+                with torch.cuda.graph(graph_prof):
+                    step()
                 prof_graph, ops.PROFILE = ops.PROFILE, None
-                graph = graph_prof
-                if world > 1:
-                    graph = torch.cuda.CUDAGraph()
-                    with torch.cuda.graph(graph):
-                        step()
                 graph.replay()
                 torch.cuda.synchronize()
                 fb.check_status()
@@ -369,8 +367,6 @@ def run_ours(args):
         sampler = ClockSampler(local) if sample_clocks else None
         if sampler:
             sampler.start()
-        if graph is None:
-            ops.PROFILE = []
         launches0 = ops.LAUNCHES
         evs, kern = [], {}
         for _ in range(steps):
@@ -383,27 +379,23 @@ def run_ours(args):
                 step()
             e1.record()
             evs.append((e0, e1))
-            if graph is not None and graph is graph_prof:
-                # the graph's event nodes are re-recorded by every replay: read this step's kernel times now
-                torch.cuda.synchronize()
-                for nm, a, c in prof_graph:
-                    kern.setdefault(nm, []).append(a.elapsed_time(c))
         barrier()
         clocks = sampler.stop() if sampler else None
-        if graph is None:
-            prof, ops.PROFILE = ops.PROFILE, None
-            launches = ops.LAUNCHES - launches0
-        else:
-            if graph is not graph_prof:  # several ranks: one replay of the graph that holds the per-kernel events
-                flush.zero_()
-                graph_prof.replay()
-                torch.cuda.synchronize()
-            prof = prof_graph  # as recorded by the last replay of the graph that holds them
-            launches = launches_per_step * steps
-        fb.check_status()
-        if not kern:
+        launches = ops.LAUNCHES - launches0 if graph is None else launches_per_step * steps
+        time.sleep(0.5)  # the timed region may have brought the board to its power limit
+        for _ in range(min(steps, 10)):  # per-kernel times, outside the timed region
+            flush.zero_()
+            if graph is None:
+                ops.PROFILE = []
+                step()
+                prof, ops.PROFILE = ops.PROFILE, None
+            else:
+                graph_prof.replay()  # re-records the graph's event nodes
+                prof = prof_graph
+            torch.cuda.synchronize()
             for nm, a, c in prof:
                 kern.setdefault(nm, []).append(a.elapsed_time(c))
+        fb.check_status()
         t = torch.tensor([a.elapsed_time(c) for a, c in evs], dtype=torch.float64, device=dev)
         if world > 1:
             dist.all_reduce(t, op=dist.ReduceOp.MAX)  # every step counts with its slowest rank
@@ -433,14 +425,14 @@ def run_ours(args):
                 "kernel_ms": kern_ms,
                 "per_kernel_tflops": {nm: FLOPS_PER_ENTRY[nm] * D * nnz_local / (kern_ms[nm] * 1e-3) / 1e12
                                       for nm in kern_ms if nm in FLOPS_PER_ENTRY}}
-    # the forward call alone (mask plan + forward kernel), this rank's share, as measured inside the timed steps
+    # the forward call alone (mask plan + forward kernel), this rank's share, from the per-kernel times
     fwd_ms = kern_ms.get("fwd", 0.0) + kern_ms.get("plan", 0.0)
     fwd = None
     if fwd_ms > 0:
         fv = 4.0 * D * nnz_local * world / (fwd_ms * 1e-3) / 1e12
         fwd = {"value": fv, "unit": "TFLOP/s", "ms": fwd_ms, "frac_of_measured": fv / (peak_tf * world),
                "frac_of_nominal": fv / (2250.0 * world),
-               "what": "forward call (mask plan + forward kernel) of rank 0's shard, from the per-kernel events of the timed steps"}
+               "what": "forward call (mask plan + forward kernel) of rank 0's shard, from per-kernel events in replays after the timed region"}
 
     # other draws of the same configuration: the headline seed holds one very long document, which raises the
     # unmasked fraction and the share of full tiles; seeds 0-2 are the ordinary case
@@ -538,11 +530,9 @@ def run_ours(args):
                            "sharding": f"{'heads' if dim == 1 else 'batches'} over {world} rank(s), {n_local} per rank",
                            "l2": "256 MiB buffer written between timed iterations",
                            "statistic": "ms_per_step and value: median of the timed steps, each step taken at its slowest rank",
-                           "timed_step": ("eager calls with per-kernel events" if not m["graph"] else
-                                          "one CUDA graph replay per step (plan, forward, backward); per-kernel events are nodes of "
-                                          "the graph, read after every timed replay" if world == 1 else
-                                          "one CUDA graph replay per step (plan, forward, backward); per-kernel times from one replay "
-                                          "of the same step with event nodes, right after the timed region"),
+                           "timed_step": ("eager calls; per-kernel times from further steps with events" if not m["graph"] else
+                                          "one CUDA graph replay per step (plan, forward, backward); per-kernel times from replays "
+                                          "of the same step with event nodes, after the timed region"),
                            "unmasked_fraction_of_causal": nnz_total / dense,
                            "dense_count_tflops": (14.0 if backward else 4.0) * D * dense / (ms_per_step * 1e-3) / 1e12},
                 "frac_of_measured_peak": value / (peak_tf * world), "frac_of_nominal_peak": value / (2250.0 * world),
