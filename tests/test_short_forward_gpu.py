@@ -166,3 +166,39 @@ def test_runs_are_dealt_out_alike_with_and_without_a_plan(fb, M, N, splits):
         results.append((o, lse))
     assert int(status.item()) == 0
     assert all(torch.equal(o, results[0][0]) and torch.equal(lse, results[0][1]) for o, lse in results[1:])
+
+
+@pytest.mark.parametrize("runs", [1, 3, "whole call"])
+def test_pinned_runs_give_a_sequence_the_same_bits_in_any_batch(fb, runs):
+    """A sequence (or a share of the heads) by itself chooses another number of runs than the whole call; with `key_runs`
+    it gives the bits that it has in the whole call, gradients included."""
+    B, H, Hk, M, N, D = 3, 16, 4, 2, 6000, 64
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v, do = [torch.randn(B, h, n, D, generator=g, device="cuda").bfloat16() for h, n in ((H, M), (Hk, N), (Hk, N), (H, M))]
+    whole = fb.forward_splits(B, H, Hk, M, N, D, q.dtype, True, 0)
+    assert whole > 1 and fb.forward_splits(1, H, Hk, M, N, D, q.dtype, True, 0) != whole
+    runs = whole if runs == "whole call" else runs
+
+    def step(*at):
+        x = [t[at].clone().requires_grad_() for t in (q, k, v)]
+        o = fb.attention(*x, True, key_runs=runs)
+        return (o.detach(), *torch.autograd.grad(o, x, do[at]))
+
+    full = step(slice(None))
+    for b in range(B):
+        assert all(torch.equal(a[b:b + 1], p) for a, p in zip(full, step(slice(b, b + 1))))
+    heads = [torch.cat([t[:, 4:8] if i in (0, 1) else t[:, 1:2]], 1) for i, t in enumerate(full)]
+    x = [t.clone().requires_grad_() for t in (q[:, 4:8], k[:, 1:2], v[:, 1:2])]
+    o = fb.attention(*x, True, key_runs=runs)
+    part = (o.detach(), *torch.autograd.grad(o, x, do[:, 4:8]))
+    assert all(torch.equal(a, p) for a, p in zip(heads, part))
+    if runs == whole:
+        assert torch.equal(full[0], fb.attention(q, k, v, True))
+    # eight arguments, as before: as many gradients
+    o = fb.FlashAttention.apply(q.requires_grad_(), k, v, True, None, None, None, 0)
+    o.backward(do)
+    # what cannot be cut is refused
+    ids = (-1 - torch.arange(N, device="cuda") // 1000).expand(B, H, N)
+    for args in ((k, k, v, False, None, ids[:, :Hk], ids[:, :Hk], 1), (q.detach().float(), k.float(), v.float(), True)):
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            fb.attention(*args, key_runs=2)

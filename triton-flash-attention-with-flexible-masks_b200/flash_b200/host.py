@@ -157,8 +157,7 @@ def attention_host(q, k, v, do=None, causal=False, sm_scale=None, eq=None, ek=No
                     k_ = k_.expand(dq_.shape[0], dq_.shape[1], k.shape[2]) if k_.shape[1] == 1 else k_
                 if direct:
                     ctx = _Ctx()
-                    ctx.fwd_splits = splits
-                    o = ops.FlashAttention.forward(ctx, dq_, dk_, dv_, causal, sm_scale, e, k_, score_func_mode)
+                    o = ops.FlashAttention.forward(ctx, dq_, dk_, dv_, causal, sm_scale, e, k_, score_func_mode, splits)
                     results = [("o", o, qa, qb)]
                     if backward:
                         gq, gk, gv = ops.FlashAttention.backward(ctx, ddo)[:3]

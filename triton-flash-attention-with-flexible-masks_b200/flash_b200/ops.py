@@ -154,7 +154,8 @@ def _stream():
 
 
 def forward_splits(B, H, Hk, M, N, D, dtype, causal, mode):
-    """Into how many runs the forward of this call cuts the keys of a query block (fa_fwd_splits)."""
+    """Into how many runs the forward of this call cuts the keys of a query block (fa_fwd_splits): `attention`'s key_runs
+    for a part of a call that is to give the bits of the whole one."""
     return _lib.load().fa_fwd_splits(ctypes.byref(_problem(B, H, Hk, M, N, D, dtype, causal, mode, 1, 1.0)))
 
 
@@ -178,7 +179,7 @@ def build_plan(prob, eq, ek, status):
 
 class FlashAttention(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, causal, sm_scale, eq, ek, score_func_mode):
+    def forward(ctx, q, k, v, causal, sm_scale, eq, ek, score_func_mode, key_runs=None):
         lib = _lib.load()
         # checks of flash_triton.py:510-520
         Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
@@ -228,9 +229,8 @@ class FlashAttention(torch.autograd.Function):
             if maybe_contiguous(Out) is not Out:
                 Out = torch.empty(q.shape, dtype=q.dtype, device=device)
             L = torch.empty((B, H, (M + 127) // 128 * 128), device=device, dtype=torch.float32)
-            # calls that cannot fill the GPU cut their keys into runs (attention_host sets the number of the
-            # whole call, so that a slice computes the same bits)
-            splits = getattr(ctx, "fwd_splits", 0) or lib.fa_fwd_splits(prob)
+            # calls that cannot fill the GPU cut their keys into runs
+            splits = key_runs or lib.fa_fwd_splits(prob)
             work, work_ptr, work_bytes = None, None, 0
             if splits > 1:
                 nbytes = ctypes.c_size_t(0)
@@ -255,6 +255,7 @@ class FlashAttention(torch.autograd.Function):
         ctx.causal = causal
         ctx.shapes = (B, H, M, D, N, Hk, num_groups, MN_GAP)
         ctx.score_func_info = (score_func_mode, )
+        ctx.n_other = 5 if key_runs is None else 6  # inputs that are not q, k, v
         return Out
 
     @staticmethod
@@ -299,7 +300,7 @@ class FlashAttention(torch.autograd.Function):
                     _lib.check(lib.fa_bwd_dq(prob, tq, tk, tv, tdo, lp, dp, tdq, plan_ptr, sp, stream), "fa_bwd_dq")
             if _SYNC_STATUS:
                 check_status(q.device)
-        return dq, dk, dv, None, None, None, None, None
+        return (dq, dk, dv) + (None,) * ctx.n_other
 
 
 # Without a causal mask the order of the queries is free. When the query ids are not grouped (every
@@ -369,8 +370,14 @@ def _attention_grouped(q, k, v, sm_scale, eq, ek):
     return _PermuteRows.apply(o_g, inverse, order, id_heads)
 
 
-def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func_mode=SCORE_FUNC_MODE0_NOPE):
+def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func_mode=SCORE_FUNC_MODE0_NOPE, key_runs=0):
     """Drop-in for flash_triton.py:640-641.
+
+    key_runs: into how many runs the forward cuts the keys. Calls without ids that cannot fill the GPU (few queries)
+    choose a number from their sizes, the batch and the SM count among them (0, `forward_splits`), so that a sequence's
+    result can differ in its last bits with what it is batched with. 1 computes every sequence in one run, whatever lies
+    beside it; another number, at most one per 128 keys, is for callers that fix it by the sequence alone or, as for
+    the shards of a call, by the whole call. Calls that cannot be cut (ids, fp32) take 0 or 1.
 
     The tensor-core kernels are built for head dims 64 and 128. For 16-bit inputs the reference's smaller
     head dims (16 and 32, flash_triton.py:512) run on the 64-wide kernels without any padded copy: the library
@@ -379,8 +386,11 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
     real columns only."""
     if (GROUP_QUERIES and score_func_mode == SCORE_FUNC_MODE1_DOC and not causal and eq is not None and ek is not None
             and q.is_cuda and q.dim() == 4 and 128 < q.shape[2] <= _lib.FA_GROUP_MAX_ROWS):
+        if key_runs > 1:
+            raise NotImplementedError("flash_b200: a call with ids is not cut into key runs")
         return _attention_grouped(q, k, v, sm_scale, eq, ek)
-    return FlashAttention.apply(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
+    args = (q, k, v, causal, sm_scale, eq, ek, score_func_mode)
+    return FlashAttention.apply(*args, key_runs) if key_runs else FlashAttention.apply(*args)
 
 
 def debug_mask(B, H, M, N, causal, eq=None, ek=None, score_func_mode=SCORE_FUNC_MODE0_NOPE, device="cuda"):
