@@ -55,7 +55,7 @@ enum fa_error {
     FA_ERR_ALIGNMENT = 3,    /* a base address or stride breaks the TMA 16-byte rules */
     FA_ERR_TENSORMAP = 4,    /* the driver refused to encode a tensor map */
     FA_ERR_LAUNCH = 5,       /* kernel launch failed (cudaGetLastError) */
-    FA_ERR_PLAN_SIZE = 6,    /* plan buffer too small / missing for FA_MODE1_DOC */
+    FA_ERR_PLAN_SIZE = 6,    /* plan buffer too small / missing for FA_MODE1_DOC, or workspace of a split forward */
     FA_ERR_NO_DRIVER = 7,    /* cuTensorMapEncodeTiled could not be resolved */
     FA_ERR_SCRATCH_LIMIT = 8 /* fa_fwd_static_plan: the plan does not fit in FA_STATIC_PLAN_BYTES */
 };

@@ -1,6 +1,6 @@
 """Forward calls without ids that are short of work: query heads of a group packed into one tile, keys cut into
-runs that are merged afterwards. Against plain attention in 64 bits; the bound is the parity tests' rule for 16-bit
-results (2e-2, or one rounding step of the result where that is larger)."""
+runs that are merged afterwards. Against plain attention in 64 bits, with a bound that scales with the result: the long
+calls' outputs and gradients are a few hundredths of the inputs."""
 import ctypes
 
 import pytest
@@ -39,9 +39,16 @@ def _exact(q, k, v, causal):
 
 
 def _close(got, want, what):
-    err, want = (got.double() - want).abs(), want.abs()
-    bound = torch.where(want < 2.56, torch.full_like(want, 2e-2), want * 2.0 ** -7)
-    assert bool((err <= bound).all()), (what, err.max().item())
+    """Row by row, by norm. Rounded to 16 bits on the way, u of a value each: P or dS, O (which enters dS through delta
+    whatever the size of the row's own gradient, hence the tensor's mean row beside the row's norm) and the result; the
+    roundings of a row's D columns and N keys are independent, and 8 is over twice the sum of the three at four standard
+    deviations of rows this long. A tile of 128 keys that is lost or counted twice is sqrt(128 / N) of an output's norm: at
+    least 0.056 here, where the bound is 16 u = 0.031 in bf16."""
+    u = 2.0 ** -9 if got.dtype == torch.bfloat16 else 2.0 ** -12
+    norm = want.norm(dim=-1)
+    bound = 8 * u * (norm + norm.square().mean().sqrt())
+    err = (got.double() - want).norm(dim=-1)
+    assert bool((err <= bound).all()), (what, (err / bound).max().item())
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -63,17 +70,19 @@ def test_short_forward(fb, case, dtype):
         _close(got.detach(), want.detach(), what)
 
 
+@pytest.mark.parametrize("H,Hk,M", [(4, 2, 300), (8, 2, 1), (4, 1, 3), (6, 2, 50)])
 @pytest.mark.parametrize("splits", [1, 2, 5, 16])
-def test_any_number_of_runs(fb, splits):
-    """Also numbers the rule would not take, among them runs that the causal bound leaves without keys; lse too."""
+def test_any_number_of_runs(fb, splits, H, Hk, M):
+    """Also numbers the rule would not take, among them runs that the causal bound leaves without keys; the lse too, of
+    packed tiles as well."""
     from flash_b200 import _lib, ops
-    B, H, Hk, M, N, D = 2, 4, 2, 300, 2048, 64
+    B, N, D = 2, 2048, 64
     lib = _lib.load()
     g = torch.Generator(device="cuda").manual_seed(3)
     q, o = torch.randn(B, H, M, D, generator=g, device="cuda").bfloat16(), torch.empty(B, H, M, D, device="cuda", dtype=torch.bfloat16)
     k, v = [torch.randn(B, Hk, N, D, generator=g, device="cuda").bfloat16() for _ in range(2)]
     prob = ops._problem(B, H, Hk, M, N, D, q.dtype, True, 0, 1, D ** -0.5)
-    lse = torch.full((B, H, 384), float("nan"), device="cuda")
+    lse = torch.full((B, H, -(-M // 128) * 128), float("nan"), device="cuda")
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     n = ctypes.c_size_t(0)
     assert lib.fa_fwd_workspace_bytes(ctypes.byref(prob), splits, ctypes.byref(n)) == 0
@@ -137,8 +146,8 @@ def test_values_that_are_not_finite_do_not_get_lost_in_a_run(fb, M, G, what):
     assert bool(((l1 - l2).abs() < 1e-4 + 1e-6 * l1.abs())[~dead].all())
     assert torch.equal(torch.isnan(o1), torch.isnan(o2))
     assert torch.equal(o1.nan_to_num(0, 0, 0).ne(0).any(3), o2.nan_to_num(0, 0, 0).ne(0).any(3))
-    fine = torch.isfinite(o1) & torch.isfinite(o2)
-    _close(o2[fine], o1[fine], "o")
+    finite = (torch.isfinite(o1) & torch.isfinite(o2)).all(3)
+    _close(o2[finite].bfloat16(), o1[finite], "o")
 
 
 @pytest.mark.parametrize("M,N,splits", [(300, 9000, 3), (1, 4000, 11)])

@@ -27,7 +27,6 @@
 #include <type_traits>
 #include "common.cuh"
 #include "params.cuh"
-#include <type_traits>
 
 namespace fa {
 
@@ -57,7 +56,7 @@ struct FwdSmem {
 };
 
 // SHORT: calls without ids whose items are too few or too empty for one item per (query block, head, batch).
-// Two things are added (fwd_short_pack and fwd_splits in api.cu say when):
+// Two things are added (fwd_pack and fwd_splits in api.cu say when):
 //  - p.pack query heads of one kv head share a tile, row g * M + i = query i of the g-th of them (at most 128
 //    rows: one decoded token of 4 heads reads the keys and values once instead of four times). The Q and O maps
 //    are 5-D, (D, M, G, Hk, B), and a box holds p.rows rows; tile rows past them are never loaded, hold whatever
