@@ -179,8 +179,8 @@ def test_runs_are_dealt_out_alike_with_and_without_a_plan(fb, M, N, splits):
 
 @pytest.mark.parametrize("runs", [1, 3, "whole call"])
 def test_pinned_runs_give_a_sequence_the_same_bits_in_any_batch(fb, runs):
-    """A sequence (or a share of the heads) by itself chooses another number of runs than the whole call; with `key_runs`
-    it gives the bits that it has in the whole call, gradients included."""
+    """A sequence (or a share of the heads) by itself chooses another number of runs than the whole call; with
+    `attention_in_runs` it gives the bits that it has in the whole call, gradients included."""
     B, H, Hk, M, N, D = 3, 16, 4, 2, 6000, 64
     g = torch.Generator(device="cuda").manual_seed(0)
     q, k, v, do = [torch.randn(B, h, n, D, generator=g, device="cuda").bfloat16() for h, n in ((H, M), (Hk, N), (Hk, N), (H, M))]
@@ -190,7 +190,7 @@ def test_pinned_runs_give_a_sequence_the_same_bits_in_any_batch(fb, runs):
 
     def step(*at):
         x = [t[at].clone().requires_grad_() for t in (q, k, v)]
-        o = fb.attention(*x, True, key_runs=runs)
+        o = fb.attention_in_runs(*x, runs, True)
         return (o.detach(), *torch.autograd.grad(o, x, do[at]))
 
     full = step(slice(None))
@@ -198,7 +198,7 @@ def test_pinned_runs_give_a_sequence_the_same_bits_in_any_batch(fb, runs):
         assert all(torch.equal(a[b:b + 1], p) for a, p in zip(full, step(slice(b, b + 1))))
     heads = [torch.cat([t[:, 4:8] if i in (0, 1) else t[:, 1:2]], 1) for i, t in enumerate(full)]
     x = [t.clone().requires_grad_() for t in (q[:, 4:8], k[:, 1:2], v[:, 1:2])]
-    o = fb.attention(*x, True, key_runs=runs)
+    o = fb.attention_in_runs(*x, runs, True)
     part = (o.detach(), *torch.autograd.grad(o, x, do[:, 4:8]))
     assert all(torch.equal(a, p) for a, p in zip(heads, part))
     if runs == whole:
@@ -206,8 +206,5 @@ def test_pinned_runs_give_a_sequence_the_same_bits_in_any_batch(fb, runs):
     # eight arguments, as before: as many gradients
     o = fb.FlashAttention.apply(q.requires_grad_(), k, v, True, None, None, None, 0)
     o.backward(do)
-    # what cannot be cut is refused
-    ids = (-1 - torch.arange(N, device="cuda") // 1000).expand(B, H, N)
-    for args in ((k, k, v, False, None, ids[:, :Hk], ids[:, :Hk], 1), (q.detach().float(), k.float(), v.float(), True)):
-        with pytest.raises((RuntimeError, NotImplementedError)):
-            fb.attention(*args, key_runs=2)
+    with pytest.raises(RuntimeError):  # what cannot be cut is refused
+        fb.attention_in_runs(q.detach().float(), k.float(), v.float(), 2, True)

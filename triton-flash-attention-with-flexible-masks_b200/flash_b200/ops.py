@@ -154,8 +154,8 @@ def _stream():
 
 
 def forward_splits(B, H, Hk, M, N, D, dtype, causal, mode):
-    """Into how many runs the forward of this call cuts the keys of a query block (fa_fwd_splits): `attention`'s key_runs
-    for a part of a call that is to give the bits of the whole one."""
+    """Into how many runs the forward of this call cuts the keys of a query block (fa_fwd_splits): `attention_in_runs`
+    takes it for a part of a call that is to give the bits of the whole one."""
     return _lib.load().fa_fwd_splits(ctypes.byref(_problem(B, H, Hk, M, N, D, dtype, causal, mode, 1, 1.0)))
 
 
@@ -370,14 +370,8 @@ def _attention_grouped(q, k, v, sm_scale, eq, ek):
     return _PermuteRows.apply(o_g, inverse, order, id_heads)
 
 
-def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func_mode=SCORE_FUNC_MODE0_NOPE, key_runs=0):
+def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func_mode=SCORE_FUNC_MODE0_NOPE):
     """Drop-in for flash_triton.py:640-641.
-
-    key_runs: into how many runs the forward cuts the keys. Calls without ids that cannot fill the GPU (few queries)
-    choose a number from their sizes, the batch and the SM count among them (0, `forward_splits`), so that a sequence's
-    result can differ in its last bits with what it is batched with. 1 computes every sequence in one run, whatever lies
-    beside it; another number, at most one per 128 keys, is for callers that fix it by the sequence alone or, as for
-    the shards of a call, by the whole call. Calls that cannot be cut (ids, fp32) take 0 or 1.
 
     The tensor-core kernels are built for head dims 64 and 128. For 16-bit inputs the reference's smaller
     head dims (16 and 32, flash_triton.py:512) run on the 64-wide kernels without any padded copy: the library
@@ -386,11 +380,18 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
     real columns only."""
     if (GROUP_QUERIES and score_func_mode == SCORE_FUNC_MODE1_DOC and not causal and eq is not None and ek is not None
             and q.is_cuda and q.dim() == 4 and 128 < q.shape[2] <= _lib.FA_GROUP_MAX_ROWS):
-        if key_runs > 1:
-            raise NotImplementedError("flash_b200: a call with ids is not cut into key runs")
         return _attention_grouped(q, k, v, sm_scale, eq, ek)
-    args = (q, k, v, causal, sm_scale, eq, ek, score_func_mode)
-    return FlashAttention.apply(*args, key_runs) if key_runs else FlashAttention.apply(*args)
+    return FlashAttention.apply(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
+
+
+def attention_in_runs(q, k, v, key_runs, causal=False, sm_scale=None):
+    """`attention` without ids, with the keys cut into `key_runs` runs in the forward.
+
+    `attention` chooses a number where a call cannot fill the GPU (few queries) from its sizes, the batch and the SM count
+    among them (`forward_splits`), so that a sequence's result can differ in its last bits with what it is batched with.
+    1 computes every sequence in one run, whatever lies beside it; another number, at most one per 128 keys (fp32: 1),
+    is for callers that fix it by the sequence alone or, for the shards of a call, by the whole call."""
+    return FlashAttention.apply(q, k, v, causal, sm_scale, None, None, SCORE_FUNC_MODE0_NOPE, int(key_runs))
 
 
 def debug_mask(B, H, M, N, causal, eq=None, ek=None, score_func_mode=SCORE_FUNC_MODE0_NOPE, device="cuda"):
