@@ -45,6 +45,8 @@ EncodeFn encode_fn() {
     return fn;
 }
 
+using ContextIdFn = CUresult (*)(CUcontext, unsigned long long*);
+
 int check_problem(const fa_problem* p) {
     if (!p) return FA_ERR_BAD_ARG;
     if (p->B <= 0 || p->H <= 0 || p->Hk <= 0 || p->M <= 0 || p->N <= 0) return FA_ERR_BAD_ARG;
@@ -328,6 +330,21 @@ int run_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, cons
 }
 
 }  // namespace
+
+namespace fa {
+uint64_t context_number() {
+    static ContextIdFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<ContextIdFn>(p);
+    });
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? uint64_t(id) + 1 : 0;  // (no context yet: 0)
+}
+}  // namespace fa
 
 extern "C" {
 

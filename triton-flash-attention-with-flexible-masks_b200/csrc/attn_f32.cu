@@ -498,7 +498,7 @@ static cudaError_t launch_f32_t(int which, const F32Params& p, cudaStream_t stre
     constexpr int fwd_smem = (S::rows + 4 * S::cols + S::p + 2 * kC) * 4;
     constexpr int bwd_smem = (2 * S::rows + 4 * S::cols + S::p + 2 * S::vec) * 4;
     static_assert(bwd_smem + kListCap <= 232448, "shared memory budget");
-    static std::atomic<uint64_t> allowed[4];
+    static SmemAllowed allowed[4];
     auto run = [&](auto kern, int smem, int rows, int heads) {
         const cudaError_t e = allow_smem(kern, smem, allowed[which]);
         if (e != cudaSuccess) return e;

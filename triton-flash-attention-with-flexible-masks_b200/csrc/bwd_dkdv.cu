@@ -656,7 +656,7 @@ static cudaError_t launch_dkdv_t(const CUtensorMap& tq, const CUtensorMap& tk, c
                                  const DkdvParams& p, int num_sms, cudaStream_t stream) {
     auto kern = bwd_dkdv_kernel<D, BF16>;
     constexpr int smem = DkdvSmem<D>::total;
-    static std::atomic<uint64_t> allowed{0};
+    static SmemAllowed allowed;
     cudaError_t e = allow_smem(kern, smem, allowed);
     if (e != cudaSuccess) return e;
     const int n_items = p.mask.L.nK * p.Hk * p.B;

@@ -577,7 +577,7 @@ static cudaError_t launch_dq_t(const CUtensorMap& tq, const CUtensorMap& tk, con
                                bool overlap, cudaStream_t stream) {
     auto kern = bwd_dq_kernel<D, BF16>;
     constexpr int smem = DqSmem<D>::total;
-    static std::atomic<uint64_t> allowed{0};
+    static SmemAllowed allowed;
     cudaError_t e = allow_smem(kern, smem, allowed);
     if (e != cudaSuccess) return e;
     const int n_items = p.mask.L.nQ * p.H * p.B;

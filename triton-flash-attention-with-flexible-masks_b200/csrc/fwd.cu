@@ -780,7 +780,7 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
                                 const CUtensorMap& to, const FwdParams& p, int num_sms, cudaStream_t stream) {
     auto kern = fwd_kernel<D, BF16, SHORT>;
     constexpr int smem = FwdSmem<D>::total;
-    static std::atomic<uint64_t> allowed{0};
+    static SmemAllowed allowed;
     cudaError_t e = allow_smem(kern, smem, allowed);
     if (e != cudaSuccess) return e;
     const int heads = SHORT ? p.H / p.G * cdiv(p.G, p.pack) : p.H;

@@ -82,18 +82,24 @@ struct F32Params {
     float scale;
 };
 
-// Lets kernels of this launch site use `bytes` of dynamic shared memory. The attribute belongs to the device: it is set
-// once per device (always to the same value, so a race between two first calls is harmless). One `done` per kernel.
+// A number for the current CUDA context that no other context of the process ever has, or 0 (api.cu).
+uint64_t context_number();
+
+// The contexts in which a kernel may already use its dynamic shared memory. One per kernel.
+struct SmemAllowed {
+    std::atomic<uint64_t> context[16] = {};
+};
+
+// Lets `kern` use `bytes` of dynamic shared memory. The attribute belongs to the context (a process may have several on
+// one device, and a device reset makes a new one), so it is set once per context, always to the same value.
 template <class Kernel>
-inline cudaError_t allow_smem(Kernel kern, int bytes, std::atomic<uint64_t>& done) {
-    int dev = -1;
-    const cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const uint64_t bit = (dev >= 0 && dev < 64) ? uint64_t(1) << dev : 0;
-    if (bit && (done.load(std::memory_order_relaxed) & bit)) return cudaSuccess;
-    const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (r == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
-    return r;
+inline cudaError_t allow_smem(Kernel kern, int bytes, SmemAllowed& allowed) {
+    const uint64_t number = context_number();
+    std::atomic<uint64_t>& slot = allowed.context[number % 16];
+    if (number && slot.load(std::memory_order_relaxed) == number) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) slot.store(number, std::memory_order_relaxed);
+    return e;
 }
 
 // Ordered compaction of per-tile flags (list[i] = flags of tile lo+i) into the visited list:
