@@ -168,7 +168,8 @@ int fa_debug_mask(const fa_problem* p, const void* plan, uint8_t* keep, uint8_t*
  * Returns FA_ERR_SCRATCH_LIMIT when the plan would not fit. The array is shared by all calls on a
  * GPU: it keeps the previous call's contents (every element read is overwritten first, nothing
  * needs clearing) and calls that overlap on the same GPU race. The first call on a device looks
- * up the array's address; make it before any stream capture on that device. */
+ * up the array's address; make it before any stream capture on that device (with several contexts on
+ * a device, so does a call in another context than the one before). */
 int fa_fwd_static_plan(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v,
                        const fa_tensor* o, float* lse, const fa_ids* eq, const fa_ids* ek, int32_t* status,
                        void* stream);

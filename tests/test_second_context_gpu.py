@@ -23,6 +23,14 @@ for dt, D in KINDS:
     x = [torch.randn(B, H, L, D, device="cuda").to(dt).requires_grad_() for _ in range(3)]
     fb.attention(*x, False, None, ids, ids, 1).sum().backward()
 fb.check_status()
+
+def static_plan(p, q, k, v, o, lse, ids, status):
+    return lib.fa_fwd_static_plan(p, q, k, v, o, lse, ids, ids, status, None)
+
+x, st = [torch.randn(B, H, L, 64, device="cuda").bfloat16() for _ in range(4)], torch.zeros(1, dtype=torch.int32, device="cuda")
+assert static_plan(ops._problem(B, H, H, L, L, 64, torch.bfloat16, False, 1, 1, 1.0), *[ops._tensor(t) for t in x],
+                   torch.empty(B, H, 384, device="cuda").data_ptr(), ops._ids(ids), st.data_ptr()) == 0
+torch.cuda.synchronize()
 cu = ctypes.CDLL("libcuda.so.1")
 assert cu.cuCtxCreate_v2(ctypes.byref(ctypes.c_void_p()), 0, 0) == 0
 
@@ -45,10 +53,11 @@ for dt, D in KINDS:
     plan = alloc(bytes(n.value))
     rc = [lib.fa_group_rows(p, ek, *rows, status, None), lib.fa_plan_build(p, ek, ek, plan, n.value, status, None),
           lib.fa_fwd(p, q, k, v, o, lse, plan, status, None),
-          lib.fa_bwd(p, q, k, v, o, do, lse, delta, dq, dk, dv, plan, status, None), cu.cuCtxSynchronize()]
+          lib.fa_bwd(p, q, k, v, o, do, lse, delta, dq, dk, dv, plan, status, None),
+          static_plan(p, q, k, v, o, lse, ek, status), cu.cuCtxSynchronize()]
     got = ctypes.c_int32(-1)
     assert cu.cuMemcpyDtoH_v2(ctypes.byref(got), ctypes.c_uint64(status), ctypes.c_size_t(4)) == 0
-    assert rc == [0] * 5 and got.value == 0, (dt, D, rc, got.value)
+    assert rc == [0] * 6 and got.value == 0, (dt, D, rc, got.value)
 print("served")
 """
 

@@ -19,36 +19,41 @@
 //  - the plan is not returned, so the backward entry points (which want the plan again) need a
 //    caller-owned plan buffer; this entry point serves forward-only use.
 //  - the first call on each device looks up the array's device address (see below); make that
-//    first call before starting any stream capture on that device.
+//    first call before starting any stream capture on that device. With several contexts on one
+//    device, so does every call in another context than the one before.
 //
 // The call itself performs no cudaMalloc / cudaFree and uses no allocating library routine.
 #include <mutex>
 #include "../../include/fa_b200.h"
-#include <cuda_runtime.h>
+#include "params.cuh"
 
 // In host code this name is only a handle for the runtime, not a device address: a kernel given
 // `g_static_plan` directly would read the wrong memory. The address kernels may use comes from
-// cudaGetSymbolAddress, looked up once per device with that device current.
+// cudaGetSymbolAddress, looked up with that device current.
 static __device__ __align__(256) int32_t g_static_plan[FA_STATIC_PLAN_BYTES / sizeof(int32_t)];
 
 namespace {
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
-int32_t* g_plan_addr[kMaxDevices] = {};
+struct {
+    uint64_t context;  // the array has an address of its own in every context of the device
+    int32_t* addr;
+} g_plan[kMaxDevices] = {};
 
-// Device address of the static plan on the current device, or null with an error code.
+// Device address of the static plan in the current context, or null with an error code.
 int static_plan_address(int32_t** out) {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return FA_ERR_LAUNCH;
+    const uint64_t context = fa::context_number();
     std::lock_guard<std::mutex> lock(g_mu);
-    if (!g_plan_addr[dev]) {
+    if (!g_plan[dev].addr || !context || g_plan[dev].context != context) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_static_plan);
         if (e != cudaSuccess || !p) return FA_ERR_LAUNCH;
-        g_plan_addr[dev] = static_cast<int32_t*>(p);
+        g_plan[dev] = {fa::context_number(), static_cast<int32_t*>(p)};
     }
-    *out = g_plan_addr[dev];
+    *out = g_plan[dev].addr;
     return FA_OK;
 }
 
