@@ -100,7 +100,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     constexpr int NST = S::NST;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
     const MaskArgs& mk = p.mask;
     const int G = p.G;
@@ -145,7 +145,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int s = 0; s < NST; ++s) {
             mbar_init(BAR(B_QFULL + s), 1); mbar_init(BAR(B_DOFULL + s), 1);
             mbar_init(BAR(B_QEMPTY + s), 2);  // S^T (warp 9) and dK (warp 10) both read the Q stage
-            mbar_init(BAR(B_DOEMPTY + s), 1); // dP^T and dV are issued by the same thread: one commit
+            mbar_init(BAR(B_DOEMPTY + s), 1); // dP^T and dV are issued by the same warp: one commit
         }
         mbar_init(BAR(B_SFULL), 1);
         mbar_init(BAR(B_SFREE), 256);
@@ -332,14 +332,15 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             // ------------------------------ MMA issuers (warps 9, 10) ------------------------------
             //   warp 9 : S^T(it) = K Q^T, as soon as the compute groups have read S^T(it-1)
             //   warp 10: dV(it) += P^T dO when P^T is in shared memory, then dK(it) += dS^T Q and
-            //            dP^T(it+1) = V dO^T when dS^T is in TMEM (dP^T overwrites dS^T: same thread)
-            // Each Q / dO stage is read by both threads, so its "empty" barrier takes two commits.
-            if (lane == 0) {
+            //            dP^T(it+1) = V dO^T when dS^T is in TMEM (dP^T overwrites dS^T: same warp)
+            // Each Q / dO stage is read by both warps' MMAs, so its "empty" barrier takes two commits.
+            {
+                const uint32_t utmem = uniform(int(tmem));
                 constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
                 constexpr uint32_t idesc_d = make_idesc(BF16, 128, D, false, true);
                 constexpr uint64_t desc_mn = desc_mn_major(S::BOX);
-                auto q_ready = [&](int gi) { return mbar_wait(BAR(B_QFULL + gi % NST), (gi / NST) & 1, ab, ST_WAIT_TIMEOUT + 44); };
-                auto do_ready = [&](int gi) { return mbar_wait(BAR(B_DOFULL + gi % NST), (gi / NST) & 1, ab, ST_WAIT_TIMEOUT + 45); };
+                auto q_ready = [&](int gi) { return mbar_wait_warp(BAR(B_QFULL + gi % NST), (gi / NST) & 1, ab, ST_WAIT_TIMEOUT + 44); };
+                auto do_ready = [&](int gi) { return mbar_wait_warp(BAR(B_DOFULL + gi % NST), (gi / NST) & 1, ab, ST_WAIT_TIMEOUT + 45); };
                 auto ss_mmas = [&](uint32_t d, uint32_t a_tile, uint32_t b_tile) {
 #pragma unroll
                     for (int kk2 = 0; kk2 < D / 16; ++kk2) {
@@ -352,64 +353,64 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 int k = 0, kk = 0, gt = 0;
                 for (;; ++k) {
                     const int s = k & 1;
-                    ok = mbar_wait(BAR(B_ITEMFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 56);
+                    ok = mbar_wait_warp(BAR(B_ITEMFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 56);
                     if (!ok) break;
-                    const int NIT = info[s * 8 + 2];
-                    if (info[s * 8 + 3] < 0) break;
+                    const int NIT = uniform(info[s * 8 + 2]);
+                    if (uniform(info[s * 8 + 3]) < 0) break;
                     if (NIT > 0 && warp == 9) {
-                        ok = mbar_wait(BAR(B_KFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
+                        ok = mbar_wait_warp(BAR(B_KFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
                         for (int it = 0; it < NIT && ok; ++it) {
                             const int gi = gt + it, st = gi % NST;
                             ok = q_ready(gi);
                             // the S^T columns are free once every compute thread has loaded the previous S^T
-                            if (ok && gi > 0) ok = mbar_wait(BAR(B_SFREE), (gi - 1) & 1, ab, ST_WAIT_TIMEOUT + 46);
+                            if (ok && gi > 0) ok = mbar_wait_warp(BAR(B_SFREE), (gi - 1) & 1, ab, ST_WAIT_TIMEOUT + 46);
                             if (!ok) break;
                             tc_fence_after();
-                            ss_mmas(tmem, sK, sQ(st));
+                            ss_mmas(utmem, sK, sQ(st));
                             umma_commit(BAR(B_QEMPTY + st));
                             umma_commit(BAR(B_SFULL));
                         }
                         if (!ok) break;
                         umma_commit(BAR(B_KEMPTY));
                     } else if (NIT > 0) {
-                        ok = mbar_wait(BAR(B_VFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
+                        ok = mbar_wait_warp(BAR(B_VFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
                         if (ok) ok = do_ready(gt);
                         if (!ok) break;
                         tc_fence_after();
-                        ss_mmas(tmem + 128u, sV, sdO(gt % NST));  // dP^T(0)
+                        ss_mmas(utmem + 128u, sV, sdO(gt % NST));  // dP^T(0)
                         umma_commit(BAR(B_DPFULL));
                         if (NIT == 1) umma_commit(BAR(B_VEMPTY));  // V may be replaced after the item's last dP^T
                         // dV(0) and dK(0) overwrite the accumulators: the previous item's epilogue must have read them
-                        if (kk > 0) ok = mbar_wait(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 58);
+                        if (kk > 0) ok = mbar_wait_warp(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 58);
                         for (int it = 0; it < NIT && ok; ++it) {
                             const int gi = gt + it, st = gi % NST;
                             const bool more = it + 1 < NIT;
                             // dV(it) += P^T dO: A = P^T from shared memory (K-major), B = dO (MN-major)
-                            ok = mbar_wait(BAR(B_PFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 47);
+                            ok = mbar_wait_warp(BAR(B_PFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 47);
                             if (!ok) break;
                             tc_fence_after();
 #pragma unroll
                             for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
                                 const uint32_t off = uint32_t(kk2 >> 2) * S::BOX + uint32_t(kk2 & 3) * 32u;
-                                umma_ss(tmem + 256u, smem_desc_at(kDescKMajor, sP + off),
+                                umma_ss(utmem + 256u, smem_desc_at(kDescKMajor, sP + off),
                                         smem_desc_at(desc_mn, sdO(st) + uint32_t(kk2) * 2048u), idesc_d, (it > 0 || kk2 > 0) ? 1u : 0u);
                             }
                             umma_commit(BAR(B_PFREE));
                             umma_commit(BAR(B_DOEMPTY + st));
                             if (more) ok = do_ready(gi + 1);
-                            if (ok) ok = mbar_wait(BAR(B_DSFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 48);
+                            if (ok) ok = mbar_wait_warp(BAR(B_DSFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 48);
                             if (!ok) break;
                             tc_fence_after();
                             // dK(it) += dS^T Q: A = dS^T from TMEM, B = Q (MN-major)
 #pragma unroll
                             for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
                                 const uint32_t acol = (kk2 < 4) ? uint32_t(kk2) * 8u : 64u + uint32_t(kk2 - 4) * 8u;
-                                umma_ts(tmem + 256u + uint32_t(D), tmem + 128u + acol,
+                                umma_ts(utmem + 256u + uint32_t(D), utmem + 128u + acol,
                                         smem_desc_at(desc_mn, sQ(st) + uint32_t(kk2) * 2048u), idesc_d, (it > 0 || kk2 > 0) ? 1u : 0u);
                             }
                             umma_commit(BAR(B_QEMPTY + st));
                             if (more) {
-                                ss_mmas(tmem + 128u, sV, sdO((gi + 1) % NST));  // dP^T(it+1)
+                                ss_mmas(utmem + 128u, sV, sdO((gi + 1) % NST));  // dP^T(it+1)
                                 umma_commit(BAR(B_DPFULL));
                                 if (it + 2 == NIT) umma_commit(BAR(B_VEMPTY));
                             }
@@ -419,7 +420,8 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     }
                     if (NIT > 0) ++kk;
                     gt += NIT;
-                    mbar_arrive(BAR(B_ITEMEMPTY + s));
+                    if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
+                    __syncwarp();
                 }
             }
         }

@@ -71,7 +71,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     constexpr int NSK = S::NSK;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
     const MaskArgs& mk = p.mask;
     const int nQ = mk.L.nQ;
@@ -292,18 +292,19 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             }
         } else {
             // ------------------------------ MMA issuers (warps 9, 10) ------------------------------
-            // Two issuing threads, so that the blocking tcgen05.mma issue and barrier round trips of
+            // Two issuing warps, so that the blocking tcgen05.mma issue and barrier round trips of
             // one stream do not delay the other:
             //   warp 9 : S(0), S(1); then per tile dQ(t) += dS K(t) followed by S(t+2) (which
-            //            overwrites dS(t): same thread, in order)
+            //            overwrites dS(t): same warp, in order)
             //   warp 10: dP(t+1) = dO V(t+1)^T as soon as dS(t) has been written (dP columns free)
             // Tiles are numbered across items (gi), so that the S buffers, the K ring, V and every
             // per-tile barrier simply carry on from one item to the next.
-            if (lane == 0) {
+            {
+                const uint32_t utmem = uniform(int(tmem));
                 constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
                 constexpr uint32_t idesc_dq = make_idesc(BF16, 128, D, false, true);
                 constexpr uint64_t desc_mn = desc_mn_major(S::BOX);
-                auto k_ready = [&](int gi) { return mbar_wait(BAR(B_KFULL + gi % NSK), (gi / NSK) & 1, ab, ST_WAIT_TIMEOUT + 24); };
+                auto k_ready = [&](int gi) { return mbar_wait_warp(BAR(B_KFULL + gi % NSK), (gi / NSK) & 1, ab, ST_WAIT_TIMEOUT + 24); };
                 auto ss_mmas = [&](uint32_t d, uint32_t a_tile, uint32_t b_tile) {
 #pragma unroll
                     for (int kk2 = 0; kk2 < D / 16; ++kk2) {
@@ -316,34 +317,34 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 int k = 0, kk = 0, gt = 0;
                 for (;; ++k) {
                     const int s = k & 1;
-                    ok = mbar_wait(BAR(B_ITEMFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 33);
+                    ok = mbar_wait_warp(BAR(B_ITEMFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 33);
                     if (!ok) break;
-                    const int T = info[s * 8 + 2];
-                    if (info[s * 8 + 3] < 0) break;
+                    const int T = uniform(info[s * 8 + 2]);
+                    if (uniform(info[s * 8 + 3]) < 0) break;
                     if (T > 0 && warp == 9) {
-                        ok = mbar_wait(BAR(B_QFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 23);
+                        ok = mbar_wait_warp(BAR(B_QFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 23);
                         const uint32_t q_tile = sQ(s);
                         for (int t = 0; t < 2 && t < T && ok; ++t) {
                             const int gi = gt + t;
                             ok = k_ready(gi);
                             if (ok) {
                                 tc_fence_after();
-                                ss_mmas(tmem + uint32_t(gi & 1) * 128u, q_tile, sK(gi % NSK));
+                                ss_mmas(utmem + uint32_t(gi & 1) * 128u, q_tile, sK(gi % NSK));
                                 umma_commit(BAR(B_SFULL + (gi & 1)));
                             }
                         }
                         // dQ(0) overwrites the accumulator: the previous item's epilogue must have read it
-                        if (ok && kk > 0) ok = mbar_wait(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 35);
+                        if (ok && kk > 0) ok = mbar_wait_warp(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 35);
                         for (int t = 0; t < T && ok; ++t) {
                             const int gi = gt + t, st = gi % NSK;
-                            ok = mbar_wait(BAR(B_DSFULL + (gi & 1)), (gi >> 1) & 1, ab, ST_WAIT_TIMEOUT + 26);
+                            ok = mbar_wait_warp(BAR(B_DSFULL + (gi & 1)), (gi >> 1) & 1, ab, ST_WAIT_TIMEOUT + 26);
                             if (!ok) break;
                             tc_fence_after();
-                            const uint32_t a = tmem + uint32_t(gi & 1) * 128u;
+                            const uint32_t a = utmem + uint32_t(gi & 1) * 128u;
 #pragma unroll
                             for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
                                 const uint32_t acol = (kk2 < 4) ? uint32_t(kk2) * 8u : 64u + uint32_t(kk2 - 4) * 8u;
-                                umma_ts(tmem + 384u, a + acol, smem_desc_at(desc_mn, sK(st) + uint32_t(kk2) * 2048u), idesc_dq,
+                                umma_ts(utmem + 384u, a + acol, smem_desc_at(desc_mn, sK(st) + uint32_t(kk2) * 2048u), idesc_dq,
                                         (t > 0 || kk2 > 0) ? 1u : 0u);
                             }
                             umma_commit(BAR(B_KEMPTY + st));
@@ -360,15 +361,15 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                         if (!ok) break;
                         umma_commit(BAR(B_DONE));
                     } else if (T > 0) {
-                        ok = mbar_wait(BAR(B_DOFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 23);
+                        ok = mbar_wait_warp(BAR(B_DOFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 23);
                         for (int t = 0; t < T && ok; ++t) {
                             const int gi = gt + t;
-                            ok = mbar_wait(BAR(B_VFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 25);
+                            ok = mbar_wait_warp(BAR(B_VFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 25);
                             // dP(gi) may overwrite the dP columns once every thread has read dP(gi-1)
-                            if (ok && gi > 0) ok = mbar_wait(BAR(B_DSFULL + ((gi - 1) & 1)), ((gi - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 26);
+                            if (ok && gi > 0) ok = mbar_wait_warp(BAR(B_DSFULL + ((gi - 1) & 1)), ((gi - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 26);
                             if (!ok) break;
                             tc_fence_after();
-                            ss_mmas(tmem + 256u, sdO, sV);
+                            ss_mmas(utmem + 256u, sdO, sV);
                             umma_commit(BAR(B_VEMPTY));
                             umma_commit(BAR(B_DPFULL));
                         }
@@ -377,7 +378,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     }
                     if (T > 0) ++kk;
                     gt += T;
-                    mbar_arrive(BAR(B_ITEMEMPTY + s));
+                    if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
+                    __syncwarp();
                 }
             }
         }

@@ -73,7 +73,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     constexpr int NS = S::NS;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
     const MaskArgs& mk = p.mask;
     const int nQ = mk.L.nQ;
@@ -303,33 +303,34 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             }
         } else {
             // ------------------------------ MMA issuers ------------------------------
-            // One issuing thread per softmax group: warp 9 owns the CTA's even visited tiles (S0 / O0),
+            // One issuing warp per softmax group: warp 9 owns the CTA's even visited tiles (S0 / O0),
             // warp 10 the odd ones (S1 / O1). The two chains touch disjoint TMEM and only share the
-            // K / V rings, so neither thread ever waits on the other group's softmax. Within a
+            // K / V rings, so neither warp ever waits on the other group's softmax. Within a
             // chain the MMAs of P*V(t) and S(t+2) are issued back to back (the tensor pipe accepts
             // only a few MMAs ahead and needs ~200 clocks to refill once drained): what S(t+2)
             // needs from TMA is waited for before P(t) is.
-            if (lane == 0) {
+            {
                 const int w = warp - 9;
+                const uint32_t utmem = uniform(int(tmem));
                 constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
                 constexpr uint32_t idesc_pv = make_idesc(BF16, 128, D, false, true);
                 constexpr uint64_t desc_v = desc_mn_major(S::BOX);
-                const uint32_t tS = tmem + uint32_t(w) * 128u;
-                const uint32_t tO = tmem + 256u + uint32_t(w) * uint32_t(D);
+                const uint32_t tS = utmem + uint32_t(w) * 128u;
+                const uint32_t tO = utmem + 256u + uint32_t(w) * uint32_t(D);
                 bool ok = true;
                 int k = 0, G = 0, cw = 0;  // cw: tiles this chain has finished (phases of its barriers)
                 int kkw = 0;               // items in which this chain had tiles (phase of its o_free barrier)
                 for (;; ++k) {
                     const int s = k & 1, use = k >> 1;
-                    ok = mbar_wait(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
+                    ok = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
                     if (!ok) break;
-                    const int T = info[s * 8 + 0];
-                    if (info[s * 8 + 2] < 0) break;
-                    ok = mbar_wait(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 3);
+                    const int T = uniform(info[s * 8 + 0]);
+                    if (uniform(info[s * 8 + 2]) < 0) break;
+                    ok = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 3);
                     if (!ok) break;
                     const uint32_t q_tile = sQ(s);
                     auto k_ready = [&](int g) {
-                        return mbar_wait(BAR(B_KFULL + (g % NS)), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 4);
+                        return mbar_wait_warp(BAR(B_KFULL + (g % NS)), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 4);
                     };
                     auto s_mmas = [&](int g) {
                         const int st = g % NS;
@@ -353,21 +354,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     for (int i = 0; i < nmine && ok; ++i, ++cw) {
                         const int g = G + t0 + 2 * i, st = g % NS;
                         const bool more = i + 1 < nmine;
-                        ok = mbar_wait(BAR(B_VFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 5);
+                        ok = mbar_wait_warp(BAR(B_VFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 5);
                         if (ok && more) ok = k_ready(g + 2);
                         // The first P*V of an item overwrites O: the epilogue of the previous item in which this
                         // chain had tiles must have read it. (The barrier counts those items only, on both
                         // sides: a chain without tiles in an item runs through it and must not find itself two
                         // phases behind, where a parity wait can no longer tell "not yet" from "done".)
-                        if (ok && i == 0 && kkw > 0) ok = mbar_wait(BAR(B_OFREE + w), (kkw - 1) & 1, ab, ST_WAIT_TIMEOUT + 14);
-                        if (ok) ok = mbar_wait(BAR(B_PHALF0 + w), cw & 1, ab, ST_WAIT_TIMEOUT + 6);
+                        if (ok && i == 0 && kkw > 0) ok = mbar_wait_warp(BAR(B_OFREE + w), (kkw - 1) & 1, ab, ST_WAIT_TIMEOUT + 14);
+                        if (ok) ok = mbar_wait_warp(BAR(B_PHALF0 + w), cw & 1, ab, ST_WAIT_TIMEOUT + 6);
                         if (!ok) break;
                         tc_fence_after();
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
                             umma_ts(tO, tS + uint32_t(kk) * 8u, smem_desc_at(desc_v, sV(st) + uint32_t(kk) * 2048u), idesc_pv,
                                     (i > 0 || kk > 0) ? 1u : 0u);
-                        ok = mbar_wait(BAR(B_PHALF1 + w), cw & 1, ab, ST_WAIT_TIMEOUT + 6);
+                        ok = mbar_wait_warp(BAR(B_PHALF1 + w), cw & 1, ab, ST_WAIT_TIMEOUT + 6);
                         if (!ok) break;
                         tc_fence_after();
 #pragma unroll
@@ -379,7 +380,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
                     G += T;
                     if (nmine > 0) ++kkw;
-                    if (ok) mbar_arrive(BAR(B_ITEMEMPTY + s));
+                    if (ok && lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
+                    __syncwarp();
                 }
             }
         }

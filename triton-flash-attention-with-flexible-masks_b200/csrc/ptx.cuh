@@ -101,6 +101,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const A
     }
 }
 
+// The same by all lanes of a converged warp: one answer for all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const Abort& ab, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, ab, code));
+}
+// A value that is the same in all lanes, in a form from which the compiler can tell.
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 // ----------------------------------------------------------------------------------------
 // TMA (bulk tensor copies; plain, never multicast)
 // ----------------------------------------------------------------------------------------
@@ -176,19 +183,29 @@ __device__ __forceinline__ void tc_wait_ld() {
 __device__ __forceinline__ void tc_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// arrive on an mbarrier once every tcgen05.mma issued so far by this thread has completed
+// The MMAs and their commits are issued by one elected lane (the same one each time) of a warp that runs the issuing code
+// converged, with uniform values: descriptors then stay in uniform registers. The same 8 SS + 8 TS MMAs of 128x128x16
+// issued inside a branch of one lane, beside eight warps of unrolled arithmetic: 150-210 clocks each, so 70-81, at 64
+// clocks of the pipe; with those warps idle both forms keep the pipe busy.
+// arrive on an mbarrier once every tcgen05.mma issued so far by the elected lane has completed
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
+    asm volatile(
+        "{\n\t"
+        ".reg .pred e;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "}\n" ::"r"(bar)
+        : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem]
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {
     asm volatile(
         "{\n\t"
-        ".reg .pred p;\n\t"
+        ".reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
         "}\n"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
@@ -198,9 +215,10 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
                                         uint32_t accumulate) {
     asm volatile(
         "{\n\t"
-        ".reg .pred p;\n\t"
+        ".reg .pred p, e;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
         "}\n"
         ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
