@@ -1,4 +1,5 @@
-"""Builds the CUDA library in-tree: csrc/*.cu -> flash_b200/libfa_b200.so (sm_100a only).
+"""Builds the CUDA library in-tree: csrc/*.cu -> flash_b200/libfa_b200.so (sm_100a only), and the native part of its
+torch binding on top of it: csrc/host.cpp -> flash_b200/_host.so.
 
 Usage: python build.py [--force]. nvcc cross-compiles without a GPU. The runtime is linked
 statically and the driver API is resolved at run time, so the library loads on a machine
@@ -8,10 +9,12 @@ import concurrent.futures
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "flash_b200", "libfa_b200.so")
+HOST_OUT = os.path.join(HERE, "flash_b200", "_host.so")
 OBJ_DIR = os.path.join(HERE, "build")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -67,7 +70,25 @@ def build(force=False, verbose=False):
                            capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_host(force)
     return OUT
+
+
+def _build_host(force):
+    src = os.path.join(CSRC, "host.cpp")
+    if not force and not _stale(HOST_OUT, [src, OUT] + _deps()):
+        return
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), cuda,
+               sysconfig.get_paths()["include"]]
+    r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", HOST_OUT, *("-I" + i for i in include),
+                        "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+                        "-L" + os.path.dirname(OUT), "-l:" + os.path.basename(OUT), "-Wl,-rpath,$ORIGIN"],
+                       capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
 
 
 if __name__ == "__main__":

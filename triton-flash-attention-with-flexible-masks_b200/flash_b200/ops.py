@@ -60,6 +60,11 @@ def _timed(name, kernels=1):
     return _UNTIMED if PROFILE is None else _Timed(name)
 
 
+def _count(kernels):
+    global LAUNCHES
+    LAUNCHES += kernels
+
+
 def _current(device):
     """A context in which `device` is the current one; nothing to do, and nothing paid, if it is already."""
     return _UNTIMED if torch.cuda.current_device() == device.index else torch.cuda.device(device)
@@ -177,72 +182,79 @@ def build_plan(prob, eq, ek, status):
     return plan
 
 
+def _host():
+    """The native host calls (csrc/host.cpp); no call runs without them."""
+    global _HOST
+    if _HOST is None:
+        _lib.load()
+        from . import _host as module
+        _HOST = module
+    return _HOST
+
+
+_HOST = None
+
+
 class FlashAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, sm_scale, eq, ek, score_func_mode, key_runs=None):
-        lib = _lib.load()
-        # checks of flash_triton.py:510-520
-        Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
-        assert Dq == Dk and Dk == Dv, "feature size of q, k, v should be equal"
-        assert Dk in {16, 32, 64, 128}
-        B, H, M, D = q.shape
-        N = k.shape[2]
-        Hk, Hv = k.shape[1], v.shape[1]
-        assert Hk == Hv, "num of heads in k and v should be equal"
-        assert H % Hk == 0, "number of heads in q must be a multiple of that in k & v"
-        num_groups = H // Hk
-        assert (N >= M) or (not causal), "KV length should be larger than M length in causal mode!"
-        MN_GAP = max(0, N - M)
-        # score mode (flash_triton.py:527-530)
-        assert (eq is None) == (ek is None)
-        if eq is None:
-            assert score_func_mode == SCORE_FUNC_MODE0_NOPE
-        assert score_func_mode in (SCORE_FUNC_MODE0_NOPE, SCORE_FUNC_MODE1_DOC)
-        if not q.is_cuda:
-            raise RuntimeError("flash_b200 runs on CUDA tensors only (there is no CPU implementation)")
-        device = q.device
-        if k.device != device or v.device != device or (eq is not None and (eq.device != device or ek.device != device)):
-            _same_device(q, k=k, v=v, eq=eq, ek=ek)
-        if k.dtype != q.dtype or v.dtype != q.dtype:
-            raise ValueError(f"flash_b200: q, k, v must share one dtype, got {q.dtype}, {k.dtype}, {v.dtype}")
-        if sm_scale is None:
-            sm_scale = 1. / math.sqrt(D)
-        if not sm_scale > 0:
-            raise NotImplementedError("flash_b200 needs sm_scale > 0")
-        q, k, v = maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v)
-        id_heads = 1
-        if score_func_mode == SCORE_FUNC_MODE1_DOC:
-            eq = _id_tensor(eq, B, H, M, "eq")
-            ek = _id_tensor(ek, B, H, N, "ek")
-            broadcast = (H == 1) or (eq.stride(1) == 0 and ek.stride(1) == 0)
-            id_heads = 1 if broadcast else H
-        with _current(device):
-            prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, id_heads, sm_scale)
-            status = _status_word(device)
+        host = _HOST or _host()
+        needs_grad = any(ctx.needs_input_grad[:3])
+        done, plan, id_heads = None, None, 1
+        if (eq is None and ek is None and score_func_mode == SCORE_FUNC_MODE0_NOPE and PROFILE is None and not _SYNC_STATUS
+                and (sm_scale is None or type(sm_scale) is float) and all(isinstance(x, torch.Tensor) for x in (q, k, v))):
+            status = _STATUS.get(q.get_device())
+            if status is not None:  # regular calls without ids and without need of a plan: one native call
+                done = host.forward(q, k, v, False, bool(causal), sm_scale, score_func_mode, 1, None, needs_grad, key_runs or 0, status)
+        if done is None:
+            # checks of flash_triton.py:510-520
+            Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
+            assert Dq == Dk and Dk == Dv, "feature size of q, k, v should be equal"
+            assert Dk in {16, 32, 64, 128}
+            B, H, M, D = q.shape
+            N = k.shape[2]
+            Hk, Hv = k.shape[1], v.shape[1]
+            assert Hk == Hv, "num of heads in k and v should be equal"
+            assert H % Hk == 0, "number of heads in q must be a multiple of that in k & v"
+            assert (N >= M) or (not causal), "KV length should be larger than M length in causal mode!"
+            # score mode (flash_triton.py:527-530)
+            assert (eq is None) == (ek is None)
+            if eq is None:
+                assert score_func_mode == SCORE_FUNC_MODE0_NOPE
+            assert score_func_mode in (SCORE_FUNC_MODE0_NOPE, SCORE_FUNC_MODE1_DOC)
+            if not q.is_cuda:
+                raise RuntimeError("flash_b200 runs on CUDA tensors only (there is no CPU implementation)")
+            device = q.device
+            if k.device != device or v.device != device or (eq is not None and (eq.device != device or ek.device != device)):
+                _same_device(q, k=k, v=v, eq=eq, ek=ek)
+            if k.dtype != q.dtype or v.dtype != q.dtype:
+                raise ValueError(f"flash_b200: q, k, v must share one dtype, got {q.dtype}, {k.dtype}, {v.dtype}")
+            if sm_scale is None:
+                sm_scale = 1. / math.sqrt(D)
+            if not sm_scale > 0:
+                raise NotImplementedError("flash_b200 needs sm_scale > 0")
+            q, k, v = maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v)
             if score_func_mode == SCORE_FUNC_MODE1_DOC:
-                plan = build_plan(prob, eq, ek, status)
-            elif lib.fa_plan_optional(prob, any(ctx.needs_input_grad[:3])):
-                plan = None  # so few items that counters would not pay
-            else:
-                plan = build_plan(prob, None, None, status)
-            Out = torch.empty_like(q)
-            if maybe_contiguous(Out) is not Out:
-                Out = torch.empty(q.shape, dtype=q.dtype, device=device)
-            L = torch.empty((B, H, (M + 127) // 128 * 128), device=device, dtype=torch.float32)
-            # calls that cannot fill the GPU cut their keys into runs
-            splits = key_runs or lib.fa_fwd_splits(prob)
-            work, work_ptr, work_bytes = None, None, 0
-            if splits > 1:
-                nbytes = ctypes.c_size_t(0)
-                _lib.check(lib.fa_fwd_workspace_bytes(prob, splits, ctypes.byref(nbytes)), "fa_fwd_workspace_bytes")
-                work = torch.empty(nbytes.value // 4, dtype=torch.float32, device=device)
-                work_ptr, work_bytes = work.data_ptr(), nbytes.value
-            with _timed("fwd", 2 if splits > 1 else 1):
-                _lib.check(lib.fa_fwd_split(prob, _tensor(q), _tensor(k), _tensor(v), _tensor(Out), L.data_ptr(),
-                                            plan.data_ptr() if plan is not None else None, splits, work_ptr, work_bytes,
-                                            status.data_ptr(), _stream()), "fa_fwd_split")
-            if _SYNC_STATUS:
-                check_status(q.device)
+                eq = _id_tensor(eq, B, H, M, "eq")
+                ek = _id_tensor(ek, B, H, N, "ek")
+                broadcast = (H == 1) or (eq.stride(1) == 0 and ek.stride(1) == 0)
+                id_heads = 1 if broadcast else H
+            with _current(device):
+                prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, id_heads, sm_scale)
+                status = _status_word(device)
+                if score_func_mode == SCORE_FUNC_MODE1_DOC:
+                    plan = build_plan(prob, eq, ek, status)
+                elif not _lib.load().fa_plan_optional(prob, needs_grad):  # else so few items that counters would not pay
+                    plan = build_plan(prob, None, None, status)
+                with _timed("fwd", 0):
+                    done = host.forward(q, k, v, True, bool(causal), float(sm_scale), score_func_mode, id_heads, plan, needs_grad,
+                                        key_runs or 0, status)
+                if done is None:
+                    raise RuntimeError("flash_b200: q, k, v are not plain [bs, H, L, D] CUDA tensors of matching shapes")
+                if _SYNC_STATUS:
+                    check_status(q.device)
+        Out, L, ctx.sm_scale, launched = done
+        _count(launched)
         # autograd context (flash_triton.py:558-562); eq/ek are kept for the saved-tensor contract,
         # the plan built from them is reused by backward
         if eq is None:
@@ -251,56 +263,62 @@ class FlashAttention(torch.autograd.Function):
             ctx.save_for_backward(q, k, v, Out, L, eq, ek)
         ctx.plan = plan
         ctx.id_heads = id_heads
-        ctx.sm_scale = sm_scale
         ctx.causal = causal
-        ctx.shapes = (B, H, M, D, N, Hk, num_groups, MN_GAP)
         ctx.score_func_info = (score_func_mode, )
         ctx.n_other = 5 if key_runs is None else 6  # inputs that are not q, k, v
         return Out
 
     @staticmethod
     def backward(ctx, do):
-        lib = _lib.load()
+        host = _HOST or _host()
         q, k, v, o, L = ctx.saved_tensors[:5]
-        sm_scale = ctx.sm_scale
-        causal = ctx.causal
-        B, H, M, D, N, Hk, num_groups, MN_GAP = ctx.shapes
         score_func_mode, = ctx.score_func_info
-        plan = ctx.plan
-        device = q.device
-        if do.device != device:
-            _same_device(q, do=do)
-        if do.dtype != q.dtype:
-            do = do.to(q.dtype)
-        do = maybe_contiguous(do)
-        with _current(device):
-            prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, ctx.id_heads, sm_scale)
-            status = _status_word(device)
-            stream = _stream()
-            plan_ptr = plan.data_ptr() if plan is not None else None
-            delta = torch.empty_like(L)
-            dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=device)
-            dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=device)
-            dq = torch.empty(q.shape, dtype=q.dtype, device=device)
-            tq, tk, tv, to, tdo = _tensor(q), _tensor(k), _tensor(v), _tensor(o), _tensor(do)
-            tdq, tdk, tdv = _tensor(dq), _tensor(dk), _tensor(dv)
-            lp, dp, sp = L.data_ptr(), delta.data_ptr(), status.data_ptr()
-            if PROFILE is None:  # the three kernels in one call
-                with _timed("bwd", 3):
-                    _lib.check(lib.fa_bwd(prob, tq, tk, tv, to, tdo, lp, dp, tdq, tdk, tdv, plan_ptr, sp, stream), "fa_bwd")
-            else:
-                # delta = rowsum(o * do) (flash_triton.py:584-592)
-                with _timed("delta"):
-                    _lib.check(lib.fa_bwd_delta(prob, to, tdo, dp, stream), "fa_bwd_delta")
-                # dk, dv (flash_triton.py:594-614, group sum of :635-637 done inside the kernel)
-                with _timed("dkdv"):
-                    _lib.check(lib.fa_bwd_dkdv(prob, tq, tk, tv, tdo, lp, dp, tdk, tdv, plan_ptr, sp, stream), "fa_bwd_dkdv")
-                # dq (flash_triton.py:616-634); every row is written by the kernel
-                with _timed("dq"):
-                    _lib.check(lib.fa_bwd_dq(prob, tq, tk, tv, tdo, lp, dp, tdq, plan_ptr, sp, stream), "fa_bwd_dq")
-            if _SYNC_STATUS:
-                check_status(q.device)
-        return (dq, dk, dv) + (None,) * ctx.n_other
+        device, plan = q.device, ctx.plan
+        rest = (bool(ctx.causal), ctx.sm_scale, score_func_mode, ctx.id_heads, plan, _status_word(device))
+        grads = None
+        if PROFILE is None:  # the three kernels in one call
+            grads = host.backward(do, q, k, v, o, L, False, *rest)
+        if grads is None:
+            if do.device != device:
+                _same_device(q, do=do)
+            if do.dtype != q.dtype:
+                do = do.to(q.dtype)
+            do = maybe_contiguous(do)
+            with _current(device):
+                grads = host.backward(do, q, k, v, o, L, True, *rest) if PROFILE is None else _backward_timed(do, q, k, v, o, L, *rest)
+                if grads is None:
+                    raise RuntimeError("flash_b200: the gradient is not a plain [bs, H, M, D] CUDA tensor")
+        if PROFILE is None:
+            _count(3)
+        if _SYNC_STATUS:
+            check_status(device)
+        return grads + (None,) * ctx.n_other
+
+
+def _backward_timed(do, q, k, v, o, L, causal, sm_scale, score_func_mode, id_heads, plan, status):
+    """The backward with its kernels launched, and timed, one by one."""
+    lib = _lib.load()
+    (B, H, M, D), (Hk, N) = q.shape, k.shape[1:3]
+    prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, id_heads, sm_scale)
+    stream = _stream()
+    plan_ptr = plan.data_ptr() if plan is not None else None
+    delta = torch.empty_like(L)
+    dk = torch.empty((B, Hk, N, D), dtype=k.dtype, device=q.device)
+    dv = torch.empty((B, Hk, N, D), dtype=v.dtype, device=q.device)
+    dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    tq, tk, tv, to, tdo = _tensor(q), _tensor(k), _tensor(v), _tensor(o), _tensor(do)
+    tdq, tdk, tdv = _tensor(dq), _tensor(dk), _tensor(dv)
+    lp, dp, sp = L.data_ptr(), delta.data_ptr(), status.data_ptr()
+    # delta = rowsum(o * do) (flash_triton.py:584-592)
+    with _timed("delta"):
+        _lib.check(lib.fa_bwd_delta(prob, to, tdo, dp, stream), "fa_bwd_delta")
+    # dk, dv (flash_triton.py:594-614, group sum of :635-637 done inside the kernel)
+    with _timed("dkdv"):
+        _lib.check(lib.fa_bwd_dkdv(prob, tq, tk, tv, tdo, lp, dp, tdk, tdv, plan_ptr, sp, stream), "fa_bwd_dkdv")
+    # dq (flash_triton.py:616-634); every row is written by the kernel
+    with _timed("dq"):
+        _lib.check(lib.fa_bwd_dq(prob, tq, tk, tv, tdo, lp, dp, tdq, plan_ptr, sp, stream), "fa_bwd_dq")
+    return dq, dk, dv
 
 
 # Without a causal mask the order of the queries is free. When the query ids are not grouped (every
