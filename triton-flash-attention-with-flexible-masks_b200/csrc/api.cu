@@ -21,7 +21,7 @@ cudaError_t launch_bwd_dq(int, bool, const CUtensorMap&, const CUtensorMap&, con
                           const CUtensorMap&, const CUtensorMap&, const DqParams&, int, bool, cudaStream_t);
 
 // fp32 path (attn_f32.cu)
-cudaError_t launch_f32(int which, int D, const F32Params& p, cudaStream_t stream);
+cudaError_t launch_f32(int which, int D, const F32Params& p, bool overlap, cudaStream_t stream);
 }  // namespace fa
 
 namespace {
@@ -267,7 +267,7 @@ size_t fwd_workspace_bytes(const fa_problem* p, int ns) {
 // fp32 inputs: which = 0 forward, 1 delta, 2 dK / dV, 3 dQ; absent tensors are null
 int run_f32(int which, const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
             const fa_tensor* d_o, const fa_tensor* dq, const fa_tensor* dk, const fa_tensor* dv, float* lse, float* delta,
-            const void* plan, void* stream) {
+            const void* plan, void* stream, bool overlap = false) {
     int rc;
     fa::F32Params fp{};
     const struct { const fa_tensor* t; fa::F32Tensor* dst; int H, L; } all[8] = {
@@ -285,7 +285,7 @@ int run_f32(int which, const fa_problem* p, const fa_tensor* q, const fa_tensor*
     fp.delta = delta;
     fp.B = p->B; fp.H = p->H; fp.Hk = p->Hk; fp.G = p->H / p->Hk;
     fp.scale = p->sm_scale;
-    return fa::launch_f32(which, p->D, fp, static_cast<cudaStream_t>(stream)) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+    return fa::launch_f32(which, p->D, fp, overlap, static_cast<cudaStream_t>(stream)) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 
 int run_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* d_o,
@@ -296,7 +296,7 @@ int run_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, cons
     if (!lse || !delta || !status) return FA_ERR_BAD_ARG;
     if (!aligned16(lse) || !aligned16(delta)) return FA_ERR_ALIGNMENT;  // read with bulk copies
     if (p->dtype == FA_FP32)
-        return run_f32(3, p, q, k, v, nullptr, d_o, dq, nullptr, nullptr, const_cast<float*>(lse), const_cast<float*>(delta), plan, stream);
+        return run_f32(3, p, q, k, v, nullptr, d_o, dq, nullptr, nullptr, const_cast<float*>(lse), const_cast<float*>(delta), plan, stream, overlap);
     if ((rc = check_tensor(q, p->B, p->H, p->M))) return rc;
     if ((rc = check_tensor(d_o, p->B, p->H, p->M))) return rc;
     if ((rc = check_tensor(dq, p->B, p->H, p->M))) return rc;

@@ -379,6 +379,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dq_kernel(const F32Params
 #pragma unroll
     for (int r = 0; r < 4; ++r)
         if (i0 + r0 + r < mk.M) Own<D>::store(dqbase + int64_t(i0 + r0 + r) * p.dq.sl, x, dqvec, acc[r], p.scale);  // flash_triton.py:425
+    wait_prerequisites();  // what follows in the stream finds dK / dV complete too
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -389,6 +390,7 @@ template <int D>
 __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Params p) {
     using S = F32Smem<D>;
     extern __shared__ __align__(16) float sm[];
+    launch_dependents();  // fa_bwd's dQ kernel reads nothing that this one writes
     float* Ks = sm;
     float* Vs = Ks + S::rows;
     float* QDs = Vs + S::rows;            // two stages of Q, dO
@@ -492,7 +494,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Para
 
 // ---------------------------------------------------------------------------------------------
 template <int D>
-static cudaError_t launch_f32_t(int which, const F32Params& p, cudaStream_t stream) {
+static cudaError_t launch_f32_t(int which, const F32Params& p, bool overlap, cudaStream_t stream) {
     using S = F32Smem<D>;
     const MaskArgs& mk = p.mask;
     constexpr int fwd_smem = (S::rows + 4 * S::cols + S::p + 2 * kC) * 4;
@@ -502,6 +504,7 @@ static cudaError_t launch_f32_t(int which, const F32Params& p, cudaStream_t stre
     auto run = [&](auto kern, int smem, int rows, int heads) {
         const cudaError_t e = allow_smem(kern, smem, allowed[which]);
         if (e != cudaSuccess) return e;
+        if (overlap) return launch_overlapping(kern, dim3(cdiv(rows, kR), heads, p.B), kF32Threads, smem, stream, p);
         kern<<<dim3(cdiv(rows, kR), heads, p.B), kF32Threads, smem, stream>>>(p);
         return cudaGetLastError();
     };
@@ -512,13 +515,17 @@ static cudaError_t launch_f32_t(int which, const F32Params& p, cudaStream_t stre
     return cudaGetLastError();
 }
 
-// which: 0 forward, 1 delta, 2 dK / dV, 3 dQ
-cudaError_t launch_f32(int which, int D, const F32Params& p, cudaStream_t stream) {
+// which: 0 forward, 1 delta, 2 dK / dV, 3 dQ. overlap: the launch directly before this one in the stream is the dK/dV
+// kernel of the same backward, and the blocks of this one (dQ) may run beside its: two fit on an SM up to D = 64, and
+// one alone leaves its FMA pipes idle most of the time. Whole backward, us, before and now: 8 heads x 512 x 64 causal 104,
+// 82; 8 heads x 1024 283, 223; 32 heads x 1024 694, 634; 2 heads x 100 36, 22; D = 128, 8 heads x 512, 160, 136 (there dQ only
+// starts on SMs that are free); 128 / 32 heads of 777 queries against 1024 keys, where dK/dV fills the GPU, 3291, 3222.
+cudaError_t launch_f32(int which, int D, const F32Params& p, bool overlap, cudaStream_t stream) {
     switch (D) {
-        case 16: return launch_f32_t<16>(which, p, stream);
-        case 32: return launch_f32_t<32>(which, p, stream);
-        case 64: return launch_f32_t<64>(which, p, stream);
-        case 128: return launch_f32_t<128>(which, p, stream);
+        case 16: return launch_f32_t<16>(which, p, overlap, stream);
+        case 32: return launch_f32_t<32>(which, p, overlap, stream);
+        case 64: return launch_f32_t<64>(which, p, overlap, stream);
+        case 128: return launch_f32_t<128>(which, p, overlap, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -588,17 +588,7 @@ static cudaError_t launch_dq_t(const CUtensorMap& tq, const CUtensorMap& tk, con
         kern<<<grid, kAttnThreads, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
         return cudaGetLastError();
     }
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kAttnThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, tdq, p);
+    return launch_overlapping(kern, dim3(grid), kAttnThreads, smem, stream, tq, tk, tv, tdo, tdq, p);
 }
 
 

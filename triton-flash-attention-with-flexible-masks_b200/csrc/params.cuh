@@ -102,20 +102,21 @@ inline cudaError_t allow_smem(Kernel kern, int bytes, SmemAllowed& allowed) {
     return e;
 }
 
-// Ordered compaction of per-tile flags (list[i] = flags of tile lo+i) into the visited list:
-// entry = (i) | flags << 10. One warp; returns the number of visited tiles.
-__device__ __forceinline__ int compact_visit_list(uint16_t* list, int n, int lane) {
-    int T = 0;
-    for (int base = 0; base < n; base += 32) {
-        const int i = base + lane;
-        const uint32_t f = (i < n) ? list[i] : 0u;
-        const uint32_t m = __ballot_sync(0xffffffffu, (f & TILE_VISIT) != 0);
-        __syncwarp();
-        if (f & TILE_VISIT) list[T + __popc(m & ((1u << lane) - 1u))] = uint16_t(uint32_t(i) | (f << 10));
-        T += __popc(m);
-        __syncwarp();
-    }
-    return T;
+// Launches `kern` so that it may start on SMs that the kernel before it in the stream has left, or leaves room on, once
+// all of that one's blocks have called launch_dependents(). `kern` ends with wait_prerequisites().
+template <class... Args>
+inline cudaError_t launch_overlapping(void (*kern)(Args...), dim3 grid, int threads, int smem, cudaStream_t stream, const Args&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 }  // namespace fa
