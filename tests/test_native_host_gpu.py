@@ -1,0 +1,63 @@
+"""The native host call takes regular calls; every other form takes the general path to the same kernels and the same bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def layouts(x):
+    B, H, L, D = x.shape
+    yield "contiguous", x.clone()
+    yield "transposed", x.transpose(1, 2).contiguous().transpose(1, 2)
+    wide = torch.zeros(B, H, L, 2 * D, dtype=x.dtype, device=x.device)
+    wide[..., ::2] = x
+    yield "last stride 2", wide[..., ::2]
+    odd = torch.zeros(x.numel() + 1, dtype=x.dtype, device=x.device)
+    odd[1:] = x.reshape(-1)
+    yield "odd rows", torch.cat([x, x[..., :4]], 3)[..., :D]
+    if x.dtype == torch.float32:  # 16-bit tensors of this kind are refused by the library, as before
+        yield "odd base", odd[1:].view(B, H, L, D)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_layouts_give_the_same_bits(dtype, mode):
+    import flash_b200 as fb
+    B, H, Hk, L, D = 2, 4, 2, 200, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, do = (torch.randn(B, h, L, D, generator=g, device="cuda").to(dtype) for h in (H, Hk, Hk, H))
+    ids = (-1 - torch.arange(L, device="cuda") // 70).expand(B, H, L) if mode else None
+
+    def step(q, k, v, do):
+        q, k, v = (x.detach().requires_grad_() for x in (q, k, v))
+        o = fb.attention(q, k, v, True, None, ids, ids, mode)
+        return (o.detach(), *torch.autograd.grad(o, (q, k, v), do))
+
+    want = step(q, k, v, do)
+    for (name, a), (_, b), (_, c), (_, d) in zip(*(layouts(x) for x in (q, k, v, do))):
+        for args in ((a, b, c, do), (q, k, v, d)):
+            for x, y in zip(step(*args), want):
+                assert torch.equal(x, y), name
+    # an expanded gradient
+    one = torch.ones((), dtype=dtype, device="cuda").expand(B, H, L, D)
+    assert all(torch.equal(x, y) for x, y in zip(step(q, k, v, one), step(q, k, v, one.contiguous())))
+
+
+def test_autograd_forms():
+    import flash_b200 as fb
+    q, k, v = (torch.randn(1, 2, 64, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t, lambda t: t):
+        o = fb.attention(q, k, v, True)
+    assert len(packed) == 5 and o.grad_fn.name() == "FlashAttentionBackward"
+    o.sum().backward()
+    with pytest.raises(RuntimeError):  # buffers freed
+        o.sum().backward()
+    with torch.no_grad():
+        assert not fb.attention(q, k, v, True).requires_grad
+    with pytest.raises(RuntimeError):  # no vmap rule
+        torch.vmap(lambda x: fb.attention(x, x, x, True))(torch.randn(2, 1, 2, 64, 64, device="cuda", dtype=torch.bfloat16))
+    with pytest.raises(NotImplementedError):
+        fb.attention(q, k, v, True, 0.0)
+    with pytest.raises(AssertionError):
+        fb.attention(q, k[:, :, :32], v[:, :, :32], True)
