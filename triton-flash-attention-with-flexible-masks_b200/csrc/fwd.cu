@@ -7,22 +7,29 @@
 // Persistent: one CTA per SM walks work items (one item = one block of 128 queries of one
 // (batch, head)); items are handed out in an order that puts the query blocks of
 // all heads side by side, so that the CTAs of one round carry almost equal work. With document
-// masks most items hold only a few tiles, so everything around the tiles is overlapped with the
-// neighbouring items: a scheduler warp prepares the next item's tile list, the producer prefetches
-// its Q / K / V, and the output tile leaves through an asynchronous TMA store.
+// masks most items hold only a few tiles, so nothing waits at the border of two items: every role walks the items at
+// its own pace, up to NQ of them apart.
 //
-// 12 warps:
+// 16 warps:
 //   warps 0-3  softmax group 0, warps 4-7 softmax group 1 (thread r of a group owns row r)
-//   warp 8     TMA producer (Q per item, K and V rings that run across items)
-//   warps 9,10 tcgen05.mma issuers, one per softmax group; warp 9 owns the TMEM allocation
-//   warp 11    item scheduler: decodes the item, classifies its candidate tiles from the mask plan
-//              and compacts the visited ones into a list in shared memory (two item slots)
-// Visited key tiles alternate between the two groups: the CTA's g-th tile (counted across its items)
-// uses score buffer S[g&1] and accumulates into O[g&1] with the group's own running max / sum for
-// the item; the two partial results are merged in the item's epilogue, the chain of the item's even
-// tiles first, so that the result does not depend on which group that was. Counting across items
-// keeps every K / V ring slot (slot g % NS, NS even) with one issuer, which waits for each of
-// its phases in turn, and lets consecutive one-tile items overlap on the two chains. TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
+//   warps 8-11 epilogue group: normalises a finished item's O, stages it and stores it
+//   warp 12    TMA producer (Q per item, K and V rings that run across items; K ahead of V)
+//   warps 13,15 tcgen05.mma issuers, of P*V and of S; warp 13 owns the TMEM allocation
+//   warp 14    item scheduler: decodes the item, classifies its candidate tiles from the mask plan
+//              and compacts the visited ones into a list in shared memory (NQ item slots)
+// The CTA's g-th visited tile (counted across its items) belongs to softmax group g & 1 and uses score buffer g % 3;
+// all tiles of an item accumulate into one O. The groups share the row's reference maximum (it is handed from tile to
+// tile through shared memory, so P of every tile is relative to the same one), and each keeps the sum of its own tiles,
+// so the result does not depend on which group had the even ones. With three score buffers S(g+3) follows P*V(g)
+// on the pipe, a tile before a group asks for it: a group goes from one tile's exponentials straight to the next tile's scores.
+// (Before, each group had an O and a maximum of its own and one score buffer, waited for its own P*V and S between two
+// tiles, and drained O itself. Forward kernel, us, before and now: 512 queries against 8192 keys, 32 / 8 heads of 128, 63.6,
+// 59.5; 2 x 32 / 8 x 3001 x 128 causal 164, 153; 16 x 8 x 577 x 32 39.2, 35.1; 4 x 16 x 4096 x 128 in documents 153, 147;
+// 32 x 32768 x 128 in 64 documents 885, 848; 16 x 32 x 8192 x 128 causal 9185, 8370; 4 x 12 x 1000 x 64 in documents 27.2,
+// 27.1; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 84.7, 85.7: there the masks bound it.)
+// What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group: 2800 clocks
+// for two tiles) and, in dense calls, the clock under the power cap (1.4-1.5 GHz).
+// TMEM columns: S [0,384), three of 128; O [384,512), two of 64 for D = 64 (consecutive items), one of 128 for D = 128.
 // P (input dtype, two values per column) overwrites the first 64 columns of its S buffer.
 #include <type_traits>
 #include "common.cuh"
@@ -30,30 +37,33 @@
 
 namespace fa {
 
-constexpr int kTurnMinTiles = 8;  // items with fewer visited tiles do not serialise their exp phases
-
 template <int D>
 struct FwdSmem {
     static constexpr int NS = (D == 128) ? 2 : 4;  // depth of the K ring and of the V ring
+    // item slots; with more, items are dealt out too far ahead (3 or 4 for D = 64: 8 x 8 x 1024 x 8192 in documents 90, 86 with 2)
+    static constexpr int NQ = 2;
+    static constexpr int NO = 128 / D;             // O accumulators
     static constexpr int TILE = kBlk * D * 2;
     static constexpr int BOX = kBlk * 64 * 2;
     static constexpr int NBOX = D / 64;
     static constexpr int NKC = 8;  // depth of the key-code ring
-    static constexpr int off_q = 0;  // two Q tiles; a slot also stages its item's O tile for the TMA store
-    static constexpr int off_k = 2 * TILE;
+    static constexpr int off_q = 0;  // NQ Q tiles; a slot also stages its item's O tile for the TMA store
+    static constexpr int off_k = NQ * TILE;
     static constexpr int off_v = off_k + NS * TILE;
-    static constexpr int off_list = off_v + NS * TILE;         // uint16 [2][kListCap]
-    static constexpr int off_qc = off_list + 2 * kListCap * 2;  // int32  [2][128] query codes
-    static constexpr int off_kc = off_qc + 2 * kBlk * 4;        // int32  [NKC][128] key codes, loaded with K on K's barrier
-    static constexpr int off_ml = off_kc + NKC * kBlk * 4;      // float  [2][2 groups][m, l][128]
-    static constexpr int off_info = off_ml + 2 * 2 * 2 * kBlk * 4;  // int32 [2][8]: T, lo, item (-1: no more items), -, query block, head, batch
-    static constexpr int off_bar = off_info + 64;
-    // item_full[2] item_empty[2] q_full[2] o_staged[2] k_full[NS] k_empty[NS] v_full[NS] v_empty[NS]
-    // s_full[2] p_half0[2] p_half1[2] pv_done[2] turn[2] o_free[2] ml_full
-    static constexpr int n_bar = 8 + 4 * NS + 12 + 1;
+    static constexpr int off_list = off_v + NS * TILE;           // uint16 [NQ][kListCap]
+    static constexpr int off_qc = off_list + NQ * kListCap * 2;  // int32  [NQ][128] query codes
+    static constexpr int off_kc = off_qc + NQ * kBlk * 4;        // int32  [NKC][128] key codes, loaded with K on K's barrier
+    static constexpr int off_ml = off_kc + NKC * kBlk * 4;       // float  [NQ][2 groups][m, l][128]
+    static constexpr int off_m = off_ml + NQ * 4 * kBlk * 4;     // float  [128] the rows' reference maximum
+    static constexpr int off_info = off_m + kBlk * 4;  // int32 [NQ][8]: T, lo, item (-1: no more items), kv head, query block, head, batch
+    static constexpr int off_bar = off_info + NQ * 32;
+    // item_full[NQ] item_empty[NQ] q_full[NQ] q_empty[NQ] ml_full[NQ] staged[NQ] k_full[NS] k_empty[NS] v_full[NS] v_empty[NS]
+    // s_full[3] p_full[3] pv_done[3] m_ready[2] o_full[NO] o_free[NO]
+    static constexpr int n_bar = 6 * NQ + 4 * NS + 9 + 2 + 2 * NO;
     static constexpr int off_misc = off_bar + n_bar * 8;  // tmem slot, abort flag
     static constexpr int total = off_misc + 16;
 };
+static_assert(FwdSmem<128>::total <= 232448 && FwdSmem<64>::total <= 232448, "shared memory budget");
 
 // SHORT: calls without ids whose items are too few or too empty for one item per (query block, head, batch).
 // Two things are added (fwd_pack and fwd_splits in api.cu say when):
@@ -66,11 +76,11 @@ struct FwdSmem {
 // Such calls are bound by reading K and V (16 tokens of 32 / 8 heads of 128 against 4500 keys: 295 MB, 45 us at the
 // copy rate; 171 us with a tile per head, 63 us packed) or, with few heads, by the longest item's chain of tiles.
 template <int D, bool BF16, bool SHORT>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+__global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdParams p) {
     using S = FwdSmem<D>;
-    constexpr int NS = S::NS;
+    constexpr int NS = S::NS, NQ = S::NQ, NO = S::NO;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -88,35 +98,44 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     volatile int* info = reinterpret_cast<volatile int*>(smem + S::off_info);
     const uint32_t bar0 = sbase + S::off_bar;
     auto BAR = [&](int i) { return bar0 + 8u * uint32_t(i); };
-    constexpr int B_ITEMFULL = 0, B_ITEMEMPTY = 2, B_QFULL = 4, B_OSTAGED = 6, B_KFULL = 8, B_KEMPTY = 8 + NS,
-                  B_VFULL = 8 + 2 * NS, B_VEMPTY = 8 + 3 * NS, B_SFULL = 8 + 4 * NS, B_PHALF0 = B_SFULL + 2,
-                  B_PHALF1 = B_SFULL + 4, B_PVDONE = B_SFULL + 6, B_TURN = B_SFULL + 8, B_OFREE = B_SFULL + 10, B_MLFULL = B_SFULL + 12;
+    constexpr int B_ITEMFULL = 0, B_ITEMEMPTY = NQ, B_QFULL = 2 * NQ, B_QEMPTY = 3 * NQ, B_MLFULL = 4 * NQ, B_STAGED = 5 * NQ, B_KFULL = 6 * NQ,
+                  B_KEMPTY = B_KFULL + NS, B_VFULL = B_KEMPTY + NS, B_VEMPTY = B_VFULL + NS, B_SFULL = B_VEMPTY + NS,
+                  B_PFULL = B_SFULL + 3, B_PVDONE = B_PFULL + 3, B_MREADY = B_PVDONE + 3, B_OFULL = B_MREADY + 2,
+                  B_OFREE = B_OFULL + NO;
+    static_assert(B_OFREE + NO == S::n_bar, "barriers");
     Abort ab{misc + 1, p.status, p.wait_limit};
 
     if (tid == 0) {
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < NQ; ++s) {
             mbar_init(BAR(B_ITEMFULL + s), 1);
-            mbar_init(BAR(B_ITEMEMPTY + s), 5);  // producer, two MMA issuers, one thread of each softmax group
+            mbar_init(BAR(B_ITEMEMPTY + s), 15);  // producer, two MMA issuers, eight softmax warps, four epilogue warps
             mbar_init(BAR(B_QFULL + s), 1);
-            mbar_init(BAR(B_OSTAGED + s), 256);
-            mbar_init(BAR(B_SFULL + s), 1);
-            mbar_init(BAR(B_PHALF0 + s), 128);
-            mbar_init(BAR(B_PHALF1 + s), 128);
-            mbar_init(BAR(B_PVDONE + s), 1);
-            mbar_init(BAR(B_TURN + s), 128);
-            mbar_init(BAR(B_OFREE + s), 256);
+            mbar_init(BAR(B_QEMPTY + s), 1);
+            mbar_init(BAR(B_MLFULL + s), 8);
+            mbar_init(BAR(B_STAGED + s), 4);
         }
-        mbar_init(BAR(B_MLFULL), 256);
         for (int s = 0; s < NS; ++s) {
             mbar_init(BAR(B_KFULL + s), 1);
             mbar_init(BAR(B_KEMPTY + s), 1);
             mbar_init(BAR(B_VFULL + s), 1);
             mbar_init(BAR(B_VEMPTY + s), 1);
         }
+        for (int s = 0; s < 3; ++s) {
+            mbar_init(BAR(B_SFULL + s), 1);
+            mbar_init(BAR(B_PFULL + s), 4);  // here and below: one arrival a warp
+            mbar_init(BAR(B_PVDONE + s), 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(BAR(B_MREADY + s), 4);
+        }
+        for (int s = 0; s < NO; ++s) {
+            mbar_init(BAR(B_OFULL + s), 1);
+            mbar_init(BAR(B_OFREE + s), 4);
+        }
         misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
         fence_mbar_init();
     }
-    if (warp == 9) {
+    if (warp == 13) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
     }
@@ -151,20 +170,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         qb = p.by_length ? mk.plan[mk.L.off_ordq + (int64_t(b) * mk.He + (mk.He == 1 ? 0 : h)) * nQ + pos] : nQ - 1 - pos;
     };
 
-    if (warp >= 8) {
-        setmaxnreg_dec<72>();
+    if (warp >= 12) {
+        setmaxnreg_dec<kFwdServiceRegs>();
         if (aborted) {
             // a previous kernel reported an error: do nothing
-        } else if (warp == 11) {
+        } else if (warp == 14) {
             // ------------------------------ item scheduler ------------------------------
             // Items are handed out in order from a counter in the plan (any CTA takes the next one: the
             // work per item varies with the mask); without counters (no plan given) they are
             // dealt out round robin in alternating direction, which evens out their sorted lengths.
             bool ok = true;
             for (int k = 0;; ++k) {
-                const int s = k & 1, use = k >> 1;
-                if (use > 0) ok = mbar_wait(BAR(B_ITEMEMPTY + s), (use - 1) & 1, ab, ST_WAIT_TIMEOUT + 11);
-                ok = __all_sync(0xffffffffu, ok);
+                const int s = k % NQ, use = k / NQ;
+                if (use > 0) ok = mbar_wait_warp(BAR(B_ITEMEMPTY + s), (use - 1) & 1, ab, ST_WAIT_TIMEOUT + 11);
                 if (!ok) break;
                 int j = 0;
                 if (lane == 0) {
@@ -210,6 +228,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     info[s * 8 + 0] = T;
                     info[s * 8 + 1] = lo;
                     info[s * 8 + 2] = j;
+                    info[s * 8 + 3] = SHORT ? h / nG : h / p.G;
                     info[s * 8 + 4] = qb;
                     info[s * 8 + 5] = h;
                     info[s * 8 + 6] = b;
@@ -217,240 +236,325 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 __syncwarp();
                 if (lane == 0) mbar_arrive(BAR(B_ITEMFULL + s));
             }
-        } else if (warp == 8) {
+        } else if (warp == 12) {
             // ------------------------------ TMA producer ------------------------------
-            if (lane == 0) {
-                tma_prefetch_desc(&tmQ);
-                tma_prefetch_desc(&tmK);
-                tma_prefetch_desc(&tmV);
-                bool ok = true;
-                int k = 0, G = 0;  // G: tiles of all earlier items (the K / V rings run across items)
-                // TMA store of the O tile the softmax groups staged in slot (kk & 1) for item kk
-                int item_qb[2] = {0, 0}, item_h[2] = {0, 0}, item_b[2] = {0, 0};  // the items in the two slots
-                auto store_o = [&](int kk) {
-                    const int s = kk & 1;
-                    if (!mbar_wait(BAR(B_OSTAGED + s), (kk >> 1) & 1, ab, ST_WAIT_TIMEOUT + 13)) return false;
-                    const int qb = item_qb[s], h = item_h[s], b = item_b[s];
+            // Two walks over the CTA's tiles: K (with its item's Q), up to kAhead tiles ahead of V. Into the next item K
+            // only goes ahead while its slot is free at once, so that the V tiles of the item at hand never wait for it.
+            // The warp runs converged with uniform values (one lane with its numbers in vector registers took 950 clocks
+            // from a load to the next, more than half a tile's time).
+            tma_prefetch_desc(&tmQ);
+            tma_prefetch_desc(&tmK);
+            tma_prefetch_desc(&tmV);
+            constexpr int kAhead = 3;
+            bool ok = true, last = false;  // last: the K walk has seen the end marker
+            int kk = -1, kt = 0, kT = 0, gk = 0, klo = 0, khk = 0, kb = 0, khe = 0;  // K walk: item, its next tile and tiles; tiles issued
+            int vk = -1, vt = 0, vT = 0, gv = 0, vlo = 0, vhk = 0, vb = 0;           // V walk
+            while (ok) {
+                while (vt == vT && vk < kk) {  // the V walk goes on to the next item
+                    if (vk >= 0 && lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + vk % NQ));
+                    ++vk;
+                    const int s = vk % NQ;
+                    vt = 0;
+                    vT = uniform(info[s * 8 + 0]);
+                    vlo = uniform(info[s * 8 + 1]);
+                    vhk = uniform(info[s * 8 + 3]);
+                    vb = uniform(info[s * 8 + 6]);
+                }
+                if (last && gv == gk) break;
+                bool do_k = !last && gk - gv < kAhead;
+                if (do_k && kt == kT) {  // the next item: its slot's last O must have left
+                    const int s = (kk + 1) % NQ, use = (kk + 1) / NQ;
+                    if (gv < gk && !(mbar_test_warp(BAR(B_ITEMFULL + s), use & 1) &&
+                                     (use == 0 || mbar_test_warp(BAR(B_QEMPTY + s), (use - 1) & 1)))) {
+                        do_k = false;
+                    } else {
+                        ok = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
+                        if (!ok) break;
+                        if (uniform(info[s * 8 + 2]) < 0) {
+                            last = true;
+                            continue;
+                        }
+                        if (use > 0) ok = mbar_wait_warp(BAR(B_QEMPTY + s), (use - 1) & 1, ab, ST_WAIT_TIMEOUT + 13);
+                        if (!ok) break;
+                        ++kk;
+                        kt = 0;
+                        kT = uniform(info[s * 8 + 0]);
+                        klo = uniform(info[s * 8 + 1]);
+                        khk = uniform(info[s * 8 + 3]);
+                        const int qb = uniform(info[s * 8 + 4]), h = uniform(info[s * 8 + 5]);
+                        kb = uniform(info[s * 8 + 6]);
+                        khe = (mk.He == 1) ? 0 : h;
+                        if constexpr (SHORT) {
+                            mbar_expect_tx_elect(BAR(B_QFULL + s), uint32_t(p.rows) * 128u * S::NBOX);
+                            for (int x = 0; x < S::NBOX; ++x)
+                                tma_load_5d_elect(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, (h % nG) * p.pack, khk, kb);
+                        } else {
+                            mbar_expect_tx_elect(BAR(B_QFULL + s), S::TILE);
+                            for (int x = 0; x < S::NBOX; ++x)
+                                tma_load_4d_elect(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, h, kb);
+                        }
+                        continue;  // (an item may have no tiles)
+                    }
+                }
+                if (do_k) {
+                    const int blk = klo + uniform(list_of(kk % NQ)[kt] & 1023), st = gk % NS, ug = gk / NS;
+                    if (ug > 0) ok = mbar_wait_warp(BAR(B_KEMPTY + st), (ug - 1) & 1, ab, ST_WAIT_TIMEOUT + 1);
+                    if (!ok) break;
+                    // The tile's key codes travel with K: they land in a ring of NKC slots and complete on
+                    // K's barrier, so whoever has seen S(g) (computed after that barrier) may read them.
+                    // Slot g % NKC was last read by the softmax of tile g - NKC, which is over: S(g - NS), which
+                    // has just released K's stage, was issued behind P*V(g - NS - 3).
+                    static_assert(S::NKC >= NS + 3, "key-code ring");
+                    mbar_expect_tx_elect(BAR(B_KFULL + st), S::TILE + (mk.mode == 1 ? kBlk * 4 : 0));
+                    for (int x = 0; x < S::NBOX; ++x)
+                        tma_load_4d_elect(sK(st) + x * S::BOX, &tmK, BAR(B_KFULL + st), x * 64, blk * kBlk, khk, kb);
+                    if (mk.mode == 1)
+                        bulk_load_1d_elect(sbase + S::off_kc + (gk % S::NKC) * (kBlk * 4),
+                                           mk.plan + mk.L.off_kc + (int64_t(kb) * mk.He + khe) * mk.L.Npad + int64_t(blk) * kBlk,
+                                           kBlk * 4, BAR(B_KFULL + st));
+                    ++kt;
+                    ++gk;
+                } else {
+                    const int blk = vlo + uniform(list_of(vk % NQ)[vt] & 1023), st = gv % NS, ug = gv / NS;
+                    if (ug > 0) ok = mbar_wait_warp(BAR(B_VEMPTY + st), (ug - 1) & 1, ab, ST_WAIT_TIMEOUT + 2);
+                    if (!ok) break;
+                    mbar_expect_tx_elect(BAR(B_VFULL + st), S::TILE);
+                    for (int x = 0; x < S::NBOX; ++x)
+                        tma_load_4d_elect(sV(st) + x * S::BOX, &tmV, BAR(B_VFULL + st), x * 64, blk * kBlk, vhk, vb);
+                    ++vt;
+                    ++gv;
+                }
+            }
+        } else {
+            // ------------------------------ MMA issuers ------------------------------
+            //   warp 13: P*V(g) when P(g) is there
+            //   warp 15: S(g), up to three tiles ahead: S(g) overwrites the buffer that P(g - 3) was read from
+            // Two warps, so that S of a later tile (and of the next item's first ones) never waits behind P of this one.
+            const uint32_t utmem = uniform(int(tmem));
+            constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
+            constexpr uint32_t idesc_pv = make_idesc(BF16, 128, D, false, true);
+            constexpr uint64_t desc_v = desc_mn_major(S::BOX);
+            bool ok = true;
+            int g = 0, no = 0;  // tiles; items with tiles
+            for (int k = 0;; ++k) {
+                const int s = k % NQ, use = k / NQ;
+                ok = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
+                if (!ok) break;
+                const int T = uniform(info[s * 8 + 0]);
+                if (uniform(info[s * 8 + 2]) < 0) break;
+                if (warp == 15) {
+                    if (T > 0) ok = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 3);
+                    for (int t = 0; t < T && ok; ++t, ++g) {
+                        const int buf = g % 3, st = g % NS;
+                        ok = mbar_wait_warp(BAR(B_KFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 4);
+                        if (ok && g >= 3) ok = mbar_wait_warp(BAR(B_PVDONE + buf), (g / 3 - 1) & 1, ab, ST_WAIT_TIMEOUT + 15);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t tS = utmem + uint32_t(buf) * 128u, q_tile = sQ(s), k_tile = sK(st);
+#pragma unroll
+                        for (int kk = 0; kk < D / 16; ++kk) {
+                            const uint32_t off = uint32_t(kk >> 2) * S::BOX + uint32_t(kk & 3) * 32u;
+                            umma_ss(tS, smem_desc_at(kDescKMajor, q_tile + off), smem_desc_at(kDescKMajor, k_tile + off), idesc_s, kk > 0);
+                        }
+                        umma_commit(BAR(B_KEMPTY + st));
+                        umma_commit(BAR(B_SFULL + buf));
+                    }
+                } else {
+                    const int o = no % NO;
+                    const uint32_t tO = utmem + 384u + uint32_t(o * D);
+                    for (int t = 0; t < T; ++t, ++g) {
+                        const int buf = g % 3, st = g % NS;
+                        const uint32_t tP = utmem + uint32_t(buf) * 128u, v_tile = sV(st);
+                        ok = mbar_wait_warp(BAR(B_VFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 5);
+                        // the first P*V of an item overwrites O: the epilogue of the last item that used it must have read it
+                        if (ok && t == 0 && no >= NO) ok = mbar_wait_warp(BAR(B_OFREE + o), (no / NO - 1) & 1, ab, ST_WAIT_TIMEOUT + 14);
+                        if (ok) ok = mbar_wait_warp(BAR(B_PFULL + buf), (g / 3) & 1, ab, ST_WAIT_TIMEOUT + 6);
+                        if (!ok) break;
+                        tc_fence_after();
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)
+                            umma_ts(tO, tP + uint32_t(kk) * 8u, smem_desc_at(desc_v, v_tile + uint32_t(kk) * 2048u), idesc_pv,
+                                    (t > 0 || kk > 0) ? 1u : 0u);
+                        umma_commit(BAR(B_VEMPTY + st));
+                        umma_commit(BAR(B_PVDONE + buf));
+                        if (t == T - 1) umma_commit(BAR(B_OFULL + o));
+                    }
+                }
+                if (!ok) break;
+                if (T > 0) ++no;
+                if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+    } else if (warp >= 8) {
+        // ------------------------------ epilogue group ------------------------------
+        setmaxnreg_dec<kFwdEpilogueRegs>();
+        const int r = tid & 127;
+        const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
+        const float c = p.scale_log2;
+        bool alive = !aborted;
+        int G = 0;   // tiles of all earlier items
+        int no = 0;  // items with tiles
+        for (int k = 0; alive; ++k) {
+            const int s = k % NQ, use = k / NQ;
+            alive = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
+            if (!alive) break;
+            const int T = info[s * 8 + 0], j = info[s * 8 + 2], qb = info[s * 8 + 4], h = info[s * 8 + 5], b = info[s * 8 + 6];
+            if (j < 0) break;
+            const int g_row = SHORT && p.pack > 1 ? r / mk.M : 0;
+            const int row = qb * kBlk + r - g_row * mk.M;
+            const int g_own = SHORT ? (h % nG) * p.pack + g_row : 0;
+            const bool valid = !SHORT || (row < mk.M && g_row < p.pack && g_own < p.G);
+            alive = mbar_wait_warp(BAR(B_MLFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 16);
+            // an item without tiles: nobody has waited for its Q load yet, and its slot is about to become the staging area
+            if (alive && T == 0) alive = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 17);
+            const int o = no % NO;
+            if (alive && T > 0) alive = mbar_wait_warp(BAR(B_OFULL + o), (no / NO) & 1, ab, ST_WAIT_TIMEOUT + 9);
+            if (!alive) break;
+            tc_fence_after();
+            const float* ml = reinterpret_cast<const float*>(smem + S::off_ml) + s * (4 * kBlk);  // [2 groups][m, l][128]
+            const int even = (G & 1) * (2 * kBlk), odd = 2 * kBlk - even;  // the groups that had the even and the odd tiles
+            const float m0 = ml[even + r], l0 = ml[even + kBlk + r], m1 = ml[odd + r], l1 = ml[odd + kBlk + r];
+            const float mt = fmaxf(m0, m1);
+            const float a0 = (m0 == -INFINITY) ? 0.f : fast_exp2((m0 - mt) * c);
+            const float a1 = (m1 == -INFINITY) ? 0.f : fast_exp2((m1 - mt) * c);
+            const float lt = l0 * a0 + l1 * a1;
+            const float inv = (lt > 0.f) ? 1.0f / lt : 0.f;
+            const bool used = (T > 0) && inv != 0.f;
+            const bool healthy = misc[1] == 0;
+            if (healthy) {
+                const float lse = (lt > 0.f) ? fmaf(mt, c, log2f(lt)) : -INFINITY;
+                if constexpr (SHORT) {
+                    const int64_t bh0 = int64_t(b) * p.H + int64_t(h / nG) * p.G;
+                    if (ns > 1) {
+                        // a run that went NaN says so: -inf would pass for a run without keys
+                        if (valid) p.part_lse[((bh0 + g_own) * mk.M + row) * ns + j % ns] = (lt == lt) ? lse : lt;
+                    } else {
+                        if (valid) p.lse[(bh0 + g_own) * mk.L.Mpad + row] = lse;
+                        // the rows past M that pad the buffer
+                        for (int g = (h % nG) * p.pack; g < min(p.G, (h % nG + 1) * p.pack); ++g)
+                            if (qb * kBlk + r >= mk.M) p.lse[(bh0 + g) * mk.L.Mpad + qb * kBlk + r] = 0.f;
+                    }
+                } else {
+                    p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + row] = lse;
+                }
+            }
+            float* part = nullptr;  // this thread's row in the workspace (SHORT, ns > 1)
+            if constexpr (SHORT) {
+                if (ns > 1 && valid && healthy)
+                    part = p.part_o + ((int64_t(j % ns) * p.B * p.H + int64_t(b) * p.H + int64_t(h / nG) * p.G + g_own) * mk.M + row) * D;
+            }
+            // The O tile is staged in this item's Q slot (Q is dead: every S MMA of the item has completed) in the
+            // 128-byte-swizzled layout of the tensor map.
+            uint8_t* stage = smem + S::off_q + s * S::TILE;
+#pragma unroll
+            for (int q = 0; q < D / 32; ++q) {
+                uint32_t x[32];
+                // tcgen05.ld is warp-collective: always executed, the values are ignored when unused
+                tmem_ld32(tmem + lane_base + 384u + uint32_t(o * D) + uint32_t(q) * 32u, x);
+                tc_wait_ld();
+                if (q == D / 32 - 1) {  // O has been read: the MMA issuer may start another item's P*V
+                    tc_fence_before();
+                    if (T > 0) mbar_arrive_warp(BAR(B_OFREE + o), lane);
+                }
+#pragma unroll
+                for (int y = 0; y < 32; ++y) x[y] = used ? __float_as_uint(__uint_as_float(x[y]) * inv) : 0u;
+                if constexpr (SHORT) {
+                    if (part) {
+#pragma unroll
+                        for (int y = 0; y < 8; ++y)
+                            *reinterpret_cast<uint4*>(part + 32 * q + 4 * y) = make_uint4(x[4 * y], x[4 * y + 1], x[4 * y + 2], x[4 * y + 3]);
+                    }
+                }
+                auto two = [&](int y) { return pack2<BF16>(__uint_as_float(x[y]), __uint_as_float(x[y + 1])); };
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int cg = 4 * q + i;  // 16-byte chunk of the row
+                    uint4* dst = reinterpret_cast<uint4*>(stage + (cg >> 3) * S::BOX + r * 128 + (((cg & 7) ^ (r & 7)) << 4));
+                    *dst = make_uint4(two(8 * i), two(8 * i + 2), two(8 * i + 4), two(8 * i + 6));
+                }
+            }
+            G += T;
+            if (T > 0) ++no;
+            fence_proxy_async();
+            mbar_arrive_warp(BAR(B_STAGED + s), lane);
+            if (warp == 8) alive = mbar_wait_warp(BAR(B_STAGED + s), use & 1, ab, ST_WAIT_TIMEOUT + 18);
+            if (!alive) break;
+            if (r == 0) {
+                if (healthy) {
                     if constexpr (SHORT) {
-                        if (ns > 1) return true;  // the rows went to the workspace
-                        for (int x = 0; x < S::NBOX; ++x)
-                            tma_store_5d(&tmO, sQ(s) + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
+                        if (ns == 1)  // else the rows went to the workspace
+                            for (int x = 0; x < S::NBOX; ++x)
+                                tma_store_5d(&tmO, sQ(s) + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
                     } else {
                         for (int x = 0; x < S::NBOX; ++x) tma_store_4d(&tmO, sQ(s) + x * S::BOX, x * 64, qb * kBlk, h, b);
                     }
                     tma_store_commit();
                     tma_store_wait_read();
-                    return true;
-                };
-                for (;; ++k) {
-                    const int s = k & 1, use = k >> 1;
-                    ok = mbar_wait(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
-                    if (!ok) break;
-                    const int T = info[s * 8 + 0], lo = info[s * 8 + 1], j = info[s * 8 + 2];
-                    if (j < 0) break;
-                    const uint16_t* list = list_of(s);
-                    const int qb = info[s * 8 + 4], h = info[s * 8 + 5], b = info[s * 8 + 6];
-                    const int hk = SHORT ? h / nG : h / p.G;
-                    const int he = (mk.He == 1) ? 0 : h;
-                    // the slot still holds the staged O tile of item k-2: send it off first
-                    if (use > 0) ok = store_o(k - 2);
-                    if (!ok) break;
-                    item_qb[s] = qb; item_h[s] = h; item_b[s] = b;
-                    if constexpr (SHORT) {
-                        mbar_expect_tx(BAR(B_QFULL + s), uint32_t(p.rows) * 128u * S::NBOX);
-                        for (int x = 0; x < S::NBOX; ++x)
-                            tma_load_5d(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, (h % nG) * p.pack, hk, b);
-                    } else {
-                        mbar_expect_tx(BAR(B_QFULL + s), S::TILE);
-                        for (int x = 0; x < S::NBOX; ++x)
-                            tma_load_4d(sQ(s) + x * S::BOX, &tmQ, BAR(B_QFULL + s), x * 64, qb * kBlk, h, b);
-                    }
-                    for (int t = 0; t <= T && ok; ++t) {  // K runs one tile ahead of V
-                        if (t < T) {
-                            const int kb = lo + (list[t] & 1023);
-                            const int g = G + t, st = g % NS, ug = g / NS;
-                            if (ug > 0) ok = mbar_wait(BAR(B_KEMPTY + st), (ug - 1) & 1, ab, ST_WAIT_TIMEOUT + 1);
-                            if (!ok) break;
-                            // The tile's key codes travel with K: they land in a ring of NKC slots and complete on
-                            // K's barrier, so whoever has seen S(g) (computed after that barrier) may read them.
-                            // Slot g % NKC was last read by the softmax of tile g - NKC, which is over: this thread
-                            // has already waited for the P*V of tile g - 2 - NS before issuing V(g - 2).
-                            mbar_expect_tx(BAR(B_KFULL + st), S::TILE + (mk.mode == 1 ? kBlk * 4 : 0));
-                            for (int x = 0; x < S::NBOX; ++x)
-                                tma_load_4d(sK(st) + x * S::BOX, &tmK, BAR(B_KFULL + st), x * 64, kb * kBlk, hk, b);
-                            if (mk.mode == 1)
-                                bulk_load_1d(sbase + S::off_kc + (g % S::NKC) * (kBlk * 4),
-                                             mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad + int64_t(kb) * kBlk,
-                                             kBlk * 4, BAR(B_KFULL + st));
-                        }
-                        if (t >= 1) {
-                            const int kb = lo + (list[t - 1] & 1023);
-                            const int g = G + t - 1, st = g % NS, ug = g / NS;
-                            if (ug > 0) ok = mbar_wait(BAR(B_VEMPTY + st), (ug - 1) & 1, ab, ST_WAIT_TIMEOUT + 2);
-                            if (!ok) break;
-                            mbar_expect_tx(BAR(B_VFULL + st), S::TILE);
-                            for (int x = 0; x < S::NBOX; ++x)
-                                tma_load_4d(sV(st) + x * S::BOX, &tmV, BAR(B_VFULL + st), x * 64, kb * kBlk, hk, b);
-                        }
-                    }
-                    G += T;
-                    if (ok) mbar_arrive(BAR(B_ITEMEMPTY + s));
                 }
-                // the last two items' tiles
-                if (ok && k >= 2) ok = store_o(k - 2);
-                if (ok && k >= 1) ok = store_o(k - 1);
-                tma_store_wait_all();
+                mbar_arrive(BAR(B_QEMPTY + s));  // the slot may take another item's Q
             }
-        } else {
-            // ------------------------------ MMA issuers ------------------------------
-            // One issuing warp per softmax group: warp 9 owns the CTA's even visited tiles (S0 / O0),
-            // warp 10 the odd ones (S1 / O1). The two chains touch disjoint TMEM and only share the
-            // K / V rings, so neither warp ever waits on the other group's softmax. Within a
-            // chain the MMAs of P*V(t) and S(t+2) are issued back to back (the tensor pipe accepts
-            // only a few MMAs ahead and needs ~200 clocks to refill once drained): what S(t+2)
-            // needs from TMA is waited for before P(t) is.
-            {
-                const int w = warp - 9;
-                const uint32_t utmem = uniform(int(tmem));
-                constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
-                constexpr uint32_t idesc_pv = make_idesc(BF16, 128, D, false, true);
-                constexpr uint64_t desc_v = desc_mn_major(S::BOX);
-                const uint32_t tS = utmem + uint32_t(w) * 128u;
-                const uint32_t tO = utmem + 256u + uint32_t(w) * uint32_t(D);
-                bool ok = true;
-                int k = 0, G = 0, cw = 0;  // cw: tiles this chain has finished (phases of its barriers)
-                int kkw = 0;               // items in which this chain had tiles (phase of its o_free barrier)
-                for (;; ++k) {
-                    const int s = k & 1, use = k >> 1;
-                    ok = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
-                    if (!ok) break;
-                    const int T = uniform(info[s * 8 + 0]);
-                    if (uniform(info[s * 8 + 2]) < 0) break;
-                    ok = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 3);
-                    if (!ok) break;
-                    const uint32_t q_tile = sQ(s);
-                    auto k_ready = [&](int g) {
-                        return mbar_wait_warp(BAR(B_KFULL + (g % NS)), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 4);
-                    };
-                    auto s_mmas = [&](int g) {
-                        const int st = g % NS;
-#pragma unroll
-                        for (int kk = 0; kk < D / 16; ++kk) {
-                            const uint32_t off = uint32_t(kk >> 2) * S::BOX + uint32_t(kk & 3) * 32u;
-                            umma_ss(tS, smem_desc_at(kDescKMajor, q_tile + off), smem_desc_at(kDescKMajor, sK(st) + off),
-                                    idesc_s, kk > 0);
-                        }
-                        umma_commit(BAR(B_KEMPTY + st));
-                        umma_commit(BAR(B_SFULL + w));
-                    };
-                    const int t0 = (G ^ w) & 1;  // this chain's first tile of the item: G + t0 has parity w
-                    const int nmine = (T > t0) ? (T - t0 + 1) / 2 : 0;
-                    if (nmine > 0) {
-                        ok = k_ready(G + t0);
-                        if (!ok) break;
-                        tc_fence_after();
-                        s_mmas(G + t0);
-                    }
-                    for (int i = 0; i < nmine && ok; ++i, ++cw) {
-                        const int g = G + t0 + 2 * i, st = g % NS;
-                        const bool more = i + 1 < nmine;
-                        ok = mbar_wait_warp(BAR(B_VFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 5);
-                        if (ok && more) ok = k_ready(g + 2);
-                        // The first P*V of an item overwrites O: the epilogue of the previous item in which this
-                        // chain had tiles must have read it. (The barrier counts those items only, on both
-                        // sides: a chain without tiles in an item runs through it and must not find itself two
-                        // phases behind, where a parity wait can no longer tell "not yet" from "done".)
-                        if (ok && i == 0 && kkw > 0) ok = mbar_wait_warp(BAR(B_OFREE + w), (kkw - 1) & 1, ab, ST_WAIT_TIMEOUT + 14);
-                        if (ok) ok = mbar_wait_warp(BAR(B_PHALF0 + w), cw & 1, ab, ST_WAIT_TIMEOUT + 6);
-                        if (!ok) break;
-                        tc_fence_after();
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            umma_ts(tO, tS + uint32_t(kk) * 8u, smem_desc_at(desc_v, sV(st) + uint32_t(kk) * 2048u), idesc_pv,
-                                    (i > 0 || kk > 0) ? 1u : 0u);
-                        ok = mbar_wait_warp(BAR(B_PHALF1 + w), cw & 1, ab, ST_WAIT_TIMEOUT + 6);
-                        if (!ok) break;
-                        tc_fence_after();
-#pragma unroll
-                        for (int kk = 4; kk < 8; ++kk)
-                            umma_ts(tO, tS + uint32_t(kk) * 8u, smem_desc_at(desc_v, sV(st) + uint32_t(kk) * 2048u), idesc_pv, 1u);
-                        umma_commit(BAR(B_VEMPTY + st));
-                        umma_commit(BAR(B_PVDONE + w));
-                        if (more) s_mmas(g + 2);
-                    }
-                    G += T;
-                    if (nmine > 0) ++kkw;
-                    if (ok && lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
-                    __syncwarp();
-                }
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
         }
+        if (r == 0) tma_store_wait_all();
         __syncwarp();
     } else {
-        setmaxnreg_inc<216>();
+        setmaxnreg_inc<kFwdSoftmaxRegs>();
         // ------------------------------ softmax groups ------------------------------
-        // Every wait is a bounded mbarrier wait: a thread whose wait was given up (alive == false)
+        // Every wait is a bounded mbarrier wait: a warp whose wait was given up (alive == false)
         // leaves the item loop at once, and nobody is left waiting for it for longer than the limit.
         const int w = warp >> 2;  // group
         const int r = tid & 127;  // row inside the block
         const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
         const float c = p.scale_log2;
-        const uint32_t tS = tmem + lane_base + uint32_t(w) * 128u;
-        const uint32_t tO = tmem + lane_base + 256u + uint32_t(w) * uint32_t(D);
+        float* m_row = reinterpret_cast<float*>(smem + S::off_m) + r;
         bool alive = !aborted;
-        int k = 0, cw = 0;  // cw: tiles this group has finished (phases of its barriers)
-        int nturn = 0;      // turns this group has taken (phase of its turn barrier)
-        int G = 0;          // tiles of all earlier items (stage / phase of the K and V rings)
-        for (; alive; ++k) {
-            const int s = k & 1, use = k >> 1;
-            alive = mbar_wait(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
-            alive = __all_sync(0xffffffffu, alive);
+        int G = 0;   // tiles of all earlier items
+        int no = 0;  // items with tiles
+        for (int k = 0; alive; ++k) {
+            const int s = k % NQ, use = k / NQ;
+            alive = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
             if (!alive) break;
             const int T = info[s * 8 + 0];
             const int lo = info[s * 8 + 1];
-            const int j = info[s * 8 + 2];
-            if (j < 0) break;
+            if (info[s * 8 + 2] < 0) break;
             const uint16_t* list = list_of(s);
-            const int qb = info[s * 8 + 4], h = info[s * 8 + 5], b = info[s * 8 + 6];
+            const int qb = info[s * 8 + 4];
             // this thread's query: row of the head, and (SHORT) which head of the group
             const int g_row = SHORT && p.pack > 1 ? r / mk.M : 0;
             const int row = qb * kBlk + r - g_row * mk.M;
-            const int g_own = SHORT ? (h % nG) * p.pack + g_row : 0;
-            const bool valid = !SHORT || (row < mk.M && g_row < p.pack && g_own < p.G);
+            const bool valid = !SHORT || (row < mk.M && g_row < p.pack && (info[s * 8 + 5] % nG) * p.pack + g_row < p.G);
             const bool active = !SHORT || __any_sync(0xffffffffu, valid);  // does this warp hold a query at all?
             const int qc = reinterpret_cast<const int*>(smem + S::off_qc)[s * kBlk + r];
-            float m_run = -INFINITY, l_run = 0.f;
-            int n_my = 0;
-            const int we = G & 1;   // the group that owns the item's even tiles
-            const int t0 = w ^ we;  // this group's first tile of the item
-            const int n_other = (t0 == 0) ? T / 2 : (T + 1) / 2;  // tiles of the other group
-            // short items: both groups simply run side by side; long items: the exp phase is taken in turns
-            const bool turns = T >= kTurnMinTiles;
-            if (turns && t0 == 1 && alive) mbar_arrive(BAR(B_TURN + we));  // the owner of tile 0 takes the first turn
+            const uint32_t tO = tmem + lane_base + 384u + uint32_t((no % NO) * D);
+            bool ready = false;  // the scores of the next tile are known to be there
+            float m_run = -INFINITY, l_run = 0.f;  // l_run: sum of this group's tiles relative to m_run
 
-            for (int t = t0; t < T && alive; t += 2, ++n_my, ++cw) {
+            for (int t = (G ^ w) & 1; t < T && alive; t += 2) {
+                const int g = G + t, buf = g % 3;
+                const uint32_t tS = tmem + lane_base + uint32_t(buf) * 128u;
                 const uint32_t entry = list[t];
                 const uint32_t fl = entry >> 10;
                 const int k0 = (lo + int(entry & 1023u)) * kBlk;
-                alive = mbar_wait(BAR(B_SFULL + w), cw & 1, ab, ST_WAIT_TIMEOUT + 7);
-                alive = __all_sync(0xffffffffu, alive);
+                if (!ready) alive = mbar_wait_warp(BAR(B_SFULL + buf), (g / 3) & 1, ab, ST_WAIT_TIMEOUT + 7);
                 if (!alive) break;
+                ready = false;
                 tc_fence_after();
                 if (SHORT && !active) {  // no row of this warp is a query: its lanes of P and O are never stored
-                    if (turns) {
-                        alive = mbar_wait(BAR(B_TURN + w), nturn & 1, ab, ST_WAIT_TIMEOUT + 10);
-                        alive = __all_sync(0xffffffffu, alive);
-                        if (!alive) break;
-                        ++nturn;
-                    }
-                    mbar_arrive(BAR(B_PHALF0 + w));
-                    mbar_arrive(BAR(B_PHALF1 + w));
-                    if (turns && (t0 == 0 ? (n_my < n_other) : (n_my + 1 < n_other))) mbar_arrive(BAR(B_TURN + (w ^ 1)));
+                    if (g > 0) alive = mbar_wait_warp(BAR(B_MREADY + (w ^ 1)), ((g - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 10);
+                    if (!alive) break;
+                    mbar_arrive_warp(BAR(B_MREADY + w), lane);
+                    mbar_arrive_warp(BAR(B_PFULL + buf), lane);
                     continue;
                 }
                 uint32_t sr[128];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) tmem_ld32(tS + uint32_t(q) * 32u, sr + q * 32);
+                // (asked early as well; needed once this tile's maximum is known)
+                const bool m_there = g == 0 || mbar_test_warp(BAR(B_MREADY + (w ^ 1)), ((g - 1) >> 1) & 1);
+                float m_prev = (m_there && t > 0) ? *m_row : -INFINITY;
                 tc_wait_ld();
                 float* sc = reinterpret_cast<float*>(sr);
 
@@ -515,198 +619,87 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 #pragma unroll
                 for (int a = 0; a < 8; ++a) mxa[a] = fmaxf(mxa[a], sc[120 + a]);
                 const float mx = fmaxf(max3(mxa[0], mxa[1], mxa[2]), max3(max3(mxa[3], mxa[4], mxa[5]), mxa[6], mxa[7]));
-                float m_new = fmaxf(m_run, mx);
-                // lazy rescale: keep the old reference point while the new maximum is within 2^8 of it
-                const bool need = (m_new - m_run) * c > 8.0f;
-                if (!need) m_new = m_run;
-                if (__any_sync(0xffffffffu, need)) {
-                    const float alpha = need ? fast_exp2((m_run - m_new) * c) : 1.0f;
-                    l_run *= alpha;
-                    if (n_my > 0) {
-                        alive = mbar_wait(BAR(B_PVDONE + w), (cw - 1) & 1, ab, ST_WAIT_TIMEOUT + 8);
-                        alive = __all_sync(0xffffffffu, alive);
-                        if (!alive) break;
-                        tc_fence_after();
-#pragma unroll
-                        for (int q = 0; q < D / 32; ++q) {
-                            uint32_t orr[32];
-                            tmem_ld32(tO + uint32_t(q) * 32u, orr);
-                            tc_wait_ld();
-#pragma unroll
-                            for (int x = 0; x < 32; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
-                            tmem_st32(tO + uint32_t(q) * 32u, orr);
-                        }
-                        tc_wait_st();
-                    }
-                }
-                m_run = m_new;
-                const float mneg = (m_run == -INFINITY) ? 0.f : -m_run * c;
-                // exp2(s*c - m*c) on packed pairs; P goes to TMEM in two halves so that the first four
-                // k-steps of P*V can start while the second half is still being exponentiated.
-                const uint64_t c2 = pack_f2(c, c), mneg2 = pack_f2(mneg, mneg);
-                uint64_t lacc0 = pack_f2(0.f, 0.f), lacc1 = lacc0;
-                // The exp phase is taken in turns (barriers turn[0], turn[1]; the owner of tile 0 first): left alone,
-                // the groups fall into lockstep, exponentiate together at half MUFU rate each and then
-                // queue their MMAs together, which halves the use of both pipes. In turns, one group
-                // exponentiates while the other group's P*V and next S run on the tensor pipe.
-                if (turns) {
-                    alive = mbar_wait(BAR(B_TURN + w), nturn & 1, ab, ST_WAIT_TIMEOUT + 10);
-                    alive = __all_sync(0xffffffffu, alive);
+                // The reference maximum comes from the tile before (the other group's) and goes to the tile after. Every
+                // tile waits, also an item's first, so that neither group is ever two phases ahead of the other's wait.
+                if (!m_there) {
+                    alive = mbar_wait_warp(BAR(B_MREADY + (w ^ 1)), ((g - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 10);
                     if (!alive) break;
-                    ++nturn;
+                    if (t > 0) m_prev = *m_row;
                 }
-                auto exp_half = [&](int half) {
+                // lazy rescale: keep the old reference point while the new maximum is within 2^8 of it
+                float m_new = fmaxf(m_prev, mx);
+                const bool need = (m_new - m_prev) * c > 8.0f;
+                if (!need) m_new = m_prev;
+                *m_row = m_new;
+                mbar_arrive_warp(BAR(B_MREADY + w), lane);
+                // O is 0 in a row that had no key yet: nothing to rescale there
+                const bool rescale = need && m_prev != -INFINITY;
+                if (__any_sync(0xffffffffu, rescale)) {
+                    const float alpha = rescale ? fast_exp2((m_prev - m_new) * c) : 1.0f;
+                    alive = mbar_wait_warp(BAR(B_PVDONE + (g - 1) % 3), ((g - 1) / 3) & 1, ab, ST_WAIT_TIMEOUT + 8);
+                    if (!alive) break;
+                    tc_fence_after();
 #pragma unroll
-                    for (int q = 2 * half; q < 2 * half + 2; ++q) {
-                        uint32_t pk[16];
+                    for (int q = 0; q < D / 16; ++q) {
+                        uint32_t orr[16];
+                        tmem_ld16(tO + uint32_t(q) * 16u, orr);
+                        tc_wait_ld();
 #pragma unroll
-                        for (int x = 0; x < 16; ++x) {
-                            const uint64_t x2 = fma_f2(pack_f2(sc[32 * q + 2 * x], sc[32 * q + 2 * x + 1]), c2, mneg2);
-                            float x0, x1;
-                            unpack_f2(x2, x0, x1);
-                            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-                            if (x & 1) lacc1 = add_f2(lacc1, pack_f2(p0, p1)); else lacc0 = add_f2(lacc0, pack_f2(p0, p1));
-                            pk[x] = pack2<BF16>(p0, p1);
-                        }
-                        tmem_st16(tS + uint32_t(q) * 16u, pk);
+                        for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
+                        tmem_st16(tO + uint32_t(q) * 16u, orr);
                     }
                     tc_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(BAR((half ? B_PHALF1 : B_PHALF0) + w));
-                };
-                exp_half(0);
-                exp_half(1);
-                // hand the turn over, unless the other group has no tile left to take it for
-                if (turns && (t0 == 0 ? (n_my < n_other) : (n_my + 1 < n_other))) mbar_arrive(BAR(B_TURN + (w ^ 1)));
+                }
+                const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * c;
+                // exp2(s*c - m*c) on packed pairs
+                const uint64_t c2 = pack_f2(c, c), mneg2 = pack_f2(mneg, mneg);
+                uint64_t lacc0 = pack_f2(0.f, 0.f), lacc1 = lacc0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) {
+                        const uint64_t x2 = fma_f2(pack_f2(sc[32 * q + 2 * x], sc[32 * q + 2 * x + 1]), c2, mneg2);
+                        float x0, x1;
+                        unpack_f2(x2, x0, x1);
+                        const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+                        if (x & 1) lacc1 = add_f2(lacc1, pack_f2(p0, p1)); else lacc0 = add_f2(lacc0, pack_f2(p0, p1));
+                        pk[x] = pack2<BF16>(p0, p1);
+                    }
+                    tmem_st16(tS + uint32_t(q) * 16u, pk);
+                }
+                tc_wait_st();
+                tc_fence_before();
+                mbar_arrive_warp(BAR(B_PFULL + buf), lane);
+                // (asked here, the answer is there when the next tile starts: about 100 clocks less than a wait for a barrier
+                // that has completed already)
+                ready = t + 2 < T && mbar_test_warp(BAR(B_SFULL + (g + 2) % 3), ((g + 2) / 3) & 1);
                 {
                     float a0, a1, b0, b1;
                     unpack_f2(lacc0, a0, a1);
                     unpack_f2(lacc1, b0, b1);
+                    // the sum so far follows the reference (the other group's tile may have moved it, too)
+                    if (m_new != m_run) l_run *= (m_run == -INFINITY) ? 0.f : fast_exp2((m_run - m_new) * c);
+                    m_run = m_new;
                     l_run += (a0 + a1) + (b0 + b1);
                 }
             }
-
-            // ------------------------------ item epilogue ------------------------------
-            // wait for this group's last P*V, then merge the two partial softmaxes
             if (!alive) break;
-            if (T == 0) {
-                // nobody has waited for this item's Q load yet, and its slot is about to become the staging
-                // area of the (all-zero) output tile: the load must have landed first
-                alive = mbar_wait(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 17);
-                alive = __all_sync(0xffffffffu, alive);
-                if (!alive) break;
-            }
-            if (n_my > 0) {
-                alive = mbar_wait(BAR(B_PVDONE + w), (cw - 1) & 1, ab, ST_WAIT_TIMEOUT + 9);
-                alive = __all_sync(0xffffffffu, alive);
-                if (!alive) break;
-            }
-            float* ml = reinterpret_cast<float*>(smem + S::off_ml) + s * (4 * kBlk);  // [2 groups][m, l][128]
-            ml[(w * 2 + 0) * kBlk + r] = m_run;
-            ml[(w * 2 + 1) * kBlk + r] = l_run;
-            tc_fence_before();
-            mbar_arrive(BAR(B_MLFULL));  // both groups are past all MMAs of this item
-            alive = mbar_wait(BAR(B_MLFULL), k & 1, ab, ST_WAIT_TIMEOUT + 16);
-            alive = __all_sync(0xffffffffu, alive);
-            if (!alive) break;
-            tc_fence_after();
-            // index 0: the chain of the item's even tiles, 1: of its odd tiles
-            const float m0 = ml[(we * 2 + 0) * kBlk + r], l0 = ml[(we * 2 + 1) * kBlk + r];
-            const float m1 = ml[((we ^ 1) * 2 + 0) * kBlk + r], l1 = ml[((we ^ 1) * 2 + 1) * kBlk + r];
-            const float mt = fmaxf(m0, m1);
-            const float a0 = (m0 == -INFINITY) ? 0.f : fast_exp2((m0 - mt) * c);
-            const float a1 = (m1 == -INFINITY) ? 0.f : fast_exp2((m1 - mt) * c);
-            const float lt = l0 * a0 + l1 * a1;
-            const float inv = (lt > 0.f) ? 1.0f / lt : 0.f;
-            const float f0 = a0 * inv, f1 = a1 * inv;
-            const bool use0 = (T > 0) && (f0 != 0.f), use1 = (T > 1) && (f1 != 0.f);
-            const bool healthy = alive && (misc[1] == 0);
-            if (w == 0 && healthy) {
-                const float lse = (lt > 0.f) ? fmaf(mt, c, log2f(lt)) : -INFINITY;
-                if constexpr (SHORT) {
-                    const int64_t bh0 = int64_t(b) * p.H + int64_t(h / nG) * p.G;
-                    if (ns > 1) {
-                        // a run that went NaN says so: -inf would pass for a run without keys
-                        if (valid) p.part_lse[((bh0 + g_own) * mk.M + row) * ns + j % ns] = (lt == lt) ? lse : lt;
-                    } else {
-                        if (valid) p.lse[(bh0 + g_own) * mk.L.Mpad + row] = lse;
-                        // the rows past M that pad the buffer
-                        for (int g = (h % nG) * p.pack; g < min(p.G, (h % nG + 1) * p.pack); ++g)
-                            if (qb * kBlk + r >= mk.M) p.lse[(bh0 + g) * mk.L.Mpad + qb * kBlk + r] = 0.f;
-                    }
-                } else {
-                    p.lse[(int64_t(b) * p.H + h) * mk.L.Mpad + row] = lse;
-                }
-            }
-            // this thread's half row: columns [w*D/2, (w+1)*D/2) of both accumulators
-            constexpr int HALF = D / 2;
-            const uint32_t c0 = uint32_t(w) * HALF;
-            uint32_t outw[HALF / 2];
-            float* part = nullptr;  // this thread's half row in the workspace (SHORT, ns > 1)
-            if constexpr (SHORT) {
-                if (ns > 1 && valid && healthy)
-                    part = p.part_o + ((int64_t(j % ns) * p.B * p.H + int64_t(b) * p.H + int64_t(h / nG) * p.G + g_own) * mk.M + row) * D + c0;
-            }
-#pragma unroll
-            for (int q = 0; q < HALF / 32; ++q) {
-                uint32_t x0[32], x1[32];
-                // tcgen05.ld is warp-collective: always executed, the values are ignored when unused
-                tmem_ld32(tmem + lane_base + 256u + uint32_t(we * D) + c0 + uint32_t(q) * 32u, x0);
-                tmem_ld32(tmem + lane_base + 256u + uint32_t((we ^ 1) * D) + c0 + uint32_t(q) * 32u, x1);
-                tc_wait_ld();
-#pragma unroll
-                for (int x = 0; x < 16; ++x) {
-                    float v0 = 0.f, v1 = 0.f;
-                    if (use0) {
-                        v0 = __uint_as_float(x0[2 * x]) * f0;
-                        v1 = __uint_as_float(x0[2 * x + 1]) * f0;
-                    }
-                    if (use1) {
-                        v0 = fmaf(__uint_as_float(x1[2 * x]), f1, v0);
-                        v1 = fmaf(__uint_as_float(x1[2 * x + 1]), f1, v1);
-                    }
-                    outw[16 * q + x] = pack2<BF16>(v0, v1);
-                    if constexpr (SHORT) {
-                        x0[2 * x] = __float_as_uint(v0);
-                        x0[2 * x + 1] = __float_as_uint(v1);
-                    }
-                }
-                if constexpr (SHORT) {
-                    if (part) {
-#pragma unroll
-                        for (int x = 0; x < 8; ++x)
-                            *reinterpret_cast<uint4*>(part + 32 * q + 4 * x) = make_uint4(x0[4 * x], x0[4 * x + 1], x0[4 * x + 2], x0[4 * x + 3]);
-                    }
-                }
-            }
-            // both accumulators have been read: the MMA issuers may start the next item's P*V
-            tc_fence_before();
-            if (T > 0) mbar_arrive(BAR(B_OFREE + we));        // the chain of the even tiles had some
-            if (T > 1) mbar_arrive(BAR(B_OFREE + (we ^ 1)));  // so had the other chain
-            // Stage the O tile in this item's Q slot (Q is dead: every S MMA of the item has
-            // completed) in the 128-byte-swizzled layout of the tensor map; the producer warp issues
-            // the TMA store when every thread has arrived, and reuses the slot once it has been read.
-            {
-                uint8_t* stage = smem + S::off_q + s * S::TILE;
-#pragma unroll
-                for (int i = 0; i < HALF / 8; ++i) {
-                    const int cg = int(c0) / 8 + i;  // 16-byte chunk of the row
-                    const int box = cg >> 3, ch = cg & 7;
-                    uint4* dst = reinterpret_cast<uint4*>(stage + box * S::BOX + r * 128 + ((ch ^ (r & 7)) << 4));
-                    *dst = make_uint4(outw[4 * i], outw[4 * i + 1], outw[4 * i + 2], outw[4 * i + 3]);
-                }
-            }
-            fence_proxy_async();
-            if (healthy) mbar_arrive(BAR(B_OSTAGED + s));  // the producer warp issues the TMA store
+            float* ml = reinterpret_cast<float*>(smem + S::off_ml) + s * (4 * kBlk) + w * (2 * kBlk) + r;
+            ml[0] = m_run;
+            ml[kBlk] = l_run;
+            mbar_arrive_warp(BAR(B_MLFULL + s), lane);
             G += T;
-            if (r == 0 && alive) mbar_arrive(BAR(B_ITEMEMPTY + s));
+            if (T > 0) ++no;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
         }
     }
 
     // ------------------------------ tear-down ------------------------------
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == 13) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }
@@ -788,7 +781,7 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
     const int heads = SHORT ? p.H / p.G * cdiv(p.G, p.pack) : p.H;
     const int n_items = p.mask.L.nQ * heads * p.B * (SHORT ? p.ns : 1);
     dim3 grid(n_items < num_sms ? n_items : num_sms);
-    kern<<<grid, kAttnThreads, smem, stream>>>(tq, tk, tv, to, p);
+    kern<<<grid, kFwdThreads, smem, stream>>>(tq, tk, tv, to, p);
     return cudaGetLastError();
 }
 
