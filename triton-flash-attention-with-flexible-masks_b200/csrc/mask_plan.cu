@@ -164,6 +164,108 @@ __global__ void __launch_bounds__(1024) plan_order_kernel(int32_t* plan, PlanLay
     }
 }
 
+// The three kernels above in one, for id rows of at most kSmallBlocks blocks: grid (He, B), 1024 threads. A warp takes a block
+// of 128 ids, its lane x the ids x, x + 32, x + 64 and x + 96; the block statistics pass through shared memory.
+// Bound by latency; the same words in the plan. us, in the three launches (their times alone, without the gaps of about 1 us
+// between them) and here: 16 blocks a row (4 x 1000 ids) 6.5, 3.4; 64 (4 x 4096) 7.6, 7.3; 72 (8 rows of 1024 and 8192) 8.6,
+// 9.1: beyond two blocks a warp the launches are no slower.
+constexpr int kSmallBlocks = 64;
+
+__device__ __forceinline__ int warp_min(int v) { return __reduce_min_sync(0xffffffffu, v); }
+__device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
+
+__global__ void __launch_bounds__(1024) plan_small_kernel(IdsView eq, IdsView ek, int32_t* plan, PlanLayout L, int gap, int causal,
+                                                          int* status) {
+    __shared__ int smin[kSmallBlocks], smax[kSmallBlocks], len[kSmallBlocks];  // query blocks, then key blocks
+    const int he = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t bh = int64_t(b) * L.He + he;
+    const int n = L.nQ + L.nK;
+    if (he == 0 && b == 0 && threadIdx.x < 128) plan[L.off_ctr + threadIdx.x] = 0;
+    for (int i = warp; i < n; i += 32) {
+        const bool is_q = i < L.nQ;
+        const int blk = is_q ? i : i - L.nQ, size = is_q ? L.M : L.N;
+        const IdsView& ids = is_q ? eq : ek;
+        long long id[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int l = blk * kBlk + e * 32 + lane;
+            id[e] = l < size ? load_id(ids, b, he, l) : 0;
+        }
+        int code[4], mn = 0x7fffffff, mx = int(-2147483647 - 1);
+        bool rise = false, fall = false, many = false;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int l = blk * kBlk + e * 32 + lane;
+            const bool valid = l < size, fits = id[e] >= -2147483648LL;
+            if (is_q) {
+                code[e] = !valid || id[e] >= 0 ? kCodeAny : fits ? int(id[e]) : int(-2147483647 - 1);
+                if (valid && !fits) atomicCAS(status, 0, ST_ID_RANGE);
+            } else {
+                code[e] = (valid && id[e] < 0 && fits) ? int(id[e]) : 0;
+            }
+            if (valid) {
+                mn = min(mn, code[e]);
+                mx = max(mx, code[e]);
+            }
+            plan[(is_q ? L.off_qc + bh * L.Mpad : L.off_kc + bh * L.Npad) + l] = code[e];
+            // against the code before: the lane's left neighbour, for lane 0 the last one of the 32 before
+            const int left = __shfl_up_sync(0xffffffffu, code[e], 1);
+            const int last = e > 0 ? __shfl_sync(0xffffffffu, code[e > 0 ? e - 1 : 0], 31) : code[e];
+            const int before = lane > 0 ? left : last;
+            if (lane > 0 || e > 0) {
+                rise |= code[e] > before;
+                fall |= code[e] < before;
+            }
+            const bool leads = __ffs(__match_any_sync(0xffffffffu, code[e])) - 1 == lane;
+            many |= __popc(__ballot_sync(0xffffffffu, leads)) > kWalkCodes;
+        }
+        mn = warp_min(mn);
+        mx = warp_max(mx);
+        const int flags = ((__any_sync(0xffffffffu, rise) && __any_sync(0xffffffffu, fall)) ? 0 : BF_MONO) | (many ? BF_MANY : 0);
+        if (lane == 0) {
+            smin[i] = mn;
+            smax[i] = mx;
+            const int64_t at = bh * (is_q ? L.nQ : L.nK) + blk;
+            plan[(is_q ? L.off_qflags : L.off_kflags) + at] = flags;
+            plan[(is_q ? L.off_qmin : L.off_kmin) + at] = mn;
+            plan[(is_q ? L.off_qmax : L.off_kmax) + at] = mx;
+        }
+    }
+    __syncthreads();
+    for (int i = warp; i < n; i += 32) {
+        const bool is_q = i < L.nQ;
+        const int blk = is_q ? i : i - L.nQ, n_other = is_q ? L.nK : L.nQ;
+        int lo = 0x7fffffff, hi = 0;
+        for (int o = lane; o < n_other; o += 32) {
+            const int qb = is_q ? blk : o, kb = is_q ? o : blk;
+            const uint32_t f = classify_tile(qb, kb, L.M, L.N, gap, causal, 1, smin[qb], smax[qb], smin[L.nQ + kb], smax[L.nQ + kb]);
+            if (f & TILE_VISIT) {
+                lo = min(lo, o);
+                hi = max(hi, o + 1);
+            }
+        }
+        lo = warp_min(lo);
+        hi = warp_max(hi);
+        if (hi == 0) lo = 0;
+        if (lane == 0) {
+            const int64_t at = bh * (is_q ? L.nQ : L.nK) + blk;
+            plan[(is_q ? L.off_kvlo : L.off_qlo) + at] = lo;
+            plan[(is_q ? L.off_kvhi : L.off_qhi) + at] = hi;
+            len[is_q ? L.nQ - 1 - blk : i] = hi - lo;  // natural position: query block nQ-1-i, key block i
+        }
+    }
+    __syncthreads();
+    const int i = threadIdx.x;  // order by counting, as in plan_order_kernel
+    if (i < n) {
+        const bool is_q = i < L.nQ;
+        const int first = is_q ? 0 : L.nQ, end = is_q ? L.nQ : n, li = len[i];
+        int rank = 0;
+        for (int j = first; j < end; ++j) rank += (len[j] > li) || (len[j] == li && j < i);
+        if (is_q) plan[L.off_ordq + bh * L.nQ + rank] = L.nQ - 1 - i;
+        else plan[L.off_ordk + bh * L.nK + rank] = i - L.nQ;
+    }
+}
+
 // grid (nK, nQ, B*He), 128 threads: one tile. A tile that the plan does not visit reports
 // keep = 0 everywhere, a tile without a flagged check reports keep = 1 for the entries that
 // check covers: exactly what the attention kernels assume.
@@ -203,6 +305,10 @@ cudaError_t launch_plan_build(const void* eq_ptr, const int64_t* eq_stride, int 
                               int causal, int* status, cudaStream_t stream) {
     IdsView q{eq_ptr, eq_stride[0], eq_stride[1], eq_stride[2], eq64};
     IdsView k{ek_ptr, ek_stride[0], ek_stride[1], ek_stride[2], ek64};
+    if (L.nQ + L.nK <= kSmallBlocks) {
+        plan_small_kernel<<<dim3(L.He, L.B), 1024, 0, stream>>>(q, k, plan, L, gap, causal, status);
+        return cudaGetLastError();
+    }
     dim3 grid(L.nQ + L.nK, L.He, L.B);
     plan_codes_kernel<<<grid, 128, 0, stream>>>(q, k, plan, L, status);
     plan_ranges_kernel<<<grid, 128, 0, stream>>>(plan, L, gap, causal);
