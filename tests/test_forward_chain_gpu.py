@@ -1,4 +1,4 @@
-"""The forward's chain of tiles: three score buffers, one accumulator, a reference maximum handed from tile to tile."""
+"""The forward's two chains of tiles: an accumulator and a running maximum each, merged at the end of an item."""
 import pytest
 import torch
 
@@ -63,3 +63,60 @@ def test_items_without_tiles_between_others(D):
     ref, absolute = reference(q, k, v, True, eq[:, None] == ids[None, :])
     check(o, ref, absolute, 16.0)
     assert not o[:, :, 256:512].any() and not o[:, :, 1280:1408].any()
+
+
+@pytest.mark.parametrize("tiles", [2, 5, 6])
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_both_chains_have_a_maximum_of_their_own(dtype, D, tiles):
+    """Each row sees one key in each of the last two tiles. Relative to their own chain's maximum both are an exact 1 in P,
+    whatever their scores are, so that P's rounding (2^-9 or 2^-12 of each) is not in the result, of which the values leave
+    little: what is left is the rounding of the result, and 2^-18 for scores and exponentials in fp32 (a score of 12 and
+    its multiple by log2(e) to 2^-21 each, the exponential to 2^-22, twice the value of one)."""
+    import flash_b200 as fb
+    B, H, M, N = 2, 80, 256, tiles * 128
+    q, k, v = (torch.zeros(B, H, n, D, device="cuda") for n in (M, N, N))
+    q[..., 0] = 1 + torch.arange(M, device="cuda") % 128 / 64
+    k[..., 0] = -200.0
+    first, second = N - 256 + 37, N - 128 + 90
+    k[:, :, first, 0], k[:, :, second, 0] = 3.0, 2.3125
+    v[:, :, first], v[:, :, second] = 1.0, -2.0
+    q, k, v = (x.to(dtype) for x in (q, k, v))
+    o = fb.attention(q, k, v, False, 1.0)
+    w = (0.6875 * q[..., :1].double()).exp()  # the first key's weight over the second's
+    ref = ((w - 2.0) / (w + 1.0)).expand(B, H, M, D)
+    unit = torch.finfo(dtype).eps / 2
+    err = (o.double() - ref).abs()
+    assert bool((err <= unit * ref.abs() * 1.01 + 2.0 ** -18).all()), err.max().item()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_values_behind_the_mask_of_a_whole_chain(value, D):
+    """A row with no key in a chain's tiles does not see what their values are, by the causal mask and by ids."""
+    import flash_b200 as fb
+    H = 4
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(1, H, n, D, generator=g, device="cuda").bfloat16() for n in (128, 192, 192))
+    v[:, :, 150] = value  # row i sees the keys up to i + 64: the first 64 rows have none in the second tile
+    o = fb.attention(q, k, v, True)
+    ref, absolute = reference(q[:, :, :64], k[:, :, :128], v[:, :, :128], True)
+    check(o[:, :, :64], ref, absolute, 16.0)
+    assert not torch.isfinite(o[:, :, 86:]).any()
+    q, k, v = (torch.randn(1, H, 256, D, generator=g, device="cuda").bfloat16() for _ in range(3))
+    ids = torch.where(torch.arange(256, device="cuda") < 100, -1, -2).expand(1, H, 256)
+    v[:, :, 200] = value  # the first 100 rows share their block with others that do have keys in the second tile
+    o = fb.attention(q, k, v, False, None, ids, ids, fb.SCORE_FUNC_MODE1_DOC)
+    check(o[:, :, :100], *reference(q[:, :, :100], k[:, :, :100], v[:, :, :100], False), 16.0)
+    assert not torch.isfinite(o[:, :, 100:]).any()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_row_whose_score_overflows_is_nan(D):
+    import flash_b200 as fb
+    q, k, v = (torch.randn(1, 4, 512, D, generator=torch.Generator(device="cuda").manual_seed(i), device="cuda").bfloat16() for i in range(3))
+    q[..., 0] = 4.0
+    k[:, :, 300] = 0.0
+    k[:, :, 300, 0] = 3e38  # a score of +inf for the rows that see this key
+    o = fb.attention(q, k, v, True)
+    assert bool(torch.isfinite(o[:, :, :300]).all()) and bool(torch.isnan(o[:, :, 300:]).all())

@@ -12,25 +12,28 @@
 //
 // 16 warps:
 //   warps 0-3  softmax group 0, warps 4-7 softmax group 1 (thread r of a group owns row r)
-//   warps 8-11 epilogue group: normalises a finished item's O, stages it and stores it
+//   warps 8-11 epilogue group: merges a finished item's two O, stages the result and stores it
 //   warp 12    TMA producer (Q per item, K and V rings that run across items; K ahead of V)
 //   warps 13,15 tcgen05.mma issuers, of P*V and of S; warp 13 owns the TMEM allocation
 //   warp 14    item scheduler: decodes the item, classifies its candidate tiles from the mask plan
 //              and compacts the visited ones into a list in shared memory (NQ item slots)
-// The CTA's g-th visited tile (counted across its items) belongs to softmax group g & 1 and uses score buffer g % 3;
-// all tiles of an item accumulate into one O. The groups share the row's reference maximum (it is handed from tile to
-// tile through shared memory, so P of every tile is relative to the same one), and each keeps the sum of its own tiles,
-// so the result does not depend on which group had the even ones. With three score buffers S(g+3) follows P*V(g)
-// on the pipe, a tile before a group asks for it: a group goes from one tile's exponentials straight to the next tile's scores.
-// (Before, each group had an O and a maximum of its own and one score buffer, waited for its own P*V and S between two
-// tiles, and drained O itself. Forward kernel, us, before and now: 512 queries against 8192 keys, 32 / 8 heads of 128, 63.6,
-// 59.5; 2 x 32 / 8 x 3001 x 128 causal 164, 153; 16 x 8 x 577 x 32 39.2, 35.1; 4 x 16 x 4096 x 128 in documents 153, 147;
-// 32 x 32768 x 128 in 64 documents 885, 848; 16 x 32 x 8192 x 128 causal 9185, 8370; 4 x 12 x 1000 x 64 in documents 27.2,
-// 27.1; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 84.7, 85.7: there the masks bound it.)
-// What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group: 2800 clocks
-// for two tiles) and, in dense calls, the clock under the power cap (1.4-1.5 GHz).
-// TMEM columns: S [0,384), three of 128; O [384,512), two of 64 for D = 64 (consecutive items), one of 128 for D = 128.
-// P (input dtype, two values per column) overwrites the first 64 columns of its S buffer.
+// The CTA's g-th visited tile (counted across its items) belongs to softmax group g & 1: two chains of tiles, each with a
+// running maximum, a sum and an accumulator O of its own for the item; the epilogue merges them, the chain of the item's even
+// tiles first, so that the result does not depend on which group that was. A chain in which a row had no key stays out of
+// the merge: what the values behind its mask are does not matter.
+// The next tile's scores are there when a group asks for them, so that it goes from one tile's exponentials straight to the
+// next: for D = 128 S has one buffer, free as soon as a group has its scores in registers, and P (input dtype, two values per
+// column) columns of its own, one place a chain; for D = 64 there are three buffers, P overwrites the first 64 columns of its
+// own, and S(g+3) follows P*V(g) on the pipe.
+// Forward kernel, us: two buffers in which P overwrites S, with the exponentials of the groups in turns | one O and one maximum
+// for both chains, three buffers | now. 2 x 32 / 8 heads x 3001 x 128 causal 198 | 157 | 154, with q and k of deviation 2
+// 261 | 330 | 228, of 4 263 | 355 | 238 (a shared maximum that moves makes either group wait for the other's P*V); 512 queries
+// against 8192 keys, 32 / 8 heads of 128, 80 | 64 | 64; 16 x 8 x 577 x 32 57 | 46 | 45; 4 x 16 x 4096 x 128 in documents
+// 176 | 147 | 152; 32 x 32768 x 128 in 64 documents 912 | 784 | 792; 16 x 32 x 8192 x 128 causal 9600 | 8000 | 8180; 4 x 12 x
+// 1000 x 64 in documents 44 | 39 | 38; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 107 | 95 | 89. The shared O
+// had errors 1 to 2 % larger as well: one entry of a row is an exact 1 in P, not one of each chain.
+// What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group) and, in
+// dense calls, the clock under the power cap (1.4-1.5 GHz); with short items the drain of two O, which the next item's P*V waits for.
 #include <type_traits>
 #include "common.cuh"
 #include "params.cuh"
@@ -42,7 +45,14 @@ struct FwdSmem {
     static constexpr int NS = (D == 128) ? 2 : 4;  // depth of the K ring and of the V ring
     // item slots; with more, items are dealt out too far ahead (3 or 4 for D = 64: 8 x 8 x 1024 x 8192 in documents 90, 86 with 2)
     static constexpr int NQ = 2;
-    static constexpr int NO = 128 / D;             // O accumulators
+    // TMEM columns: D = 128: S [0,128), two P of 64; D = 64: three S of 128, P in the first half of its S. Then the O of each chain.
+    // (Three S and two O of 128 do not fit; one S and two P for D = 64, too: 4 x 16 x 4096 x 64 causal 247 us for 223.)
+    static constexpr bool POWN = D == 128;   // P has columns of its own
+    static constexpr int NP = POWN ? 2 : 3;  // places for P
+    static constexpr int tmem_o = POWN ? 256 : 384;
+    static_assert(tmem_o + 2 * D <= 512, "TMEM columns");
+    static __device__ int tmem_s(int g) { return POWN ? 0 : g % 3 * 128; }
+    static __device__ int tmem_p(int g) { return POWN ? 128 + (g & 1) * 64 : g % 3 * 128; }
     static constexpr int TILE = kBlk * D * 2;
     static constexpr int BOX = kBlk * 64 * 2;
     static constexpr int NBOX = D / 64;
@@ -54,12 +64,11 @@ struct FwdSmem {
     static constexpr int off_qc = off_list + NQ * kListCap * 2;  // int32  [NQ][128] query codes
     static constexpr int off_kc = off_qc + NQ * kBlk * 4;        // int32  [NKC][128] key codes, loaded with K on K's barrier
     static constexpr int off_ml = off_kc + NKC * kBlk * 4;       // float  [NQ][2 groups][m, l][128]
-    static constexpr int off_m = off_ml + NQ * 4 * kBlk * 4;     // float  [128] the rows' reference maximum
-    static constexpr int off_info = off_m + kBlk * 4;  // int32 [NQ][8]: T, lo, item (-1: no more items), kv head, query block, head, batch
+    static constexpr int off_info = off_ml + NQ * 4 * kBlk * 4;  // int32 [NQ][8]: T, lo, item (-1: no more items), kv head, query block, head, batch
     static constexpr int off_bar = off_info + NQ * 32;
     // item_full[NQ] item_empty[NQ] q_full[NQ] q_empty[NQ] ml_full[NQ] staged[NQ] k_full[NS] k_empty[NS] v_full[NS] v_empty[NS]
-    // s_full[3] p_full[3] pv_done[3] m_ready[2] o_full[NO] o_free[NO]
-    static constexpr int n_bar = 6 * NQ + 4 * NS + 9 + 2 + 2 * NO;
+    // s_full[4] s_free[2] p_full[NP] pv_done[NP] o_full[2] o_free[2]
+    static constexpr int n_bar = 6 * NQ + 4 * NS + 6 + 2 * NP + 4;
     static constexpr int off_misc = off_bar + n_bar * 8;  // tmem slot, abort flag
     static constexpr int total = off_misc + 16;
 };
@@ -80,7 +89,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdParams p) {
     using S = FwdSmem<D>;
-    constexpr int NS = S::NS, NQ = S::NQ, NO = S::NO;
+    constexpr int NS = S::NS, NQ = S::NQ, NP = S::NP;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -100,9 +109,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     auto BAR = [&](int i) { return bar0 + 8u * uint32_t(i); };
     constexpr int B_ITEMFULL = 0, B_ITEMEMPTY = NQ, B_QFULL = 2 * NQ, B_QEMPTY = 3 * NQ, B_MLFULL = 4 * NQ, B_STAGED = 5 * NQ, B_KFULL = 6 * NQ,
                   B_KEMPTY = B_KFULL + NS, B_VFULL = B_KEMPTY + NS, B_VEMPTY = B_VFULL + NS, B_SFULL = B_VEMPTY + NS,
-                  B_PFULL = B_SFULL + 3, B_PVDONE = B_PFULL + 3, B_MREADY = B_PVDONE + 3, B_OFULL = B_MREADY + 2,
-                  B_OFREE = B_OFULL + NO;
-    static_assert(B_OFREE + NO == S::n_bar, "barriers");
+                  B_SFREE = B_SFULL + 4, B_PFULL = B_SFREE + 2, B_PVDONE = B_PFULL + NP, B_OFULL = B_PVDONE + NP, B_OFREE = B_OFULL + 2;
+    static_assert(B_OFREE + 2 == S::n_bar, "barriers");
     Abort ab{misc + 1, p.status, p.wait_limit};
 
     if (tid == 0) {
@@ -120,15 +128,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             mbar_init(BAR(B_VFULL + s), 1);
             mbar_init(BAR(B_VEMPTY + s), 1);
         }
-        for (int s = 0; s < 3; ++s) {
-            mbar_init(BAR(B_SFULL + s), 1);
+        for (int s = 0; s < 4; ++s) mbar_init(BAR(B_SFULL + s), 1);
+        for (int s = 0; s < NP; ++s) {
             mbar_init(BAR(B_PFULL + s), 4);  // here and below: one arrival a warp
             mbar_init(BAR(B_PVDONE + s), 1);
         }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(BAR(B_MREADY + s), 4);
-        }
-        for (int s = 0; s < NO; ++s) {
+            mbar_init(BAR(B_SFREE + s), 4);
             mbar_init(BAR(B_OFULL + s), 1);
             mbar_init(BAR(B_OFREE + s), 4);
         }
@@ -302,8 +308,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     if (!ok) break;
                     // The tile's key codes travel with K: they land in a ring of NKC slots and complete on
                     // K's barrier, so whoever has seen S(g) (computed after that barrier) may read them.
-                    // Slot g % NKC was last read by the softmax of tile g - NKC, which is over: S(g - NS), which
-                    // has just released K's stage, was issued behind P*V(g - NS - 3).
+                    // Slot g % NKC was last read by the softmax of tile g - NKC, which is over: S(g - NS), which has just
+                    // released K's stage, was issued behind P*V(g - NS - 3) or, where P has columns of its own, when both groups had
+                    // read the scores of tiles g - NS - 1 and g - NS - 2, hence were done with those up to g - NS - 3.
                     static_assert(S::NKC >= NS + 3, "key-code ring");
                     mbar_expect_tx_elect(BAR(B_KFULL + st), S::TILE + (mk.mode == 1 ? kBlk * 4 : 0));
                     for (int x = 0; x < S::NBOX; ++x)
@@ -328,14 +335,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         } else {
             // ------------------------------ MMA issuers ------------------------------
             //   warp 13: P*V(g) when P(g) is there
-            //   warp 15: S(g), up to three tiles ahead: S(g) overwrites the buffer that P(g - 3) was read from
+            //   warp 15: S(g) when its buffer is free
             // Two warps, so that S of a later tile (and of the next item's first ones) never waits behind P of this one.
             const uint32_t utmem = uniform(int(tmem));
             constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
             constexpr uint32_t idesc_pv = make_idesc(BF16, 128, D, false, true);
             constexpr uint64_t desc_v = desc_mn_major(S::BOX);
             bool ok = true;
-            int g = 0, no = 0;  // tiles; items with tiles
+            int G = 0;           // tiles of all earlier items
+            int n0 = 0, n1 = 0;  // items in which the chains had tiles
             for (int k = 0;; ++k) {
                 const int s = k % NQ, use = k / NQ;
                 ok = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
@@ -344,44 +352,49 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 if (uniform(info[s * 8 + 2]) < 0) break;
                 if (warp == 15) {
                     if (T > 0) ok = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 3);
-                    for (int t = 0; t < T && ok; ++t, ++g) {
-                        const int buf = g % 3, st = g % NS;
+                    for (int g = G; g < G + T && ok; ++g) {
+                        const int st = g % NS;
                         ok = mbar_wait_warp(BAR(B_KFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 4);
-                        if (ok && g >= 3) ok = mbar_wait_warp(BAR(B_PVDONE + buf), (g / 3 - 1) & 1, ab, ST_WAIT_TIMEOUT + 15);
+                        // the buffer: its scores have been read, or the P that took their place
+                        if (S::POWN && ok && g > 0) ok = mbar_wait_warp(BAR(B_SFREE + ((g - 1) & 1)), ((g - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 15);
+                        if (!S::POWN && ok && g >= NP) ok = mbar_wait_warp(BAR(B_PVDONE + g % NP), (g / NP - 1) & 1, ab, ST_WAIT_TIMEOUT + 15);
                         if (!ok) break;
                         tc_fence_after();
-                        const uint32_t tS = utmem + uint32_t(buf) * 128u, q_tile = sQ(s), k_tile = sK(st);
+                        const uint32_t tS = utmem + uint32_t(S::tmem_s(g)), q_tile = sQ(s), k_tile = sK(st);
 #pragma unroll
                         for (int kk = 0; kk < D / 16; ++kk) {
                             const uint32_t off = uint32_t(kk >> 2) * S::BOX + uint32_t(kk & 3) * 32u;
                             umma_ss(tS, smem_desc_at(kDescKMajor, q_tile + off), smem_desc_at(kDescKMajor, k_tile + off), idesc_s, kk > 0);
                         }
                         umma_commit(BAR(B_KEMPTY + st));
-                        umma_commit(BAR(B_SFULL + buf));
+                        umma_commit(BAR(B_SFULL + (g & 3)));
                     }
                 } else {
-                    const int o = no % NO;
-                    const uint32_t tO = utmem + 384u + uint32_t(o * D);
-                    for (int t = 0; t < T; ++t, ++g) {
-                        const int buf = g % 3, st = g % NS;
-                        const uint32_t tP = utmem + uint32_t(buf) * 128u, v_tile = sV(st);
+                    for (int t = 0; t < T; ++t) {
+                        const int g = G + t, st = g % NS, w = g & 1;
+                        const uint32_t tO = utmem + uint32_t(S::tmem_o + w * D), tP = utmem + uint32_t(S::tmem_p(g)), v_tile = sV(st);
                         ok = mbar_wait_warp(BAR(B_VFULL + st), (g / NS) & 1, ab, ST_WAIT_TIMEOUT + 5);
-                        // the first P*V of an item overwrites O: the epilogue of the last item that used it must have read it
-                        if (ok && t == 0 && no >= NO) ok = mbar_wait_warp(BAR(B_OFREE + o), (no / NO - 1) & 1, ab, ST_WAIT_TIMEOUT + 14);
-                        if (ok) ok = mbar_wait_warp(BAR(B_PFULL + buf), (g / 3) & 1, ab, ST_WAIT_TIMEOUT + 6);
+                        // The first P*V of a chain in an item overwrites its O: the epilogue of the last item that used it must have
+                        // read it. (o_full and o_free count the items in which the chain had tiles, on both sides.)
+                        const int n = w ? n1 : n0;
+                        if (ok && t < 2 && n > 0) ok = mbar_wait_warp(BAR(B_OFREE + w), (n - 1) & 1, ab, ST_WAIT_TIMEOUT + 14);
+                        if (ok) ok = mbar_wait_warp(BAR(B_PFULL + g % NP), (g / NP) & 1, ab, ST_WAIT_TIMEOUT + 6);
                         if (!ok) break;
                         tc_fence_after();
 #pragma unroll
                         for (int kk = 0; kk < 8; ++kk)
                             umma_ts(tO, tP + uint32_t(kk) * 8u, smem_desc_at(desc_v, v_tile + uint32_t(kk) * 2048u), idesc_pv,
-                                    (t > 0 || kk > 0) ? 1u : 0u);
+                                    (t > 1 || kk > 0) ? 1u : 0u);
                         umma_commit(BAR(B_VEMPTY + st));
-                        umma_commit(BAR(B_PVDONE + buf));
-                        if (t == T - 1) umma_commit(BAR(B_OFULL + o));
+                        umma_commit(BAR(B_PVDONE + g % NP));
+                        if (t + 2 >= T) {  // the chain's last tile
+                            umma_commit(BAR(B_OFULL + w));
+                            if (w) ++n1; else ++n0;
+                        }
                     }
                 }
                 if (!ok) break;
-                if (T > 0) ++no;
+                G += T;
                 if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
                 __syncwarp();
             }
@@ -394,8 +407,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
         const float c = p.scale_log2;
         bool alive = !aborted;
-        int G = 0;   // tiles of all earlier items
-        int no = 0;  // items with tiles
+        int G = 0;           // tiles of all earlier items
+        int n0 = 0, n1 = 0;  // items in which the chains of group 0 and 1 had tiles
         for (int k = 0; alive; ++k) {
             const int s = k % NQ, use = k / NQ;
             alive = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
@@ -409,19 +422,23 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             alive = mbar_wait_warp(BAR(B_MLFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 16);
             // an item without tiles: nobody has waited for its Q load yet, and its slot is about to become the staging area
             if (alive && T == 0) alive = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 17);
-            const int o = no % NO;
-            if (alive && T > 0) alive = mbar_wait_warp(BAR(B_OFULL + o), (no / NO) & 1, ab, ST_WAIT_TIMEOUT + 9);
+            const int we = G & 1;  // the chain that had the item's even tiles: index 0 below, 1 the other one
+            const int i0 = we ? n1 : n0, i1 = we ? n0 : n1;
+            if (alive && T > 0) alive = mbar_wait_warp(BAR(B_OFULL + we), i0 & 1, ab, ST_WAIT_TIMEOUT + 9);
+            if (alive && T > 1) alive = mbar_wait_warp(BAR(B_OFULL + (we ^ 1)), i1 & 1, ab, ST_WAIT_TIMEOUT + 9);
             if (!alive) break;
             tc_fence_after();
             const float* ml = reinterpret_cast<const float*>(smem + S::off_ml) + s * (4 * kBlk);  // [2 groups][m, l][128]
-            const int even = (G & 1) * (2 * kBlk), odd = 2 * kBlk - even;  // the groups that had the even and the odd tiles
+            const int even = we * (2 * kBlk), odd = 2 * kBlk - even;
             const float m0 = ml[even + r], l0 = ml[even + kBlk + r], m1 = ml[odd + r], l1 = ml[odd + kBlk + r];
             const float mt = fmaxf(m0, m1);
             const float a0 = (m0 == -INFINITY) ? 0.f : fast_exp2((m0 - mt) * c);
             const float a1 = (m1 == -INFINITY) ? 0.f : fast_exp2((m1 - mt) * c);
             const float lt = l0 * a0 + l1 * a1;
             const float inv = (lt > 0.f) ? 1.0f / lt : 0.f;
-            const bool used = (T > 0) && inv != 0.f;
+            const float f0 = a0 * inv, f1 = a1 * inv;
+            // a chain in which the row had no key takes no part, whatever the values behind its mask are
+            const bool use0 = (T > 0) && (f0 != 0.f), use1 = (T > 1) && (f1 != 0.f);
             const bool healthy = misc[1] == 0;
             if (healthy) {
                 const float lse = (lt > 0.f) ? fmaf(mt, c, log2f(lt)) : -INFINITY;
@@ -448,35 +465,44 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             // The O tile is staged in this item's Q slot (Q is dead: every S MMA of the item has completed) in the
             // 128-byte-swizzled layout of the tensor map.
             uint8_t* stage = smem + S::off_q + s * S::TILE;
+            const uint32_t tO0 = tmem + lane_base + uint32_t(S::tmem_o + we * D), tO1 = tmem + lane_base + uint32_t(S::tmem_o + (we ^ 1) * D);
 #pragma unroll
-            for (int q = 0; q < D / 32; ++q) {
-                uint32_t x[32];
+            for (int q = 0; q < D / 16; ++q) {
+                uint32_t x0[16], x1[16];
                 // tcgen05.ld is warp-collective: always executed, the values are ignored when unused
-                tmem_ld32(tmem + lane_base + 384u + uint32_t(o * D) + uint32_t(q) * 32u, x);
+                tmem_ld16(tO0 + uint32_t(q) * 16u, x0);
+                tmem_ld16(tO1 + uint32_t(q) * 16u, x1);
                 tc_wait_ld();
-                if (q == D / 32 - 1) {  // O has been read: the MMA issuer may start another item's P*V
+                if (q == D / 16 - 1) {  // O has been read: the MMA issuers may start another item's P*V
                     tc_fence_before();
-                    if (T > 0) mbar_arrive_warp(BAR(B_OFREE + o), lane);
+                    if (T > 0) mbar_arrive_warp(BAR(B_OFREE + we), lane);
+                    if (T > 1) mbar_arrive_warp(BAR(B_OFREE + (we ^ 1)), lane);
                 }
 #pragma unroll
-                for (int y = 0; y < 32; ++y) x[y] = used ? __float_as_uint(__uint_as_float(x[y]) * inv) : 0u;
+                for (int y = 0; y < 16; ++y) {
+                    float v = 0.f;
+                    if (use0) v = __uint_as_float(x0[y]) * f0;
+                    if (use1) v = fmaf(__uint_as_float(x1[y]), f1, v);
+                    x0[y] = __float_as_uint(v);
+                }
                 if constexpr (SHORT) {
                     if (part) {
 #pragma unroll
-                        for (int y = 0; y < 8; ++y)
-                            *reinterpret_cast<uint4*>(part + 32 * q + 4 * y) = make_uint4(x[4 * y], x[4 * y + 1], x[4 * y + 2], x[4 * y + 3]);
+                        for (int y = 0; y < 4; ++y)
+                            *reinterpret_cast<uint4*>(part + 16 * q + 4 * y) = make_uint4(x0[4 * y], x0[4 * y + 1], x0[4 * y + 2], x0[4 * y + 3]);
                     }
                 }
-                auto two = [&](int y) { return pack2<BF16>(__uint_as_float(x[y]), __uint_as_float(x[y + 1])); };
+                auto two = [&](int y) { return pack2<BF16>(__uint_as_float(x0[y]), __uint_as_float(x0[y + 1])); };
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int cg = 4 * q + i;  // 16-byte chunk of the row
+                for (int i = 0; i < 2; ++i) {
+                    const int cg = 2 * q + i;  // 16-byte chunk of the row
                     uint4* dst = reinterpret_cast<uint4*>(stage + (cg >> 3) * S::BOX + r * 128 + (((cg & 7) ^ (r & 7)) << 4));
                     *dst = make_uint4(two(8 * i), two(8 * i + 2), two(8 * i + 4), two(8 * i + 6));
                 }
             }
             G += T;
-            if (T > 0) ++no;
+            n0 += (we ? T > 1 : T > 0) ? 1 : 0;
+            n1 += (we ? T > 0 : T > 1) ? 1 : 0;
             fence_proxy_async();
             mbar_arrive_warp(BAR(B_STAGED + s), lane);
             if (warp == 8) alive = mbar_wait_warp(BAR(B_STAGED + s), use & 1, ab, ST_WAIT_TIMEOUT + 18);
@@ -509,10 +535,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         const int r = tid & 127;  // row inside the block
         const uint32_t lane_base = uint32_t((warp & 3) * 32) << 16;
         const float c = p.scale_log2;
-        float* m_row = reinterpret_cast<float*>(smem + S::off_m) + r;
+        const uint32_t tO = tmem + lane_base + uint32_t(S::tmem_o + w * D);
         bool alive = !aborted;
-        int G = 0;   // tiles of all earlier items
-        int no = 0;  // items with tiles
+        int G = 0;  // tiles of all earlier items
         for (int k = 0; alive; ++k) {
             const int s = k % NQ, use = k / NQ;
             alive = mbar_wait_warp(BAR(B_ITEMFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 12);
@@ -528,34 +553,37 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             const bool valid = !SHORT || (row < mk.M && g_row < p.pack && (info[s * 8 + 5] % nG) * p.pack + g_row < p.G);
             const bool active = !SHORT || __any_sync(0xffffffffu, valid);  // does this warp hold a query at all?
             const int qc = reinterpret_cast<const int*>(smem + S::off_qc)[s * kBlk + r];
-            const uint32_t tO = tmem + lane_base + 384u + uint32_t((no % NO) * D);
-            bool ready = false;  // the scores of the next tile are known to be there
-            float m_run = -INFINITY, l_run = 0.f;  // l_run: sum of this group's tiles relative to m_run
+            const int t0 = (G ^ w) & 1;  // this group's first tile of the item
+            float m_run = -INFINITY, l_run = 0.f;
 
-            for (int t = (G ^ w) & 1; t < T && alive; t += 2) {
-                const int g = G + t, buf = g % 3;
-                const uint32_t tS = tmem + lane_base + uint32_t(buf) * 128u;
+            for (int t = t0; t < T && alive; t += 2) {
                 const uint32_t entry = list[t];
                 const uint32_t fl = entry >> 10;
                 const int k0 = (lo + int(entry & 1023u)) * kBlk;
-                if (!ready) alive = mbar_wait_warp(BAR(B_SFULL + buf), (g / 3) & 1, ab, ST_WAIT_TIMEOUT + 7);
+                const int g = G + t;
+                const uint32_t tS = tmem + lane_base + uint32_t(S::tmem_s(g)), tP = tmem + lane_base + uint32_t(S::tmem_p(g));
+                // P*V of the group's tile before: it has read its P and added to O
+                auto pv_before = [&] { return g < 2 || mbar_wait_warp(BAR(B_PVDONE + (g - 2) % NP), ((g - 2) / NP) & 1, ab, ST_WAIT_TIMEOUT + 8); };
+                alive = mbar_wait_warp(BAR(B_SFULL + (g & 3)), (g >> 2) & 1, ab, ST_WAIT_TIMEOUT + 7);
                 if (!alive) break;
-                ready = false;
                 tc_fence_after();
                 if (SHORT && !active) {  // no row of this warp is a query: its lanes of P and O are never stored
-                    if (g > 0) alive = mbar_wait_warp(BAR(B_MREADY + (w ^ 1)), ((g - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 10);
-                    if (!alive) break;
-                    mbar_arrive_warp(BAR(B_MREADY + w), lane);
-                    mbar_arrive_warp(BAR(B_PFULL + buf), lane);
+                    if (S::POWN) {
+                        mbar_arrive_warp(BAR(B_SFREE + w), lane);
+                        alive = pv_before();
+                        if (!alive) break;
+                    }
+                    mbar_arrive_warp(BAR(B_PFULL + g % NP), lane);
                     continue;
                 }
                 uint32_t sr[128];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) tmem_ld32(tS + uint32_t(q) * 32u, sr + q * 32);
-                // (asked early as well; needed once this tile's maximum is known)
-                const bool m_there = g == 0 || mbar_test_warp(BAR(B_MREADY + (w ^ 1)), ((g - 1) >> 1) & 1);
-                float m_prev = (m_there && t > 0) ? *m_row : -INFINITY;
                 tc_wait_ld();
+                if (S::POWN) {
+                    tc_fence_before();
+                    mbar_arrive_warp(BAR(B_SFREE + w), lane);  // the next tile's scores may overwrite these
+                }
                 float* sc = reinterpret_cast<float*>(sr);
 
                 if (fl & (TILE_BOUND | TILE_DOC)) {
@@ -570,7 +598,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         lim = jmax - k0;
                     }
                     const bool doc = (fl & TILE_DOC) && qc < 0;  // a row with qc >= 0 passes the id check everywhere
-                    const int* kcs = reinterpret_cast<const int*>(smem + S::off_kc + ((G + t) % S::NKC) * (kBlk * 4));
+                    const int* kcs = reinterpret_cast<const int*>(smem + S::off_kc + (g % S::NKC) * (kBlk * 4));
                     // (the key codes completed on K's barrier, before the S MMA whose result was just read)
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -619,38 +647,38 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 #pragma unroll
                 for (int a = 0; a < 8; ++a) mxa[a] = fmaxf(mxa[a], sc[120 + a]);
                 const float mx = fmaxf(max3(mxa[0], mxa[1], mxa[2]), max3(max3(mxa[3], mxa[4], mxa[5]), mxa[6], mxa[7]));
-                // The reference maximum comes from the tile before (the other group's) and goes to the tile after. Every
-                // tile waits, also an item's first, so that neither group is ever two phases ahead of the other's wait.
-                if (!m_there) {
-                    alive = mbar_wait_warp(BAR(B_MREADY + (w ^ 1)), ((g - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 10);
-                    if (!alive) break;
-                    if (t > 0) m_prev = *m_row;
-                }
+                float m_new = fmaxf(m_run, mx);
                 // lazy rescale: keep the old reference point while the new maximum is within 2^8 of it
-                float m_new = fmaxf(m_prev, mx);
-                const bool need = (m_new - m_prev) * c > 8.0f;
-                if (!need) m_new = m_prev;
-                *m_row = m_new;
-                mbar_arrive_warp(BAR(B_MREADY + w), lane);
-                // O is 0 in a row that had no key yet: nothing to rescale there
-                const bool rescale = need && m_prev != -INFINITY;
-                if (__any_sync(0xffffffffu, rescale)) {
-                    const float alpha = rescale ? fast_exp2((m_prev - m_new) * c) : 1.0f;
-                    alive = mbar_wait_warp(BAR(B_PVDONE + (g - 1) % 3), ((g - 1) / 3) & 1, ab, ST_WAIT_TIMEOUT + 8);
+                const bool need = (m_new - m_run) * c > 8.0f;
+                if (!need) m_new = m_run;
+                if (S::POWN) {  // this tile's P overwrites that one's
+                    alive = pv_before();
                     if (!alive) break;
                     tc_fence_after();
-#pragma unroll
-                    for (int q = 0; q < D / 16; ++q) {
-                        uint32_t orr[16];
-                        tmem_ld16(tO + uint32_t(q) * 16u, orr);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
-                        tmem_st16(tO + uint32_t(q) * 16u, orr);
-                    }
-                    tc_wait_st();
                 }
-                const float mneg = (m_new == -INFINITY) ? 0.f : -m_new * c;
+                if (__any_sync(0xffffffffu, need)) {
+                    const float alpha = need ? fast_exp2((m_run - m_new) * c) : 1.0f;
+                    l_run *= alpha;
+                    if (t > t0) {
+                        if (!S::POWN) {
+                            alive = pv_before();
+                            if (!alive) break;
+                            tc_fence_after();
+                        }
+#pragma unroll
+                        for (int q = 0; q < D / 16; ++q) {
+                            uint32_t orr[16];
+                            tmem_ld16(tO + uint32_t(q) * 16u, orr);
+                            tc_wait_ld();
+#pragma unroll
+                            for (int x = 0; x < 16; ++x) orr[x] = __float_as_uint(__uint_as_float(orr[x]) * alpha);
+                            tmem_st16(tO + uint32_t(q) * 16u, orr);
+                        }
+                        tc_wait_st();
+                    }
+                }
+                m_run = m_new;
+                const float mneg = (m_run == -INFINITY) ? 0.f : -m_run * c;
                 // exp2(s*c - m*c) on packed pairs
                 const uint64_t c2 = pack_f2(c, c), mneg2 = pack_f2(mneg, mneg);
                 uint64_t lacc0 = pack_f2(0.f, 0.f), lacc1 = lacc0;
@@ -666,21 +694,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         if (x & 1) lacc1 = add_f2(lacc1, pack_f2(p0, p1)); else lacc0 = add_f2(lacc0, pack_f2(p0, p1));
                         pk[x] = pack2<BF16>(p0, p1);
                     }
-                    tmem_st16(tS + uint32_t(q) * 16u, pk);
+                    tmem_st16(tP + uint32_t(q) * 16u, pk);
                 }
                 tc_wait_st();
                 tc_fence_before();
-                mbar_arrive_warp(BAR(B_PFULL + buf), lane);
-                // (asked here, the answer is there when the next tile starts: about 100 clocks less than a wait for a barrier
-                // that has completed already)
-                ready = t + 2 < T && mbar_test_warp(BAR(B_SFULL + (g + 2) % 3), ((g + 2) / 3) & 1);
+                mbar_arrive_warp(BAR(B_PFULL + g % NP), lane);
                 {
                     float a0, a1, b0, b1;
                     unpack_f2(lacc0, a0, a1);
                     unpack_f2(lacc1, b0, b1);
-                    // the sum so far follows the reference (the other group's tile may have moved it, too)
-                    if (m_new != m_run) l_run *= (m_run == -INFINITY) ? 0.f : fast_exp2((m_run - m_new) * c);
-                    m_run = m_new;
                     l_run += (a0 + a1) + (b0 + b1);
                 }
             }
@@ -690,7 +712,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             ml[kBlk] = l_run;
             mbar_arrive_warp(BAR(B_MLFULL + s), lane);
             G += T;
-            if (T > 0) ++no;
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR(B_ITEMEMPTY + s));
         }
