@@ -61,3 +61,15 @@ def test_autograd_forms():
         fb.attention(q, k, v, True, 0.0)
     with pytest.raises(AssertionError):
         fb.attention(q, k[:, :, :32], v[:, :, :32], True)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_negative_number_of_runs_is_refused(dtype):
+    import flash_b200 as fb
+    q, k, v = (torch.randn(1, 4, 300, 64, device="cuda").to(dtype) for _ in range(3))
+    o = fb.attention(q, k, v, True)
+    for x in (q, torch.cat([q, q[..., :4]], 3)[..., :64]):  # the native call, the general code
+        for runs in (-1, -3):
+            with pytest.raises(RuntimeError, match="bad argument"):
+                fb.attention_in_runs(x, k, v, runs, True)
+        assert torch.equal(fb.attention_in_runs(x, k, v, 0, True), o)  # 0: as `attention` chooses

@@ -80,7 +80,7 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, bool prepa
         if (!taken_as_is(o)) o = at::empty(q.sizes(), q.options());
         const auto f32 = q.options().dtype(at::kFloat);
         lse = at::empty({p.B, p.H, fa_padded_rows(p.M)}, f32);
-        splits = key_runs > 0 ? key_runs : fa_fwd_splits(&p);
+        splits = key_runs != 0 ? key_runs : fa_fwd_splits(&p);  // (a number below 1 is the library's to refuse)
         Tensor work;
         size_t bytes = 0;
         if (splits > 1) {
