@@ -73,3 +73,18 @@ def test_a_negative_number_of_runs_is_refused(dtype):
             with pytest.raises(RuntimeError, match="bad argument"):
                 fb.attention_in_runs(x, k, v, runs, True)
         assert torch.equal(fb.attention_in_runs(x, k, v, 0, True), o)  # 0: as `attention` chooses
+
+
+@pytest.mark.parametrize("kind", [float, bool, torch.tensor])
+def test_the_mode_may_be_any_number(kind):
+    import flash_b200 as fb
+    q, k, v, do = (torch.randn(1, 4, 300, 64, device="cuda").bfloat16() for _ in range(4))
+    ids = (-1 - torch.arange(300, device="cuda") // 70).expand(1, 4, 300)
+
+    def step(e, mode):
+        x = [t.clone().requires_grad_() for t in (q, k, v)]
+        o = fb.attention(*x, True, None, e, e, mode)
+        return (o.detach(), *torch.autograd.grad(o, x, do))
+
+    for e, mode in ((None, 0), (ids, 0), (ids, 1)):
+        assert all(torch.equal(a, b) for a, b in zip(step(e, kind(mode)), step(e, mode)))

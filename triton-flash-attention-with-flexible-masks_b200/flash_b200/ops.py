@@ -205,7 +205,7 @@ class FlashAttention(torch.autograd.Function):
                 and (sm_scale is None or type(sm_scale) is float) and all(isinstance(x, torch.Tensor) for x in (q, k, v))):
             status = _STATUS.get(q.get_device())
             if status is not None:  # regular calls without ids and without need of a plan: one native call
-                done = host.forward(q, k, v, False, bool(causal), sm_scale, score_func_mode, 1, None, needs_grad, key_runs or 0, status)
+                done = host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs or 0, status)
         if done is None:
             # checks of flash_triton.py:510-520
             Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
@@ -222,6 +222,7 @@ class FlashAttention(torch.autograd.Function):
             if eq is None:
                 assert score_func_mode == SCORE_FUNC_MODE0_NOPE
             assert score_func_mode in (SCORE_FUNC_MODE0_NOPE, SCORE_FUNC_MODE1_DOC)
+            score_func_mode = int(score_func_mode)
             if not q.is_cuda:
                 raise RuntimeError("flash_b200 runs on CUDA tensors only (there is no CPU implementation)")
             device = q.device
@@ -264,7 +265,7 @@ class FlashAttention(torch.autograd.Function):
         ctx.plan = plan
         ctx.id_heads = id_heads
         ctx.causal = causal
-        ctx.score_func_info = (score_func_mode, )
+        ctx.score_func_info = (int(score_func_mode), )
         ctx.n_other = 5 if key_runs is None else 6  # inputs that are not q, k, v
         return Out
 
