@@ -88,3 +88,25 @@ def test_the_mode_may_be_any_number(kind):
 
     for e, mode in ((None, 0), (ids, 0), (ids, 1)):
         assert all(torch.equal(a, b) for a, b in zip(step(e, kind(mode)), step(e, mode)))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_longer_keys_and_values_are_read_as_far_as_the_call_goes(dtype):
+    import flash_b200 as fb
+    B, H, Hk, M, N, D = 2, 4, 2, 200, 230, 64
+    q, k, v, do = (torch.randn(b, h, n, D, device="cuda").to(dtype) for b, h, n in ((B, H, M), (B + 1, Hk, N), (B + 2, Hk, N + 10), (B, H, M)))
+
+    def step(k, v):
+        x = q.clone().requires_grad_()
+        o = fb.attention(x, k, v, True)
+        return o.detach(), *torch.autograd.grad(o, x, do)
+
+    assert all(torch.equal(a, b) for a, b in zip(step(k, v), step(k[:B], v[:B, :, :N])))
+    for x in (k, v):  # a gradient of theirs would have the wrong shape
+        with pytest.raises(RuntimeError, match="invalid gradient"):
+            x.requires_grad_()
+            fb.attention(q, k, v, True).backward(do)
+        x.requires_grad_(False)
+    for a, b in ((k[:1], v), (k, v[:1]), (k, v[:, :, :N - 1])):
+        with pytest.raises(RuntimeError):
+            fb.attention(q, a, b, True)

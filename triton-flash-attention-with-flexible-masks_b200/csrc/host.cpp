@@ -46,7 +46,8 @@ bool plain_cuda(const Tensor& t) {
 }
 
 // Fills `p`, or says that the call is not a regular one on the current device. `prepared`: ops.maybe_contiguous has seen the
-// tensors already, and what the library does not take of what it returned the library refuses.
+// tensors already, and what the library does not take of what it returned the library refuses. There k and v may have more
+// batches, and v more keys, than q and k ask for: the first ones are read.
 bool regular(const Tensor& q, const Tensor& k, const Tensor& v, bool prepared, bool causal, double sm_scale, int mode, int id_heads,
              fa_problem& p) {
     if (!plain_cuda(q) || !plain_cuda(k) || !plain_cuda(v)) return false;
@@ -55,7 +56,8 @@ bool regular(const Tensor& q, const Tensor& k, const Tensor& v, bool prepared, b
     if (k.device() != q.device() || v.device() != q.device() || q.get_device() != c10::cuda::current_device()) return false;
     const int64_t B = q.size(0), H = q.size(1), M = q.size(2), D = q.size(3), Hk = k.size(1), N = k.size(2);
     if (D != 16 && D != 32 && D != 64 && D != 128) return false;
-    if (k.sizes() != v.sizes() || k.size(0) != B || k.size(3) != D) return false;
+    if (k.size(3) != D || v.size(1) != Hk || v.size(3) != D) return false;
+    if (prepared ? k.size(0) < B || v.size(0) < B || v.size(2) < N : k.size(0) != B || v.size(0) != B || v.size(2) != N) return false;
     if (B < 1 || H < 1 || M < 1 || Hk < 1 || N < 1 || B > 65535 || H > 65535 || M > INT32_MAX || N > INT32_MAX) return false;
     if (H % Hk != 0 || (causal && N < M) || !(sm_scale > 0)) return false;
     if (!prepared && (!taken_as_is(q) || !taken_as_is(k) || !taken_as_is(v))) return false;
@@ -107,8 +109,8 @@ py::object backward(const Tensor& d_o, const Tensor& q, const Tensor& k, const T
     {
         py::gil_scoped_release free;
         Tensor delta = at::empty_like(lse);
-        dk = at::empty(k.sizes(), k.options());
-        dv = at::empty(v.sizes(), v.options());
+        dk = at::empty({p.B, p.Hk, p.N, p.D}, k.options());
+        dv = at::empty({p.B, p.Hk, p.N, p.D}, v.options());
         dq = at::empty(q.sizes(), q.options());
         const fa_tensor tq = view(q), tk = view(k), tv = view(v), to = view(o), tdo = view(d_o), tdq = view(dq), tdk = view(dk),
                         tdv = view(dv);
