@@ -110,3 +110,19 @@ def test_longer_keys_and_values_are_read_as_far_as_the_call_goes(dtype):
     for a, b in ((k[:1], v), (k, v[:1]), (k, v[:, :, :N - 1])):
         with pytest.raises(RuntimeError):
             fb.attention(q, a, b, True)
+
+
+class _Tagged(torch.Tensor):
+    pass
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_a_tensor_subclass_gives_one(mode):
+    import flash_b200 as fb
+    q, k, v = (torch.randn(2, 4, 200, 64, device="cuda").bfloat16() for _ in range(3))
+    ids = (-1 - torch.arange(200, device="cuda") // 70).expand(2, 4, 200) if mode else None
+    want = fb.attention(q, k, v, True, None, ids, ids, mode)
+    for x in (q, q.transpose(1, 2).contiguous().transpose(1, 2), torch.cat([q, q[..., :4]], 3)[..., :64]):
+        o = fb.attention(x.as_subclass(_Tagged), k, v, True, None, ids, ids, mode)
+        assert type(o) is _Tagged and torch.equal(o.as_subclass(torch.Tensor), want)
+    assert type(fb.attention(torch.nn.Parameter(q), k, v, True, None, ids, ids, mode)) is torch.Tensor

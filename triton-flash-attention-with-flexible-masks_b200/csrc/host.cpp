@@ -67,9 +67,11 @@ bool regular(const Tensor& q, const Tensor& k, const Tensor& v, bool prepared, b
 
 void* current_stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
-// (o, lse, scale, kernels launched), or None. Unprepared calls without a plan are taken only if it would gain nothing.
+// (o, lse, scale, kernels launched), or None. Unprepared calls without a plan are taken only if it would gain nothing. `out`: a
+// tensor like q for the result, given where q is of a subclass of torch.Tensor.
 py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, bool prepared, bool causal, std::optional<double> scale, int mode,
-                   int id_heads, const std::optional<Tensor>& plan, bool backward, int key_runs, const Tensor& status) {
+                   int id_heads, const std::optional<Tensor>& plan, bool backward, int key_runs, const Tensor& status,
+                   const std::optional<Tensor>& out) {
     fa_problem p;
     const double sm_scale = scale ? *scale : 1.0 / std::sqrt(double(q.dim() == 4 ? q.size(3) : 1));
     if (!regular(q, k, v, prepared, causal, sm_scale, mode, id_heads, p)) return py::none();
@@ -78,7 +80,7 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, bool prepa
     int splits = 1;
     {
         py::gil_scoped_release free;
-        o = at::empty_like(q);
+        o = out ? *out : at::empty_like(q);
         if (!taken_as_is(o)) o = at::empty(q.sizes(), q.options());
         const auto f32 = q.options().dtype(at::kFloat);
         lse = at::empty({p.B, p.H, fa_padded_rows(p.M)}, f32);

@@ -195,6 +195,11 @@ def _host():
 _HOST = None
 
 
+def _like_subclass(q):
+    """The result's tensor for a q of a subclass of torch.Tensor, so that it is one of them, too; else None."""
+    return None if type(q) in (torch.Tensor, torch.nn.Parameter) else torch.empty_like(q)
+
+
 class FlashAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, sm_scale, eq, ek, score_func_mode, key_runs=None):
@@ -205,7 +210,8 @@ class FlashAttention(torch.autograd.Function):
                 and (sm_scale is None or type(sm_scale) is float) and all(isinstance(x, torch.Tensor) for x in (q, k, v))):
             status = _STATUS.get(q.get_device())
             if status is not None:  # regular calls without ids and without need of a plan: one native call
-                done = host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs or 0, status)
+                done = host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs or 0, status,
+                                    _like_subclass(q))
         if done is None:
             # checks of flash_triton.py:510-520
             Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
@@ -249,7 +255,7 @@ class FlashAttention(torch.autograd.Function):
                     plan = build_plan(prob, None, None, status)
                 with _timed("fwd", 0):
                     done = host.forward(q, k, v, True, bool(causal), float(sm_scale), score_func_mode, id_heads, plan, needs_grad,
-                                        key_runs or 0, status)
+                                        key_runs or 0, status, _like_subclass(q))
                 if done is None:
                     raise RuntimeError("flash_b200: q, k, v are not plain [bs, H, L, D] CUDA tensors of matching shapes")
                 if _SYNC_STATUS:
