@@ -126,3 +126,12 @@ def test_a_tensor_subclass_gives_one(mode):
         o = fb.attention(x.as_subclass(_Tagged), k, v, True, None, ids, ids, mode)
         assert type(o) is _Tagged and torch.equal(o.as_subclass(torch.Tensor), want)
     assert type(fb.attention(torch.nn.Parameter(q), k, v, True, None, ids, ids, mode)) is torch.Tensor
+
+
+def test_tracing_is_refused():
+    """A trace would hold the allocation of the result and not the kernel that fills it."""
+    import flash_b200 as fb
+    x = torch.randn(1, 4, 200, 64, device="cuda").bfloat16()
+    fb.attention(x, x, x, True)
+    with pytest.raises(AssertionError):
+        torch.jit.trace(lambda q: fb.attention(q, q, q, True), x, check_trace=False)
