@@ -135,3 +135,16 @@ def test_tracing_is_refused():
     fb.attention(x, x, x, True)
     with pytest.raises(AssertionError):
         torch.jit.trace(lambda q: fb.attention(q, q, q, True), x, check_trace=False)
+
+
+def test_negated_views():
+    import flash_b200 as fb
+    q, k, v, do = (torch.randn(1, 4, 200, 64, device="cuda").bfloat16() for _ in range(4))
+
+    def step(q, do):
+        q = q.detach().requires_grad_()
+        o = fb.attention(q, k, v, True)
+        return o.detach(), *torch.autograd.grad(o, q, do)
+
+    want = step(-q, -do)
+    assert all(torch.equal(a, b) for a, b in zip(step(torch._neg_view(q), torch._neg_view(do)), want))

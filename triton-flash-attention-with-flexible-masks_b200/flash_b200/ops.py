@@ -109,7 +109,8 @@ def check_status(device=None):
 
 def maybe_contiguous(x):
     """flash_triton.py:435-437, extended by the TMA rules: last stride 1, 16-byte aligned base,
-    other strides positive multiples of 8 elements."""
+    other strides positive multiples of 8 elements, no pending negation."""
+    x = x.resolve_neg()
     ok = x.data_ptr() % 16 == 0
     if ok and x.is_contiguous() and x.shape[-1] % 8 == 0:
         return x
