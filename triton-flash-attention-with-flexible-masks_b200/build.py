@@ -7,6 +7,7 @@ without a CUDA driver (its entry points then return an error instead of computin
 """
 import concurrent.futures
 import os
+import shutil
 import subprocess
 import sys
 import sysconfig
@@ -74,14 +75,19 @@ def build(force=False, verbose=False):
     return OUT
 
 
+def _cuda_include():
+    """The toolkit's headers, beside the nvcc that NVCC names, by a path or by a name on PATH."""
+    nvcc = os.path.realpath(shutil.which(NVCC) or NVCC)
+    return os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")
+
+
 def _build_host(force):
     src = os.path.join(CSRC, "host.cpp")
     if not force and not _stale(HOST_OUT, [src, OUT] + _deps()):
         return
     import torch
     root = os.path.dirname(torch.__file__)
-    cuda = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
-    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), cuda,
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), _cuda_include(),
                sysconfig.get_paths()["include"]]
     r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", HOST_OUT, *("-I" + i for i in include),
                         "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
