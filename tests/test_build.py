@@ -1,4 +1,5 @@
 """The in-tree build (nvcc and g++ run here without a GPU)."""
+import importlib.util
 import os
 import shutil
 
@@ -14,3 +15,19 @@ def test_cuda_headers_are_found_for_any_form_of_NVCC(monkeypatch, name):
         nvcc = os.path.basename(nvcc)
     monkeypatch.setattr(build, "NVCC", nvcc)
     assert os.path.exists(os.path.join(build._cuda_include(), "cuda_runtime_api.h"))
+
+
+@pytest.mark.parametrize("torch_there", [False, True])
+def test_the_library_alone_needs_no_torch(monkeypatch, torch_there):
+    def no_host(force):
+        raise AssertionError("the host module was built")
+
+    monkeypatch.setattr(build, "_build_host", no_host)
+    if torch_there:
+        assert build.build(host=False) == build.OUT
+        with pytest.raises(AssertionError):
+            build.build()
+    else:
+        find = importlib.util.find_spec
+        monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
+        assert build.build() == build.OUT

@@ -1,11 +1,13 @@
 """Builds the CUDA library in-tree: csrc/*.cu -> flash_b200/libfa_b200.so (sm_100a only), and the native part of its
 torch binding on top of it: csrc/host.cpp -> flash_b200/_host.so.
 
-Usage: python build.py [--force]. nvcc cross-compiles without a GPU. The runtime is linked
+Usage: python build.py [--force] [--library]. With --library, and where torch is not installed, the CUDA library alone is
+built: it is all that users of the C ABI need, and links and includes nothing of torch's or Python's. nvcc cross-compiles without a GPU. The runtime is linked
 statically and the driver API is resolved at run time, so the library loads on a machine
 without a CUDA driver (its entry points then return an error instead of computing).
 """
 import concurrent.futures
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -51,7 +53,7 @@ def _compile(src):
     return obj, r.stderr
 
 
-def build(force=False, verbose=False):
+def build(force=False, verbose=False, host=True):
     os.makedirs(OBJ_DIR, exist_ok=True)
     srcs = _sources()
     if force:
@@ -71,7 +73,8 @@ def build(force=False, verbose=False):
                            capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    _build_host(force)
+    if host and importlib.util.find_spec("torch") is not None:
+        _build_host(force)
     return OUT
 
 
@@ -98,4 +101,4 @@ def _build_host(force):
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose=True))
+    print(build(force="--force" in sys.argv, verbose=True, host="--library" not in sys.argv))
