@@ -31,3 +31,17 @@ def test_the_library_alone_needs_no_torch(monkeypatch, torch_there):
         find = importlib.util.find_spec
         monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
         assert build.build() == build.OUT
+
+
+def test_the_host_module_is_stale_for_another_torch_or_python(monkeypatch):
+    import sysconfig
+    import torch
+    build.build()
+    assert not build._host_stale()
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0.1")
+        assert build._host_stale()
+    with monkeypatch.context() as m:
+        m.setattr(sysconfig, "get_config_var", lambda name: "cpython-300")
+        assert build._host_stale()
+    assert not build._host_stale()

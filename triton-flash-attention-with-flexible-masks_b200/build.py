@@ -19,6 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "flash_b200", "libfa_b200.so")
 HOST_OUT = os.path.join(HERE, "flash_b200", "_host.so")
 OBJ_DIR = os.path.join(HERE, "build")
+HOST_TAG = os.path.join(OBJ_DIR, "host.tag")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -84,20 +85,40 @@ def _cuda_include():
     return os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")
 
 
+def _host_tag():
+    """What the host module is bound to besides its sources: this Python and the C++ interface of this torch."""
+    import torch
+    return f"{sysconfig.get_config_var('SOABI')} torch {torch.__version__} abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}\n"
+
+
+def _host_stale():
+    if _stale(HOST_OUT, [os.path.join(CSRC, "host.cpp"), OUT] + _deps()) or not os.path.exists(HOST_TAG):
+        return True
+    with open(HOST_TAG) as f:
+        return f.read() != _host_tag()
+
+
 def _build_host(force):
-    src = os.path.join(CSRC, "host.cpp")
-    if not force and not _stale(HOST_OUT, [src, OUT] + _deps()):
+    if not force and not _host_stale():
         return
     import torch
+    src = os.path.join(CSRC, "host.cpp")
     root = os.path.dirname(torch.__file__)
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), _cuda_include(),
                sysconfig.get_paths()["include"]]
-    r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", HOST_OUT, *("-I" + i for i in include),
+    part = f"{HOST_OUT}.{os.getpid()}"  # moved into place when it is whole: another process may be loading the module
+    r = subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", part, *("-I" + i for i in include),
+                        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
                         "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
                         "-L" + os.path.dirname(OUT), "-l:" + os.path.basename(OUT), "-Wl,-rpath,$ORIGIN"],
                        capture_output=True, text=True)
     if r.returncode != 0:
+        if os.path.exists(part):
+            os.remove(part)
         raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
+    os.replace(part, HOST_OUT)
+    with open(HOST_TAG, "w") as f:
+        f.write(_host_tag())
 
 
 if __name__ == "__main__":
