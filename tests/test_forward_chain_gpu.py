@@ -33,7 +33,7 @@ def check(o, ref, absolute, scale):
 @pytest.mark.parametrize("growing", [False, True], ids=["flat", "growing"])
 def test_tiles_and_moving_maximum(tiles, D, growing):
     """`growing`: every tile's scores exceed the last one's by more than the slack of the lazy rescale in half of the
-    rows, and fall in the others, so that each tile of one group moves the maximum that the other group goes on from."""
+    rows, and fall in the others, so that each tile moves its chain's maximum."""
     import flash_b200 as fb
     B, H, M, N = 2, 40, 256, tiles * 128 - 5  # more items than SMs, whose tiles start at even and odd places of the ring
     g = torch.Generator(device="cuda").manual_seed(tiles * D)
@@ -46,6 +46,54 @@ def test_tiles_and_moving_maximum(tiles, D, growing):
     o = fb.attention(q, k, v)
     check(o, *reference(q, k, v, False), scale=16.0 + (12.0 * tiles if growing else 0))
     assert torch.equal(o, fb.attention(q, k, v))
+
+
+def growing_inputs(B, H, Hk, M, N, D, dtype, seed):
+    """Scores that rise from tile to tile by more than the slack of the lazy rescale in half of the rows and fall in the
+    others, twice over, so that both chains rescale, too, when they have come down."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(B, h, n, D, generator=g, device="cuda") for h, n in ((H, M), (Hk, N), (Hk, N)))
+    q[..., 0] = torch.where(torch.arange(M, device="cuda") % 2 == 0, 1.0, -1.0) * D ** 0.5
+    k[..., 0] = torch.arange(N, device="cuda") // 128 % 4 * 12.0
+    return [x.to(dtype) for x in (q, k, v)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("form", ["full", "causal", "ids"])
+@pytest.mark.parametrize("tiles", [1, 3, 6])
+def test_many_items_a_cta_while_the_maximum_moves(tiles, form, D, dtype):
+    """Six items a CTA on 148 SMs: the item slots, the accumulators and the barriers of both are used again several times,
+    by items of an even, an odd and (ids, causal) a varying number of tiles."""
+    import flash_b200 as fb
+    B, H, M, N = 4, 112, 256, tiles * 128 - (0 if tiles == 1 else 5)
+    M = min(M, N)
+    H = H * 256 // (-(-M // 128) * 128)
+    q, k, v = growing_inputs(B, H, H, M, N, D, dtype, tiles * D)
+    keep, args = None, (form != "full",)
+    if form == "ids":
+        ek = -1 - torch.arange(N, device="cuda") // 170
+        eq = ek[N - M:].clone()
+        eq[::50] = 3  # attends to all
+        keep = (eq[:, None] >= 0) | (eq[:, None] == ek)
+        args = (True, None, eq.expand(B, H, M), ek.expand(B, H, N), fb.SCORE_FUNC_MODE1_DOC)
+    o = fb.attention(q, k, v, *args)
+    for b in range(B):
+        check(o[b:b + 1], *reference(q[b:b + 1], k[b:b + 1], v[b:b + 1], form != "full", keep), scale=16.0 + 48.0)
+    assert torch.equal(o, fb.attention(q, k, v, *args))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("runs", [1, 3])
+def test_many_packed_items_while_the_maximum_moves(runs, D):
+    import flash_b200 as fb
+    B, H, Hk, M, N = 100, 32, 8, 16, 1400
+    q, k, v = growing_inputs(B, H, Hk, M, N, D, torch.bfloat16, D)
+    o = fb.attention_in_runs(q, k, v, runs, True)
+    for b in range(0, B, 20):
+        part = slice(b, b + 20)
+        ke, ve = (x[part].repeat_interleave(H // Hk, 1) for x in (k, v))
+        check(o[part], *reference(q[part], ke, ve, True), scale=16.0 + 48.0)
 
 
 @pytest.mark.parametrize("D", [64, 128])

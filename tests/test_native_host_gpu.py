@@ -148,3 +148,57 @@ def test_negated_views():
 
     want = step(-q, -do)
     assert all(torch.equal(a, b) for a, b in zip(step(torch._neg_view(q), torch._neg_view(do)), want))
+
+
+class _Recorder:
+    """The native host calls, with what each was asked and whether it took the call: (direction, prepared, taken)."""
+
+    def __init__(self, host):
+        self.host, self.calls = host, []
+
+    def forward(self, *args):
+        done = self.host.forward(*args)
+        self.calls.append(("forward", args[3], done is not None))
+        return done
+
+    def backward(self, *args):
+        done = self.host.backward(*args)
+        self.calls.append(("backward", args[6], done is not None))
+        return done
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_which_calls_take_the_native_route(monkeypatch, dtype):
+    """Regular calls are taken as they are, in both directions; the others are declined once and taken when they have
+    been prepared."""
+    import flash_b200 as fb
+    from flash_b200 import ops
+    B, H, L, D = 2, 4, 200, 64
+    q, k, v, do = (torch.randn(B, H, L, D, device="cuda").to(dtype) for _ in range(4))
+    fb.attention(q, k, v, True)  # (the first call on a device makes its status word on the general path)
+    recorder = _Recorder(ops._host())
+    monkeypatch.setattr(ops, "_HOST", recorder)
+
+    def route(q, k, v, do):
+        recorder.calls.clear()
+        x = [t.detach().requires_grad_() for t in (q, k, v)]
+        fb.attention(*x, True).backward(do)
+        return list(recorder.calls)
+
+    forward, backward = [("forward", False, True)], [("backward", False, True)]
+    general_forward = [("forward", False, False), ("forward", True, True)]
+    general_backward = [("backward", False, False), ("backward", True, True)]
+    regular = ("contiguous", "transposed")
+    for (name, a), (_, b), (_, c), (_, d) in zip(*(layouts(x) for x in (q, k, v, do))):
+        assert route(a, b, c, do) == (forward if name in regular else general_forward) + backward, name
+        assert route(q, k, v, d) == forward + (backward if name in regular else general_backward), name
+    assert route(q, k, v, torch.ones((), dtype=dtype, device="cuda").expand(B, H, L, D)) == forward + general_backward
+    assert route(q, k, v, do.to(torch.float64)) == forward + backward  # (autograd casts it first)
+    with torch.no_grad():
+        recorder.calls.clear()
+        fb.attention(q, k, v, True)
+        assert recorder.calls == forward
+        ids = (-1 - torch.arange(L, device="cuda") // 70).expand(B, H, L)
+        recorder.calls.clear()
+        fb.attention(q, k, v, True, None, ids, ids, fb.SCORE_FUNC_MODE1_DOC)  # ids: a plan is built first
+        assert recorder.calls == [("forward", True, True)]
