@@ -24,7 +24,9 @@
  *    the call that passed the id (its result may mask that query wrongly); later calls run.
  *  - one bounded wait lasts at most 5e8 SM clocks (about 0.25 s); the environment variable
  *    FA_B200_WAIT_LIMIT_CLOCKS (>= 10000), read when the library is first used, replaces the limit,
- *    e.g. on hosts where several contexts time-share the GPU.
+ *    e.g. on hosts where several contexts time-share the GPU. The scheduler of a kernel waits for as
+ *    long as one of its work items takes (up to 1024 tiles of 128 x 128, in fa_bwd_dkdv for each head
+ *    of a group, some 3000 clocks each): a limit below that can end valid calls.
  */
 #ifndef FA_B200_H_
 #define FA_B200_H_

@@ -1,4 +1,8 @@
 """The forward's two chains of tiles: an accumulator and a running maximum each, merged at the end of an item."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -168,3 +172,20 @@ def test_a_row_whose_score_overflows_is_nan(D):
     k[:, :, 300, 0] = 3e38  # a score of +inf for the rows that see this key
     o = fb.attention(q, k, v, True)
     assert bool(torch.isfinite(o[:, :, :300]).all()) and bool(torch.isnan(o[:, :, 300:]).all())
+
+
+def test_an_item_may_last_longer_than_the_limit_of_a_wait(repo_root):
+    """An item of 1024 tiles takes over a million clocks, five times the limit set here, and no wait within it more than a
+    twentieth of the limit: the epilogue group, which waits for the whole item, goes by its tiles."""
+    code = """
+import torch, flash_b200 as fb
+q = torch.randn(1, 2, 128, 64, device="cuda").bfloat16()
+k, v = (torch.randn(1, 2, 131072, 64, device="cuda").bfloat16() for _ in range(2))
+o = fb.attention_in_runs(q, k, v, 1)
+fb.check_status()
+assert bool(torch.isfinite(o).all())
+"""
+    path = os.path.join(repo_root, "triton-flash-attention-with-flexible-masks_b200")
+    env = dict(os.environ, FA_B200_WAIT_LIMIT_CLOCKS="200000", PYTHONPATH=path + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]

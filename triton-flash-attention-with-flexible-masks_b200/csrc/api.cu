@@ -191,11 +191,12 @@ constexpr float kLog2e = 1.4426950408889634f;
 // Limit of one bounded wait inside the kernels, in SM clocks: FA_B200_WAIT_LIMIT_CLOCKS if set to a
 // number >= 10000 when the library is first used, else the built-in default.
 long long wait_limit_clocks() {
+    constexpr long long kMost = 1LL << 50;  // a week; a wait for a whole item multiplies it by the item's tiles
     static const long long v = [] {
         const char* e = getenv("FA_B200_WAIT_LIMIT_CLOCKS");
         if (e) {
             const long long x = atoll(e);
-            if (x >= 10000) return x;
+            if (x >= 10000) return x < kMost ? x : kMost;
         }
         return fa::kWaitLimitClocks;
     }();

@@ -419,7 +419,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             const int row = qb * kBlk + r - g_row * mk.M;
             const int g_own = SHORT ? (h % nG) * p.pack + g_row : 0;
             const bool valid = !SHORT || (row < mk.M && g_row < p.pack && g_own < p.G);
-            alive = mbar_wait_warp(BAR(B_MLFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 16);
+            // the only wait here that lasts as long as an item: it allows each of the tiles what another wait may last
+            const Abort item{ab.flag, ab.status, ab.limit * (T + 1)};
+            alive = mbar_wait_warp(BAR(B_MLFULL + s), use & 1, item, ST_WAIT_TIMEOUT + 16);
             // an item without tiles: nobody has waited for its Q load yet, and its slot is about to become the staging area
             if (alive && T == 0) alive = mbar_wait_warp(BAR(B_QFULL + s), use & 1, ab, ST_WAIT_TIMEOUT + 17);
             const int we = G & 1;  // the chain that had the item's even tiles: index 0 below, 1 the other one
