@@ -99,6 +99,10 @@ int fa_plan_bytes(const fa_problem* p, size_t* bytes);
  * no longer than through a plan's counters. Results are the same bits with and without a plan. */
 int fa_plan_optional(const fa_problem* p, int32_t backward);
 
+/* With ids fa_plan_build launches one kernel for at most this many blocks of 128 queries and of 128
+ * keys together, else three. */
+#define FA_PLAN_ONE_KERNEL_BLOCKS 64
+
 /* Builds the mask plan from eq [B,H,M] / ek [B,H,N]: 32-bit id codes, per-128-block id
  * min/max, per-block ranges of blocks that hold at least one unmasked entry, and a few work
  * counters through which the CTAs of fa_fwd / fa_bwd_dkdv / fa_bwd_dq share out their work.

@@ -163,3 +163,10 @@ def test_group_and_permute_rows_check_their_arguments():
     assert lib.fa_permute_rows(ctypes.byref(p), ctypes.byref(t), ctypes.byref(t), None, None) == 1
     t.stride[2] = 132  # a row stride that is not a whole number of 16-byte units
     assert lib.fa_permute_rows(ctypes.byref(p), ctypes.byref(t), ctypes.byref(t), ptr, None) == 3
+
+
+@pytest.mark.parametrize("name", ["FA_GROUP_MAX_ROWS", "FA_PLAN_ONE_KERNEL_BLOCKS", "FA_BF16", "FA_FP16", "FA_FP32", "FA_ID_NONE", "FA_ID_INT32", "FA_ID_INT64"])
+def test_constants_are_those_of_the_header(repo_root, name):
+    text = open(os.path.join(repo_root, "include", "fa_b200.h")).read()
+    value = re.search(rf"\b{name}\b\s*=?\s*(\d+)", text)
+    assert int(value.group(1)) == getattr(_lib, name)

@@ -2,6 +2,7 @@
 // kernel that materialises keep / tile-class decisions with the attention kernels' own
 // predicate. The reference has no counterpart (it evaluates every tile inside the causal
 // bound, flash_triton.py:94-129); the rule encoded is flash_triton.py:114.
+#include "../../include/fa_b200.h"
 #include "common.cuh"
 
 namespace fa {
@@ -166,10 +167,11 @@ __global__ void __launch_bounds__(1024) plan_order_kernel(int32_t* plan, PlanLay
 
 // The three kernels above in one, for id rows of at most kSmallBlocks blocks: grid (He, B), 1024 threads. A warp takes a block
 // of 128 ids, its lane x the ids x, x + 32, x + 64 and x + 96; the block statistics pass through shared memory.
-// Bound by latency; the same words in the plan. us, in the three launches (their times alone, without the gaps of about 1 us
-// between them) and here: 16 blocks a row (4 x 1000 ids) 6.5, 3.4; 64 (4 x 4096) 7.6, 7.3; 72 (8 rows of 1024 and 8192) 8.6,
-// 9.1: beyond two blocks a warp the launches are no slower.
-constexpr int kSmallBlocks = 64;
+// Bound by latency; the same words in the plan. us a plan in a replayed graph, gaps between launches included, by three launches
+// and here: 16 blocks a row, 4 rows 6.6, 3.7; 32 blocks 6.7, 4.8; 64 blocks, 1 row 6.3, 7.0; 4 rows 7.0, 7.2; 32 rows 9.0, 7.3;
+// 72 blocks, 1 row 7.1, 8.4; 8 rows 7.5, 8.4; 32 rows 9.7, 8.5; 128 blocks, 8 rows 8.0, 12.4; 32 rows 12.8, 12.4. Up to two blocks
+// a warp it is as fast or faster on the device, and saves the host two launches; beyond, only with 32 rows or more.
+constexpr int kSmallBlocks = FA_PLAN_ONE_KERNEL_BLOCKS;
 
 __device__ __forceinline__ int warp_min(int v) { return __reduce_min_sync(0xffffffffu, v); }
 __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }

@@ -11,6 +11,7 @@ LIB_PATH = os.path.join(_HERE, "libfa_b200.so")
 FA_BF16, FA_FP16, FA_FP32 = 0, 1, 2
 FA_ID_NONE, FA_ID_INT32, FA_ID_INT64 = 0, 1, 2
 FA_GROUP_MAX_ROWS = 16384
+FA_PLAN_ONE_KERNEL_BLOCKS = 64
 
 EXPORTS = (
     "fa_version", "fa_error_string", "fa_padded_rows", "fa_plan_bytes", "fa_plan_build", "fa_fwd",

@@ -177,7 +177,8 @@ def build_plan(prob, eq, ek, status):
                                      status.data_ptr(), _stream()), "fa_plan_build")
         return plan
     ieq, iek = _ids(eq), _ids(ek)
-    with _timed("plan", 1 if (prob.M + 127) // 128 + (prob.N + 127) // 128 <= 64 else 3):  # kSmallBlocks in mask_plan.cu
+    blocks = (prob.M + 127) // 128 + (prob.N + 127) // 128
+    with _timed("plan", 1 if blocks <= _lib.FA_PLAN_ONE_KERNEL_BLOCKS else 3):
         _lib.check(lib.fa_plan_build(prob, ieq, iek, plan.data_ptr(),
                                      nbytes.value, status.data_ptr(), _stream()), "fa_plan_build")
     return plan
