@@ -139,11 +139,10 @@ int make_map_grouped(CUtensorMap* out, const fa_tensor* t, const fa_problem* p, 
 
 // Query heads of a group that share one 128-row tile in the forward: as many as fit, for calls without ids whose
 // queries fill at most half a tile. K and V are then read once for all of them, and there are fewer tiles in all. With a
-// tile per head and packed (and split, where fwd_splits says so), us, 32 / 8 heads of 128: 16 sequences against 3000 keys,
-// 1 query 115, 40.2; 16 queries 115, 41.2; 32 queries 117, 41.8; 64 queries 117, 70.0; against 128 keys 22.9, 9.7; 25.0,
-// 10.5; 25.0, 10.6; 26.6, 18.8; 64 sequences of 64 queries against 2000 keys 270, 156; one sequence of 64 against 512 keys
-// 14.8, 12.4, where packing leaves most SMs idle. No call of the sweep (1 to 64 queries, 1 to 64 sequences, 128 to 8192
-// keys) got slower.
+// tile per head and packed (and split, where fwd_splits says so), us between events in a graph, 32 / 8 heads of 128: 16
+// sequences against 3000 keys, 1 query 91, 42; 16 queries 92, 42; 32 queries 92, 44; 64 queries 94, 62; against 128 keys 20,
+// 14; 23, 14; 23, 16; 23, 18; 64 sequences of 64 queries against 2000 keys 223, 139. One sequence of 64 against 512 keys,
+// where packing leaves most SMs idle, is the exception: 14, 16.
 int fwd_pack(const fa_problem* p) {
     const int G = p->H / p->Hk;
     if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32 || p->M > fa::kBlk / 2) return 1;
@@ -238,11 +237,11 @@ int sm_count() {
 // Runs into which the forward cuts each item's key tiles, for calls without ids that have fewer items than the GPU
 // has SMs. A round of items costs its tiles plus about 4 tile times of fill, drain and epilogue; the second
 // kernel and the fp32 rows cost about 6 more. At most two items per SM, which bounds the workspace at 20 MB.
-// One token, 32 / 8 heads of 128, us with 1 run and with the number taken here: 32768 keys 240, 37.7 (18 runs; best of
-// 1, 2, 4, 8, 16: 37.0 with 16); 4096 keys 36.5, 16.7 (16; best); 1024 keys 14.9 (1; best 12.6 with 4); 4 sequences
-// of 8192 keys 67.5, 34.1 (4; best); 8 of them 71.2, 52.0 (2; best). 300 queries against 9000 keys: 16 / 4 heads 77.4, 39.9
-// (3; 2 runs 49.2, 4 runs 56.9), 32 / 8 heads 78.0, 71.8 (3; 2 runs 94.1, 4 runs 82.0). 1000 x 1000 of 8 heads of 64: 14.6
-// (1; 2 runs 18.1).
+// One token, 32 / 8 heads of 128, us between events in a graph with 1 run and with the number taken here: 32768 keys 190, 40.5
+// (18 runs; best of 1, 2, 4, 8, 16: 40.4 with 16); 4096 keys 34, 22 (16; best 20 with 8); 1024 keys 18 (1; 2 and 4 the same); 4
+// sequences of 8192 keys 58, 36 (4; best); 8 of them 63, 54 (2; best). 300 queries against 9000 keys: 16 / 4 heads 63, 38 (3;
+// 2 runs 46, 4 runs 53), 32 / 8 heads 65, 67 (3; 2 runs 83, 4 runs 75): the model's costs are those of an
+// earlier forward, whose chain of tiles was slower. 1000 x 1000 of 8 heads of 64: 16 (1; 2 runs 24).
 int fwd_splits(const fa_problem* p, int sms) {
     if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32) return 1;
     const int pack = fwd_pack(p);
@@ -385,7 +384,7 @@ int fa_plan_bytes(const fa_problem* p, size_t* bytes) {
     return FA_OK;
 }
 
-// A split forward may have two runs per SM, still dealt out in a fixed order: 32 / 8 heads of 300 queries, 9000 keys in
+// A split forward may have two runs per SM, still dealt out in a fixed order (times of an earlier forward): 32 / 8 heads of 300 queries, 9000 keys in
 // 3 runs 72.6 us, 72.7 us through the counters of a plan that is there, 76.8 us with the clearing of its counters;
 // 12 tokens of 32 / 8 heads, 16384 keys in 3 runs 129.6, 130.1 and 134.2 us; 24 heads of 500, 16000 keys 114.9, 114.8, 118.4.
 int fa_plan_optional(const fa_problem* p, int32_t backward) {

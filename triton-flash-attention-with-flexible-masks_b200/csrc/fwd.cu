@@ -25,13 +25,14 @@
 // next: for D = 128 S has one buffer, free as soon as a group has its scores in registers, and P (input dtype, two values per
 // column) columns of its own, one place a chain; for D = 64 there are three buffers, P overwrites the first 64 columns of its
 // own, and S(g+3) follows P*V(g) on the pipe.
-// Forward kernel, us: two buffers in which P overwrites S, with the exponentials of the groups in turns | one O and one maximum
-// for both chains, three buffers | now. 2 x 32 / 8 heads x 3001 x 128 causal 198 | 157 | 154, with q and k of deviation 2
-// 261 | 330 | 228, of 4 263 | 355 | 238 (a shared maximum that moves makes either group wait for the other's P*V); 512 queries
-// against 8192 keys, 32 / 8 heads of 128, 80 | 64 | 64; 16 x 8 x 577 x 32 57 | 46 | 45; 4 x 16 x 4096 x 128 in documents
-// 176 | 147 | 152; 32 x 32768 x 128 in 64 documents 912 | 784 | 792; 16 x 32 x 8192 x 128 causal 9600 | 8000 | 8180; 4 x 12 x
-// 1000 x 64 in documents 44 | 39 | 38; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 107 | 95 | 89. The shared O
-// had errors 1 to 2 % larger as well: one entry of a row is an exact 1 in P, not one of each chain.
+// Forward kernel, us between events in a graph (some 4 more than the kernel alone): two buffers in which P overwrites S, with
+// the exponentials of the groups in turns | one O and one maximum for both chains, three buffers | now. 2 x 32 / 8 heads x
+// 3001 x 128 causal 195 | 154 | 152, with q and k of deviation 2 242 | 322 | 198, of 4 229 | 303 | 204 (a shared maximum that
+// moves makes either group wait for the other's P*V); 512 queries against 8192 keys, 32 / 8 heads of 128, 77 | 61 | 61, deviation
+// 3 86 | 99 | 67; 16 x 8 x 577 x 32 45 | 37 | 37; 4 x 16 x 4096 x 128 in documents 174 | 145 | 151, deviation 3 184 | 206 | 163;
+// 32 x 32768 x 128 in 64 documents 908 | 776 | 786; 16 x 32 x 8192 x 128 causal 9520 | 7760 | 7690; 4 x 16 x 4096 x 64 causal
+// 249 | 201 | 192; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 94 | 83 | 79. The shared O had errors 1 to 2 %
+// larger as well: one entry of a row is an exact 1 in P, not one of each chain.
 // What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group) and, in
 // dense calls, the clock under the power cap (1.4-1.5 GHz); with short items the drain of two O, which the next item's P*V waits for.
 #include <type_traits>
@@ -83,7 +84,7 @@ static_assert(FwdSmem<128>::total <= 232448 && FwdSmem<64>::total <= 232448, "sh
 //  - an item's tiles are cut into p.ns runs that are items of their own. With ns > 1 the normalised fp32 rows
 //    and their log-sum-exp go to the workspace, and fwd_combine_kernel merges them.
 // Such calls are bound by reading K and V (16 tokens of 32 / 8 heads of 128 against 4500 keys: 295 MB, 45 us at the
-// copy rate; 171 us with a tile per head, 63 us packed) or, with few heads, by the longest item's chain of tiles.
+// copy rate; 127 us with a tile per head, 55 us packed) or, with few heads, by the longest item's chain of tiles.
 template <int D, bool BF16, bool SHORT>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,

@@ -2,7 +2,7 @@
 // descriptors, and the launches of fa_b200.h. The autograd node stays in Python (ops.py), and so do all messages: a
 // call that is not regular (another layout, device, shape or type than the kernels take as they are) is declined with
 // None, and ops.py's general code copies, asks or raises. Bound by per-call overhead: a forward of 8 heads of 200
-// queries took 27 us of host time around 9 us of kernel through ctypes.
+// queries took 27 us of host time around 8 us of kernel through ctypes.
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <torch/csrc/utils/pybind.h>
