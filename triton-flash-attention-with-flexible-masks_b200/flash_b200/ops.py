@@ -199,7 +199,11 @@ _HOST = None
 
 def _like_subclass(q):
     """The result's tensor for a q of a subclass of torch.Tensor, so that it is one of them, too; else None."""
-    return None if type(q) in (torch.Tensor, torch.nn.Parameter) else torch.empty_like(q)
+    return None if type(q) in _PLAIN else torch.empty_like(q)
+
+
+# looked up once: a short call's host time is what bounds it
+_TENSOR, _PLAIN, _tracing_state = torch.Tensor, (torch.Tensor, torch.nn.Parameter), torch._C._get_tracing_state
 
 
 class FlashAttention(torch.autograd.Function):
@@ -209,8 +213,8 @@ class FlashAttention(torch.autograd.Function):
         needs_grad = any(ctx.needs_input_grad[:3])
         done, plan, id_heads = None, None, 1
         if (eq is None and ek is None and score_func_mode == SCORE_FUNC_MODE0_NOPE and PROFILE is None and not _SYNC_STATUS
-                and (sm_scale is None or type(sm_scale) is float) and all(isinstance(x, torch.Tensor) for x in (q, k, v))
-                and torch._C._get_tracing_state() is None):  # torch.jit.trace would record allocations and no kernel: the checks below refuse it
+                and (sm_scale is None or type(sm_scale) is float) and isinstance(q, _TENSOR) and isinstance(k, _TENSOR)
+                and isinstance(v, _TENSOR) and _tracing_state() is None):  # (a trace would hold no kernel: the checks below refuse it)
             status = _STATUS.get(q.get_device())
             if status is not None:  # regular calls without ids and without need of a plan: one native call
                 done = host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs or 0, status,
