@@ -202,3 +202,44 @@ def test_which_calls_take_the_native_route(monkeypatch, dtype):
         recorder.calls.clear()
         fb.attention(q, k, v, True, None, ids, ids, fb.SCORE_FUNC_MODE1_DOC)  # ids: a plan is built first
         assert recorder.calls == [("forward", True, True)]
+
+
+def test_no_autograd_node_changes_nothing():
+    """Calls that need no gradient go without a node: the same bits, messages and refusals as with one."""
+    import flash_b200 as fb
+    import torch.autograd.forward_ad as fwad
+    q, k, v = (torch.randn(2, 4, 200, 64, device="cuda").bfloat16() for _ in range(3))
+    want = fb.attention(q.clone().requires_grad_(), k, v, True)
+    assert want.requires_grad
+    with torch.no_grad():
+        got = fb.attention(q.clone().requires_grad_(), k, v, True)
+    with torch.inference_mode():
+        frozen = fb.attention(q, k, v, True)
+    for o in (got, frozen, fb.attention(q, k, v, True)):
+        assert not o.requires_grad and o.grad_fn is None and torch.equal(o, want)
+    assert frozen.is_inference()
+    for bad, error in (((q, k[:, :, :32], v[:, :, :32]), AssertionError), ((q, k.half(), v), ValueError), ((q, k.cpu(), v), ValueError)):
+        with pytest.raises(error):
+            fb.attention(*bad, True)
+    with pytest.raises(RuntimeError):
+        torch.vmap(lambda x: fb.attention(x, x, x, True))(torch.randn(2, 1, 2, 64, 64, device="cuda").bfloat16())
+    with torch.no_grad(), fwad.dual_level(), pytest.raises(Exception, match="jvp"):
+        fb.attention(fwad.make_dual(q, q), k, v, True)
+    with pytest.raises(Exception):
+        torch.func.jvp(lambda x: fb.attention(x, k, v, True), (q,), (q,))
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64, torch.int16])
+def test_ids_of_any_form_give_the_same_bits(dtype):
+    """Broadcast over the heads or not, strided or not, of a type that the library takes or one that is converted first."""
+    import flash_b200 as fb
+    B, H, L = 2, 4, 200
+    q, k, v = (torch.randn(B, H, L, 64, device="cuda").bfloat16() for _ in range(3))
+    ids = (-1 - torch.arange(L, device="cuda") // 70).to(dtype)
+    want = fb.attention(q, k, v, True, None, ids.long().expand(B, H, L), ids.long().expand(B, H, L), 1)
+    full = ids.expand(B, H, L).contiguous()
+    for e in (ids.expand(B, H, L), full, full.transpose(0, 2).contiguous().transpose(0, 2), torch.stack([full, full], -1)[..., 0]):
+        assert torch.equal(fb.attention(q, k, v, True, None, e, e, 1), want)
+    for bad in (ids.expand(B, 1, L), ids[:-1].expand(B, H, L - 1), ids.expand(B, H, L).float()):
+        with pytest.raises(AssertionError):
+            fb.attention(q, k, v, True, None, ids.expand(B, H, L), bad, 1)

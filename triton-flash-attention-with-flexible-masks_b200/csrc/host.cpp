@@ -67,6 +67,37 @@ bool regular(const Tensor& q, const Tensor& k, const Tensor& v, bool prepared, b
 
 void* current_stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
+// Would ops.maybe_contiguous return all three as they are? (Where this says no, ops.py goes by that.)
+bool as_is(const Tensor& q, const Tensor& k, const Tensor& v) {
+    return plain_cuda(q) && plain_cuda(k) && plain_cuda(v) && taken_as_is(q) && taken_as_is(k) && taken_as_is(v);
+}
+
+// How many heads the ids of a call have, 1 or H, where they are as the library takes them; 0: ops.py looks, converts or refuses.
+int64_t id_heads(const Tensor& eq, const Tensor& ek, int64_t B, int64_t H, int64_t M, int64_t N) {
+    for (const Tensor* t : {&eq, &ek})
+        if (!t->is_cuda() || t->layout() != at::kStrided || t->dim() != 3 || t->is_neg() || t->size(0) != B || t->size(1) != H ||
+            t->size(2) != (t == &eq ? M : N) || (t->scalar_type() != at::kInt && t->scalar_type() != at::kLong))
+            return 0;
+    return H == 1 || (eq.stride(1) == 0 && ek.stride(1) == 0) ? 1 : H;
+}
+
+// The plan of a call (ops.build_plan): its memory and the launches that fill it. `problem` is the address of an fa_problem; the
+// ids, if any, are int32 or int64 tensors [B, H, M] and [B, H, N] that ops.py has checked.
+Tensor plan(uintptr_t problem, const std::optional<Tensor>& eq, const std::optional<Tensor>& ek, const Tensor& status) {
+    const fa_problem* p = reinterpret_cast<const fa_problem*>(problem);
+    auto ids = [](const Tensor& t) {
+        return fa_ids{t.const_data_ptr(), {t.stride(0), t.stride(1), t.stride(2)}, t.scalar_type() == at::kInt ? FA_ID_INT32 : FA_ID_INT64};
+    };
+    py::gil_scoped_release free;
+    size_t bytes = 0;
+    check(fa_plan_bytes(p, &bytes), "fa_plan_bytes");
+    Tensor plan = at::empty({int64_t(bytes / 4)}, status.options());
+    const fa_ids q = eq ? ids(*eq) : fa_ids{}, k = ek ? ids(*ek) : fa_ids{};
+    check(fa_plan_build(p, eq ? &q : nullptr, ek ? &k : nullptr, plan.data_ptr(), bytes, status.data_ptr<int>(), current_stream(status)),
+          "fa_plan_build");
+    return plan;
+}
+
 // (o, lse, scale, kernels launched), or None. Unprepared calls without a plan are taken only if it would gain nothing. `out`: a
 // tensor like q for the result, given where q is of a subclass of torch.Tensor.
 py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, bool prepared, bool causal, std::optional<double> scale, int mode,
@@ -126,6 +157,9 @@ py::object backward(const Tensor& d_o, const Tensor& q, const Tensor& k, const T
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+    m.def("as_is", &as_is);
+    m.def("id_heads", &id_heads);
+    m.def("plan", &plan);
     m.def("forward", &forward);
     m.def("backward", &backward);
 }

@@ -165,36 +165,31 @@ def forward_splits(B, H, Hk, M, N, D, dtype, causal, mode):
     return _lib.load().fa_fwd_splits(ctypes.byref(_problem(B, H, Hk, M, N, D, dtype, causal, mode, 1, 1.0)))
 
 
+def _plan_kernels(M, N):
+    return 1 if (M + 127) // 128 + (N + 127) // 128 <= _lib.FA_PLAN_ONE_KERNEL_BLOCKS else 3
+
+
 def build_plan(prob, eq, ek, status):
     """Mask plan: int32 device buffer consumed by the forward and backward kernels. With ids it
     holds their codes and block statistics; without (eq is None) only the kernels' work counters."""
-    lib = _lib.load()
-    nbytes = ctypes.c_size_t(0)
-    _lib.check(lib.fa_plan_bytes(prob, ctypes.byref(nbytes)), "fa_plan_bytes")
-    plan = torch.empty(max(nbytes.value // 4, 1), dtype=torch.int32, device=status.device)
+    make = _PLAN or _host().plan
     if eq is None:
-        _lib.check(lib.fa_plan_build(prob, None, None, plan.data_ptr(), nbytes.value,
-                                     status.data_ptr(), _stream()), "fa_plan_build")
-        return plan
-    ieq, iek = _ids(eq), _ids(ek)
-    blocks = (prob.M + 127) // 128 + (prob.N + 127) // 128
-    with _timed("plan", 1 if blocks <= _lib.FA_PLAN_ONE_KERNEL_BLOCKS else 3):
-        _lib.check(lib.fa_plan_build(prob, ieq, iek, plan.data_ptr(),
-                                     nbytes.value, status.data_ptr(), _stream()), "fa_plan_build")
-    return plan
+        return make(ctypes.addressof(prob), None, None, status)
+    with _timed("plan", _plan_kernels(prob.M, prob.N)):
+        return make(ctypes.addressof(prob), eq, ek, status)
 
 
 def _host():
     """The native host calls (csrc/host.cpp); no call runs without them."""
-    global _HOST
+    global _HOST, _PLAN, _AS_IS, _ID_HEADS
     if _HOST is None:
         _lib.load()
         from . import _host as module
-        _HOST = module
+        _HOST, _PLAN, _AS_IS, _ID_HEADS = module, module.plan, module.as_is, module.id_heads
     return _HOST
 
 
-_HOST = None
+_HOST = _PLAN = _AS_IS = _ID_HEADS = None
 
 
 def _like_subclass(q):
@@ -204,6 +199,18 @@ def _like_subclass(q):
 
 # looked up once: a short call's host time is what bounds it
 _TENSOR, _PLAIN, _tracing_state = torch.Tensor, (torch.Tensor, torch.nn.Parameter), torch._C._get_tracing_state
+_grad_enabled, _transforms, _forward_ad = torch.is_grad_enabled, torch._C._functorch.peek_interpreter_stack, torch.autograd.forward_ad
+
+
+def _native_forward(host, q, k, v, causal, sm_scale, needs_grad, key_runs):
+    """One native call for a regular call without ids and without need of a plan; None for any other."""
+    if (PROFILE is not None or _SYNC_STATUS or not (sm_scale is None or type(sm_scale) is float)
+            or _tracing_state() is not None):  # (a trace would hold no kernel: the general code's checks refuse it)
+        return None
+    status = _STATUS.get(q.get_device())
+    if status is None:
+        return None
+    return host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs, status, _like_subclass(q))
 
 
 class FlashAttention(torch.autograd.Function):
@@ -212,21 +219,18 @@ class FlashAttention(torch.autograd.Function):
         host = _HOST or _host()
         needs_grad = any(ctx.needs_input_grad[:3])
         done, plan, id_heads = None, None, 1
-        if (eq is None and ek is None and score_func_mode == SCORE_FUNC_MODE0_NOPE and PROFILE is None and not _SYNC_STATUS
-                and (sm_scale is None or type(sm_scale) is float) and isinstance(q, _TENSOR) and isinstance(k, _TENSOR)
-                and isinstance(v, _TENSOR) and _tracing_state() is None):  # (a trace would hold no kernel: the checks below refuse it)
-            status = _STATUS.get(q.get_device())
-            if status is not None:  # regular calls without ids and without need of a plan: one native call
-                done = host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs or 0, status,
-                                    _like_subclass(q))
+        if (eq is None and ek is None and score_func_mode == SCORE_FUNC_MODE0_NOPE and isinstance(q, _TENSOR) and isinstance(k, _TENSOR)
+                and isinstance(v, _TENSOR)):
+            done = _native_forward(host, q, k, v, causal, sm_scale, needs_grad, key_runs or 0)
         if done is None:
             # checks of flash_triton.py:510-520
-            Dq, Dk, Dv = q.shape[-1], k.shape[-1], v.shape[-1]
+            q_shape, k_shape, v_shape = q.shape, k.shape, v.shape
+            Dq, Dk, Dv = q_shape[-1], k_shape[-1], v_shape[-1]
             assert Dq == Dk and Dk == Dv, "feature size of q, k, v should be equal"
             assert Dk in {16, 32, 64, 128}
-            B, H, M, D = q.shape
-            N = k.shape[2]
-            Hk, Hv = k.shape[1], v.shape[1]
+            B, H, M, D = q_shape
+            N = k_shape[2]
+            Hk, Hv = k_shape[1], v_shape[1]
             assert Hk == Hv, "num of heads in k and v should be equal"
             assert H % Hk == 0, "number of heads in q must be a multiple of that in k & v"
             assert (N >= M) or (not causal), "KV length should be larger than M length in causal mode!"
@@ -247,12 +251,15 @@ class FlashAttention(torch.autograd.Function):
                 sm_scale = 1. / math.sqrt(D)
             if not sm_scale > 0:
                 raise NotImplementedError("flash_b200 needs sm_scale > 0")
-            q, k, v = maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v)
+            if not _AS_IS(q, k, v):
+                q, k, v = maybe_contiguous(q), maybe_contiguous(k), maybe_contiguous(v)
             if score_func_mode == SCORE_FUNC_MODE1_DOC:
-                eq = _id_tensor(eq, B, H, M, "eq")
-                ek = _id_tensor(ek, B, H, N, "ek")
-                broadcast = (H == 1) or (eq.stride(1) == 0 and ek.stride(1) == 0)
-                id_heads = 1 if broadcast else H
+                id_heads = _ID_HEADS(eq, ek, B, H, M, N)
+                if not id_heads:
+                    eq = _id_tensor(eq, B, H, M, "eq")
+                    ek = _id_tensor(ek, B, H, N, "ek")
+                    broadcast = (H == 1) or (eq.stride(1) == 0 and ek.stride(1) == 0)
+                    id_heads = 1 if broadcast else H
             with _current(device):
                 prob = _problem(B, H, Hk, M, N, D, q.dtype, causal, score_func_mode, id_heads, sm_scale)
                 status = _status_word(device)
@@ -413,6 +420,16 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
     if (GROUP_QUERIES and score_func_mode == SCORE_FUNC_MODE1_DOC and not causal and eq is not None and ek is not None
             and q.is_cuda and q.dim() == 4 and 128 < q.shape[2] <= _lib.FA_GROUP_MAX_ROWS):
         return _attention_grouped(q, k, v, sm_scale, eq, ek)
+    # A call that needs no gradient has no use for an autograd node, a third of a short call's host time. (Transforms of
+    # torch.func and forward-mode gradients need it for their messages, subclasses for their hooks.)
+    if (eq is None and ek is None and type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(score_func_mode) is int
+            and score_func_mode == SCORE_FUNC_MODE0_NOPE and _HOST is not None
+            and not (_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))
+            and _transforms() is None and _forward_ad._current_level < 0):
+        done = _native_forward(_HOST, q, k, v, causal, sm_scale, False, 0)
+        if done is not None:
+            _count(done[3])
+            return done[0]
     return FlashAttention.apply(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
 
 
