@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
     float* Ps = KVs + 4 * S::cols;
     int* codes = reinterpret_cast<int*>(Ps + S::p);  // two stages
     __shared__ uint8_t visited[kListCap];
+    follow_stream();
     const MaskArgs& mk = p.mask;
     const int i0 = int(gridDim.x - 1 - blockIdx.x) * kR, h = blockIdx.y, b = blockIdx.z, hk = h / p.G;  // long rows first
     const int he = (mk.He == 1) ? 0 : h;
@@ -286,6 +287,7 @@ __global__ void __launch_bounds__(kF32Threads) f32_fwd_kernel(const F32Params p)
 // delta = rowsum(o * dO) (flash_triton.py:161-165): grid (ceil(M / 4), H, B), one warp per row
 template <int D>
 __global__ void __launch_bounds__(128) f32_delta_kernel(const F32Params p) {
+    follow_stream();
     const int i = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int h = blockIdx.y, b = blockIdx.z;
     if (i >= p.mask.L.Mpad) return;
@@ -390,7 +392,7 @@ template <int D>
 __global__ void __launch_bounds__(kF32Threads) f32_bwd_dkdv_kernel(const F32Params p) {
     using S = F32Smem<D>;
     extern __shared__ __align__(16) float sm[];
-    launch_dependents();  // fa_bwd's dQ kernel reads nothing that this one writes
+    follow_stream();  // (in this order: fa_bwd's dQ kernel reads nothing that this one writes, but delta, which is complete now)
     float* Ks = sm;
     float* Vs = Ks + S::rows;
     float* QDs = Vs + S::rows;            // two stages of Q, dO
@@ -504,15 +506,15 @@ static cudaError_t launch_f32_t(int which, const F32Params& p, bool overlap, cud
     auto run = [&](auto kern, int smem, int rows, int heads) {
         const cudaError_t e = allow_smem(kern, smem, allowed[which]);
         if (e != cudaSuccess) return e;
-        if (overlap) return launch_overlapping(kern, dim3(cdiv(rows, kR), heads, p.B), kF32Threads, smem, stream, p);
-        kern<<<dim3(cdiv(rows, kR), heads, p.B), kF32Threads, smem, stream>>>(p);
+        const dim3 grid(cdiv(rows, kR), heads, p.B);
+        if (which != 3 || overlap) return launch_overlapping(kern, grid, kF32Threads, smem, stream, p);
+        kern<<<grid, kF32Threads, smem, stream>>>(p);
         return cudaGetLastError();
     };
     if (which == 0) return run(f32_fwd_kernel<D>, fwd_smem, mk.M, p.H);
     if (which == 2) return run(f32_bwd_dkdv_kernel<D>, bwd_smem, mk.N, p.Hk);
     if (which == 3) return run(f32_bwd_dq_kernel<D>, bwd_smem, mk.M, p.H);
-    f32_delta_kernel<D><<<dim3(unsigned(mk.L.Mpad / 4), p.H, p.B), 128, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapping(f32_delta_kernel<D>, dim3(unsigned(mk.L.Mpad / 4), p.H, p.B), 128, 0, stream, p);
 }
 
 // which: 0 forward, 1 delta, 2 dK / dV, 3 dQ. overlap: the launch directly before this one in the stream is the dK/dV

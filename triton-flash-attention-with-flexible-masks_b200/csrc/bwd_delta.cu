@@ -12,6 +12,7 @@ namespace fa {
 // with head dims 16 and 32 only the first 2 or 4 threads of a row have any).
 template <int D, bool BF16>
 __global__ void __launch_bounds__(128) bwd_delta_kernel(const DeltaParams p) {
+    follow_stream();
     const int h = blockIdx.y, b = blockIdx.z;
     const int row = blockIdx.x * 16 + (threadIdx.x >> 3);
     const int part = threadIdx.x & 7;
@@ -53,20 +54,11 @@ __global__ void __launch_bounds__(128) bwd_delta_kernel(const DeltaParams p) {
 
 cudaError_t launch_bwd_delta(const DeltaParams& p, cudaStream_t stream) {
     dim3 grid(unsigned(p.Mpad / 16), p.H, p.B);
-    if (p.D == 128) {
-        if (p.bf16) bwd_delta_kernel<128, true><<<grid, 128, 0, stream>>>(p);
-        else bwd_delta_kernel<128, false><<<grid, 128, 0, stream>>>(p);
-    } else if (p.D == 32) {
-        if (p.bf16) bwd_delta_kernel<32, true><<<grid, 128, 0, stream>>>(p);
-        else bwd_delta_kernel<32, false><<<grid, 128, 0, stream>>>(p);
-    } else if (p.D == 16) {
-        if (p.bf16) bwd_delta_kernel<16, true><<<grid, 128, 0, stream>>>(p);
-        else bwd_delta_kernel<16, false><<<grid, 128, 0, stream>>>(p);
-    } else {
-        if (p.bf16) bwd_delta_kernel<64, true><<<grid, 128, 0, stream>>>(p);
-        else bwd_delta_kernel<64, false><<<grid, 128, 0, stream>>>(p);
-    }
-    return cudaGetLastError();
+    auto run = [&](auto kern) { return launch_overlapping(kern, grid, 128, 0, stream, p); };
+    if (p.D == 128) return run(p.bf16 ? bwd_delta_kernel<128, true> : bwd_delta_kernel<128, false>);
+    if (p.D == 32) return run(p.bf16 ? bwd_delta_kernel<32, true> : bwd_delta_kernel<32, false>);
+    if (p.D == 16) return run(p.bf16 ? bwd_delta_kernel<16, true> : bwd_delta_kernel<16, false>);
+    return run(p.bf16 ? bwd_delta_kernel<64, true> : bwd_delta_kernel<64, false>);
 }
 
 }  // namespace fa

@@ -165,14 +165,14 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             mbar_init(BAR(B_ITEMFULL + s), 1);
             mbar_init(BAR(B_ITEMEMPTY + s), 18);  // producer, MMA issuer, sixteen compute warps
         }
-        misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
         fence_mbar_init();
-        launch_dependents();  // fa_bwd's dQ kernel reads nothing that this one writes
     }
     if (warp == 17) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
     }
+    follow_stream();  // (in this order: fa_bwd's dQ kernel reads nothing that this one writes, but delta, which is complete now)
+    if (tid == 0) misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -670,8 +670,7 @@ static cudaError_t launch_dkdv_t(const CUtensorMap& tq, const CUtensorMap& tk, c
     if (e != cudaSuccess) return e;
     const int n_items = p.mask.L.nK * p.Hk * p.B;
     const int grid = n_items < num_sms ? n_items : num_sms;
-    kern<<<grid, kDkdvThreads, smem, stream>>>(tq, tk, tv, tdo, tdk, tdv, p);
-    return cudaGetLastError();
+    return launch_overlapping(kern, dim3(grid), kDkdvThreads, smem, stream, tq, tk, tv, tdo, tdk, tdv, p);
 }
 
 

@@ -126,6 +126,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
         fence_mbar_init();
     }
+    launch_dependents();  // what follows in the stream waits for this kernel's end, hence for the dK/dV kernel's
     if (warp == 9) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
@@ -593,8 +594,8 @@ static cudaError_t launch_dq_t(const CUtensorMap& tq, const CUtensorMap& tk, con
 
 
 // overlap: the launch directly before this one in the stream is the dK/dV kernel of the same backward, and the CTAs of
-// this one may take the SMs that it has already left. It reads nothing that dK/dV writes; delta and the plan are older
-// than the dK/dV launch, which is not a programmatic one. Whole steps, replayed as graphs: 4 x 12 heads x 1000 x 64
+// this one may take the SMs that it has already left. It reads nothing that dK/dV writes; delta and the plan were complete
+// before a block of dK/dV let this launch begin. Whole steps, replayed as graphs: 4 x 12 heads x 1000 x 64
 // packed 104.7 -> 94.0 us, 16 x 8 x 577 x 32 150.4 -> 143.3 us, 2 x 32 / 8 x 3001 x 128 causal 749 -> 708 us; where
 // dK/dV has many small items, which leave no tail, the same within the noise.
 cudaError_t launch_bwd_dq(int D, bool bf16, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,

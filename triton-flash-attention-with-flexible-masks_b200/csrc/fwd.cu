@@ -139,13 +139,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             mbar_init(BAR(B_OFULL + s), 1);
             mbar_init(BAR(B_OFREE + s), 4);
         }
-        misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
         fence_mbar_init();
     }
     if (warp == 13) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
     }
+    follow_stream();
+    if (tid == 0) misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -743,6 +744,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
 // in fp32 in the order of the parts. Bound by latency: at most 20 MB are read (fwd_splits in api.cu), mostly from L2.
 template <bool BF16>
 __global__ void __launch_bounds__(256) fwd_combine_kernel(const CombineParams p) {
+    follow_stream();
     const int64_t row = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);  // of the [B, H, M] rows
     const int lane = threadIdx.x & 31;
     const int64_t rows = int64_t(p.B) * p.H * p.M;
@@ -788,9 +790,7 @@ __global__ void __launch_bounds__(256) fwd_combine_kernel(const CombineParams p)
 
 cudaError_t launch_fwd_combine(bool bf16, const CombineParams& p, cudaStream_t stream) {
     const unsigned grid = unsigned((int64_t(p.B) * p.H * p.M + 7) / 8);
-    if (bf16) fwd_combine_kernel<true><<<grid, 256, 0, stream>>>(p);
-    else fwd_combine_kernel<false><<<grid, 256, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapping(bf16 ? fwd_combine_kernel<true> : fwd_combine_kernel<false>, dim3(grid), 256, 0, stream, p);
 }
 
 // ---- host launcher (called from api.cu) -------------------------------------------------
@@ -805,8 +805,7 @@ static cudaError_t launch_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, co
     const int heads = SHORT ? p.H / p.G * cdiv(p.G, p.pack) : p.H;
     const int n_items = p.mask.L.nQ * heads * p.B * (SHORT ? p.ns : 1);
     dim3 grid(n_items < num_sms ? n_items : num_sms);
-    kern<<<grid, kFwdThreads, smem, stream>>>(tq, tk, tv, to, p);
-    return cudaGetLastError();
+    return launch_overlapping(kern, grid, kFwdThreads, smem, stream, tq, tk, tv, to, p);
 }
 
 

@@ -37,6 +37,7 @@ constexpr int kSortThreads = 1024;
 __global__ void __launch_bounds__(kSortThreads) group_rows_kernel(IdRows eq, int M, int P, int He, int32_t* order,
                                                                   int32_t* inverse, int32_t* grouped, int* status) {
     extern __shared__ __align__(16) unsigned long long keys[];
+    fa::follow_stream();
     const int he = blockIdx.x, b = blockIdx.y;
     const int64_t row = (int64_t(b) * He + he) * M;
     for (int i = threadIdx.x; i < P; i += kSortThreads) {
@@ -94,6 +95,7 @@ struct RowTensor {
 // writes whole 128-byte (or longer) stretches.
 __global__ void __launch_bounds__(256) permute_rows_kernel(RowTensor t, const int32_t* index, int M, int H, int He,
                                                            int vec, int64_t total) {
+    fa::follow_stream();
     const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (g >= total) return;
     const int c = int(g % vec);
@@ -136,9 +138,9 @@ extern "C" int fa_group_rows(const fa_problem* p, const fa_ids* eq, int32_t* ord
     if (fa::allow_smem(group_rows_kernel, int(FA_GROUP_MAX_ROWS * sizeof(unsigned long long)), allowed) != cudaSuccess)
         return FA_ERR_LAUNCH;
     const IdRows rows{eq->ptr, eq->stride[0], eq->stride[1], eq->stride[2], eq->dtype == FA_ID_INT64};
-    group_rows_kernel<<<dim3(p->id_heads, p->B), kSortThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        rows, p->M, P, p->id_heads, order, inverse, grouped_ids, status);
-    return cudaGetLastError() == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+    const cudaError_t e = fa::launch_overlapping(group_rows_kernel, dim3(p->id_heads, p->B), kSortThreads, int(smem),
+                                                 static_cast<cudaStream_t>(stream), rows, p->M, P, p->id_heads, order, inverse, grouped_ids, status);
+    return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 
 extern "C" int fa_permute_rows(const fa_problem* p, const fa_tensor* src, const fa_tensor* dst, const int32_t* index,
@@ -162,7 +164,7 @@ extern "C" int fa_permute_rows(const fa_problem* p, const fa_tensor* src, const 
     const int64_t blocks = (total + 255) / 256;
     if (blocks > 0x7fffffffLL) return FA_ERR_UNSUPPORTED;
     const int He = (p->mode == FA_MODE1_DOC) ? p->id_heads : 1;
-    permute_rows_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(t, index, p->M, p->H, He, vec,
-                                                                                         total);
-    return cudaGetLastError() == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+    const cudaError_t e = fa::launch_overlapping(permute_rows_kernel, dim3(unsigned(blocks)), 256, 0, static_cast<cudaStream_t>(stream), t, index,
+                                                 p->M, p->H, He, vec, total);
+    return e == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }

@@ -4,6 +4,7 @@
 // bound, flash_triton.py:94-129); the rule encoded is flash_triton.py:114.
 #include "../../include/fa_b200.h"
 #include "common.cuh"
+#include "params.cuh"
 
 namespace fa {
 
@@ -42,6 +43,7 @@ __device__ __forceinline__ int block_reduce_max(int v, int* scratch) {
 __global__ void __launch_bounds__(128) plan_codes_kernel(IdsView eq, IdsView ek, int32_t* plan, PlanLayout L,
                                                          int* status) {
     __shared__ int scratch[4];
+    follow_stream();
     const int he = blockIdx.y, b = blockIdx.z;
     const int64_t bh = int64_t(b) * L.He + he;
     const bool is_q = int(blockIdx.x) < L.nQ;
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(128) plan_codes_kernel(IdsView eq, IdsView ek,
 // one key block over query blocks.
 __global__ void __launch_bounds__(128) plan_ranges_kernel(int32_t* plan, PlanLayout L, int gap, int causal) {
     __shared__ int scratch[4];
+    follow_stream();
     const int he = blockIdx.y, b = blockIdx.z;
     const int64_t bh = int64_t(b) * L.He + he;
     const bool is_q = int(blockIdx.x) < L.nQ;
@@ -144,6 +147,7 @@ __global__ void __launch_bounds__(128) plan_ranges_kernel(int32_t* plan, PlanLay
 // come before it.
 __global__ void __launch_bounds__(1024) plan_order_kernel(int32_t* plan, PlanLayout L) {
     __shared__ int len[kListCap];
+    follow_stream();
     const bool is_q = blockIdx.x == 0;
     const int he = blockIdx.y, b = blockIdx.z;
     const int64_t bh = int64_t(b) * L.He + he;
@@ -179,6 +183,7 @@ __device__ __forceinline__ int warp_max(int v) { return __reduce_max_sync(0xffff
 __global__ void __launch_bounds__(1024) plan_small_kernel(IdsView eq, IdsView ek, int32_t* plan, PlanLayout L, int gap, int causal,
                                                           int* status) {
     __shared__ int smin[kSmallBlocks], smax[kSmallBlocks], len[kSmallBlocks];  // query blocks, then key blocks
+    follow_stream();
     const int he = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t bh = int64_t(b) * L.He + he;
     const int n = L.nQ + L.nK;
@@ -308,14 +313,13 @@ cudaError_t launch_plan_build(const void* eq_ptr, const int64_t* eq_stride, int 
     IdsView q{eq_ptr, eq_stride[0], eq_stride[1], eq_stride[2], eq64};
     IdsView k{ek_ptr, ek_stride[0], ek_stride[1], ek_stride[2], ek64};
     if (L.nQ + L.nK <= kSmallBlocks) {
-        plan_small_kernel<<<dim3(L.He, L.B), 1024, 0, stream>>>(q, k, plan, L, gap, causal, status);
-        return cudaGetLastError();
+        return launch_overlapping(plan_small_kernel, dim3(L.He, L.B), 1024, 0, stream, q, k, plan, L, gap, causal, status);
     }
     dim3 grid(L.nQ + L.nK, L.He, L.B);
-    plan_codes_kernel<<<grid, 128, 0, stream>>>(q, k, plan, L, status);
-    plan_ranges_kernel<<<grid, 128, 0, stream>>>(plan, L, gap, causal);
-    plan_order_kernel<<<dim3(2, L.He, L.B), 1024, 0, stream>>>(plan, L);
-    return cudaGetLastError();
+    cudaError_t e = launch_overlapping(plan_codes_kernel, grid, 128, 0, stream, q, k, plan, L, status);
+    if (e == cudaSuccess) e = launch_overlapping(plan_ranges_kernel, grid, 128, 0, stream, plan, L, gap, causal);
+    if (e == cudaSuccess) e = launch_overlapping(plan_order_kernel, dim3(2, L.He, L.B), 1024, 0, stream, plan, L);
+    return e;
 }
 
 cudaError_t launch_debug_mask(const MaskArgs& a, uint8_t* keep, uint8_t* tile_class, cudaStream_t stream) {

@@ -340,8 +340,14 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 
 // Programmatic launch: the next kernel of the stream, if it was launched that way, may start once every block of this
 // grid has said so (or left); and the wait, in that kernel, for the kernel before it to be complete. No-ops otherwise.
+// A kernel that begins with follow_stream() touches no memory that others use before the kernel before it, and all that is older,
+// is complete; the next one may then set itself up (barriers, tensor memory, its blocks' launch) while this one runs.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void follow_stream() {
+    wait_prerequisites();
+    launch_dependents();
+}
 
 // ----------------------------------------------------------------------------------------
 // descriptors
