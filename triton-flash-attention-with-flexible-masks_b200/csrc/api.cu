@@ -318,6 +318,7 @@ int run_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, cons
     qp.B = p->B;
     qp.H = p->H;
     qp.G = p->H / p->Hk;
+    qp.ksteps = p->D / 16;
     qp.gh = head_group(p, p->H * p->B);
     qp.by_length = (p->mode == FA_MODE1_DOC && int64_t(fa::cdiv(p->M, fa::kBlk) * p->H * p->B) < 32 * int64_t(sms)) ? 1 : 0;
     qp.scale_log2 = p->sm_scale * kLog2e;
@@ -544,6 +545,7 @@ int fa_bwd_dkdv(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, con
     kp.H = p->H;
     kp.Hk = p->Hk;
     kp.G = p->H / p->Hk;
+    kp.ksteps = p->D / 16;
     kp.gh = head_group(p, p->Hk * p->B);
     kp.by_length = (p->mode == FA_MODE1_DOC && int64_t(fa::cdiv(p->N, fa::kBlk) * p->Hk * p->B) < 32 * int64_t(sms)) ? 1 : 0;
     kp.scale_log2 = p->sm_scale * kLog2e;

@@ -51,6 +51,9 @@ struct DkdvParams {
     const float* delta;  // [B, H, Mpad]
     MaskArgs mask;
     int B, H, Hk, G;
+    // Head dim / 16. The columns that 64-wide tiles have beyond it are zeros, and S and dP leave them out: 16 x 8 heads x 577 x 32, dK/dV
+    // 46.5 -> 45.5 us, dQ 40.6 -> 39.8. (The forward's S, which nothing waits for, was no faster.)
+    int ksteps;
     int gh;  // kv heads per scheduling group
     int by_length;  // take the blocks of a head in the plan's sorted order (few items per CTA)
     float scale_log2, sm_scale;
@@ -63,6 +66,7 @@ struct DqParams {
     const float* delta;
     MaskArgs mask;
     int B, H, G;
+    int ksteps;  // as in DkdvParams
     int gh;  // heads per scheduling group
     int by_length;  // take the blocks of a head in the plan's sorted order (few items per CTA)
     float scale_log2, sm_scale;
