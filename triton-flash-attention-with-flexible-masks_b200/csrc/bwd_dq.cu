@@ -7,8 +7,7 @@
 //              [64g, 64g+64) of every tile
 //   warp 8     TMA producer (per item Q with the per-row LSE / delta, and dO; K ring; V) and the TMA
 //              store of a finished item's dQ
-//   warp 9     tcgen05.mma issuer for S and dQ; owns the TMEM allocation
-//   warp 10    tcgen05.mma issuer for dP
+//   warps 9,10 tcgen05.mma issuers (10: dP at D = 64); warp 9 owns the TMEM allocation
 //   warp 11    scheduler: per item, the range of candidate key blocks and their codes
 // Q has two slots (item parity); a slot also stages its item's dQ for the TMA store, so the next
 // item's Q, K and first S tiles do not wait for the epilogue. dO, V and the dP columns are single
@@ -69,6 +68,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
               const __grid_constant__ CUtensorMap tmdQ, const DqParams p) {
     using S = DqSmem<D>;
     constexpr int NSK = S::NSK;
+    constexpr bool kOne = D == 128;  // one warp issues all MMAs
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -111,7 +111,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
             mbar_init(BAR(B_ITEMFULL + s), 1);
-            mbar_init(BAR(B_ITEMEMPTY + s), 11);  // producer, two MMA issuers, eight compute warps
+            mbar_init(BAR(B_ITEMEMPTY + s), kOne ? 10 : 11);  // producer, MMA issuers, eight compute warps
             mbar_init(BAR(B_QFULL + s), 1);
             mbar_init(BAR(B_STAGED + s), 256);
             mbar_init(BAR(B_SFULL + s), 1);
@@ -291,15 +291,15 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 if (ok && k >= 2) ok = store_dq(k - 2);
                 if (ok && k >= 1) ok = store_dq(k - 1);
             }
-        } else {
-            // ------------------------------ MMA issuers (warps 9, 10) ------------------------------
-            // Two issuing warps, so that the blocking tcgen05.mma issue and barrier round trips of
-            // one stream do not delay the other:
-            //   warp 9 : S(0), S(1); then per tile dQ(t) += dS K(t) followed by S(t+2) (which
-            //            overwrites dS(t): same warp, in order)
-            //   warp 10: dP(t+1) = dO V(t+1)^T as soon as dS(t) has been written (dP columns free)
-            // Tiles are numbered across items (gi), so that the S buffers, the K ring, V and every
-            // per-tile barrier simply carry on from one item to the next.
+        } else if (!kOne || warp == 9) {
+            // ------------------------------ MMA issuers (warp 9; at D = 64 also 10) ------------------------------
+            // When dS(t) has been written: dQ(t) += dS K(t), dP(t+1) (over dP(t), which has been read), S(t+2) (over dS(t)). At D = 128 one
+            // warp issues them in this order, that in which the pipe should take them: with a warp of its own dP(t+1) shared the pipe with
+            // both others, and all three came late (2 x 32 / 8 heads x 3001 x 128 causal 249 -> 237 us, 4 x 16 x 4096 x 128 in documents
+            // 161 -> 155, 32 x 32768 x 128 in 64 documents 1027 -> 990; dP(t+1) first, 257, 165 and 1061: it may still wait for V). At D = 64 the
+            // products are half as long and their issue is what counts: dP has a warp of its own (16 x 8 x 577 x 32 40.5 us, 41.7 with one).
+            // Tiles are numbered across items (gi), so that the S buffers, the K ring, V and every per-tile barrier simply carry on from one
+            // item to the next.
             {
                 const uint32_t utmem = uniform(int(tmem));
                 constexpr uint32_t idesc_s = make_idesc(BF16, 128, 128, false, false);
@@ -323,18 +323,30 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     if (!ok) break;
                     const int T = uniform(info[s * 8 + 2]);
                     if (uniform(info[s * 8 + 3]) < 0) break;
+                    auto issue_dp = [&](int t) {
+                        if (!mbar_wait_warp(BAR(B_VFULL), (gt + t) & 1, ab, ST_WAIT_TIMEOUT + 25)) return false;
+                        tc_fence_after();
+                        ss_mmas(utmem + 256u, sdO, sV);
+                        if (!kOne) umma_commit(BAR(B_VEMPTY));
+                        umma_commit(BAR(B_DPFULL));
+                        if (kOne) umma_commit(BAR(B_VEMPTY));
+                        if (t + 1 == T) umma_commit(BAR(B_DOEMPTY));
+                        return true;
+                    };
                     if (T > 0 && warp == 9) {
-                        ok = mbar_wait_warp(BAR(B_QFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 23);
-                        const uint32_t q_tile = sQ(s);
-                        for (int t = 0; t < 2 && t < T && ok; ++t) {
+                        auto issue_s = [&](int t) {
                             const int gi = gt + t;
-                            ok = k_ready(gi);
-                            if (ok) {
-                                tc_fence_after();
-                                ss_mmas(utmem + uint32_t(gi & 1) * 128u, q_tile, sK(gi % NSK));
-                                umma_commit(BAR(B_SFULL + (gi & 1)));
-                            }
-                        }
+                            if (!k_ready(gi)) return false;
+                            tc_fence_after();
+                            ss_mmas(utmem + uint32_t(gi & 1) * 128u, sQ(s), sK(gi % NSK));
+                            umma_commit(BAR(B_SFULL + (gi & 1)));
+                            return true;
+                        };
+                        ok = mbar_wait_warp(BAR(B_QFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 23);
+                        if (ok) ok = issue_s(0);
+                        if (kOne && ok) ok = mbar_wait_warp(BAR(B_DOFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 23);
+                        if (kOne && ok) ok = issue_dp(0);
+                        if (ok && T > 1) ok = issue_s(1);
                         // dQ(0) overwrites the accumulator: the previous item's epilogue must have read it
                         if (ok && kk > 0) ok = mbar_wait_warp(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 35);
                         for (int t = 0; t < T && ok; ++t) {
@@ -350,33 +362,21 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                                         (t > 0 || kk2 > 0) ? 1u : 0u);
                             }
                             umma_commit(BAR(B_KEMPTY + st));
+                            if (kOne && t + 1 < T) ok = issue_dp(t + 1);
                             // K(t+2) reuses the stage that dQ(t-1) releases, so it is waited for only now
-                            if (t + 2 < T) {
-                                ok = k_ready(gi + 2);
-                                if (ok) {
-                                    tc_fence_after();
-                                    ss_mmas(a, q_tile, sK((gi + 2) % NSK));
-                                    umma_commit(BAR(B_SFULL + (gi & 1)));
-                                }
-                            }
+                            if (ok && t + 2 < T) ok = issue_s(t + 2);
                         }
                         if (!ok) break;
                         umma_commit(BAR(B_DONE));
-                    } else if (T > 0) {
+                    } else if (T > 0) {  // warp 10
                         ok = mbar_wait_warp(BAR(B_DOFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 23);
                         for (int t = 0; t < T && ok; ++t) {
                             const int gi = gt + t;
-                            ok = mbar_wait_warp(BAR(B_VFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 25);
                             // dP(gi) may overwrite the dP columns once every thread has read dP(gi-1)
-                            if (ok && gi > 0) ok = mbar_wait_warp(BAR(B_DSFULL + ((gi - 1) & 1)), ((gi - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 26);
-                            if (!ok) break;
-                            tc_fence_after();
-                            ss_mmas(utmem + 256u, sdO, sV);
-                            umma_commit(BAR(B_VEMPTY));
-                            umma_commit(BAR(B_DPFULL));
+                            if (gi > 0) ok = mbar_wait_warp(BAR(B_DSFULL + ((gi - 1) & 1)), ((gi - 1) >> 1) & 1, ab, ST_WAIT_TIMEOUT + 26);
+                            if (ok) ok = issue_dp(t);
                         }
                         if (!ok) break;
-                        umma_commit(BAR(B_DOEMPTY));
                     }
                     if (T > 0) ++kk;
                     gt += T;
