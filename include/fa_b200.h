@@ -113,6 +113,9 @@ int fa_plan_optional(const fa_problem* p, int32_t backward);
 int fa_plan_build(const fa_problem* p, const fa_ids* eq, const fa_ids* ek, void* plan, size_t plan_bytes,
                   int32_t* status, void* stream);
 
+/* All launches but that of a separate fa_bwd_dq are programmatic: a kernel sets itself up while the one before it in the stream
+ * ends, and waits for that one's end before it reads or writes memory. Seen from the stream nothing changes. */
+
 /* Forward (replaces flash_triton.py:541). o has q's shape; lse is [B, H, fa_padded_rows(M)] fp32,
  * log2-domain log-sum-exp of the scaled scores (flash_triton.py:133), -inf for a row with no
  * unmasked key (whose output row is 0). plan may be NULL when mode == FA_MODE0_NOPE (here and in

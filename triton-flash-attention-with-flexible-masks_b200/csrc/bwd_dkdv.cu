@@ -629,7 +629,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
             }
             if (!ok) break;
-            // both accumulators have been read: warp 10 may start the next item's dV / dK
+            // both accumulators have been read: warp 17 may start the next item's dV / dK
             tc_fence_before();
             if (NIT > 0) {
                 mbar_arrive_warp(BAR(B_ACCFREE), lane);

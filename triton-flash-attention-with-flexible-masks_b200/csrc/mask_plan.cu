@@ -172,9 +172,9 @@ __global__ void __launch_bounds__(1024) plan_order_kernel(int32_t* plan, PlanLay
 // The three kernels above in one, for id rows of at most kSmallBlocks blocks: grid (He, B), 1024 threads. A warp takes a block
 // of 128 ids, its lane x the ids x, x + 32, x + 64 and x + 96; the block statistics pass through shared memory.
 // Bound by latency; the same words in the plan. us a plan in a replayed graph, gaps between launches included, by three launches
-// and here: 16 blocks a row, 4 rows 6.6, 3.7; 32 blocks 6.7, 4.8; 64 blocks, 1 row 6.3, 7.0; 4 rows 7.0, 7.2; 32 rows 9.0, 7.3;
-// 72 blocks, 1 row 7.1, 8.4; 8 rows 7.5, 8.4; 32 rows 9.7, 8.5; 128 blocks, 8 rows 8.0, 12.4; 32 rows 12.8, 12.4. Up to two blocks
-// a warp it is as fast or faster on the device, and saves the host two launches; beyond, only with 32 rows or more.
+// (each set up while the one before it ends) and here: 16 blocks a row, 4 rows 5.4, 3.1; 32 blocks 5.6, 4.2; 64 blocks, 4 rows 5.6, 6.7; 8
+// rows 6.1, 6.7; 32 rows 8.1, 6.8; 72 blocks, 8 rows 6.2, 8.7; 32 rows 8.3, 8.9; 128 blocks, 8 rows 7.1, 11.7; 32 rows 12.2, 11.8. On the device it is
+// faster up to one block a warp, or with 32 rows; from there to two blocks a warp it costs up to 1 us and saves the host two launches.
 constexpr int kSmallBlocks = FA_PLAN_ONE_KERNEL_BLOCKS;
 
 __device__ __forceinline__ int warp_min(int v) { return __reduce_min_sync(0xffffffffu, v); }
