@@ -74,6 +74,8 @@ struct FwdSmem {
     static constexpr int total = off_misc + 16;
 };
 static_assert(FwdSmem<128>::total <= 232448 && FwdSmem<64>::total <= 232448, "shared memory budget");
+// No two blocks of these kernels share an SM, and its tensor memory, though the next launch may start while this one ends.
+static_assert(FwdSmem<128>::total > 116736 && FwdSmem<64>::total > 116736, "shares an SM");
 
 // SHORT: calls without ids whose items are too few or too empty for one item per (query block, head, batch).
 // Two things are added (fwd_pack and fwd_splits in api.cu say when):
