@@ -167,15 +167,16 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         fence_mbar_init();
     }
+    wait_prerequisites();
     if (warp == 17) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
     }
-    follow_stream();  // (in this order: fa_bwd's dQ kernel reads nothing that this one writes, but delta, which is complete now)
     if (tid == 0) misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    launch_dependents();  // (fa_bwd's dQ kernel reads nothing that this one writes, but delta, which is complete since the wait)
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
     // an earlier launch on this device ran into a time-out that the host has not yet cleared

@@ -126,7 +126,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
         fence_mbar_init();
     }
-    launch_dependents();  // what follows in the stream waits for this kernel's end, hence for the dK/dV kernel's
+    // (an overlapped launch does not wait here: the dK/dV kernel's blocks hold their tensor memory since before it could begin)
     if (warp == 9) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
@@ -134,6 +134,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    launch_dependents();  // what follows in the stream waits for this kernel's end, hence for the dK/dV kernel's
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
     // Item k of this CTA. Items are handed out in order from a counter in the plan (any CTA takes the next one: the work

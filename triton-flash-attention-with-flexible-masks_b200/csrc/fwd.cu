@@ -74,7 +74,9 @@ struct FwdSmem {
     static constexpr int total = off_misc + 16;
 };
 static_assert(FwdSmem<128>::total <= 232448 && FwdSmem<64>::total <= 232448, "shared memory budget");
-// No two blocks of these kernels share an SM, and its tensor memory, though the next launch may start while this one ends.
+// No two blocks of the library's kernels share an SM, and its tensor memory, though the next launch may start while this one ends.
+// (Beside a block of head dim 64 another library's may have room; the order in which each of the kernels waits, allocates and lets
+// the next one begin keeps that one's allocation from mattering.)
 static_assert(FwdSmem<128>::total > 116736 && FwdSmem<64>::total > 116736, "shares an SM");
 
 // SHORT: calls without ids whose items are too few or too empty for one item per (query block, head, batch).
@@ -143,15 +145,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         }
         fence_mbar_init();
     }
+    wait_prerequisites();
     if (warp == 13) {
         tmem_alloc(sbase + S::off_misc, 512);
         tmem_relinquish();
     }
-    follow_stream();
     if (tid == 0) misc[1] = (status_is_fatal(*reinterpret_cast<volatile int*>(p.status)) || (sbase & 1023u) != 0) ? 1 : 0;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    launch_dependents();
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
     // an earlier launch on this device ran into a time-out that the host has not yet cleared

@@ -110,8 +110,8 @@ inline cudaError_t allow_smem(Kernel kern, int bytes, SmemAllowed& allowed) {
 }
 
 // Launches `kern` so that it may start on SMs that the kernel before it in the stream has left, or leaves room on, once
-// all of that one's blocks have called launch_dependents() or left. `kern` begins with follow_stream(), or, where it needs nothing
-// of that kernel, ends with wait_prerequisites().
+// all of that one's blocks have called launch_dependents() or left. `kern` begins with follow_stream() (or with its two parts around
+// the allocation of tensor memory), or, where it needs nothing of that kernel, ends with wait_prerequisites().
 // Nearly all launches are of this kind: the gap from one kernel to the next, 2 to 3 us with a kernel's setup, shrinks to about 1.
 template <class... Params, class... Args>
 inline cudaError_t launch_overlapping(void (*kern)(Params...), dim3 grid, int threads, int smem, cudaStream_t stream, const Args&... args) {

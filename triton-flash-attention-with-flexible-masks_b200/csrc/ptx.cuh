@@ -341,7 +341,10 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // Programmatic launch: the next kernel of the stream, if it was launched that way, may start once every block of this
 // grid has said so (or left); and the wait, in that kernel, for the kernel before it to be complete. No-ops otherwise.
 // A kernel that begins with follow_stream() touches no memory that others use before the kernel before it, and all that is older,
-// is complete; the next one may then set itself up (barriers, tensor memory, its blocks' launch) while this one runs.
+// is complete; the next one may then set itself up (barriers, its blocks' launch) while this one runs.
+// A kernel that allocates tensor memory does so between the two, and lets the next one begin behind the barrier that follows: an
+// allocation waits, without a limit, for the columns that another block of the SM holds. A block that waited there for a kernel
+// that comes after it in the stream, or held columns that the one before it still has to get, would wait for ever.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void follow_stream() {
