@@ -32,3 +32,9 @@ def test_no_other_kernel_allocates_tensor_memory():
     for name in sorted(os.listdir(CSRC)):
         if name not in ("fwd.cu", "bwd_dkdv.cu", "bwd_dq.cu", "ptx.cuh"):
             assert "tmem_alloc(" not in _code(name), name
+
+
+@pytest.mark.parametrize("name", sorted(n for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh"))))
+def test_no_loads_that_ask_for_read_only_memory(name):
+    """A kernel begins while the one before it still writes what it is going to read."""
+    assert not re.search(r"__ldg\b|__restrict__|ld\.global(\.\w+)*\.nc\b", _code(name))

@@ -25,8 +25,8 @@ __global__ void __launch_bounds__(128) bwd_delta_kernel(const DeltaParams p) {
                             2 * (int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh + int64_t(row) * p.d_o.sl + part * PER);
 #pragma unroll
         for (int v = 0; v < PER / 8; ++v) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(po) + v);
-            const uint4 g = __ldg(reinterpret_cast<const uint4*>(pd) + v);
+            const uint4 a = reinterpret_cast<const uint4*>(po)[v];
+            const uint4 g = reinterpret_cast<const uint4*>(pd)[v];
             const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
             const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll

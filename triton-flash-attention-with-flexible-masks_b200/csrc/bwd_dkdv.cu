@@ -477,7 +477,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const float2* vdelta = reinterpret_cast<const float2*>(p.delta + (int64_t(b) * p.H + hk * G + cg) * mk.L.Mpad + q0 + 2 * (lane & 3));
                 float2 delta[4];
 #pragma unroll
-                for (int n = 0; n < 4; ++n) delta[n] = __ldg(vdelta + 4 * n);
+                for (int n = 0; n < 4; ++n) delta[n] = vdelta[4 * n];
 
                 // keep(x) = (cmin <= x < cmax) & (qc[x] >= 0 | qc[x] == kc) as a 32-bit mask, worked out before the
                 // scores are there
@@ -486,9 +486,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 if (flagged) {
                     if (fl_doc) {
                         const int64_t bh_ids = int64_t(b) * mk.He + ((mk.He == 1) ? 0 : hk * G + cg);
-                        if (kc_g != cg) { kc = __ldg(mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + j); kc_g = cg; }
+                        if (kc_g != cg) { kc = mk.plan[mk.L.off_kc + bh_ids * mk.L.Npad + j]; kc_g = cg; }
                         const int* qcs = mk.plan + mk.L.off_qc + bh_ids * mk.L.Mpad + q0;
-                        const int qc = __ldg(qcs + lane);
+                        const int qc = qcs[lane];
                         keep = codes_equal(qcs, qc, kc, many) | __ballot_sync(0xffffffffu, qc >= 0);
                     }
                     if (fl_range) {

@@ -410,7 +410,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             const int row = qb * kBlk + r;
             const int q0 = qb * kBlk;
             const int64_t bh_ids = int64_t(b) * mk.He + he;
-            const int qc = (mk.mode == 1) ? __ldg(mk.plan + mk.L.off_qc + bh_ids * mk.L.Mpad + row) : 0;
+            const int qc = (mk.mode == 1) ? mk.plan[mk.L.off_qc + bh_ids * mk.L.Mpad + row] : 0;
             // Q's barrier also covers the rows' LSE and delta; the slot is this item's staging area later
             ok = mbar_wait(BAR(B_QFULL + s), (k >> 1) & 1, ab, ST_WAIT_TIMEOUT + 36);
             ok = __all_sync(0xffffffffu, ok);
@@ -434,7 +434,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 if (flagged) {
                     if (fl_doc) {
                         const int* kcs = mk.plan + mk.L.off_kc + bh_ids * mk.L.Npad + k0;
-                        const int kc0 = __ldg(kcs + lane), kc1 = __ldg(kcs + 32 + lane);
+                        const int kc0 = kcs[lane], kc1 = kcs[32 + lane];
                         const uint32_t same0 = codes_equal(kcs, kc0, qc, many), same1 = codes_equal(kcs + 32, kc1, qc, many);
                         if (qc < 0) {  // a row with qc >= 0 passes the id check everywhere
                             keep[0] = same0;

@@ -212,7 +212,7 @@ __device__ __forceinline__ uint32_t codes_equal(const int32_t* codes, int code, 
         const int4* c4 = reinterpret_cast<const int4*>(codes);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const int4 c = __ldg(c4 + u);
+            const int4 c = c4[u];
             mine |= (c.x == own ? 1u << (4 * u) : 0u) | (c.y == own ? 2u << (4 * u) : 0u) |
                     (c.z == own ? 4u << (4 * u) : 0u) | (c.w == own ? 8u << (4 * u) : 0u);
         }

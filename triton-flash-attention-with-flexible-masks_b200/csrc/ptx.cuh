@@ -342,6 +342,8 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // grid has said so (or left); and the wait, in that kernel, for the kernel before it to be complete. No-ops otherwise.
 // A kernel that begins with follow_stream() touches no memory that others use before the kernel before it, and all that is older,
 // is complete; the next one may then set itself up (barriers, its blocks' launch) while this one runs.
+// The kernel has begun by then, so that what the one before it writes is not read-only for as long as it lives: no kernel reads
+// global memory by __ldg or through __restrict__, whose loads (ld.global.nc) ask for that and need not stay behind the wait.
 // A kernel that allocates tensor memory does so between the two, and lets the next one begin behind the barrier that follows: an
 // allocation waits, without a limit, for the columns that another block of the SM holds. A block that waited there for a kernel
 // that comes after it in the stream, or held columns that the one before it still has to get, would wait for ever.
