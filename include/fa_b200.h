@@ -113,8 +113,11 @@ int fa_plan_optional(const fa_problem* p, int32_t backward);
 int fa_plan_build(const fa_problem* p, const fa_ids* eq, const fa_ids* ek, void* plan, size_t plan_bytes,
                   int32_t* status, void* stream);
 
-/* All launches but that of a separate fa_bwd_dq are programmatic: a kernel sets itself up while the one before it in the stream
- * ends, and waits for that one's end before it reads or writes memory. Seen from the stream nothing changes. */
+/* Launches. The kernels are launched programmatically, but for the debug entry points' and that of a separate fa_bwd_dq: a kernel sets
+ * itself up while the one before it in the stream ends, and waits for that one's end before it reads or writes memory. The one exception
+ * is the dQ kernel of fa_bwd, which reads, takes work from the plan's counters and writes dq beside the dK/dV kernel and waits for it
+ * only at its end (see fa_bwd for what may not share memory). What comes after a call in its stream finds the call's results complete; a
+ * programmatic kernel of the caller's does so behind its own wait (griddepcontrol.wait). */
 
 /* Forward (replaces flash_triton.py:541). o has q's shape; lse is [B, H, fa_padded_rows(M)] fp32,
  * log2-domain log-sum-exp of the scaled scores (flash_triton.py:133), -inf for a row with no
@@ -151,8 +154,10 @@ int fa_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const
               const fa_tensor* d_o, const float* lse, const float* delta, const fa_tensor* dq,
               const void* plan, int32_t* status, void* stream);
 
-/* fa_bwd_delta, fa_bwd_dkdv and fa_bwd_dq in this order; stops at the first that fails. The dQ kernel (16-bit types)
- * is launched so that it may start on SMs that the dK/dV kernel has left; it ends after it. */
+/* fa_bwd_delta, fa_bwd_dkdv and fa_bwd_dq in this order; stops at the first that fails. The dQ kernel is launched so
+ * that it may run on SMs that the dK/dV kernel has left, or (fp32) beside its blocks; it ends after it. So dq, dk and dv must share no
+ * memory with one another, nor with q, k, v, d_o, lse, delta or the plan (the three calls one by one ask that of the
+ * tensors of each call only). */
 int fa_bwd(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* o,
            const fa_tensor* d_o, const float* lse, float* delta, const fa_tensor* dq, const fa_tensor* dk,
            const fa_tensor* dv, const void* plan, int32_t* status, void* stream);
