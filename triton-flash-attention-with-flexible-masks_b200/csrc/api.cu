@@ -235,13 +235,14 @@ int sm_count() {
 }
 
 // Runs into which the forward cuts each item's key tiles, for calls without ids that have fewer items than the GPU
-// has SMs. A round of items costs its tiles plus about 4 tile times of fill, drain and epilogue; the second
-// kernel and the fp32 rows cost about 6 more. At most two items per SM, which bounds the workspace at 20 MB.
-// One token, 32 / 8 heads of 128, us between events in a graph with 1 run and with the number taken here: 32768 keys 190, 40.5
-// (18 runs; best of 1, 2, 4, 8, 16: 40.4 with 16); 4096 keys 34, 22 (16; best 20 with 8); 1024 keys 18 (1; 2 and 4 the same); 4
-// sequences of 8192 keys 58, 36 (4; best); 8 of them 63, 54 (2; best). 300 queries against 9000 keys: 16 / 4 heads 63, 38 (3;
-// 2 runs 46, 4 runs 53), 32 / 8 heads 65, 67 (3; 2 runs 83, 4 runs 75): the model's costs are those of an
-// earlier forward, whose chain of tiles was slower. 1000 x 1000 of 8 heads of 64: 16 (1; 2 runs 24).
+// has SMs. A round of items is taken to cost its tiles plus 4 tile times of fill, drain and epilogue, the second
+// kernel and the fp32 rows 6 more (fitted to an earlier forward). At most two items per SM, which bounds the workspace at 20 MB.
+// One token, 32 / 8 heads of 128, us a call in a replayed graph with 1 run and with the number taken here, and the best of 1, 2, 3, 4, 6,
+// 8, 12, 16: 32768 keys 186, 35.2 (18 runs; 34.0 with 16); 4096 keys 29, 16.5 (16; 15.5 with 8); 1024 keys 12.9 (1; 12.2 with 3 or 4);
+// 4 sequences of 8192 keys 53, 30.6 (4, the best); 8 of them 58, 48 (2, the best); 16 of 4500 51 (1, the best). 300 queries against 9000
+// keys: 16 / 4 heads 58, 34 (3, the best; 2 runs 41, 4 runs 47), 32 / 8 heads 63, 61 (3, the best; 2 runs 74, 4 runs 71); 512 against
+// 8192, 32 / 8 heads 56 (1, the best; 2 runs 73). 64 against 4000, 16 heads 30, 18.5 (8; 17.6 with 6). Heads of 64: 1000 x 1000 of 8
+// heads 12 (1, the best; 2 runs 17), 2 x 16 heads of 200 against 3000 22.8, 22.5 (2, the best).
 int fwd_splits(const fa_problem* p, int sms) {
     if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32) return 1;
     const int pack = fwd_pack(p);

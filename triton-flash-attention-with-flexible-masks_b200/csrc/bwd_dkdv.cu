@@ -254,7 +254,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             }
         } else if (warp == 16) {
             // ------------------------------ TMA producer ------------------------------
-            // (converged, with uniform values: with two stages of Q the time from "Q is free" to the next Q is on the way of S^T)
+            // (converged, with uniform values: from a branch of one lane a load takes up to 950 clocks to issue)
             tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
             tma_prefetch_desc(&tmdK); tma_prefetch_desc(&tmdV);
             bool ok = true;
@@ -589,10 +589,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (!ok) break;
             tc_fence_after();
             {
-                // dV and dK * sm_scale (flash_triton.py:313) go out through shared memory: each thread
-                // writes its half rows into the dO and Q ring stage of the item's last tile (dead: all MMAs
-                // of the item are complete) in the tensor maps' 128-byte-swizzled layout; the producer warp
-                // issues the TMA stores, which clip rows >= N.
+                // dV and dK * sm_scale (flash_triton.py:313) go out through shared memory: each thread writes its quarter of a
+                // row of dV into the dO ring stage of the item's last tile, and of dK into the Q ring stage (dead: the last dV,
+                // and then the last dK, MMAs are complete) in the tensor maps' 128-byte-swizzled layout; the producer warp issues
+                // the TMA stores, which clip rows >= N.
                 const int last = gt + NIT + NQ * NDO - 1;  // (of an earlier item, if this one has no tiles)
                 constexpr int COLS = D / 4;  // of a warp
                 const uint32_t c0 = uint32_t(w) * COLS;

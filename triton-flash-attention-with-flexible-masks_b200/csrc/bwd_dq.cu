@@ -297,7 +297,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             // When dS(t) has been written: dQ(t) += dS K(t), dP(t+1) (over dP(t), which has been read), S(t+2) (over dS(t)). At D = 128 one
             // warp issues them in this order, that in which the pipe should take them: with a warp of its own dP(t+1) shared the pipe with
             // both others, and all three came late (2 x 32 / 8 heads x 3001 x 128 causal 249 -> 237 us, 4 x 16 x 4096 x 128 in documents
-            // 161 -> 155, 32 x 32768 x 128 in 64 documents 1027 -> 990; dP(t+1) first, 257, 165 and 1061: it may still wait for V). At D = 64 the
+            // 161 -> 155, 32 x 32768 x 128 in 64 documents 1029 -> 992; dP(t+1) first, 257, 165 and 1061: it may still wait for V). At D = 64 the
             // products are half as long and their issue is what counts: dP has a warp of its own (16 x 8 x 577 x 32 40.5 us, 41.7 with one).
             // Tiles are numbered across items (gi), so that the S buffers, the K ring, V and every per-tile barrier simply carry on from one
             // item to the next.

@@ -195,17 +195,19 @@ __device__ __forceinline__ bool keep_entry(int i, int j, int qc, int kc, int N, 
 // Masks of 32 columns, one bit per column, for the flagged tiles of the backward kernels. They are worked out while the
 // kernels wait for the scores, with one coalesced read of the codes; after the exponentials one select per entry is
 // left, and a chunk whose bits are 0 in every row of a warp is not exponentiated at all. Against compares per entry
-// (and codes read by every thread) on the way from S to P: dK/dV 210 -> 194 us and dQ 118 -> 111 us with 8 x 8 heads of
-// 1024 queries, 8192 keys in 8 documents; 250 -> 242 and 168 -> 163 us with 4 x 16 heads x 4096 in up to 16 documents.
+// (and codes read by every thread) on the way from S to P, with eight compute warps in both kernels: dK/dV 210 -> 194 us and dQ
+// 118 -> 111 us with 8 x 8 heads of 1024 queries, 8192 keys in 8 documents; 250 -> 242 and 168 -> 163 us with 4 x 16 heads x 4096 in
+// up to 16 documents.
 // The forward keeps its compares: the same masks there cost dense tiles 2 % (registers) for 2 % on packed ones.
 __device__ __forceinline__ uint32_t first_bits(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1u; }
 
 // Bit x of the result: codes[x] (32 of them, 16-byte aligned; `code` is the lane's own) equals this thread's `own`. All
 // lanes of the warp take part. A walk over the distinct codes of the chunk costs a shuffle and a vote for each (one to
 // three with packed documents); reading and comparing all 32 costs the same whatever they are. `many`, from the plan's
-// BF_MANY, says which: backward of 4 x 16 heads x 4096 x 128 with ids drawn at random from 4 (walk) 1095 us, from 6, 8
-// or 40 (compare) 1077 us, and 1182, 1504 and 1504 us with a walk of at most six codes and shuffles beyond; random
-// runs of 10 (four or five codes, walk) 961 us, 1007 us with a compare; compares after the scores: 1163 us for all.
+// BF_MANY (more than five codes in 32), says which. Backward of 4 x 16 heads x 4096 x 128 causal, us, always by a walk | always by a
+// compare | as the plan says: ids drawn at random from 4 939 | 936 | 955, from 6 1098 | 1034 | 1038, from 8 1161 | 1047 | 1065, from 40
+// 1658 | 1044 | 1053; random runs of 10 835 | 957 | 930; documents of 500 300 | 311 | 291. Head dim 64: from 4 930 | 885 | 907, from 40
+// 1591 | 855 | 864, runs 736 | 738 | 750, documents 218 | 230 | 219.
 __device__ __forceinline__ uint32_t codes_equal(const int32_t* codes, int code, int own, bool many) {
     uint32_t mine = 0u;
     if (many) {

@@ -174,7 +174,8 @@ __global__ void __launch_bounds__(1024) plan_order_kernel(int32_t* plan, PlanLay
 // Bound by latency; the same words in the plan. us a plan in a replayed graph, gaps between launches included, by three launches
 // (each set up while the one before it ends) and here: 16 blocks a row, 4 rows 5.4, 3.1; 32 blocks 5.6, 4.2; 64 blocks, 4 rows 5.6, 6.7; 8
 // rows 6.1, 6.7; 32 rows 8.1, 6.8; 72 blocks, 8 rows 6.2, 8.7; 32 rows 8.3, 8.9; 128 blocks, 8 rows 7.1, 11.7; 32 rows 12.2, 11.8. On the device it is
-// faster up to one block a warp, or with 32 rows; from there to two blocks a warp it costs up to 1 us and saves the host two launches.
+// faster up to one block a warp, and up to two with 32 rows. With 33 to 64 blocks and few rows it is slower, by up to 1.1 us, but saves
+// the host two launches (a call with ids and its gradients is bound by the host up to some 2000 tokens): the line is drawn there.
 constexpr int kSmallBlocks = FA_PLAN_ONE_KERNEL_BLOCKS;
 
 __device__ __forceinline__ int warp_min(int v) { return __reduce_min_sync(0xffffffffu, v); }

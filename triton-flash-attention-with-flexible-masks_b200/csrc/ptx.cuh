@@ -75,7 +75,7 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 
 // Default limit of one wait, in SM clocks (~0.25 s at 2 GHz). Legitimate waits in these kernels last a few tile times
 // (microseconds), except the item schedulers', for a slot whose item is at work: up to 1024 tiles in the forward and dQ, and
-// as many for each head of a group in dK/dV, of 1400 to 3100 clocks each. But a CTA that is time-sliced out (another
+// as many for each head of a group in dK/dV, of 1400 to 3000 clocks each. But a CTA that is time-sliced out (another
 // context on the GPU, a profiler replay) sees the clock run on: hosts that share a GPU between
 // contexts can raise the limit (FA_B200_WAIT_LIMIT_CLOCKS, read by the library when it is loaded).
 constexpr long long kWaitLimitClocks = 500LL * 1000 * 1000;
