@@ -1,12 +1,17 @@
 // The host side of a regular `attention()` call in one native call each way: allocations, the problem and tensor
-// descriptors, and the launches of fa_b200.h. The autograd node stays in Python (ops.py), and so do all messages: a
-// call that is not regular (another layout, device, shape or type than the kernels take as they are) is declined with
-// None, and ops.py's general code copies, asks or raises. Bound by per-call overhead: a forward of 8 heads of 200
-// queries took 27 us of host time around 8 us of kernel through ctypes.
-#include <c10/cuda/CUDAStream.h>
+// descriptors, the launches of fa_b200.h and the autograd node. The general code and its node stay in Python (ops.py), and so do all
+// messages: a call that is not regular (another layout, device, shape or type than the kernels take as they are) is declined with
+// None, and ops.py copies, asks or raises. Bound by per-call overhead: a forward of 8 heads of 200
+// queries took 27 us of host time around 8 us of kernel through ctypes; a training step's forward and
+// backward 113 us with the node in Python, 88 with the one below.
+#include <ATen/SavedTensorHooks.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 #include <torch/types.h>
+#include <atomic>
 #include <cmath>
 #include "../../include/fa_b200.h"
 
@@ -81,21 +86,69 @@ int64_t id_heads(const Tensor& eq, const Tensor& ek, int64_t B, int64_t H, int64
     return H == 1 || (eq.stride(1) == 0 && ek.stride(1) == 0) ? 1 : H;
 }
 
-// The plan of a call (ops.build_plan): its memory and the launches that fill it. `problem` is the address of an fa_problem; the
-// ids, if any, are int32 or int64 tensors [B, H, M] and [B, H, N] that ops.py has checked.
-Tensor plan(uintptr_t problem, const std::optional<Tensor>& eq, const std::optional<Tensor>& ek, const Tensor& status) {
-    const fa_problem* p = reinterpret_cast<const fa_problem*>(problem);
-    auto ids = [](const Tensor& t) {
-        return fa_ids{t.const_data_ptr(), {t.stride(0), t.stride(1), t.stride(2)}, t.scalar_type() == at::kInt ? FA_ID_INT32 : FA_ID_INT64};
-    };
-    py::gil_scoped_release free;
+fa_ids id_view(const Tensor& t) {
+    return fa_ids{t.const_data_ptr(), {t.stride(0), t.stride(1), t.stride(2)}, t.scalar_type() == at::kInt ? FA_ID_INT32 : FA_ID_INT64};
+}
+
+// The plan of a call: its memory and the launches that fill it. eq and ek, if any, are int32 or int64 tensors [B, H, M] and [B, H, N].
+Tensor build_plan(const fa_problem& p, const Tensor* eq, const Tensor* ek, const Tensor& status) {
     size_t bytes = 0;
-    check(fa_plan_bytes(p, &bytes), "fa_plan_bytes");
+    check(fa_plan_bytes(&p, &bytes), "fa_plan_bytes");
     Tensor plan = at::empty({int64_t(bytes / 4)}, status.options());
-    const fa_ids q = eq ? ids(*eq) : fa_ids{}, k = ek ? ids(*ek) : fa_ids{};
-    check(fa_plan_build(p, eq ? &q : nullptr, ek ? &k : nullptr, plan.data_ptr(), bytes, status.data_ptr<int>(), current_stream(status)),
+    const fa_ids q = eq ? id_view(*eq) : fa_ids{}, k = ek ? id_view(*ek) : fa_ids{};
+    check(fa_plan_build(&p, eq ? &q : nullptr, ek ? &k : nullptr, plan.data_ptr(), bytes, status.data_ptr<int>(), current_stream(status)),
           "fa_plan_build");
     return plan;
+}
+
+// ops.build_plan. `problem` is the address of an fa_problem; ops.py has checked the ids.
+Tensor plan(uintptr_t problem, const std::optional<Tensor>& eq, const std::optional<Tensor>& ek, const Tensor& status) {
+    py::gil_scoped_release free;
+    return build_plan(*reinterpret_cast<const fa_problem*>(problem), eq ? &*eq : nullptr, ek ? &*ek : nullptr, status);
+}
+
+struct Outputs {
+    Tensor o, lse;
+    int splits;
+};
+
+// The forward's allocations and launches for a problem that `regular` has filled.
+Outputs launch_forward(const fa_problem& p, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& plan, int key_runs,
+                       const Tensor& status, const std::optional<Tensor>& out) {
+    Outputs r;
+    r.o = out ? *out : at::empty_like(q);
+    if (!taken_as_is(r.o)) r.o = at::empty(q.sizes(), q.options());
+    const auto f32 = q.options().dtype(at::kFloat);
+    r.lse = at::empty({p.B, p.H, fa_padded_rows(p.M)}, f32);
+    r.splits = key_runs != 0 ? key_runs : fa_fwd_splits(&p);  // (a number below 1 is the library's to refuse)
+    Tensor work;
+    size_t bytes = 0;
+    if (r.splits > 1) {
+        check(fa_fwd_workspace_bytes(&p, r.splits, &bytes), "fa_fwd_workspace_bytes");
+        work = at::empty({int64_t(bytes / 4)}, f32);
+    }
+    const fa_tensor tq = view(q), tk = view(k), tv = view(v), to = view(r.o);
+    check(fa_fwd_split(&p, &tq, &tk, &tv, &to, r.lse.data_ptr<float>(), plan.defined() ? plan.data_ptr() : nullptr, r.splits,
+                       work.defined() ? work.data_ptr() : nullptr, bytes, status.data_ptr<int>(), current_stream(q)),
+          "fa_fwd_split");
+    return r;
+}
+
+// dq, dk, dv. q, k, v, o, lse and the problem are those of a forward, d_o is like q.
+std::array<Tensor, 3> launch_backward(const fa_problem& p, const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v,
+                                      const Tensor& o, const Tensor& lse, const Tensor& plan, const Tensor& status) {
+    Tensor delta = at::empty_like(lse);
+    Tensor dk = at::empty({p.B, p.Hk, p.N, p.D}, k.options()), dv = at::empty({p.B, p.Hk, p.N, p.D}, v.options());
+    Tensor dq = at::empty(q.sizes(), q.options());
+    const fa_tensor tq = view(q), tk = view(k), tv = view(v), to = view(o), tdo = view(d_o), tdq = view(dq), tdk = view(dk), tdv = view(dv);
+    check(fa_bwd(&p, &tq, &tk, &tv, &to, &tdo, lse.data_ptr<float>(), delta.data_ptr<float>(), &tdq, &tdk, &tdv,
+                 plan.defined() ? plan.data_ptr() : nullptr, status.data_ptr<int>(), current_stream(q)),
+          "fa_bwd");
+    return {std::move(dq), std::move(dk), std::move(dv)};
+}
+
+bool like_query(const Tensor& d_o, const Tensor& q) {
+    return plain_cuda(d_o) && d_o.scalar_type() == q.scalar_type() && d_o.device() == q.device() && d_o.sizes() == q.sizes();
 }
 
 // (o, lse, scale, kernels launched), or None. Unprepared calls without a plan are taken only if it would gain nothing. `out`: a
@@ -107,27 +160,12 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, bool prepa
     const double sm_scale = scale ? *scale : 1.0 / std::sqrt(double(q.dim() == 4 ? q.size(3) : 1));
     if (!regular(q, k, v, prepared, causal, sm_scale, mode, id_heads, p)) return py::none();
     if (!plan && (mode != FA_MODE0_NOPE || (!prepared && !fa_plan_optional(&p, backward)))) return py::none();
-    Tensor o, lse;
-    int splits = 1;
+    Outputs r;
     {
         py::gil_scoped_release free;
-        o = out ? *out : at::empty_like(q);
-        if (!taken_as_is(o)) o = at::empty(q.sizes(), q.options());
-        const auto f32 = q.options().dtype(at::kFloat);
-        lse = at::empty({p.B, p.H, fa_padded_rows(p.M)}, f32);
-        splits = key_runs != 0 ? key_runs : fa_fwd_splits(&p);  // (a number below 1 is the library's to refuse)
-        Tensor work;
-        size_t bytes = 0;
-        if (splits > 1) {
-            check(fa_fwd_workspace_bytes(&p, splits, &bytes), "fa_fwd_workspace_bytes");
-            work = at::empty({int64_t(bytes / 4)}, f32);
-        }
-        const fa_tensor tq = view(q), tk = view(k), tv = view(v), to = view(o);
-        check(fa_fwd_split(&p, &tq, &tk, &tv, &to, lse.data_ptr<float>(), plan ? plan->data_ptr() : nullptr, splits,
-                           work.defined() ? work.data_ptr() : nullptr, bytes, status.data_ptr<int>(), current_stream(q)),
-              "fa_fwd_split");
+        r = launch_forward(p, q, k, v, plan ? *plan : Tensor(), key_runs, status, out);
     }
-    return py::make_tuple(std::move(o), std::move(lse), sm_scale, splits > 1 ? 2 : 1);
+    return py::make_tuple(std::move(r.o), std::move(r.lse), sm_scale, r.splits > 1 ? 2 : 1);
 }
 
 // (dq, dk, dv), or None. q, k, v, o, lse and the numbers are those of a forward.
@@ -135,24 +173,98 @@ py::object backward(const Tensor& d_o, const Tensor& q, const Tensor& k, const T
                     bool prepared, bool causal, double sm_scale, int mode, int id_heads, const std::optional<Tensor>& plan,
                     const Tensor& status) {
     fa_problem p;
-    if (!regular(q, k, v, true, causal, sm_scale, mode, id_heads, p) || !plain_cuda(d_o) || d_o.scalar_type() != q.scalar_type() ||
-        d_o.device() != q.device() || d_o.sizes() != q.sizes() || (!prepared && !taken_as_is(d_o)))
+    if (!regular(q, k, v, true, causal, sm_scale, mode, id_heads, p) || !like_query(d_o, q) || (!prepared && !taken_as_is(d_o)))
         return py::none();
-    Tensor dq, dk, dv;
+    std::array<Tensor, 3> g;
     {
         py::gil_scoped_release free;
-        Tensor delta = at::empty_like(lse);
-        dk = at::empty({p.B, p.Hk, p.N, p.D}, k.options());
-        dv = at::empty({p.B, p.Hk, p.N, p.D}, v.options());
-        dq = at::empty(q.sizes(), q.options());
-        const fa_tensor tq = view(q), tk = view(k), tv = view(v), to = view(o), tdo = view(d_o), tdq = view(dq), tdk = view(dk),
-                        tdv = view(dv);
-        check(fa_bwd(&p, &tq, &tk, &tv, &to, &tdo, lse.data_ptr<float>(), delta.data_ptr<float>(), &tdq, &tdk, &tdv,
-                     plan ? plan->data_ptr() : nullptr, status.data_ptr<int>(), current_stream(q)),
-              "fa_bwd");
+        g = launch_backward(p, d_o, q, k, v, o, lse, plan ? *plan : Tensor(), status);
     }
-    return py::make_tuple(std::move(dq), std::move(dk), std::move(dv));
+    return py::make_tuple(std::move(g[0]), std::move(g[1]), std::move(g[2]));
 }
+
+// Kernels launched by `attend` and its gradients (ops.LAUNCHES).
+std::atomic<int64_t> n_launched{0};
+
+// What a regular call is, besides q, k and v.
+struct Call {
+    fa_problem p;
+    const Tensor *eq, *ek;  // null without ids
+    const Tensor& status;
+    bool needs_grad;
+    int plan_kernels;
+};
+
+// The autograd node of a regular call: what ops.FlashAttention does, without Python on the way of the gradients, whose thread would
+// have to be given the interpreter first. Saves the same tensors; the plan is the node's own.
+struct FlashAttention : torch::autograd::Function<FlashAttention> {
+    static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Call& c) {
+        Tensor plan;
+        Outputs r;
+        {
+            py::gil_scoped_release free;
+            if (c.eq || !fa_plan_optional(&c.p, c.needs_grad)) plan = build_plan(c.p, c.eq, c.ek, c.status);
+            r = launch_forward(c.p, q, k, v, plan, 0, c.status, std::nullopt);
+        }
+        n_launched += (c.eq ? c.plan_kernels : 0) + (r.splits > 1 ? 2 : 1);
+        if (c.needs_grad) {
+            torch::autograd::variable_list saved{q, k, v, r.o, r.lse};
+            if (c.eq) {
+                saved.push_back(*c.eq);
+                saved.push_back(*c.ek);
+            }
+            ctx->save_for_backward(std::move(saved));
+            ctx->saved_data["plan"] = plan;
+            ctx->saved_data["status"] = c.status;
+            ctx->saved_data["causal"] = int64_t(c.p.causal);
+            ctx->saved_data["mode"] = int64_t(c.p.mode);
+            ctx->saved_data["id_heads"] = int64_t(c.p.id_heads);
+            ctx->saved_data["scale"] = double(c.p.sm_scale);
+        }
+        return r.o;
+    }
+
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
+        const c10::cuda::CUDAGuard device(q.device());
+        auto& data = ctx->saved_data;
+        fa_problem p;
+        TORCH_CHECK(regular(q, k, v, true, data["causal"].toInt() != 0, data["scale"].toDouble(), int(data["mode"].toInt()),
+                            int(data["id_heads"].toInt()), p),
+                    "flash_b200: the saved q, k, v are not plain [bs, H, L, D] CUDA tensors of matching shapes");
+        Tensor d_o = grads[0];
+        if (d_o.scalar_type() != q.scalar_type()) d_o = d_o.to(q.scalar_type());
+        d_o = d_o.resolve_neg();
+        TORCH_CHECK(like_query(d_o, q), "flash_b200: the gradient is not a plain [bs, H, M, D] CUDA tensor");
+        if (!taken_as_is(d_o)) d_o = d_o.contiguous();  // (ops.maybe_contiguous)
+        auto g = launch_backward(p, d_o, q, k, v, saved[3], saved[4], data["plan"].toTensor(), data["status"].toTensor());
+        n_launched += 3;
+        return {std::move(g[0]), std::move(g[1]), std::move(g[2]), Tensor()};
+    }
+};
+
+// The whole of a regular call, its gradients included; None: ops.py takes it another way. Saved-tensor hooks count what is saved and by whom, so
+// that their calls take ops.FlashAttention.
+py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, std::optional<double> scale, const std::optional<Tensor>& eq,
+                  const std::optional<Tensor>& ek, int mode, const Tensor& status) {
+    fa_problem p;
+    const double sm_scale = scale ? *scale : 1.0 / std::sqrt(double(q.dim() == 4 ? q.size(3) : 1));
+    if (eq.has_value() != ek.has_value() || mode != (eq ? FA_MODE1_DOC : FA_MODE0_NOPE)) return py::none();
+    if (!regular(q, k, v, false, causal, sm_scale, mode, 1, p)) return py::none();
+    if (eq) {
+        if (eq->device() != q.device() || ek->device() != q.device()) return py::none();
+        p.id_heads = int(id_heads(*eq, *ek, p.B, p.H, p.M, p.N));
+        if (p.id_heads == 0) return py::none();
+    }
+    if (at::SavedTensorDefaultHooks::get_hooks()) return py::none();
+    const bool needs_grad = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
+    const int plan_kernels = (p.M + 127) / 128 + (p.N + 127) / 128 <= FA_PLAN_ONE_KERNEL_BLOCKS ? 1 : 3;
+    const Call call{p, eq ? &*eq : nullptr, ek ? &*ek : nullptr, status, needs_grad, plan_kernels};
+    return py::cast(FlashAttention::apply(q, k, v, call));
+}
+
+int64_t launched() { return n_launched; }
 
 }  // namespace
 
@@ -162,4 +274,6 @@ PYBIND11_MODULE(_host, m) {
     m.def("plan", &plan);
     m.def("forward", &forward);
     m.def("backward", &backward);
+    m.def("attend", &attend);
+    m.def("launched", &launched);
 }

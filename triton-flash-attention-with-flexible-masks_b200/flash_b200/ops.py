@@ -24,9 +24,15 @@ _DTYPES = {torch.bfloat16: _lib.FA_BF16, torch.float16: _lib.FA_FP16, torch.floa
 _STATUS = {}  # device index -> int32[1] status word
 _SYNC_STATUS = os.environ.get("FA_B200_SYNC_STATUS", "0") not in ("", "0")
 # When set to a list, every kernel launch appends (name, start_event, end_event) recorded on the
-# launching stream, and LAUNCHES counts the library's kernels. Used by the benchmark only.
+# launching stream. LAUNCHES (below) counts the library's kernels. Used by the benchmark only.
 PROFILE = None
-LAUNCHES = 0
+_launches = 0
+
+
+def __getattr__(name):
+    if name == "LAUNCHES":
+        return _launches + (_HOST.launched() if _HOST is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 class _Timed:
@@ -55,14 +61,14 @@ _UNTIMED = contextlib.nullcontext()
 
 
 def _timed(name, kernels=1):
-    global LAUNCHES
-    LAUNCHES += kernels
+    global _launches
+    _launches += kernels
     return _UNTIMED if PROFILE is None else _Timed(name)
 
 
 def _count(kernels):
-    global LAUNCHES
-    LAUNCHES += kernels
+    global _launches
+    _launches += kernels
 
 
 def _current(device):
@@ -179,6 +185,9 @@ def build_plan(prob, eq, ek, status):
         return make(ctypes.addressof(prob), eq, ek, status)
 
 
+_own_build_plan = build_plan
+
+
 def _host():
     """The native host calls (csrc/host.cpp); no call runs without them."""
     global _HOST, _PLAN, _AS_IS, _ID_HEADS
@@ -213,7 +222,22 @@ def _native_forward(host, q, k, v, causal, sm_scale, needs_grad, key_runs):
     return host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs, status, _like_subclass(q))
 
 
+def _native_attend(q, k, v, causal, sm_scale, eq, ek, score_func_mode):
+    """A regular call with whatever plan and node it needs, in one native call; None for any other."""
+    attend = getattr(_HOST, "attend", None)
+    if (attend is None or build_plan is not _own_build_plan  # (somebody's own plan or host calls)
+            or PROFILE is not None or _SYNC_STATUS or not (sm_scale is None or type(sm_scale) is float)
+            or _tracing_state() is not None or not (eq is None or type(eq) in _PLAIN) or not (ek is None or type(ek) in _PLAIN)):
+        return None
+    status = _STATUS.get(q.get_device())
+    if status is None:
+        return None
+    return attend(q, k, v, bool(causal), sm_scale, eq, ek, score_func_mode, status)
+
+
 class FlashAttention(torch.autograd.Function):
+    """The autograd node of every call that `attend` (csrc/host.cpp) does not take."""
+
     @staticmethod
     def forward(ctx, q, k, v, causal, sm_scale, eq, ek, score_func_mode, key_runs=None):
         host = _HOST or _host()
@@ -420,17 +444,23 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
     if (GROUP_QUERIES and score_func_mode == SCORE_FUNC_MODE1_DOC and not causal and eq is not None and ek is not None
             and q.is_cuda and q.dim() == 4 and 128 < q.shape[2] <= _lib.FA_GROUP_MAX_ROWS):
         return _attention_grouped(q, k, v, sm_scale, eq, ek)
-    # A call that needs no gradient has no use for an autograd node, which is a third of a short call's host time: 8 heads of 200 queries
-    # take 13.6 us a call with it, 9.7 without. (Transforms of torch.func and forward-mode gradients need it for their messages,
-    # subclasses for their hooks.)
-    if (eq is None and ek is None and type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(score_func_mode) is int
-            and score_func_mode == SCORE_FUNC_MODE0_NOPE and _HOST is not None
-            and not (_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))
+    # Regular calls go to the library in one native call, with a native autograd node where a gradient is needed. A small training step is
+    # bound by its host time: 4 x 12 heads x 1000 x 64 in documents 113 us for 92 of kernels with the node of this module (its backward waits for
+    # the interpreter in the engine's thread), 88 with the native one. Transforms of torch.func and forward-mode gradients need
+    # the node of this module for their messages, subclasses for their hooks, and a trace for its refusal.
+    if (_HOST is not None and type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(score_func_mode) is int
             and _transforms() is None and _forward_ad._current_level < 0):
-        done = _native_forward(_HOST, q, k, v, causal, sm_scale, False, 0)
-        if done is not None:
-            _count(done[3])
-            return done[0]
+        if (eq is None and ek is None and score_func_mode == SCORE_FUNC_MODE0_NOPE
+                and not (_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))):
+            # no node at all: 8 heads of 200 queries take 13.6 us a call with the one of this module, 9.7 without
+            done = _native_forward(_HOST, q, k, v, causal, sm_scale, False, 0)
+            if done is not None:
+                _count(done[3])
+                return done[0]
+        else:
+            done = _native_attend(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
+            if done is not None:
+                return done
     return FlashAttention.apply(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
 
 
