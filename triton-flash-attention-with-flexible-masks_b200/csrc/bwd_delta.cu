@@ -8,57 +8,75 @@
 
 namespace fa {
 
-// 8 threads per row, 16 rows per CTA of 128 threads; each thread reads D/8 contiguous elements (at least 8:
-// with head dims 16 and 32 only the first 2 or 4 threads of a row have any).
+// D / 8 neighbouring threads read a row, 16 bytes of O and of dO each, so that a warp's load covers whole 128-byte lines, and each thread
+// has the loads of its kRows rows in flight before it uses the first. Bound by HBM.
+// us, eight threads a row with 2 x D / 8 elements and one row each | now: 16 x 8 x 577 x 32 6.5 | 2.8, 8 x 8 x 1024 x 64
+// 5.5 | 3.5, 4 x 12 x 1000 x 64 4.4 | 2.8; D = 128, where HBM has always been the bound, 4 x 16 x 4096 37 | 36 and 32 x 32768 109 | 106
+// (the wait for the forward's last blocks included); two or eight rows a thread 36 and 39, 106 and 112.
+template <int D>
+struct DeltaShape {
+    static constexpr int kThreads = 256, kLanes = D / 8, kRows = (D == 128 ? 4 : D == 64 ? 4 : 2);
+    static constexpr int kStep = kThreads / kLanes;     // rows that the block's threads read together
+    static constexpr int kBlockRows = kStep * kRows;
+};
+
 template <int D, bool BF16>
-__global__ void __launch_bounds__(128) bwd_delta_kernel(const DeltaParams p) {
+__global__ void __launch_bounds__(256) bwd_delta_kernel(const DeltaParams p) {
+    using S = DeltaShape<D>;
     follow_stream();
     const int h = blockIdx.y, b = blockIdx.z;
-    const int row = blockIdx.x * 16 + (threadIdx.x >> 3);
-    const int part = threadIdx.x & 7;
-    constexpr int PER = (D >= 64) ? D / 8 : 8;  // elements per thread: 16 (D=128) or 8
-    float acc = 0.f;
-    if (row < p.M && part * PER < D) {
-        const uint8_t* po = static_cast<const uint8_t*>(p.o.ptr) +
-                            2 * (int64_t(b) * p.o.sb + int64_t(h) * p.o.sh + int64_t(row) * p.o.sl + part * PER);
-        const uint8_t* pd = static_cast<const uint8_t*>(p.d_o.ptr) +
-                            2 * (int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh + int64_t(row) * p.d_o.sl + part * PER);
+    const int row0 = blockIdx.x * S::kBlockRows + int(threadIdx.x) / S::kLanes;
+    const int part = int(threadIdx.x) % S::kLanes;
+    const uint16_t* po = static_cast<const uint16_t*>(p.o.ptr) + int64_t(b) * p.o.sb + int64_t(h) * p.o.sh + part * 8;
+    const uint16_t* pd = static_cast<const uint16_t*>(p.d_o.ptr) + int64_t(b) * p.d_o.sb + int64_t(h) * p.d_o.sh + part * 8;
+    uint4 a[S::kRows], g[S::kRows];
 #pragma unroll
-        for (int v = 0; v < PER / 8; ++v) {
-            const uint4 a = reinterpret_cast<const uint4*>(po)[v];
-            const uint4 g = reinterpret_cast<const uint4*>(pd)[v];
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
-            const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                float a0, a1, g0, g1;
-                if constexpr (BF16) {
-                    a0 = __uint_as_float(aw[k] << 16); a1 = __uint_as_float(aw[k] & 0xffff0000u);
-                    g0 = __uint_as_float(gw[k] << 16); g1 = __uint_as_float(gw[k] & 0xffff0000u);
-                } else {
-                    const __half2 ah = *reinterpret_cast<const __half2*>(&aw[k]);
-                    const __half2 gh = *reinterpret_cast<const __half2*>(&gw[k]);
-                    a0 = __low2float(ah); a1 = __high2float(ah);
-                    g0 = __low2float(gh); g1 = __high2float(gh);
-                }
-                acc = fmaf(a0, g0, acc);
-                acc = fmaf(a1, g1, acc);
-            }
+    for (int r = 0; r < S::kRows; ++r) {
+        const int row = row0 + r * S::kStep;
+        a[r] = g[r] = make_uint4(0, 0, 0, 0);
+        if (row < p.M) {
+            a[r] = *reinterpret_cast<const uint4*>(po + int64_t(row) * p.o.sl);
+            g[r] = *reinterpret_cast<const uint4*>(pd + int64_t(row) * p.d_o.sl);
         }
     }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-    if (part == 0 && row < p.Mpad) p.delta[(int64_t(b) * p.H + h) * p.Mpad + row] = acc;
+#pragma unroll
+    for (int r = 0; r < S::kRows; ++r) {
+        const uint32_t aw[4] = {a[r].x, a[r].y, a[r].z, a[r].w};
+        const uint32_t gw[4] = {g[r].x, g[r].y, g[r].z, g[r].w};
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float a0, a1, g0, g1;
+            if constexpr (BF16) {
+                a0 = __uint_as_float(aw[k] << 16); a1 = __uint_as_float(aw[k] & 0xffff0000u);
+                g0 = __uint_as_float(gw[k] << 16); g1 = __uint_as_float(gw[k] & 0xffff0000u);
+            } else {
+                const __half2 ah = *reinterpret_cast<const __half2*>(&aw[k]);
+                const __half2 gh = *reinterpret_cast<const __half2*>(&gw[k]);
+                a0 = __low2float(ah); a1 = __high2float(ah);
+                g0 = __low2float(gh); g1 = __high2float(gh);
+            }
+            acc = fmaf(a0, g0, acc);
+            acc = fmaf(a1, g1, acc);
+        }
+#pragma unroll
+        for (int o = 1; o < S::kLanes; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        const int row = row0 + r * S::kStep;
+        if (part == 0 && row < p.Mpad) p.delta[(int64_t(b) * p.H + h) * p.Mpad + row] = acc;
+    }
+}
+
+template <int D>
+static cudaError_t launch_delta_t(const DeltaParams& p, cudaStream_t stream) {
+    const dim3 grid(unsigned((p.Mpad + DeltaShape<D>::kBlockRows - 1) / DeltaShape<D>::kBlockRows), p.H, p.B);
+    return launch_overlapping(p.bf16 ? bwd_delta_kernel<D, true> : bwd_delta_kernel<D, false>, grid, DeltaShape<D>::kThreads, 0, stream, p);
 }
 
 cudaError_t launch_bwd_delta(const DeltaParams& p, cudaStream_t stream) {
-    dim3 grid(unsigned(p.Mpad / 16), p.H, p.B);
-    auto run = [&](auto kern) { return launch_overlapping(kern, grid, 128, 0, stream, p); };
-    if (p.D == 128) return run(p.bf16 ? bwd_delta_kernel<128, true> : bwd_delta_kernel<128, false>);
-    if (p.D == 32) return run(p.bf16 ? bwd_delta_kernel<32, true> : bwd_delta_kernel<32, false>);
-    if (p.D == 16) return run(p.bf16 ? bwd_delta_kernel<16, true> : bwd_delta_kernel<16, false>);
-    return run(p.bf16 ? bwd_delta_kernel<64, true> : bwd_delta_kernel<64, false>);
+    if (p.D == 128) return launch_delta_t<128>(p, stream);
+    if (p.D == 64) return launch_delta_t<64>(p, stream);
+    if (p.D == 32) return launch_delta_t<32>(p, stream);
+    return launch_delta_t<16>(p, stream);
 }
 
 }  // namespace fa
