@@ -118,6 +118,52 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     static_assert(B_OFREE + 2 == S::n_bar, "barriers");
     Abort ab{misc + 1, p.status, p.wait_limit};
 
+    // item -> (query block, head, batch). Heads are taken in groups of p.gh; inside a group the query
+    // blocks go from the last one down (with a causal mask: long ones first) and the heads of the
+    // group vary fastest. The CTAs thus work on neighbouring query blocks of a few heads at a time:
+    // few enough that their K / V streams stay in L2, enough that not all CTAs pull the same lines.
+    auto decode = [&](int j, int& qb, int& h, int& b) {
+        const int per = p.gh * nQ;                 // items of a full group of heads
+        const int grp = j / per, rem = j - grp * per;
+        const int gsz = min(p.gh, HB - grp * p.gh);  // heads in this group (the last one may be smaller)
+        const int pos = rem / gsz, bh = grp * p.gh + (rem - pos * gsz);
+        b = bh / HP;
+        h = bh - b * HP;
+        // few items per CTA: longest first (sorted in the plan), so that no long item is left for the end
+        qb = p.by_length ? mk.plan[mk.L.off_ordq + (int64_t(b) * mk.He + (mk.He == 1 ? 0 : h)) * nQ + pos] : nQ - 1 - pos;
+    };
+    // What the scheduler finds out about item j before it has a slot for it; in `flags` the class of candidate tile lo + lane.
+    struct Item {
+        int j, qb, h, b, lo, n;
+        uint32_t flags;
+        int4 qc;
+    };
+    auto classify = [&](const Item& it, int i) {
+        return i < it.n ? classify_from_plan(mk, it.b, (mk.He == 1) ? 0 : it.h, it.qb, it.lo + i) & (TILE_VISIT | TILE_BOUND | TILE_DOC | TILE_KMONO) : 0u;
+    };
+    auto prepare = [&](int j) {
+        Item it;
+        it.j = j;
+        const int sp = SHORT ? j % ns : 0;  // which run of the item's tiles
+        decode(SHORT ? j / ns : j, it.qb, it.h, it.b);
+        const int he = (mk.He == 1) ? 0 : it.h;
+        int lo, hi;
+        kv_range(mk, it.b, he, it.qb, lo, hi);
+        int n = hi - lo;
+        if constexpr (SHORT) {  // no ids: every tile of the range is visited
+            const int first = int(int64_t(n) * sp / ns);
+            n = int(int64_t(n) * (sp + 1) / ns) - first;
+            lo += first;
+        }
+        it.lo = lo;
+        it.n = n < kListCap ? n : kListCap;  // the host refuses problems that could exceed the cap
+        it.qc = make_int4(0, 0, 0, 0);
+        if (mk.mode == 1)
+            it.qc = *reinterpret_cast<const int4*>(mk.plan + mk.L.off_qc + (int64_t(it.b) * mk.He + he) * mk.L.Mpad + int64_t(it.qb) * kBlk + lane * 4);
+        it.flags = classify(it, lane);
+        return it;
+    };
+
     if (tid == 0) {
         for (int s = 0; s < NQ; ++s) {
             mbar_init(BAR(B_ITEMFULL + s), 1);
@@ -145,6 +191,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         }
         fence_mbar_init();
     }
+    // Without ids the scheduler knows its first item before the kernel may touch memory.
+    Item item;
+    if (warp == 14 && mk.mode == 0) item = prepare(int(blockIdx.x));
     wait_prerequisites();
     if (warp == 13) {
         tmem_alloc(sbase + S::off_misc, 512);
@@ -168,41 +217,33 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     auto sK = [&](int s) { return sbase + S::off_k + uint32_t(s) * S::TILE; };
     auto sV = [&](int s) { return sbase + S::off_v + uint32_t(s) * S::TILE; };
     auto list_of = [&](int s) { return reinterpret_cast<const uint16_t*>(smem + S::off_list) + s * kListCap; };
-    // item -> (query block, head, batch). Heads are taken in groups of p.gh; inside a group the query
-    // blocks go from the last one down (with a causal mask: long ones first) and the heads of the
-    // group vary fastest. The CTAs thus work on neighbouring query blocks of a few heads at a time:
-    // few enough that their K / V streams stay in L2, enough that not all CTAs pull the same lines.
-    auto decode = [&](int j, int& qb, int& h, int& b) {
-        const int per = p.gh * nQ;                 // items of a full group of heads
-        const int grp = j / per, rem = j - grp * per;
-        const int gsz = min(p.gh, HB - grp * p.gh);  // heads in this group (the last one may be smaller)
-        const int pos = rem / gsz, bh = grp * p.gh + (rem - pos * gsz);
-        b = bh / HP;
-        h = bh - b * HP;
-        // few items per CTA: longest first (sorted in the plan), so that no long item is left for the end
-        qb = p.by_length ? mk.plan[mk.L.off_ordq + (int64_t(b) * mk.He + (mk.He == 1 ? 0 : h)) * nQ + pos] : nQ - 1 - pos;
-    };
-
     if (warp >= 12) {
         setmaxnreg_dec<kFwdServiceRegs>();
         if (aborted) {
             // a previous kernel reported an error: do nothing
         } else if (warp == 14) {
             // ------------------------------ item scheduler ------------------------------
-            // Items are handed out in order from a counter in the plan (any CTA takes the next one: the
-            // work per item varies with the mask); without counters (no plan given) they are
-            // dealt out round robin in alternating direction, which evens out their sorted lengths.
+            // The first item of a CTA is its own number; the others are handed out in order from a counter in the plan (any CTA
+            // takes the next one: the work per item varies with the mask); without counters (no plan given) they are dealt out
+            // round robin in alternating direction, which evens out their sorted lengths. us, every item from the counter | the first
+            // one known, without ids before the wait: 8 x 200 x 64 7.42 | 7.10, 4 x 12 x 1000 x 64 in documents 24.4 | 22.5, 8 x 8 x 1024 x 8192 x
+            // 64 in documents 75.2 | 71.4, 4 x 16 x 4096 x 128 in documents 153 | 148, 16 x 8 x 577 x 32 31.1 | 31.5. An item taken, and what the
+            // plan says about it read, while the one before it still holds the slot leaves no pause between items, but is dealt out
+            // too far ahead: 28.1 for 27.8, 75.6 for 76.5, 157 for 154. (dK/dV gains nothing from a first item of its own.)
             bool ok = true;
+            int j = int(blockIdx.x);
             for (int k = 0;; ++k) {
                 const int s = k % NQ, use = k / NQ;
                 if (use > 0) ok = mbar_wait_warp(BAR(B_ITEMEMPTY + s), (use - 1) & 1, ab, ST_WAIT_TIMEOUT + 11);
                 if (!ok) break;
-                int j = 0;
-                if (lane == 0) {
-                    if (ctr) j = int(atomicAdd(ctr, 1u));
-                    else j = k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
+                if (k > 0) {
+                    if (lane == 0) {
+                        if (ctr) j = int(gridDim.x + atomicAdd(ctr, 1u));
+                        else j = k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
+                    }
+                    j = __shfl_sync(0xffffffffu, j, 0);
                 }
-                j = __shfl_sync(0xffffffffu, j, 0);
+                if ((k > 0 || mk.mode != 0) && j < n_items) item = prepare(j);
                 if (j >= n_items) {  // end marker
                     if (lane == 0) {
                         info[s * 8 + 2] = -1;
@@ -210,41 +251,24 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
                     break;
                 }
-                int qb, h, b;
-                const int sp = SHORT ? j % ns : 0;  // which run of the item's tiles
-                decode(SHORT ? j / ns : j, qb, h, b);
-                const int he = (mk.He == 1) ? 0 : h;
-                int lo, hi;
-                kv_range(mk, b, he, qb, lo, hi);
-                int n = hi - lo;
-                if constexpr (SHORT) {  // no ids: every tile of the range is visited
-                    const int first = int(int64_t(n) * sp / ns);
-                    n = int(int64_t(n) * (sp + 1) / ns) - first;
-                    lo += first;
-                }
-                if (n > kListCap) n = kListCap;  // the host refuses problems that could exceed the cap
                 uint16_t* list = reinterpret_cast<uint16_t*>(smem + S::off_list) + s * kListCap;
                 int T = 0;
-                for (int base = 0; base < n; base += 32) {
+                for (int base = 0; base < item.n; base += 32) {
                     const int i = base + lane;
-                    const uint32_t f = (i < n) ? classify_from_plan(mk, b, he, qb, lo + i) & (TILE_VISIT | TILE_BOUND | TILE_DOC | TILE_KMONO) : 0u;
+                    const uint32_t f = base == 0 ? item.flags : classify(item, i);
                     const uint32_t m = __ballot_sync(0xffffffffu, (f & TILE_VISIT) != 0);
                     if (f & TILE_VISIT) list[T + __popc(m & ((1u << lane) - 1u))] = uint16_t(uint32_t(i) | (f << 10));
                     T += __popc(m);
                 }
-                int4 qc4 = make_int4(0, 0, 0, 0);
-                if (mk.mode == 1)
-                    qc4 = *reinterpret_cast<const int4*>(mk.plan + mk.L.off_qc + (int64_t(b) * mk.He + he) * mk.L.Mpad +
-                                                         int64_t(qb) * kBlk + lane * 4);
-                reinterpret_cast<int4*>(smem + S::off_qc)[s * 32 + lane] = qc4;
+                reinterpret_cast<int4*>(smem + S::off_qc)[s * 32 + lane] = item.qc;
                 if (lane == 0) {
                     info[s * 8 + 0] = T;
-                    info[s * 8 + 1] = lo;
+                    info[s * 8 + 1] = item.lo;
                     info[s * 8 + 2] = j;
-                    info[s * 8 + 3] = SHORT ? h / nG : h / p.G;
-                    info[s * 8 + 4] = qb;
-                    info[s * 8 + 5] = h;
-                    info[s * 8 + 6] = b;
+                    info[s * 8 + 3] = SHORT ? item.h / nG : item.h / p.G;
+                    info[s * 8 + 4] = item.qb;
+                    info[s * 8 + 5] = item.h;
+                    info[s * 8 + 6] = item.b;
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(BAR(B_ITEMFULL + s));
