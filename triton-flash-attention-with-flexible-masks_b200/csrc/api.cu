@@ -21,7 +21,7 @@ cudaError_t launch_bwd_dq(int, bool, const CUtensorMap&, const CUtensorMap&, con
                           const CUtensorMap&, const CUtensorMap&, const DqParams&, int, bool, cudaStream_t);
 
 // fp32 path (attn_f32.cu)
-cudaError_t launch_f32(int which, int D, const F32Params& p, bool overlap, cudaStream_t stream);
+cudaError_t launch_f32(int which, int D, const F32Params& p, bool overlap, int sms, cudaStream_t stream);
 }  // namespace fa
 
 namespace {
@@ -286,7 +286,9 @@ int run_f32(int which, const fa_problem* p, const fa_tensor* q, const fa_tensor*
     fp.delta = delta;
     fp.B = p->B; fp.H = p->H; fp.Hk = p->Hk; fp.G = p->H / p->Hk;
     fp.scale = p->sm_scale;
-    return fa::launch_f32(which, p->D, fp, overlap, static_cast<cudaStream_t>(stream)) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
+    const int sms = sm_count();
+    if (sms <= 0) return FA_ERR_LAUNCH;
+    return fa::launch_f32(which, p->D, fp, overlap, sms, static_cast<cudaStream_t>(stream)) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
 }
 
 int run_bwd_dq(const fa_problem* p, const fa_tensor* q, const fa_tensor* k, const fa_tensor* v, const fa_tensor* d_o,
