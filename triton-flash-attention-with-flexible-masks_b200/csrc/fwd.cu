@@ -191,6 +191,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         }
         fence_mbar_init();
     }
+    if constexpr (SHORT) {
+        // Rows without a query are multiplied all the same, and zeros take less power than what lies in shared and tensor memory: 16
+        // tokens of 32 / 8 heads of 128 against 4500 keys, call after call under the power cap, 55.8 us -> 53.9 (51.4 without the cap, both).
+        for (int i = tid; i < NQ * S::TILE / 16; i += kFwdThreads) reinterpret_cast<uint4*>(smem + S::off_q)[i] = make_uint4(0, 0, 0, 0);
+        fence_proxy_async();
+    }
     // Without ids the scheduler knows its first item before the kernel may touch memory.
     Item item;
     if (warp == 14 && mk.mode == 0) item = prepare(int(blockIdx.x));
@@ -570,6 +576,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         const float c = p.scale_log2;
         const uint32_t tO = tmem + lane_base + uint32_t(S::tmem_o + w * D);
         bool alive = !aborted;
+        if (SHORT && S::POWN) {  // P of the rows without a query
+            uint32_t zero[32] = {};
+            tmem_st32(tmem + lane_base + uint32_t(S::tmem_p(w)), zero);
+            tmem_st32(tmem + lane_base + uint32_t(S::tmem_p(w)) + 32u, zero);
+            tc_wait_st();
+            tc_fence_before();
+        }
         int G = 0;  // tiles of all earlier items
         for (int k = 0; alive; ++k) {
             const int s = k % NQ, use = k / NQ;
