@@ -9,6 +9,7 @@
 namespace fa {
 cudaError_t launch_plan_build(const void*, const int64_t*, int, const void*, const int64_t*, int, int32_t*,
                               const PlanLayout&, int, int, int*, cudaStream_t);
+cudaError_t launch_plan_clear(int32_t*, int, cudaStream_t);
 cudaError_t launch_debug_mask(const MaskArgs&, uint8_t*, uint8_t*, cudaStream_t);
 cudaError_t launch_fwd(int, bool, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&,
                        const FwdParams&, int, cudaStream_t);
@@ -408,7 +409,7 @@ int fa_plan_build(const fa_problem* p, const fa_ids* eq, const fa_ids* ek, void*
         if (!plan) return FA_OK;
         if (reinterpret_cast<uintptr_t>(plan) % 16 != 0) return FA_ERR_ALIGNMENT;
         if (plan_bytes < kCtrWords * sizeof(int32_t)) return FA_ERR_PLAN_SIZE;
-        return cudaMemsetAsync(plan, 0, kCtrWords * sizeof(int32_t), static_cast<cudaStream_t>(stream)) == cudaSuccess
+        return fa::launch_plan_clear(static_cast<int32_t*>(plan), int(kCtrWords), static_cast<cudaStream_t>(stream)) == cudaSuccess
                    ? FA_OK : FA_ERR_LAUNCH;
     }
     if (!eq || !ek || !eq->ptr || !ek->ptr || !plan || !status) return FA_ERR_BAD_ARG;

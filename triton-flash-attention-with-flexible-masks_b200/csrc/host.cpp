@@ -206,7 +206,7 @@ struct FlashAttention : torch::autograd::Function<FlashAttention> {
             if (c.eq || !fa_plan_optional(&c.p, c.needs_grad)) plan = build_plan(c.p, c.eq, c.ek, c.status);
             r = launch_forward(c.p, q, k, v, plan, 0, c.status, std::nullopt);
         }
-        n_launched += (c.eq ? c.plan_kernels : 0) + (r.splits > 1 ? 2 : 1);
+        n_launched += (plan.defined() ? c.plan_kernels : 0) + (r.splits > 1 ? 2 : 1);
         if (c.needs_grad) {
             torch::autograd::variable_list saved{q, k, v, r.o, r.lse};
             if (c.eq) {
@@ -259,7 +259,7 @@ py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, bool causal
     }
     if (at::SavedTensorDefaultHooks::get_hooks()) return py::none();
     const bool needs_grad = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
-    const int plan_kernels = (p.M + 127) / 128 + (p.N + 127) / 128 <= FA_PLAN_ONE_KERNEL_BLOCKS ? 1 : 3;
+    const int plan_kernels = !eq || (p.M + 127) / 128 + (p.N + 127) / 128 <= FA_PLAN_ONE_KERNEL_BLOCKS ? 1 : 3;
     const Call call{p, eq ? &*eq : nullptr, ek ? &*ek : nullptr, status, needs_grad, plan_kernels};
     return py::cast(FlashAttention::apply(q, k, v, call));
 }

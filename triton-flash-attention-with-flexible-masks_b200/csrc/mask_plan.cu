@@ -307,6 +307,13 @@ __global__ void __launch_bounds__(128) debug_mask_kernel(MaskArgs a, uint8_t* ke
     }
 }
 
+// The plan of a call without ids: its work counters. A kernel, for a memset in the stream keeps the kernels before and behind it from
+// overlapping: 16 x 8 x 577 x 32, forward and backward, 115.0 -> 111.0 us.
+__global__ void plan_clear_kernel(int32_t* ctr) {
+    follow_stream();
+    ctr[threadIdx.x] = 0;
+}
+
 // ---- host launchers (called from api.cu) ------------------------------------------------
 cudaError_t launch_plan_build(const void* eq_ptr, const int64_t* eq_stride, int eq64, const void* ek_ptr,
                               const int64_t* ek_stride, int ek64, int32_t* plan, const PlanLayout& L, int gap,
@@ -321,6 +328,10 @@ cudaError_t launch_plan_build(const void* eq_ptr, const int64_t* eq_stride, int 
     if (e == cudaSuccess) e = launch_overlapping(plan_ranges_kernel, grid, 128, 0, stream, plan, L, gap, causal);
     if (e == cudaSuccess) e = launch_overlapping(plan_order_kernel, dim3(2, L.He, L.B), 1024, 0, stream, plan, L);
     return e;
+}
+
+cudaError_t launch_plan_clear(int32_t* ctr, int words, cudaStream_t stream) {
+    return launch_overlapping(plan_clear_kernel, dim3(1), words, 0, stream, ctr);
 }
 
 cudaError_t launch_debug_mask(const MaskArgs& a, uint8_t* keep, uint8_t* tile_class, cudaStream_t stream) {

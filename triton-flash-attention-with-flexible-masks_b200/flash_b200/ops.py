@@ -180,6 +180,7 @@ def build_plan(prob, eq, ek, status):
     holds their codes and block statistics; without (eq is None) only the kernels' work counters."""
     make = _PLAN or _host().plan
     if eq is None:
+        _count(1)
         return make(ctypes.addressof(prob), None, None, status)
     with _timed("plan", _plan_kernels(prob.M, prob.N)):
         return make(ctypes.addressof(prob), eq, ek, status)
