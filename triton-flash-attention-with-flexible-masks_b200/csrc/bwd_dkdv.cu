@@ -376,58 +376,58 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     const int NIT = uniform(info[s * 8 + 2]);
                     if (uniform(info[s * 8 + 3]) < 0) break;
                     if (NIT > 0) {
-                        auto issue_s = [&](int it) {
-                            const int gi = gt + it, st = gi % NQ;
-                            if (!q_ready(gi)) return false;
-                            tc_fence_after();
-                            ss_mmas(utmem + S::s_col(gi), sK, sQ(st));
-                            umma_commit(BAR(B_SFULL + gi % NSB));
-                            if (it + 1 == NIT) umma_commit(BAR(B_KEMPTY));
-                            return true;
-                        };
-                        auto issue_dp = [&](int it) {
-                            const int gi = gt + it, st = gi % NDO;
-                            if (!do_ready(gi)) return false;
-                            tc_fence_after();
-                            ss_mmas(utmem + 128u, sV, sdO(st));
-                            umma_commit(BAR(B_DPFULL));
-                            if (it + 1 == NIT) umma_commit(BAR(B_VEMPTY));
-                            return true;
-                        };
+                        // Steps before tile 0 issue what the first tiles' dV and dK stand behind: each product is written once, for the sake of
+                        // the instruction caches.
                         ok = mbar_wait_warp(BAR(B_KFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
-                        if (ok) ok = issue_s(0);
-                        if (ok) ok = mbar_wait_warp(BAR(B_VFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
-                        if (ok) ok = issue_dp(0);
-                        for (int it = 1; it < NSB && it < NIT && ok; ++it) ok = issue_s(it);
-                        // dV(0) and dK(0) overwrite the accumulators: the previous item's epilogue must have read them
-                        if (ok && kk > 0) ok = mbar_wait_warp(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 58);
-                        for (int it = 0; it < NIT && ok; ++it) {
+                        for (int it = -NSB; it < NIT && ok; ++it) {
                             const int gi = gt + it;
-                            // dV += P^T dO: A = P^T from TMEM (a warp's P lies over its own S), B = dO (MN-major)
-                            ok = mbar_wait_warp(BAR(B_PFULL + gi % NSB), (gi / NSB) & 1, ab, ST_WAIT_TIMEOUT + 47);
-                            if (!ok) break;
-                            tc_fence_after();
+                            if (it >= 0) {
+                                // dV(0) and dK(0) overwrite the accumulators: the previous item's epilogue must have read them
+                                if (it == 0 && kk > 0) ok = mbar_wait_warp(BAR(B_ACCFREE), (kk - 1) & 1, ab, ST_WAIT_TIMEOUT + 58);
+                                // dV += P^T dO: A = P^T from TMEM (a warp's P lies over its own S), B = dO (MN-major)
+                                if (ok) ok = mbar_wait_warp(BAR(B_PFULL + gi % NSB), (gi / NSB) & 1, ab, ST_WAIT_TIMEOUT + 47);
+                                if (!ok) break;
+                                tc_fence_after();
 #pragma unroll
-                            for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
-                                const uint32_t acol = uint32_t(kk2 >> 1) * 32u + uint32_t(kk2 & 1) * 8u;
-                                umma_ts(utmem + 256u, utmem + S::s_col(gi) + acol, smem_desc_at(desc_mn, sdO(gi % NDO) + uint32_t(kk2) * 2048u),
-                                        idesc_d, (it > 0 || kk2 > 0) ? 1u : 0u);
+                                for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
+                                    const uint32_t acol = uint32_t(kk2 >> 1) * 32u + uint32_t(kk2 & 1) * 8u;
+                                    umma_ts(utmem + 256u, utmem + S::s_col(gi) + acol, smem_desc_at(desc_mn, sdO(gi % NDO) + uint32_t(kk2) * 2048u),
+                                            idesc_d, (it > 0 || kk2 > 0) ? 1u : 0u);
+                                }
+                                umma_commit(BAR(B_DOEMPTY + gi % NDO));
+                                if (it + 1 == NIT) umma_commit(BAR(B_DVDONE));
                             }
-                            umma_commit(BAR(B_DOEMPTY + gi % NDO));
-                            if (it + 1 == NIT) umma_commit(BAR(B_DVDONE));
-                            if (it + NSB < NIT) ok = issue_s(it + NSB);
-                            // dK += dS^T Q: A = dS^T from TMEM (a warp's dS lies over its own dP), B = Q (MN-major)
-                            if (ok) ok = mbar_wait_warp(BAR(B_DSFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 48);
-                            if (!ok) break;
-                            tc_fence_after();
+                            if (it + NSB < NIT) {  // S^T(it + NSB)
+                                const int gs = gi + NSB;
+                                ok = q_ready(gs);
+                                if (!ok) break;
+                                tc_fence_after();
+                                ss_mmas(utmem + S::s_col(gs), sK, sQ(gs % NQ));
+                                umma_commit(BAR(B_SFULL + gs % NSB));
+                                if (it + NSB + 1 == NIT) umma_commit(BAR(B_KEMPTY));
+                            }
+                            if (it >= 0) {
+                                // dK += dS^T Q: A = dS^T from TMEM (a warp's dS lies over its own dP), B = Q (MN-major)
+                                ok = mbar_wait_warp(BAR(B_DSFULL), gi & 1, ab, ST_WAIT_TIMEOUT + 48);
+                                if (!ok) break;
+                                tc_fence_after();
 #pragma unroll
-                            for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
-                                const uint32_t acol = uint32_t(kk2 >> 1) * 32u + uint32_t(kk2 & 1) * 8u;
-                                umma_ts(utmem + 256u + uint32_t(D), utmem + 128u + acol, smem_desc_at(desc_mn, sQ(gi % NQ) + uint32_t(kk2) * 2048u),
-                                        idesc_d, (it > 0 || kk2 > 0) ? 1u : 0u);
+                                for (int kk2 = 0; kk2 < kBlk / 16; ++kk2) {
+                                    const uint32_t acol = uint32_t(kk2 >> 1) * 32u + uint32_t(kk2 & 1) * 8u;
+                                    umma_ts(utmem + 256u + uint32_t(D), utmem + 128u + acol, smem_desc_at(desc_mn, sQ(gi % NQ) + uint32_t(kk2) * 2048u),
+                                            idesc_d, (it > 0 || kk2 > 0) ? 1u : 0u);
+                                }
+                                umma_commit(BAR(B_QEMPTY + gi % NQ));
                             }
-                            umma_commit(BAR(B_QEMPTY + gi % NQ));
-                            if (it + 1 < NIT) ok = issue_dp(it + 1);
+                            if (it >= -1 && it + 1 < NIT) {  // dP^T(it + 1)
+                                if (it < 0) ok = mbar_wait_warp(BAR(B_VFULL), kk & 1, ab, ST_WAIT_TIMEOUT + 43);
+                                if (ok) ok = do_ready(gi + 1);
+                                if (!ok) break;
+                                tc_fence_after();
+                                ss_mmas(utmem + 128u, sV, sdO((gi + 1) % NDO));
+                                umma_commit(BAR(B_DPFULL));
+                                if (it + 2 == NIT) umma_commit(BAR(B_VEMPTY));
+                            }
                         }
                         if (!ok) break;
                         umma_commit(BAR(B_DKDONE));
