@@ -192,13 +192,12 @@ __device__ __forceinline__ bool keep_entry(int i, int j, int qc, int kc, int N, 
     return keep;
 }
 
-// Masks of 32 columns, one bit per column, for the flagged tiles of the backward kernels. They are worked out while the
-// kernels wait for the scores, with one coalesced read of the codes; after the exponentials one select per entry is
+// Masks of 32 columns, one bit per column, for the flagged tiles. The backward kernels work them out while they
+// wait for the scores, with one coalesced read of the codes; after the exponentials one select per entry is
 // left, and a chunk whose bits are 0 in every row of a warp is not exponentiated at all. Against compares per entry
 // (and codes read by every thread) on the way from S to P, with eight compute warps in both kernels: dK/dV 210 -> 194 us and dQ
 // 118 -> 111 us with 8 x 8 heads of 1024 queries, 8192 keys in 8 documents; 250 -> 242 and 168 -> 163 us with 4 x 16 heads x 4096 in
 // up to 16 documents.
-// The forward keeps its compares: the same masks there cost dense tiles 2 % (registers) for 2 % on packed ones.
 __device__ __forceinline__ uint32_t first_bits(int n) { return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1u; }
 
 // Bit x of the result: codes[x] (32 of them, 16-byte aligned; `code` is the lane's own) equals this thread's `own`. All

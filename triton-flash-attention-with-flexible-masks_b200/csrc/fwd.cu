@@ -41,6 +41,9 @@
 
 namespace fa {
 
+// In an item's list of tiles a flag is one of six bits: TILE_KMANY has the place of TILE_QTAIL, which the forward does not ask for.
+constexpr uint32_t LIST_KMANY = TILE_QTAIL;
+
 template <int D>
 struct FwdSmem {
     static constexpr int NS = (D == 128) ? 2 : 4;  // depth of the K ring and of the V ring
@@ -139,7 +142,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         int4 qc;
     };
     auto classify = [&](const Item& it, int i) {
-        return i < it.n ? classify_from_plan(mk, it.b, (mk.He == 1) ? 0 : it.h, it.qb, it.lo + i) & (TILE_VISIT | TILE_BOUND | TILE_DOC | TILE_KMONO) : 0u;
+        return i < it.n ? classify_from_plan(mk, it.b, (mk.He == 1) ? 0 : it.h, it.qb, it.lo + i) & (TILE_VISIT | TILE_BOUND | TILE_DOC | TILE_KMONO | TILE_KMANY) : 0u;
     };
     auto prepare = [&](int j) {
         Item it;
@@ -263,7 +266,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     const int i = base + lane;
                     const uint32_t f = base == 0 ? item.flags : classify(item, i);
                     const uint32_t m = __ballot_sync(0xffffffffu, (f & TILE_VISIT) != 0);
-                    if (f & TILE_VISIT) list[T + __popc(m & ((1u << lane) - 1u))] = uint16_t(uint32_t(i) | (f << 10));
+                    if (f & TILE_VISIT) list[T + __popc(m & ((1u << lane) - 1u))] = uint16_t(uint32_t(i) | ((f & ~TILE_KMANY) | ((f & TILE_KMANY) ? LIST_KMANY : 0u)) << 10);
                     T += __popc(m);
                 }
                 reinterpret_cast<int4*>(smem + S::off_qc)[s * 32 + lane] = item.qc;
@@ -505,7 +508,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             // 128-byte-swizzled layout of the tensor map.
             uint8_t* stage = smem + S::off_q + s * S::TILE;
             const uint32_t tO0 = tmem + lane_base + uint32_t(S::tmem_o + we * D), tO1 = tmem + lane_base + uint32_t(S::tmem_o + (we ^ 1) * D);
-#pragma unroll
+            // (rolled: an eighth of the code to fetch for each item. 4 x 16 x 4096 x 128 in documents 152 -> 146 us a forward)
+#pragma unroll 1
             for (int q = 0; q < D / 16; ++q) {
                 uint32_t x0[16], x1[16];
                 // tcgen05.ld is warp-collective: always executed, the values are ignored when unused
@@ -633,52 +637,38 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 float* sc = reinterpret_cast<float*>(sr);
 
                 if (fl & (TILE_BOUND | TILE_DOC)) {
-                    // keep(x) = (x <= lim) & (qc >= 0 | kc[x] == qc). The compare + select per entry is
-                    // ALU work that costs as much as the tile's MMAs, so it is done per 32-key chunk
-                    // where possible: a chunk is kept or masked as a whole when it lies entirely on
-                    // one side of the bound and (for monotone key codes) holds one single document.
+                    // keep(x) = (x <= lim) & (qc >= 0 | kc[x] == qc) as 32-bit masks, one select per entry behind them. The ids' part is worked
+                    // out by a loop over the four chunks: unrolled, with a case of its own for each kind of chunk, this was most of
+                    // the softmax warps' code, and fetching it cost more than running it. us a forward, so | now: 8 x 8 x 1024 x 8192 x 64 in
+                    // documents 72.7 | 62.5, 4 x 12 x 1000 x 64 21.1 | 19.1, 4 x 16 x 4096 x 128 154 | 142, with ids drawn at random from 40 383 | 338,
+                    // 32 x 32768 x 128 in 64 documents 870 | 827, 16 x 8 x 577 x 32 without ids 29.1 | 28.1.
                     int lim = kBlk - 1;
                     if (fl & TILE_BOUND) {
                         int jmax = mk.N - 1;
                         if (mk.causal) jmax = min(jmax, row + mk.gap);
                         lim = jmax - k0;
                     }
-                    const bool doc = (fl & TILE_DOC) && qc < 0;  // a row with qc >= 0 passes the id check everywhere
-                    const int* kcs = reinterpret_cast<const int*>(smem + S::off_kc + (g % S::NKC) * (kBlk * 4));
                     // (the key codes completed on K's barrier, before the S MMA whose result was just read)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        int state = 0;  // this row in chunk q: 0 keep all, 1 mask all, 2 entry by entry
-                        if (32 * q > lim) state = 1;
-                        else if (32 * q + 31 > lim) state = 2;
-                        if (doc && state != 1) {
-                            if (fl & TILE_KMONO) {
-                                const int kf = kcs[32 * q], kl = kcs[32 * q + 31];
-                                if (kf != kl) state = 2;
-                                else if (kf != qc) state = 1;
-                            } else {
-                                state = 2;
+                    const int* kcs = reinterpret_cast<const int*>(smem + S::off_kc + (g % S::NKC) * (kBlk * 4));
+                    uint32_t same[4] = {~0u, ~0u, ~0u, ~0u};
+                    if (fl & TILE_DOC) {
+                        if ((fl & TILE_KMONO) && kcs[0] == kcs[kBlk - 1]) {  // one code in the block
+                            if (qc < 0 && kcs[0] != qc) same[0] = same[1] = same[2] = same[3] = 0u;
+                        } else {
+#pragma unroll 1
+                            for (int q = 0; q < 4; ++q) {
+                                uint32_t m = codes_equal(kcs + 32 * q, kcs[32 * q + lane], qc, (fl & LIST_KMANY) != 0);
+                                if (qc >= 0) m = ~0u;  // such a row passes the id check everywhere
+                                if (q == 0) same[0] = m; else if (q == 1) same[1] = m; else if (q == 2) same[2] = m; else same[3] = m;
                             }
                         }
-                        if (!__any_sync(0xffffffffu, state == 2)) {
-                            if (state == 1) {
+                    }
 #pragma unroll
-                                for (int x = 0; x < 32; ++x) sc[32 * q + x] = -INFINITY;
-                            }
-                        } else if (doc) {
-                            const int4* kc4 = reinterpret_cast<const int4*>(kcs + 32 * q);
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t keep = first_bits(lim + 1 - 32 * q) & same[q];
+                        if (__any_sync(0xffffffffu, keep != ~0u)) {
 #pragma unroll
-                            for (int u = 0; u < 8; ++u) {
-                                const int4 kc = kc4[u];
-                                const int x = 32 * q + 4 * u;
-                                sc[x + 0] = (kc.x == qc && x + 0 <= lim) ? sc[x + 0] : -INFINITY;
-                                sc[x + 1] = (kc.y == qc && x + 1 <= lim) ? sc[x + 1] : -INFINITY;
-                                sc[x + 2] = (kc.z == qc && x + 2 <= lim) ? sc[x + 2] : -INFINITY;
-                                sc[x + 3] = (kc.w == qc && x + 3 <= lim) ? sc[x + 3] : -INFINITY;
-                            }
-                        } else {
-#pragma unroll
-                            for (int x = 0; x < 32; ++x) sc[32 * q + x] = (32 * q + x <= lim) ? sc[32 * q + x] : -INFINITY;
+                            for (int x = 0; x < 32; ++x) sc[32 * q + x] = (keep & (1u << x)) ? sc[32 * q + x] : -INFINITY;
                         }
                     }
                 }
