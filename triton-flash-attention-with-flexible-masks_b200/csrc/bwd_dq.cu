@@ -418,10 +418,12 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             const float lse = reinterpret_cast<const float*>(smem + S::off_vec + s * S::VEC)[r];
             const float delta = reinterpret_cast<const float*>(smem + S::off_vec + s * S::VEC)[kBlk + r];
 
-            int cc = wk.first_from(0);
-            for (int t = 0; t < T && ok; ++t, cc = wk.first_from(cc + 1)) {
+            int cc = -1;
+            for (int t = 0; t < T && ok; ++t) {
                 const int gi = gt + t;
-                const uint32_t code = wk.code(cc);
+                uint32_t code;
+#pragma unroll 1
+                do code = wk.code(++cc); while (code == QC_SKIP);
                 const bool fl_doc = code >= QC_DOC, many = code == QC_DOCMANY;
                 const int kb0 = (lo + cc) * kBlk;
                 const int kb1 = min(kb0 + kBlk, mk.N);
