@@ -5,7 +5,6 @@
 
 namespace fa {
 
-constexpr int kAttnThreads = 384;  // dQ: 3 warpgroups: two compute groups, one producer / MMA group
 constexpr int kDkdvThreads = 608;  // dK / dV: sixteen compute warps and the producer, MMA and scheduler warps
 // forward: 4 warpgroups, two softmax groups, an epilogue group, a producer / MMA group. Registers a thread after setmaxnreg
 constexpr int kFwdThreads = 512, kFwdSoftmaxRegs = 192, kFwdEpilogueRegs = 80, kFwdServiceRegs = 48;
