@@ -33,7 +33,11 @@
 // 32 x 32768 x 128 in 64 documents 908 | 776 | 786; 16 x 32 x 8192 x 128 causal 9520 | 7760 | 7690; 4 x 16 x 4096 x 64 causal
 // 249 | 201 | 192; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 94 | 83 | 79. The shared O had errors 1 to 2 %
 // larger as well: one entry of a row is an exact 1 in P, not one of each chain.
-// What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group) and, in
+// Since then the code was made smaller (loops that are not unrolled, masks by a loop, shorter waits) and a block's first item is known at once, us, that "now" | at
+// present: 2 x 32 / 8 x 3001 170 | 162, 512 against 8192 58.0 | 56.5, 16 x 8 x 577 x 32 31.1 | 27.9, 4 x 16 x 4096 x 128 in documents 152 | 136, 32 x
+// 32768 x 128 870 | 812, 16 x 32 x 8192 x 128 8470 | 8030, 8 x 8 x 1024 x 8192 x 64 75.2 | 62.5, 4 x 12 x 1000 x 64 in documents 24.4 | 19.2.
+// What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group, and fetching their own straight code), at D = 128 the
+// 64 KB of K and V that each tile brings from L2 (52 B a clock and SM; half of them would take dense calls 5 % less time), and, in
 // dense calls, the clock under the power cap (1.4-1.5 GHz); with short items the drain of two O, which the next item's P*V waits for.
 #include <type_traits>
 #include "common.cuh"
