@@ -200,28 +200,29 @@ struct Call {
 struct FlashAttention : torch::autograd::Function<FlashAttention> {
     static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Call& c) {
         Tensor plan;
-        Outputs r;
-        {
-            py::gil_scoped_release free;
-            if (c.eq || !fa_plan_optional(&c.p, c.needs_grad)) plan = build_plan(c.p, c.eq, c.ek, c.status);
-            r = launch_forward(c.p, q, k, v, plan, 0, c.status, std::nullopt);
+        Outputs r = launch(q, k, v, c, plan);
+        torch::autograd::variable_list saved{q, k, v, r.o, r.lse};
+        if (c.eq) {
+            saved.push_back(*c.eq);
+            saved.push_back(*c.ek);
         }
-        n_launched += (plan.defined() ? c.plan_kernels : 0) + (r.splits > 1 ? 2 : 1);
-        if (c.needs_grad) {
-            torch::autograd::variable_list saved{q, k, v, r.o, r.lse};
-            if (c.eq) {
-                saved.push_back(*c.eq);
-                saved.push_back(*c.ek);
-            }
-            ctx->save_for_backward(std::move(saved));
-            ctx->saved_data["plan"] = plan;
-            ctx->saved_data["status"] = c.status;
-            ctx->saved_data["causal"] = int64_t(c.p.causal);
-            ctx->saved_data["mode"] = int64_t(c.p.mode);
-            ctx->saved_data["id_heads"] = int64_t(c.p.id_heads);
-            ctx->saved_data["scale"] = double(c.p.sm_scale);
-        }
+        ctx->save_for_backward(std::move(saved));
+        ctx->saved_data["plan"] = plan;
+        ctx->saved_data["status"] = c.status;
+        ctx->saved_data["causal"] = int64_t(c.p.causal);
+        ctx->saved_data["mode"] = int64_t(c.p.mode);
+        ctx->saved_data["id_heads"] = int64_t(c.p.id_heads);
+        ctx->saved_data["scale"] = double(c.p.sm_scale);
         return r.o;
+    }
+
+    // The plan, where the call needs one, and the forward.
+    static Outputs launch(const Tensor& q, const Tensor& k, const Tensor& v, const Call& c, Tensor& plan) {
+        py::gil_scoped_release free;
+        if (c.eq || !fa_plan_optional(&c.p, c.needs_grad)) plan = build_plan(c.p, c.eq, c.ek, c.status);
+        Outputs r = launch_forward(c.p, q, k, v, plan, 0, c.status, std::nullopt);
+        n_launched += (plan.defined() ? c.plan_kernels : 0) + (r.splits > 1 ? 2 : 1);
+        return r;
     }
 
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
@@ -257,11 +258,13 @@ py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, bool causal
         p.id_heads = int(id_heads(*eq, *ek, p.B, p.H, p.M, p.N));
         if (p.id_heads == 0) return py::none();
     }
-    if (at::SavedTensorDefaultHooks::get_hooks()) return py::none();
     const bool needs_grad = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
+    if (needs_grad && at::SavedTensorDefaultHooks::get_hooks()) return py::none();
     const int plan_kernels = !eq || (p.M + 127) / 128 + (p.N + 127) / 128 <= FA_PLAN_ONE_KERNEL_BLOCKS ? 1 : 3;
     const Call call{p, eq ? &*eq : nullptr, ek ? &*ek : nullptr, status, needs_grad, plan_kernels};
-    return py::cast(FlashAttention::apply(q, k, v, call));
+    if (needs_grad) return py::cast(FlashAttention::apply(q, k, v, call));
+    Tensor plan;
+    return py::cast(FlashAttention::launch(q, k, v, call, plan).o);
 }
 
 int64_t launched() { return n_launched; }

@@ -209,7 +209,7 @@ def _like_subclass(q):
 
 # looked up once: a short call's host time is what bounds it
 _TENSOR, _PLAIN, _tracing_state = torch.Tensor, (torch.Tensor, torch.nn.Parameter), torch._C._get_tracing_state
-_grad_enabled, _transforms, _forward_ad = torch.is_grad_enabled, torch._C._functorch.peek_interpreter_stack, torch.autograd.forward_ad
+_transforms, _forward_ad = torch._C._functorch.peek_interpreter_stack, torch.autograd.forward_ad
 
 
 def _native_forward(host, q, k, v, causal, sm_scale, needs_grad, key_runs):
@@ -221,19 +221,6 @@ def _native_forward(host, q, k, v, causal, sm_scale, needs_grad, key_runs):
     if status is None:
         return None
     return host.forward(q, k, v, False, bool(causal), sm_scale, SCORE_FUNC_MODE0_NOPE, 1, None, needs_grad, key_runs, status, _like_subclass(q))
-
-
-def _native_attend(q, k, v, causal, sm_scale, eq, ek, score_func_mode):
-    """A regular call with whatever plan and node it needs, in one native call; None for any other."""
-    attend = getattr(_HOST, "attend", None)
-    if (attend is None or build_plan is not _own_build_plan  # (somebody's own plan or host calls)
-            or PROFILE is not None or _SYNC_STATUS or not (sm_scale is None or type(sm_scale) is float)
-            or _tracing_state() is not None or not (eq is None or type(eq) in _PLAIN) or not (ek is None or type(ek) in _PLAIN)):
-        return None
-    status = _STATUS.get(q.get_device())
-    if status is None:
-        return None
-    return attend(q, k, v, bool(causal), sm_scale, eq, ek, score_func_mode, status)
 
 
 class FlashAttention(torch.autograd.Function):
@@ -449,17 +436,14 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
     # bound by its host time: 4 x 12 heads x 1000 x 64 in documents 113 us for 92 of kernels with the node of this module (its backward waits for
     # the interpreter in the engine's thread), 88 with the native one. Transforms of torch.func and forward-mode gradients need
     # the node of this module for their messages, subclasses for their hooks, and a trace for its refusal.
-    if (_HOST is not None and type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(score_func_mode) is int
-            and _transforms() is None and _forward_ad._current_level < 0):
-        if (eq is None and ek is None and score_func_mode == SCORE_FUNC_MODE0_NOPE
-                and not (_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad))):
-            # no node at all: 8 heads of 200 queries take 13.6 us a call with the one of this module, 9.7 without
-            done = _native_forward(_HOST, q, k, v, causal, sm_scale, False, 0)
-            if done is not None:
-                _count(done[3])
-                return done[0]
-        else:
-            done = _native_attend(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
+    # Without a gradient there is no node at all: 8 heads of 200 queries took 13.6 us a call with the one of this module, 7.5 now.
+    if (type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(score_func_mode) is int and (eq is None or type(eq) in _PLAIN)
+            and (ek is None or type(ek) in _PLAIN) and (sm_scale is None or type(sm_scale) is float) and PROFILE is None and not _SYNC_STATUS
+            and build_plan is _own_build_plan  # (not somebody's own)
+            and _transforms() is None and _forward_ad._current_level < 0 and _tracing_state() is None):
+        attend, status = getattr(_HOST, "attend", None), _STATUS.get(q.get_device())
+        if attend is not None and status is not None:
+            done = attend(q, k, v, bool(causal), sm_scale, eq, ek, score_func_mode, status)
             if done is not None:
                 return done
     return FlashAttention.apply(q, k, v, causal, sm_scale, eq, ek, score_func_mode)
