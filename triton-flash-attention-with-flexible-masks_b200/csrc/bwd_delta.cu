@@ -10,12 +10,12 @@ namespace fa {
 
 // D / 8 neighbouring threads read a row, 16 bytes of O and of dO each, so that a warp's load covers whole 128-byte lines, and each thread
 // has the loads of its kRows rows in flight before it uses the first. Bound by HBM.
-// us, eight threads a row with 2 x D / 8 elements and one row each | now: 16 x 8 x 577 x 32 6.5 | 2.8, 8 x 8 x 1024 x 64
-// 5.5 | 3.5, 4 x 12 x 1000 x 64 4.4 | 2.8; D = 128, where HBM has always been the bound, 4 x 16 x 4096 37 | 36 and 32 x 32768 109 | 106
-// (the wait for the forward's last blocks included); two or eight rows a thread 36 and 39, 106 and 112.
+// us between events in a graph, eight threads a row with 2 x D / 8 elements and one row each | now: 16 x 8 x 577 x 32 6.1 | 2.8, 8 x 8 x 1024 x 64
+// 5.2 | 3.3, 4 x 12 x 1000 x 64 4.1 | 3.0, 2 x 32 x 3001 x 128 16.2 | 14.2, 32 x 32768 x 128 96.7 | 83.1 (6.5 TB/s), 4 x 16 x 4096 x 128 21.1 | 21.2; one row
+// a thread 18.3 and 103 in the fourth and fifth, four rows 21.7 in the last.
 template <int D>
 struct DeltaShape {
-    static constexpr int kThreads = 256, kLanes = D / 8, kRows = (D == 128 ? 4 : D == 64 ? 4 : 2);
+    static constexpr int kThreads = 256, kLanes = D / 8, kRows = 2;
     static constexpr int kStep = kThreads / kLanes;     // rows that the block's threads read together
     static constexpr int kBlockRows = kStep * kRows;
 };
