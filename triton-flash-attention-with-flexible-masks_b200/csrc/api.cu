@@ -237,13 +237,13 @@ int sm_count() {
 
 // Runs into which the forward cuts each item's key tiles, for calls without ids that have fewer items than the GPU
 // has SMs. A round of items is taken to cost its tiles plus 4 tile times of fill, drain and epilogue, the second
-// kernel and the fp32 rows 6 more (fitted to an earlier forward). At most two items per SM, which bounds the workspace at 20 MB.
-// One token, 32 / 8 heads of 128, us a call in a replayed graph with 1 run and with the number taken here, and the best of 1, 2, 3, 4, 6,
-// 8, 12, 16: 32768 keys 186, 35.2 (18 runs; 34.0 with 16); 4096 keys 29, 16.5 (16; 15.5 with 8); 1024 keys 12.9 (1; 12.2 with 3 or 4);
-// 4 sequences of 8192 keys 53, 30.6 (4, the best); 8 of them 58, 48 (2, the best); 16 of 4500 51 (1, the best). 300 queries against 9000
-// keys: 16 / 4 heads 58, 34 (3, the best; 2 runs 41, 4 runs 47), 32 / 8 heads 63, 61 (3, the best; 2 runs 74, 4 runs 71); 512 against
-// 8192, 32 / 8 heads 56 (1, the best; 2 runs 73). 64 against 4000, 16 heads 30, 18.5 (8; 17.6 with 6). Heads of 64: 1000 x 1000 of 8
-// heads 12 (1, the best; 2 runs 17), 2 x 16 heads of 200 against 3000 22.8, 22.5 (2, the best).
+// kernel and the fp32 rows 6 more. At most two items per SM, which bounds the workspace at 20 MB.
+// One token, 32 / 8 heads of 128, us a call in a replayed graph with 1 run and with the number taken here, and the best of 1, 2, 3, 4, 5, 6,
+// 8, 10, 12, 16, 18: 32768 keys (heads of 64) 173, 21.2 (18 runs; 20.9 with 16); 16384 95, 17.3 (16, the best); 4096 28.6, 12.7 (16, the best); 1024 12.3 (1; 11.2
+// with 4); 4 sequences of 8192 keys 52.6, 29.1 (4, the best); 8 of them 56.7, 47.5 (2, the best); 12 of 3000 30.7 (1, the best). 300 queries against 9000
+// keys: 16 / 4 heads 57.4, 33.7 (3, the best; 2 runs 40.6, 4 runs 45.2), 32 / 8 heads 59.2, 57.5 (3, the best; 2 runs 72.6, 4 runs 64.9); 512 against
+// 2000, 32 / 8 heads 19.9 (1, the best; 2 runs 36.0). 64 against 4000, 16 heads 29.3, 16.6 (8; 16.0 with 6), 40 against 2000, 32 / 8 heads 18.8, 16.0 (8; 15.0 with 4),
+// 500 against 3000, 16 heads 24.6, 25.5 (2). Heads of 64: 1024 x 1024 of 8 heads 11.3 (1, the best; 2 runs 16.3).
 int fwd_splits(const fa_problem* p, int sms) {
     if (p->mode != FA_MODE0_NOPE || p->dtype == FA_FP32) return 1;
     const int pack = fwd_pack(p);
