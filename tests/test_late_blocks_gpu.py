@@ -74,3 +74,27 @@ def test_forward(busy, form, counters):
 
     launch()
     late_blocks(busy, launch, (o, lse[..., :M]), (o.clone(), lse[..., :M].clone()), status)
+
+
+@pytest.mark.parametrize("counters", [False, True])
+def test_dkdv(busy, counters):
+    from flash_b200 import _lib, ops
+    lib = _lib.load()
+    B, H, Hk, M, N, D = 1, 16, 16, 32768, 1200, 128
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, do = (torch.randn(B, h, n, D, generator=g, device="cuda").bfloat16() for h, n in ((H, M), (Hk, N), (Hk, N), (H, M)))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    prob = ops._problem(B, H, Hk, M, N, D, q.dtype, False, 0, 1, D ** -0.5)
+    plan = ops.build_plan(prob, None, None, status) if counters else None
+    o, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    lse, delta = (torch.empty(B, H, lib.fa_padded_rows(M), device="cuda") for _ in range(2))
+    tq, tk, tv, to, tdo = [ops._tensor(t) for t in (q, k, v, o, do)]
+    assert lib.fa_fwd(prob, tq, tk, tv, to, lse.data_ptr(), None, status.data_ptr(), ops._stream()) == 0
+    assert lib.fa_bwd_delta(prob, to, tdo, delta.data_ptr(), ops._stream()) == 0
+
+    def launch():
+        assert lib.fa_bwd_dkdv(prob, tq, tk, tv, tdo, lse.data_ptr(), delta.data_ptr(), ops._tensor(dk), ops._tensor(dv),
+                               plan.data_ptr() if counters else None, status.data_ptr(), ops._stream()) == 0
+
+    launch()
+    late_blocks(busy, launch, (dk, dv), (dk.clone(), dv.clone()), status)

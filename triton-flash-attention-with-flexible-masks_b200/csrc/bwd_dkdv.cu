@@ -193,8 +193,24 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     launch_dependents();  // (fa_bwd's dQ kernel reads nothing that this one writes, but delta, which is complete since the wait)
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
+    // Item k of this CTA. Items are handed out in order from a counter in the plan (any CTA takes the next one: the
+    // work per item varies with the mask); without counters (no plan given) they are
+    // dealt out round robin in alternating direction, which evens out their sorted lengths.
+    auto take = [&](int k) {
+        if (ctr) return int(atomicAdd(ctr, 1u));
+        return k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
+    };
     // an earlier launch on this device ran into a time-out that the host has not yet cleared
-    if (aborted && (sbase & 1023u) == 0) nan_fill_outputs(smem + S::off_k, S::NBOX, &tmdK, &tmdV, nK, p.Hk, p.B);
+    if (aborted && (sbase & 1023u) == 0)
+        nan_fill_items(smem + S::off_k, S::NBOX, n_items, take, [&](int j, int lane) {
+            int kb, hk, b;
+            decode(j, kb, hk, b);
+            if (lane == 0)
+                for (int x = 0; x < S::NBOX; ++x) {
+                    tma_store_4d(&tmdK, smem_u32(smem + S::off_k) + x * S::BOX, x * 64, kb * kBlk, hk, b);
+                    tma_store_4d(&tmdV, smem_u32(smem + S::off_k) + x * S::BOX, x * 64, kb * kBlk, hk, b);
+                }
+        });
 
     if (warp >= 16) {
         if (aborted) {
@@ -202,9 +218,6 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             // ------------------------------ scheduler ------------------------------
             // Item k goes to slot k & 1: range [lo, lo + n) of candidate query blocks (union over the
             // group's heads), a 2-bit code per candidate, and the number of tiles.
-            // Items are handed out in order from a counter in the plan (any CTA takes the next one: the
-            // work per item varies with the mask); without counters (no plan given) they are
-            // dealt out round robin in alternating direction, which evens out their sorted lengths.
             bool ok = true;
             for (int k = 0;; ++k) {
                 const int s = k & 1, use = k >> 1;
@@ -212,10 +225,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 int j = 0;
-                if (lane == 0) {
-                    if (ctr) j = int(atomicAdd(ctr, 1u));
-                    else j = k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
-                }
+                if (lane == 0) j = take(k);
                 j = __shfl_sync(0xffffffffu, j, 0);
                 if (j >= n_items) {  // end marker
                     if (lane == 0) {

@@ -255,32 +255,6 @@ __device__ __forceinline__ void nan_fill_items(uint8_t* tile, int nbox, int n_it
     }
 }
 
-// A launch that finds the device's status word set by an earlier time-out computes nothing. It fills
-// its outputs with NaN (0xFFFF is a NaN in bf16 and in fp16), so that what it leaves behind cannot be
-// mistaken for a result. Called by all threads of the CTA; `tile` is nbox * 16 KB of shared memory,
-// 1024-byte aligned; m1 may be null. Tiles are [128 rows, 64 * nbox columns] of a [B, H, L, D] tensor.
-__device__ __forceinline__ void nan_fill_outputs(uint8_t* tile, int nbox, const CUtensorMap* m0, const CUtensorMap* m1,
-                                                 int n_blk, int n_h, int n_b) {
-    constexpr int kBox = kBlk * 64 * 2;
-    for (int i = threadIdx.x; i < nbox * kBox / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(tile)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-    fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t src = smem_u32(tile);
-        const int n = n_blk * n_h * n_b;
-        for (int j = blockIdx.x; j < n; j += gridDim.x) {
-            const int blk = j % n_blk, h = (j / n_blk) % n_h, b = j / (n_blk * n_h);
-            for (int x = 0; x < nbox; ++x) {
-                tma_store_4d(m0, src + x * kBox, x * 64, blk * kBlk, h, b);
-                if (m1) tma_store_4d(m1, src + x * kBox, x * 64, blk * kBlk, h, b);
-            }
-            tma_store_commit();
-        }
-        tma_store_wait_all();
-    }
-}
-
 // Device-side view of a [B, H, L, D] tensor for plain (non-TMA) stores.
 struct OutTensor {
     void* ptr;
