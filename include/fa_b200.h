@@ -188,7 +188,7 @@ int fa_fwd_static_plan(const fa_problem* p, const fa_tensor* q, const fa_tensor*
                        const fa_tensor* o, float* lse, const fa_ids* eq, const fa_ids* ek, int32_t* status,
                        void* stream);
 
-/* Largest query length fa_group_rows sorts (one CTA sorts a row in shared memory). */
+/* Largest query length fa_group_rows sorts (the longer rows in the shared memory of one CTA each). */
 #define FA_GROUP_MAX_ROWS 16384
 
 /* Grouping of the queries by id for calls WITHOUT a causal mask, where the order of the query rows is
@@ -198,7 +198,8 @@ int fa_fwd_static_plan(const fa_problem* p, const fa_tensor* q, const fa_tensor*
  * their places. Writes three int32 arrays [B, id_heads, M], contiguous: `order` (grouped position ->
  * caller's position), `inverse` (caller's position -> grouped position) and `grouped_ids` (the ids in
  * grouped order; pass them as the eq of fa_plan_build). p->M <= FA_GROUP_MAX_ROWS, else
- * FA_ERR_UNSUPPORTED. An id below -2^31 sets status 200 as in fa_plan_build. */
+ * FA_ERR_UNSUPPORTED. An id below -2^31 sets status 200 as in fa_plan_build. One of the outputs may take the
+ * place of a contiguous int32 eq (each row is read before its results are written); other overlaps are not supported. */
 int fa_group_rows(const fa_problem* p, const fa_ids* eq, int32_t* order, int32_t* inverse, int32_t* grouped_ids,
                   int32_t* status, void* stream);
 

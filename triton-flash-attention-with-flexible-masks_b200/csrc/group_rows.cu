@@ -56,6 +56,15 @@ __device__ __forceinline__ uint32_t sort_code(const IdRows& eq, int b, int he, i
 // 8.1 | 8.5.
 constexpr int kRankRows = 4096, kRankThreads = 256, kRankBlock = 64;
 constexpr int64_t kRankCodes = 49152;  // id rows x M up to which counting is faster
+
+// Does the range of bytes that holds the ids meet that of the int32 array `out` of n elements?
+bool overlaps(const IdRows& eq, int B, int He, int M, const int32_t* out, int64_t n) {
+    const int64_t item = eq.is64 ? 8 : 4, last[3] = {(B - 1) * eq.sb, (He - 1) * eq.sh, (M - 1) * eq.sl};
+    int64_t lo = 0, hi = 0;  // of the offsets, in elements
+    for (int64_t x : last) (x < 0 ? lo : hi) += x;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(eq.ptr), o = reinterpret_cast<uintptr_t>(out);
+    return base + lo * item < o + n * 4 && o < base + (hi + 1) * item;
+}
 __global__ void __launch_bounds__(kRankThreads) group_rank_kernel(IdRows eq, int M, int He, int32_t* order, int32_t* inverse,
                                                                   int32_t* grouped, int* status) {
     __shared__ uint4 codes4[kRankRows / 4];
@@ -185,7 +194,11 @@ extern "C" int fa_group_rows(const fa_problem* p, const fa_ids* eq, int32_t* ord
     if (eq->dtype != FA_ID_INT32 && eq->dtype != FA_ID_INT64) return FA_ERR_BAD_ARG;
     if (p->M > FA_GROUP_MAX_ROWS) return FA_ERR_UNSUPPORTED;
     const IdRows rows{eq->ptr, eq->stride[0], eq->stride[1], eq->stride[2], eq->dtype == FA_ID_INT64};
-    if (p->M <= kRankRows && int64_t(p->id_heads) * p->B * p->M <= kRankCodes) {
+    const int64_t n = int64_t(p->id_heads) * p->B * p->M;
+    // The counting kernel's blocks read a row while others write its results; the network's block has read its row when it writes.
+    const bool apart = !overlaps(rows, p->B, p->id_heads, p->M, order, n) && !overlaps(rows, p->B, p->id_heads, p->M, inverse, n) &&
+                       !overlaps(rows, p->B, p->id_heads, p->M, grouped_ids, n);
+    if (p->M <= kRankRows && n <= kRankCodes && apart) {
         const dim3 grid(fa::cdiv(p->M, kRankBlock), p->id_heads, p->B);
         return fa::launch_overlapping(group_rank_kernel, grid, kRankThreads, 0, static_cast<cudaStream_t>(stream), rows, p->M, p->id_heads, order,
                                       inverse, grouped_ids, status) == cudaSuccess ? FA_OK : FA_ERR_LAUNCH;
