@@ -156,20 +156,27 @@ struct F32Acc {
 #pragma unroll
             for (int k = 0; k < N; ++k) v[i][k] = mul_f2(v[i][k], pack_f2(f[2 * i], f[2 * i + 1]));
     }
-    // += sum_c P[c][row] * V[c][own column k], P being the warp's own (put_p)
-    __device__ __forceinline__ void add(const float* P, const float* V, int x) {
-        constexpr int LD = D + 4;
+    // += sum_c P[c][row] * V[c][own column k], P being the warp's own (put_p). kHalves: over lo <= c < hi only
+    template <bool kHalves>
+    __device__ __forceinline__ void add(const float* P, const float* V, int x, int lo, int hi) {
+        if (!kHalves || (lo <= 0 && hi >= kC)) {
 #pragma unroll 8
-        for (int c = 0; c < kC; ++c) {
-            float own[N];
-            Own<D>::load(V + c * LD, x, own);
-            const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(P + c * kRW);
+            for (int c = 0; c < kC; ++c) add_column(P, V, x, c);
+        } else {
+            hi = min(hi, kC);
+#pragma unroll 4
+            for (int c = max(lo, 0); c < hi; ++c) add_column(P, V, x, c);
+        }
+    }
+    __device__ __forceinline__ void add_column(const float* P, const float* V, int x, int c) {
+        float own[N];
+        Own<D>::load(V + c * (D + 4), x, own);
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(P + c * kRW);
 #pragma unroll
-            for (int k = 0; k < N; ++k) {
-                const uint64_t o2 = pack_f2(own[k], own[k]);
-                v[0][k] = fma_f2(w.x, o2, v[0][k]);
-                v[1][k] = fma_f2(w.y, o2, v[1][k]);
-            }
+        for (int k = 0; k < N; ++k) {
+            const uint64_t o2 = pack_f2(own[k], own[k]);
+            v[0][k] = fma_f2(w.x, o2, v[0][k]);
+            v[1][k] = fma_f2(w.y, o2, v[1][k]);
         }
     }
     __device__ __forceinline__ void row(int r, float (&out)[N]) const {
@@ -223,7 +230,7 @@ __device__ __forceinline__ int code_k(const MaskArgs& mk, int b, int he, int j) 
 // forward: grid (ceil(M / 32), H, B)
 // ---------------------------------------------------------------------------------------------
 template <int D, int R>
-__global__ void __launch_bounds__(threads(R)) f32_fwd_kernel(const F32Params p) {
+__global__ void __launch_bounds__(threads(R), R == 32 && D <= 32 ? 4 : 0) f32_fwd_kernel(const F32Params p) {
     using S = F32Smem<D, R>;
     extern __shared__ __align__(16) float sm[];
     float* Qs = sm;
@@ -243,6 +250,12 @@ __global__ void __launch_bounds__(threads(R)) f32_fwd_kernel(const F32Params p) 
     const bool kvec = rows_aligned(kbase, p.k.sl), vvec = rows_aligned(vbase, p.v.sl);
     const int32_t* kcodes = mk.mode == 1 ? mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad : nullptr;
     const int end = mk.causal ? min(mk.N, i0 + R + mk.gap) : mk.N;  // keys beyond the last row's causal bound
+    // In a block of 32 rows those beyond the first half's: the values there stay out of its P V, for a product with a P of 0 may be NaN.
+    // What a NaN or an infinity reaches then does not go by the size of the blocks, which goes by what a sequence is batched with. us, forward and
+    // forward with backward, products over the whole tile | over what the half sees: 4 x 8 heads x 1024 x 64 causal 179, 726 | 177, 712, not causal
+    // 324, 1342 | 324, 1329; 4 x 8 x 1024 x 128 causal 363, 1462 | 359, 1466; 8 x 16 x 512 x 32 causal 121, 496 | 119, 488, not causal 205, 855 | 208, 859
+    // (four blocks of head dims up to 32 share an SM only while a thread has 64 registers: 211 with three).
+    const int end_half = mk.causal && r0 < 16 ? i0 + 16 + mk.gap : mk.N + kC;
     auto fetch = [&](int j0, int st) {
         load_tile<D, kC, R>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, end);
         load_tile<D, kC, R>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, end);
@@ -297,7 +310,7 @@ __global__ void __launch_bounds__(threads(R)) f32_fwd_kernel(const F32Params p) 
         acc.scale(alpha);
         put_p(Ps, x, s);
         __syncwarp();
-        acc.add(Ps, Ks + S::cols, x);
+        acc.template add<R == 32>(Ps, Ks + S::cols, x, 0, end_half - j0);
         __syncthreads();  // the stage may be refilled
         j0 = jn;
     }
@@ -358,6 +371,7 @@ __global__ void __launch_bounds__(threads(R)) f32_bwd_dq_kernel(const F32Params 
     const bool kvec = rows_aligned(kbase, p.k.sl), vvec = rows_aligned(vbase, p.v.sl);
     const int32_t* kcodes = mk.mode == 1 ? mk.plan + mk.L.off_kc + (int64_t(b) * mk.He + he) * mk.L.Npad : nullptr;
     const int end = mk.causal ? min(mk.N, i0 + R + mk.gap) : mk.N;  // keys beyond the last row's causal bound
+    const int end_half = mk.causal && r0 < 16 ? i0 + 16 + mk.gap : mk.N + kC;  // (see the forward)
     auto fetch = [&](int j0, int st) {
         load_tile<D, kC, R>(KVs + st * 2 * S::cols, kbase, p.k.sl, kvec, j0, end);
         load_tile<D, kC, R>(KVs + (st * 2 + 1) * S::cols, vbase, p.v.sl, vvec, j0, end);
@@ -405,7 +419,7 @@ __global__ void __launch_bounds__(threads(R)) f32_bwd_dq_kernel(const F32Params 
         }
         put_p(Ps, x, dp);
         __syncwarp();
-        acc.add(Ps, Ks, x);  // dQ += dS K (flash_triton.py:420)
+        acc.template add<R == 32>(Ps, Ks, x, 0, end_half - j0);  // dQ += dS K (flash_triton.py:420)
         __syncthreads();
         j0 = jn;
     }
@@ -450,6 +464,7 @@ __global__ void __launch_bounds__(threads(R)) f32_bwd_dkdv_kernel(const F32Param
     dv.clear();
     // first query row that can see key j0 under the causal mask (flash_triton.py:214-218)
     const int first = mk.causal ? max(0, j0 - mk.gap) : 0;
+    const int first_half = mk.causal && r0 >= 16 ? j0 + 16 - mk.gap : 0;  // the same for the second half of 32 keys (see the forward)
     for (int g = 0; g < p.G; ++g) {
         const int h = hk * p.G + g;
         const int he = (mk.He == 1) ? 0 : h;
@@ -507,11 +522,11 @@ __global__ void __launch_bounds__(threads(R)) f32_bwd_dkdv_kernel(const F32Param
             }
             put_p(Ps, x, s);
             __syncwarp();
-            dv.add(Ps, dOs, x);  // dV += P^T dO (flash_triton.py:291)
+            dv.template add<R == 32>(Ps, dOs, x, first_half - i0, kC);  // dV += P^T dO (flash_triton.py:291)
             __syncwarp();
             put_p(Ps, x, dp);
             __syncwarp();
-            dk.add(Ps, Qs, x);   // dK += dS^T Q (flash_triton.py:308)
+            dk.template add<R == 32>(Ps, Qs, x, first_half - i0, kC);   // dK += dS^T Q (flash_triton.py:308)
             __syncthreads();
             i0 = in;
         }
