@@ -9,6 +9,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_cpp_function.h>
 #include <torch/csrc/utils/pybind.h>
 #include <torch/types.h>
 #include <atomic>
@@ -189,6 +190,7 @@ std::atomic<int64_t> n_launched{0};
 // What a regular call is, besides q, k and v.
 struct Call {
     fa_problem p;
+    double sm_scale;
     const Tensor *eq, *ek;  // null without ids
     const Tensor& status;
     bool needs_grad;
@@ -212,7 +214,7 @@ struct FlashAttention : torch::autograd::Function<FlashAttention> {
         ctx->saved_data["causal"] = int64_t(c.p.causal);
         ctx->saved_data["mode"] = int64_t(c.p.mode);
         ctx->saved_data["id_heads"] = int64_t(c.p.id_heads);
-        ctx->saved_data["scale"] = double(c.p.sm_scale);
+        ctx->saved_data["scale"] = c.sm_scale;
         return r.o;
     }
 
@@ -261,13 +263,62 @@ py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, bool causal
     const bool needs_grad = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
     if (needs_grad && at::SavedTensorDefaultHooks::get_hooks()) return py::none();
     const int plan_kernels = !eq || (p.M + 127) / 128 + (p.N + 127) / 128 <= FA_PLAN_ONE_KERNEL_BLOCKS ? 1 : 3;
-    const Call call{p, eq ? &*eq : nullptr, ek ? &*ek : nullptr, status, needs_grad, plan_kernels};
+    const Call call{p, sm_scale, eq ? &*eq : nullptr, ek ? &*ek : nullptr, status, needs_grad, plan_kernels};
     if (needs_grad) return py::cast(FlashAttention::apply(q, k, v, call));
     Tensor plan;
     return py::cast(FlashAttention::launch(q, k, v, call, plan).o);
 }
 
 int64_t launched() { return n_launched; }
+
+// What `grad_fn` of a regular call shows to Python: what it shows of ops.FlashAttention (the reference's contract, flash_triton.py:558-562).
+using Node = torch::autograd::CppNode<FlashAttention>;
+
+Node& node_of(PyObject* self) { return static_cast<Node&>(*reinterpret_cast<torch::autograd::THPCppFunction*>(self)->cdata); }
+
+using Shown = py::object (*)(Node&);
+
+PyObject* show(PyObject* self, void* get) {
+    HANDLE_TH_ERRORS
+    return reinterpret_cast<Shown>(get)(node_of(self)).release().ptr();
+    END_HANDLE_TH_ERRORS
+}
+
+PyGetSetDef property(const char* name, Shown get) { return {name, show, nullptr, nullptr, reinterpret_cast<void*>(get)}; }
+
+PyObject* node_name(PyObject*, PyObject*) { return PyUnicode_FromString("FlashAttentionBackward"); }
+
+void register_node() {
+    using namespace torch::autograd;
+    static PyGetSetDef properties[] = {
+        {"next_functions", THPCppFunction_next_functions, nullptr, nullptr, nullptr},
+        {"requires_grad", THPCppFunction_requires_grad, nullptr, nullptr, nullptr},
+        {"metadata", THPCppFunction_metadata, nullptr, nullptr, nullptr},
+        {"_input_metadata", THPCppFunction_input_metadata, nullptr, nullptr, nullptr},
+        property("saved_tensors", [](Node& n) -> py::object { return py::tuple(py::cast(n.ctx_.get_saved_variables())); }),
+        property("needs_input_grad", [](Node& n) -> py::object {
+            py::tuple t(8);  // of attention()'s arguments
+            for (size_t i = 0; i < 8; ++i) t[i] = py::bool_(i < 3 && n.should_compute_output(i));
+            return t;
+        }),
+        property("sm_scale", [](Node& n) -> py::object { return py::cast(n.ctx_.saved_data["scale"].toDouble()); }),
+        property("causal", [](Node& n) -> py::object { return py::cast(n.ctx_.saved_data["causal"].toInt() != 0); }),
+        property("score_func_info", [](Node& n) -> py::object { return py::make_tuple(n.ctx_.saved_data["mode"].toInt()); }),
+        property("id_heads", [](Node& n) -> py::object { return py::cast(n.ctx_.saved_data["id_heads"].toInt()); }),
+        property("plan", [](Node& n) -> py::object { return py::cast(n.ctx_.saved_data["plan"].toTensor()); }),  // (None where there is none)
+        {nullptr, nullptr, nullptr, nullptr, nullptr},
+    };
+    static PyMethodDef methods[] = {
+        {"name", node_name, METH_NOARGS, nullptr},
+        {"register_hook", THPCppFunction_register_hook, METH_O, nullptr},
+        {"register_prehook", THPCppFunction_register_prehook, METH_O, nullptr},
+        {"_register_hook_dict", THPCppFunction_register_hook_dict, METH_O, nullptr},
+        {"_sequence_nr", THPCppFunction_sequence_nr, METH_NOARGS, nullptr},
+        {nullptr, nullptr, 0, nullptr},
+    };
+    static PyTypeObject type{PyVarObject_HEAD_INIT(nullptr, 0)};
+    registerCppFunction(typeid(Node), _initFunctionPyTypeObject(type, "flash_b200._host.FlashAttentionNode", properties, methods));
+}
 
 }  // namespace
 
@@ -279,4 +330,5 @@ PYBIND11_MODULE(_host, m) {
     m.def("backward", &backward);
     m.def("attend", &attend);
     m.def("launched", &launched);
+    register_node();
 }

@@ -441,7 +441,10 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
             and (ek is None or type(ek) in _PLAIN) and (sm_scale is None or type(sm_scale) is float) and PROFILE is None and not _SYNC_STATUS
             and build_plan is _own_build_plan  # (not somebody's own)
             and _transforms() is None and _forward_ad._current_level < 0 and _tracing_state() is None):
-        attend, status = getattr(_HOST, "attend", None), _STATUS.get(q.get_device())
+        host, status = _HOST, _STATUS.get(q.get_device())
+        if status is None and q.is_cuda:  # the first call on a device gets the same node as the others
+            host, status = host or _host(), _status_word(q.device)
+        attend = getattr(host, "attend", None)
         if attend is not None and status is not None:
             done = attend(q, k, v, bool(causal), sm_scale, eq, ek, score_func_mode, status)
             if done is not None:
