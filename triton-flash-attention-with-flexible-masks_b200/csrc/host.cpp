@@ -250,11 +250,13 @@ struct FlashAttention : torch::autograd::Function<FlashAttention> {
 // The whole of a regular call, its gradients included; None: ops.py takes it another way. Saved-tensor hooks count what is saved and by whom, so
 // that their calls take ops.FlashAttention.
 py::object attend(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, std::optional<double> scale, const std::optional<Tensor>& eq,
-                  const std::optional<Tensor>& ek, int mode, const Tensor& status) {
+                  const std::optional<Tensor>& ek, const py::int_& score_mode, const Tensor& status) {
     fa_problem p;
+    int beyond = 0;  // (a number of any size: what no mode has is for ops.py to refuse)
+    const long mode = PyLong_AsLongAndOverflow(score_mode.ptr(), &beyond);
     const double sm_scale = scale ? *scale : 1.0 / std::sqrt(double(q.dim() == 4 ? q.size(3) : 1));
-    if (eq.has_value() != ek.has_value() || mode != (eq ? FA_MODE1_DOC : FA_MODE0_NOPE)) return py::none();
-    if (!regular(q, k, v, false, causal, sm_scale, mode, 1, p)) return py::none();
+    if (beyond != 0 || eq.has_value() != ek.has_value() || mode != (eq ? FA_MODE1_DOC : FA_MODE0_NOPE)) return py::none();
+    if (!regular(q, k, v, false, causal, sm_scale, int(mode), 1, p)) return py::none();
     if (eq) {
         if (eq->device() != q.device() || ek->device() != q.device()) return py::none();
         p.id_heads = int(id_heads(*eq, *ek, p.B, p.H, p.M, p.N));
