@@ -227,7 +227,7 @@ __device__ __forceinline__ int code_k(const MaskArgs& mk, int b, int he, int j) 
 }
 
 // ---------------------------------------------------------------------------------------------
-// forward: grid (ceil(M / 32), H, B)
+// forward: grid (H, B, ceil(M / R))
 // ---------------------------------------------------------------------------------------------
 template <int D, int R>
 __global__ void __launch_bounds__(threads(R), R == 32 && D <= 32 ? 4 : 0) f32_fwd_kernel(const F32Params p) {
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(128) f32_delta_kernel(const F32Params p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// dQ: grid (ceil(M / 32), H, B). rows = queries, columns = keys
+// dQ: grid (H, B, ceil(M / R)). rows = queries, columns = keys
 // ---------------------------------------------------------------------------------------------
 template <int D, int R>
 __global__ void __launch_bounds__(threads(R)) f32_bwd_dq_kernel(const F32Params p) {
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(threads(R)) f32_bwd_dq_kernel(const F32Params 
 }
 
 // ---------------------------------------------------------------------------------------------
-// dK, dV: grid (ceil(N / 32), Hk, B). rows = keys, columns = queries; the query heads of the group
+// dK, dV: grid (Hk, B, ceil(N / R)). rows = keys, columns = queries; the query heads of the group
 // are walked one after the other, so the group sum (flash_triton.py:635-637) needs no second pass
 // ---------------------------------------------------------------------------------------------
 template <int D, int R>

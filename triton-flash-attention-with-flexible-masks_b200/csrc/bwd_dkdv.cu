@@ -130,14 +130,13 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // blocks go in order (with a causal mask: long ones first) and the heads of the group vary
     // fastest. The CTAs thus work on neighbouring key blocks of a few heads at a time: few enough
     // that their Q / dO streams stay in L2, enough that not all CTAs pull the same lines.
-    const int HB = p.Hk * p.B;
-    auto decode = [&](int j, int& kb, int& hk, int& b) {
-        const int per = p.gh * nK;
+    auto decode = [&](int j, int& kb, int& hk, int& b, int gh, int nk, int heads, int batches) {
+        const int per = gh * nk;
         const int grp = j / per, rem = j - grp * per;
-        const int gsz = min(p.gh, HB - grp * p.gh);
-        const int pos = rem / gsz, bh = grp * p.gh + (rem - pos * gsz);
-        hk = bh % p.Hk;
-        b = bh / p.Hk;
+        const int gsz = min(gh, heads * batches - grp * gh);
+        const int pos = rem / gsz, bh = grp * gh + (rem - pos * gsz);
+        hk = bh % heads;
+        b = bh / heads;
         // few items per CTA: longest first (sorted in the plan), so that no long item is left for the end
         kb = p.by_length ? mk.plan[mk.L.off_ordk + (int64_t(b) * mk.He + (mk.He == 1 ? 0 : hk * G)) * nK + pos] : pos;
     };
@@ -193,24 +192,29 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     launch_dependents();  // (fa_bwd's dQ kernel reads nothing that this one writes, but delta, which is complete since the wait)
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
-    // Item k of this CTA. Items are handed out in order from a counter in the plan (any CTA takes the next one: the
-    // work per item varies with the mask); without counters (no plan given) they are
-    // dealt out round robin in alternating direction, which evens out their sorted lengths.
-    auto take = [&](int k) {
-        if (ctr) return int(atomicAdd(ctr, 1u));
-        return k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
-    };
-    // an earlier launch on this device ran into a time-out that the host has not yet cleared
-    if (aborted && (sbase & 1023u) == 0)
-        nan_fill_items(smem + S::off_k, S::NBOX, n_items, take, [&](int j, int lane) {
-            int kb, hk, b;
-            decode(j, kb, hk, b);
-            if (lane == 0)
+    // An earlier launch on this device ran into a time-out that the host has not yet cleared: the CTA fills its items of the fixed order with NaN
+    // (see nan_fill_items; with counters any other CTA may have taken them, and if none does they are everybody's). The numbers for it are hidden
+    // from the compiler, which kept them in registers throughout, 96 for 84 and 28 bytes spilled: 4 x 16 x 4096 x 128 in documents 221 us for 186;
+    // with this behind the roles instead 187, 4 x 16 x 4096 x 64 causal 315 for 310.
+    if (aborted && (sbase & 1023u) == 0) {
+        for (int i = tid; i < S::NBOX * S::BOX / 16; i += kDkdvThreads) reinterpret_cast<uint4*>(smem + S::off_k)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        fence_proxy_async();
+        __syncthreads();
+        int gh = p.gh, nk = nK, heads = p.Hk, batches = p.B;
+        asm volatile("" : "+r"(gh), "+r"(nk), "+r"(heads), "+r"(batches));
+        if (tid == 0) {
+            for (int k = 0, j; (j = item_in_order(k)) < n_items; ++k) {
+                int kb, hk, b;
+                decode(j, kb, hk, b, gh, nk, heads, batches);
                 for (int x = 0; x < S::NBOX; ++x) {
-                    tma_store_4d(&tmdK, smem_u32(smem + S::off_k) + x * S::BOX, x * 64, kb * kBlk, hk, b);
-                    tma_store_4d(&tmdV, smem_u32(smem + S::off_k) + x * S::BOX, x * 64, kb * kBlk, hk, b);
+                    tma_store_4d(&tmdK, sK + x * S::BOX, x * 64, kb * kBlk, hk, b);
+                    tma_store_4d(&tmdV, sK + x * S::BOX, x * 64, kb * kBlk, hk, b);
                 }
-        });
+                tma_store_commit();
+            }
+            tma_store_wait_all();
+        }
+    }
 
     if (warp >= 16) {
         if (aborted) {
@@ -218,6 +222,9 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             // ------------------------------ scheduler ------------------------------
             // Item k goes to slot k & 1: range [lo, lo + n) of candidate query blocks (union over the
             // group's heads), a 2-bit code per candidate, and the number of tiles.
+            // Items are handed out in order from a counter in the plan (any CTA takes the next one: the
+            // work per item varies with the mask); without counters (no plan given) they are
+            // dealt out round robin in alternating direction, which evens out their sorted lengths.
             bool ok = true;
             for (int k = 0;; ++k) {
                 const int s = k & 1, use = k >> 1;
@@ -225,7 +232,10 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 int j = 0;
-                if (lane == 0) j = take(k);
+                if (lane == 0) {
+                    if (ctr) j = int(atomicAdd(ctr, 1u));
+                    else j = item_in_order(k);
+                }
                 j = __shfl_sync(0xffffffffu, j, 0);
                 if (j >= n_items) {  // end marker
                     if (lane == 0) {
@@ -235,7 +245,7 @@ bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     break;
                 }
                 int kb, hk, b;
-                decode(j, kb, hk, b);
+                decode(j, kb, hk, b, p.gh, nK, p.Hk, p.B);
                 int lo = 0x7fffffff, hi = 0;
                 {
                     const int ng = (mk.He == 1) ? 1 : G;

@@ -230,6 +230,11 @@ __device__ __forceinline__ uint32_t codes_equal(const int32_t* codes, int code, 
     return mine;
 }
 
+// Item k of a CTA that takes its items in a fixed order: round robin in alternating direction, which evens out their sorted lengths.
+__device__ __forceinline__ int item_in_order(int k) {
+    return k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
+}
+
 // A CTA that finds the device's status word set by an earlier time-out computes nothing. It fills what it would have computed with
 // NaN (0xFFFF is a NaN in bf16 and in fp16), so that what it leaves behind cannot be mistaken for a result: that, and only that, for the
 // CTAs of a launch may disagree about the word (the time-out may come, on another stream, while they start). Called by all threads;
