@@ -151,11 +151,10 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // dK/dV kernel may have CTAs that started before that kernel's time-out and CTAs that started after it, so those
     // that see it fill the items that they would have computed, and only those.
     if (aborted && (sbase & 1023u) == 0)
-        nan_fill_items(smem + S::off_q, S::NBOX, n_items, take, [&](int j, int lane) {
-            int qb, h, b;
-            decode(j, qb, h, b);
-            if (lane == 0)
-                for (int x = 0; x < S::NBOX; ++x) tma_store_4d(&tmdQ, smem_u32(smem + S::off_q) + x * S::BOX, x * 64, qb * kBlk, h, b);
+        nan_fill_items(smem + S::off_q, S::NBOX, &tmdQ, [&](int k, int& qb, int& h, int& b) {
+            const int j = take(k);
+            if (j < n_items) decode(j, qb, h, b);
+            return j < n_items;
         });
 
     if (warp >= NW) {

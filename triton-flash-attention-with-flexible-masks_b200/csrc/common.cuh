@@ -237,26 +237,23 @@ __device__ __forceinline__ int item_in_order(int k) {
 
 // A CTA that finds the device's status word set by an earlier time-out computes nothing. It fills what it would have computed with
 // NaN (0xFFFF is a NaN in bf16 and in fp16), so that what it leaves behind cannot be mistaken for a result: that, and only that, for the
-// CTAs of a launch may disagree about the word (the time-out may come, on another stream, while they start). Called by all threads;
-// `tile` is nbox * 16 KB of shared memory, 1024-byte aligned. take(k) gives the CTA's k-th item, n_items or more behind the last one;
-// fill(item, lane) is called by all lanes of warp 0 and stores the item's tile, by lane 0.
-template <class Take, class Fill>
-__device__ __forceinline__ void nan_fill_items(uint8_t* tile, int nbox, int n_items, Take take, Fill fill) {
+// CTAs of a launch may disagree about the word (the time-out may come, on another stream, while they start). next(k, blk, h, b) gives the k-th
+// tile to fill, or false behind the last one; tiles are [128 rows, 64 * nbox columns] of a [B, H, L, D] tensor. Called by all threads
+// of the CTA; `tile` is nbox * 16 KB of shared memory, 1024-byte aligned.
+template <class Next>
+__device__ __forceinline__ void nan_fill_items(uint8_t* tile, int nbox, const CUtensorMap* m, Next next) {
     constexpr int kBox = kBlk * 64 * 2;
     for (int i = threadIdx.x; i < nbox * kBox / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(tile)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
     fence_proxy_async();
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        for (int k = 0;; ++k) {
-            const int j = __shfl_sync(0xffffffffu, lane == 0 ? take(k) : 0, 0);
-            if (j >= n_items) break;
-            fill(j, lane);
-            if (lane == 0) tma_store_commit();
+    if (threadIdx.x == 0) {
+        int blk, h, b;
+        for (int k = 0; next(k, blk, h, b); ++k) {
+            for (int x = 0; x < nbox; ++x) tma_store_4d(m, smem_u32(tile) + x * kBox, x * 64, blk * kBlk, h, b);
+            tma_store_commit();
         }
-        if (lane == 0) tma_store_wait_all();
-        __syncwarp();
+        tma_store_wait_all();
     }
 }
 

@@ -227,22 +227,35 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         if (ctr) return int(gridDim.x + atomicAdd(ctr, 1u));
         return k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
     };
-    // an earlier launch on this device ran into a time-out that the host has not yet cleared (with ns > 1 the combine kernel fills the output)
+    // An earlier launch on this device ran into a time-out that the host has not yet cleared: the items that the CTA would have computed are filled
+    // with NaN (see nan_fill_items), and their LSE. (With ns > 1 the combine kernel fills the output.)
     if (aborted && (sbase & 1023u) == 0 && ns == 1) {
-        nan_fill_items(smem + S::off_q, S::NBOX, n_items, take, [&](int j, int lane) {
-            int qb, h, b;
-            decode(j, qb, h, b);
-            const int h0 = SHORT ? h / nG * p.G + (h % nG) * p.pack : h, n_h = SHORT ? min(p.pack, p.G - (h % nG) * p.pack) : 1;
-            if (lane == 0)
-                for (int x = 0; x < S::NBOX; ++x) {
-                    if constexpr (SHORT) tma_store_5d(&tmO, smem_u32(smem + S::off_q) + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
-                    else tma_store_4d(&tmO, smem_u32(smem + S::off_q) + x * S::BOX, x * 64, qb * kBlk, h, b);
+        for (int i = tid; i < S::TILE / 16; i += kFwdThreads) reinterpret_cast<uint4*>(smem + S::off_q)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        fence_proxy_async();
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t tile = sbase + S::off_q;
+            for (int k = 0;; ++k) {
+                const int j = __shfl_sync(0xffffffffu, lane == 0 ? take(k) : 0, 0);
+                if (j >= n_items) break;
+                int qb, h, b;
+                decode(j, qb, h, b);
+                const int h0 = SHORT ? h / nG * p.G + (h % nG) * p.pack : h, n_h = SHORT ? min(p.pack, p.G - (h % nG) * p.pack) : 1;
+                if (lane == 0) {
+                    for (int x = 0; x < S::NBOX; ++x) {
+                        if constexpr (SHORT) tma_store_5d(&tmO, tile + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
+                        else tma_store_4d(&tmO, tile + x * S::BOX, x * 64, qb * kBlk, h, b);
+                    }
+                    tma_store_commit();
                 }
-            for (int i = lane; i < n_h * kBlk; i += 32) {  // the rows past M pad the buffer
-                const int row = qb * kBlk + i % kBlk;
-                p.lse[(int64_t(b) * p.H + h0 + i / kBlk) * mk.L.Mpad + row] = row < mk.M ? __int_as_float(-1) : 0.f;
+                for (int i = lane; i < n_h * kBlk; i += 32) {  // the rows past M pad the buffer
+                    const int row = qb * kBlk + i % kBlk;
+                    p.lse[(int64_t(b) * p.H + h0 + i / kBlk) * mk.L.Mpad + row] = row < mk.M ? __int_as_float(-1) : 0.f;
+                }
             }
-        });
+            if (lane == 0) tma_store_wait_all();
+            __syncwarp();
+        }
     }
 
     auto sQ = [&](int s) { return sbase + S::off_q + uint32_t(s) * S::TILE; };
