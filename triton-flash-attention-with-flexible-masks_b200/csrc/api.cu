@@ -389,9 +389,13 @@ int fa_plan_bytes(const fa_problem* p, size_t* bytes) {
     return FA_OK;
 }
 
-// A split forward may have two runs per SM, still dealt out in a fixed order (times of an earlier forward): 32 / 8 heads of 300 queries, 9000 keys in
-// 3 runs 72.6 us, 72.7 us through the counters of a plan that is there, 76.8 us with the clearing of its counters;
-// 12 tokens of 32 / 8 heads, 16384 keys in 3 runs 129.6, 130.1 and 134.2 us; 24 heads of 500, 16000 keys 114.9, 114.8, 118.4.
+// While the items fit on the SMs at once there is nothing to share out. us in replayed graphs, without | through the counters of a plan that is there |
+// with the clearing of its counters: forward of 8 x 200 x 64 causal 10.9 | 12.4 | 12.4, of 16 x 1024 x 64 16.5 | 17.1 | 17.8, of 4 x 4096 x 128 36.3 | 36.9 | 37.2;
+// forward and backward of the three 24.0 | - | 26.1, 45.1 | - | 49.1, 106.9 | - | 118. A split forward may have two runs per SM, dealt out in a fixed
+// order: 32 / 8 heads of 300 queries, 9000 keys in 3 runs 65.2 | 66.0 | 66.2; 12 tokens of 32 / 8 heads, 16384 keys in 3 runs 129.5 | 130.1 | 131; 24 heads of 500,
+// 16000 keys 98.6 | 98.6 | 100.6. Beyond the line the counters even out calls whose items are alike (forward and backward of 10 x 2048 x 64 without a mask
+// 125 | - | 107, of 2 x 16 x 577 x 64 59.6 | - | 55.0), and cost those of up to two rounds with a causal mask, whose fixed order pairs long with short
+// items (10 x 2048 x 128 74.3 | - | 87.5, 20 x 1024 x 64 46.6 | - | 55.8, 2 x 16 x 1024 x 64 55.7 | - | 62.4). (One line for all of them: the rule asks for no mask.)
 int fa_plan_optional(const fa_problem* p, int32_t backward) {
     if (check_problem(p) || p->mode != FA_MODE0_NOPE) return 0;
     if (p->dtype == FA_FP32) return 1;

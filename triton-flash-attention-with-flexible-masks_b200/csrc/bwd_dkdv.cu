@@ -27,9 +27,10 @@
 // in 64 documents 1351 | 1225; 8 x 8 x 1024 x 8192 x 64, queries of 8 documents, 172 | 135; 16 x 8 x 577 x 32 54 | 45; 4 x 12 x 1000 x 64
 // in documents 35 | 30. In between: sixteen warps with P^T in shared memory 273 / 195 / 1267 / 138 / 45 / 31, a tile's shared memory traffic being 2980
 // wavefronts then; two MMA warps, so that dK may come between dV and S^T, 305 / 201 / 1320 / 142 / 46 / 30.
-// With shorter waits, products written once and a shorter walk, us between events in a graph, before | now: 8 x 8 x 1024 x 8192 x 64 134 | 119, 16 x 8 x
-// 577 x 32 42.2 | 40.1, 4 x 12 x 1000 x 64 in documents 28.4 | 28.2, 4 x 16 x 4096 x 128 in documents 213 | 213 (under the power cap), 32 x 32768 x 128
-// 1414 | 1380.
+// Since then shorter waits, products written once and a shorter walk. Both builds in turn, replayed graphs of one launch, some 30 after a pause (so above the
+// power cap), other documents than above, us, that "sixteen" | now: 2 x 32 / 8 x 3001 261 | 264, 4 x 16 x 4096 x 128 in documents 186 | 185, 32 x 32768 x 128
+// in 64 documents 588 | 572, 8 x 8 x 1024 x 8192 x 64 143 | 129, 16 x 8 x 577 x 32 47.4 | 45.4, 4 x 12 x 1000 x 64 in documents 33.1 | 32.7, 4 x 16 x 4096 x 64
+// causal 309 | 309.
 #include "common.cuh"
 #include "params.cuh"
 

@@ -33,9 +33,11 @@
 // 32 x 32768 x 128 in 64 documents 908 | 776 | 786; 16 x 32 x 8192 x 128 causal 9520 | 7760 | 7690; 4 x 16 x 4096 x 64 causal
 // 249 | 201 | 192; 8 x 8 x 1024 x 8192 x 64, queries of random documents, 94 | 83 | 79. The shared O had errors 1 to 2 %
 // larger as well: one entry of a row is an exact 1 in P, not one of each chain.
-// Since then the code was made smaller (loops that are not unrolled, masks by a loop, shorter waits) and a block's first item is known at once, us, that "now" | at
-// present: 2 x 32 / 8 x 3001 170 | 162, 512 against 8192 58.0 | 56.5, 16 x 8 x 577 x 32 31.1 | 27.9, 4 x 16 x 4096 x 128 in documents 152 | 136, 32 x
-// 32768 x 128 870 | 812, 16 x 32 x 8192 x 128 8470 | 8030, 8 x 8 x 1024 x 8192 x 64 75.2 | 62.5, 4 x 12 x 1000 x 64 in documents 24.4 | 19.2.
+// Since then the code was made smaller (loops that are not unrolled, masks by a loop, shorter waits) and a block's first item is known at once. Both builds in turn,
+// replayed graphs of one launch, some 30 after a pause (so above the power cap but for the last), other documents than above, us, that "now" | at present: 2 x 32 / 8 x
+// 3001 153 | 142, 512 against 8192 63.8 | 61.8, 16 x 8 x 577 x 32 36.6 | 33.1, 4 x 16 x 4096 x 128 in documents 146 | 122, 32 x 32768 x 128 in 64 documents
+// 484 | 387, 4 x 16 x 4096 x 64 causal 192 | 180, 8 x 8 x 1024 x 8192 x 64 105 | 91.5, 4 x 12 x 1000 x 64 in documents 30.9 | 24.8; long series of
+// 16 x 32 x 8192 x 128, under the cap, 8370 | 8150.
 // What bounds it: the softmax warps (scores out of TMEM, maximum, 1024 clocks of MUFU for a tile of each group, and fetching their own straight code), at D = 128 the
 // 64 KB of K and V that each tile brings from L2 (52 B a clock and SM; half of them would take dense calls 5 % less time), and, in
 // dense calls, the clock under the power cap (1.4-1.5 GHz); with short items the drain of two O, which the next item's P*V waits for.
@@ -90,8 +92,8 @@ static_assert(FwdSmem<128>::total > 116736 && FwdSmem<64>::total > 116736, "shar
 // Two things are added (fwd_pack and fwd_splits in api.cu say when):
 //  - p.pack query heads of one kv head share a tile, row g * M + i = query i of the g-th of them (at most 128
 //    rows: one decoded token of 4 heads reads the keys and values once instead of four times). The Q and O maps
-//    are 5-D, (D, M, G, Hk, B), and a box holds p.rows rows; tile rows past them are never loaded, hold whatever
-//    was there and only ever reach results that are not stored. Warps without a valid row skip the softmax.
+//    are 5-D, (D, M, G, Hk, B), and a box holds p.rows rows; tile rows past them are never loaded. They
+//    start as zeros, may later hold what an earlier item staged there, and only ever reach results that are not stored. Warps without a valid row skip the softmax.
 //  - an item's tiles are cut into p.ns runs that are items of their own. With ns > 1 the normalised fp32 rows
 //    and their log-sum-exp go to the workspace, and fwd_combine_kernel merges them.
 // Such calls are bound by reading K and V (16 tokens of 32 / 8 heads of 128 against 4500 keys: 295 MB, 45 us at the
@@ -141,7 +143,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     };
     // What the scheduler finds out about item j before it has a slot for it; in `flags` the class of candidate tile lo + lane.
     struct Item {
-        int j, qb, h, b, lo, n;
+        int qb, h, b, lo, n;
         uint32_t flags;
         int4 qc;
     };
@@ -150,7 +152,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     };
     auto prepare = [&](int j) {
         Item it;
-        it.j = j;
         const int sp = SHORT ? j % ns : 0;  // which run of the item's tiles
         decode(SHORT ? j / ns : j, it.qb, it.h, it.b);
         const int he = (mk.He == 1) ? 0 : it.h;

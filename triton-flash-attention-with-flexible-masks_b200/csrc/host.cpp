@@ -2,8 +2,8 @@
 // descriptors, the launches of fa_b200.h and the autograd node. The general code and its node stay in Python (ops.py), and so do all
 // messages: a call that is not regular (another layout, device, shape or type than the kernels take as they are) is declined with
 // None, and ops.py copies, asks or raises. Bound by per-call overhead: a forward of 8 heads of 200
-// queries took 27 us of host time around 8 us of kernel through ctypes; a training step's forward and
-// backward 113 us with the node in Python, 88 with the one below.
+// queries took 27 us of host time around 8 us of kernel through ctypes; a training step of 4 x 12
+// heads x 1000 x 64 in documents 122 us with the node in Python, 92 with the one below, around some 70 of kernels.
 #include <ATen/SavedTensorHooks.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>

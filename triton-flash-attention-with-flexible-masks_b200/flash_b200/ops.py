@@ -433,8 +433,8 @@ def attention(q, k, v, causal=False, sm_scale=None, eq=None, ek=None, score_func
             and q.is_cuda and q.dim() == 4 and 128 < q.shape[2] <= _lib.FA_GROUP_MAX_ROWS):
         return _attention_grouped(q, k, v, sm_scale, eq, ek)
     # Regular calls go to the library in one native call, with a native autograd node where a gradient is needed. A small training step is
-    # bound by its host time: 4 x 12 heads x 1000 x 64 in documents 113 us for 92 of kernels with the node of this module (its backward waits for
-    # the interpreter in the engine's thread), 88 with the native one. Transforms of torch.func and forward-mode gradients need
+    # bound by its host time: 4 x 12 heads x 1000 x 64 in documents, some 70 us of kernels, 122 us a step with the node of this module (its backward waits for
+    # the interpreter in the engine's thread), 92 with the native one. Transforms of torch.func and forward-mode gradients need
     # the node of this module for their messages, subclasses for their hooks, and a trace for its refusal.
     # Without a gradient there is no node at all: 8 heads of 200 queries took 13.6 us a call with the one of this module, 7.5 now.
     if (type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(score_func_mode) is int and (eq is None or type(eq) in _PLAIN)
