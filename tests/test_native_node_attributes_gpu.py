@@ -57,3 +57,33 @@ assert type(first.grad_fn) is type(second.grad_fn) and torch.equal(first, second
     env = dict(os.environ, PYTHONPATH=path + os.pathsep + os.environ.get("PYTHONPATH", ""))
     r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_saved_tensors_while_another_thread_frees_them():
+    import threading
+    import flash_b200 as fb
+    x = [torch.randn(1, 2, 200, 64, device="cuda").bfloat16().requires_grad_() for _ in range(3)]
+    do = torch.randn_like(x[0])
+    for _ in range(50):
+        o = fb.attention(*x, True)
+        node, wrong, begun = o.grad_fn, [], threading.Event()
+
+        def look():
+            begun.set()
+            while True:
+                try:
+                    if len(node.saved_tensors) != 5:
+                        wrong.append("tensors missing")
+                except RuntimeError as e:
+                    if "second time" not in str(e):
+                        wrong.append(str(e))
+                    return
+
+        threads = [threading.Thread(target=look) for _ in range(3)]
+        for t in threads:
+            t.start()
+        begun.wait()
+        torch.autograd.grad(o, x, do)
+        for t in threads:
+            t.join()
+        assert not wrong

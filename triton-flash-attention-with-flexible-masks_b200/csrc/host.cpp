@@ -278,6 +278,16 @@ using Node = torch::autograd::CppNode<FlashAttention>;
 
 Node& node_of(PyObject* self) { return static_cast<Node&>(*reinterpret_cast<torch::autograd::THPCppFunction*>(self)->cdata); }
 
+// The engine's thread gives the saved tensors up, behind the node's lock, without the interpreter: so they are asked for.
+torch::autograd::variable_list saved_tensors(Node& n) {
+    struct Open : torch::autograd::Node {
+        static std::mutex& lock_of(torch::autograd::Node& n) { return n.*(&Open::mutex_); }
+    };
+    py::gil_scoped_release free;
+    const std::lock_guard<std::mutex> lock(Open::lock_of(n));
+    return n.ctx_.get_saved_variables();
+}
+
 using Shown = py::object (*)(Node&);
 
 PyObject* show(PyObject* self, void* get) {
@@ -297,7 +307,7 @@ void register_node() {
         {"requires_grad", THPCppFunction_requires_grad, nullptr, nullptr, nullptr},
         {"metadata", THPCppFunction_metadata, nullptr, nullptr, nullptr},
         {"_input_metadata", THPCppFunction_input_metadata, nullptr, nullptr, nullptr},
-        property("saved_tensors", [](Node& n) -> py::object { return py::tuple(py::cast(n.ctx_.get_saved_variables())); }),
+        property("saved_tensors", [](Node& n) -> py::object { return py::tuple(py::cast(saved_tensors(n))); }),
         property("needs_input_grad", [](Node& n) -> py::object {
             py::tuple t(8);  // of attention()'s arguments
             for (size_t i = 0; i < 8; ++i) t[i] = py::bool_(i < 3 && n.should_compute_output(i));
