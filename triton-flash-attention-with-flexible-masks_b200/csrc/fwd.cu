@@ -220,42 +220,32 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     launch_dependents();
     const uint32_t tmem = uint32_t(misc[0]);
     const bool aborted = misc[1] != 0;
-    // Item k of this CTA. The first one is its own number; the others are handed out in order from a counter in the plan (any CTA takes
-    // the next one: the work per item varies with the mask); without counters (no plan given) they are dealt out round robin in
-    // alternating direction, which evens out their sorted lengths.
-    auto take = [&](int k) {
-        if (k == 0) return int(blockIdx.x);
-        if (ctr) return int(gridDim.x + atomicAdd(ctr, 1u));
-        return k * int(gridDim.x) + ((k & 1) ? int(gridDim.x) - 1 - int(blockIdx.x) : int(blockIdx.x));
-    };
-    // An earlier launch on this device ran into a time-out that the host has not yet cleared: the items that the CTA would have computed are filled
-    // with NaN (see nan_fill_items), and their LSE. (With ns > 1 the combine kernel fills the output.)
+    // An earlier launch on this device ran into a time-out that the host has not yet cleared: the CTA fills its items of the fixed order with NaN, and
+    // their LSE (see nan_fill_items; with counters any other CTA may have taken all but the first, and if none does they are everybody's. With ns > 1
+    // the combine kernel fills the output). By one thread: by a warp, and by the items of the counter, the code cost each launch
+    // 0.08 us (8 x 200 x 64 6.52 for 6.44), behind the roles it cost long calls 1 % (32 x 32768 x 128 in 64 documents 395 us for 391; 392 now).
     if (aborted && (sbase & 1023u) == 0 && ns == 1) {
         for (int i = tid; i < S::TILE / 16; i += kFwdThreads) reinterpret_cast<uint4*>(smem + S::off_q)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
         fence_proxy_async();
         __syncthreads();
-        if (warp == 0) {
-            const uint32_t tile = sbase + S::off_q;
-            for (int k = 0;; ++k) {
-                const int j = __shfl_sync(0xffffffffu, lane == 0 ? take(k) : 0, 0);
-                if (j >= n_items) break;
+        if (tid == 0) {
+#pragma unroll 1
+            for (int k = 0, j; (j = item_in_order(k)) < n_items; ++k) {
                 int qb, h, b;
                 decode(j, qb, h, b);
                 const int h0 = SHORT ? h / nG * p.G + (h % nG) * p.pack : h, n_h = SHORT ? min(p.pack, p.G - (h % nG) * p.pack) : 1;
-                if (lane == 0) {
-                    for (int x = 0; x < S::NBOX; ++x) {
-                        if constexpr (SHORT) tma_store_5d(&tmO, tile + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
-                        else tma_store_4d(&tmO, tile + x * S::BOX, x * 64, qb * kBlk, h, b);
-                    }
-                    tma_store_commit();
+                for (int x = 0; x < S::NBOX; ++x) {
+                    if constexpr (SHORT) tma_store_5d(&tmO, sbase + S::off_q + x * S::BOX, x * 64, qb * kBlk, (h % nG) * p.pack, h / nG, b);
+                    else tma_store_4d(&tmO, sbase + S::off_q + x * S::BOX, x * 64, qb * kBlk, h, b);
                 }
-                for (int i = lane; i < n_h * kBlk; i += 32) {  // the rows past M pad the buffer
+                tma_store_commit();
+#pragma unroll 1
+                for (int i = 0; i < n_h * kBlk; ++i) {  // the rows past M pad the buffer
                     const int row = qb * kBlk + i % kBlk;
                     p.lse[(int64_t(b) * p.H + h0 + i / kBlk) * mk.L.Mpad + row] = row < mk.M ? __int_as_float(-1) : 0.f;
                 }
             }
-            if (lane == 0) tma_store_wait_all();
-            __syncwarp();
+            tma_store_wait_all();
         }
     }
 
@@ -269,7 +259,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             // a previous kernel reported an error: do nothing
         } else if (warp == 14) {
             // ------------------------------ item scheduler ------------------------------
-            // us, every item from the counter | the first one known, without ids before the wait: 8 x 200 x 64 7.42 | 7.10, 4 x 12 x 1000 x 64 in documents 24.4 | 22.5, 8 x 8 x 1024 x 8192 x
+            // The first item of a CTA is its own number; the others are handed out in order from a counter in the plan (any CTA
+            // takes the next one: the work per item varies with the mask); without counters (no plan given) they are dealt out
+            // round robin in alternating direction, which evens out their sorted lengths. us, every item from the counter | the first
+            // one known, without ids before the wait: 8 x 200 x 64 7.42 | 7.10, 4 x 12 x 1000 x 64 in documents 24.4 | 22.5, 8 x 8 x 1024 x 8192 x
             // 64 in documents 75.2 | 71.4, 4 x 16 x 4096 x 128 in documents 153 | 148, 16 x 8 x 577 x 32 31.1 | 31.5. An item taken, and what the
             // plan says about it read, while the one before it still holds the slot leaves no pause between items, but is dealt out
             // too far ahead: 28.1 for 27.8, 75.6 for 76.5, 157 for 154. (dK/dV gains nothing from a first item of its own.)
@@ -280,7 +273,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 if (use > 0) ok = mbar_wait_warp(BAR(B_ITEMEMPTY + s), (use - 1) & 1, ab, ST_WAIT_TIMEOUT + 11);
                 if (!ok) break;
                 if (k > 0) {
-                    if (lane == 0) j = take(k);
+                    if (lane == 0) {
+                        if (ctr) j = int(gridDim.x + atomicAdd(ctr, 1u));
+                        else j = item_in_order(k);
+                    }
                     j = __shfl_sync(0xffffffffu, j, 0);
                 }
                 if ((k > 0 || mk.mode != 0) && j < n_items) item = prepare(j);
